@@ -242,7 +242,10 @@ def vnl_apply(proj, dion, becp_, hpsi_inout):
     rdt = torch.float64 if dt == F64 else torch.float32
     dion = _c(torch.as_tensor(dion, device="cuda").to(rdt), "dion")
     esz = 16 if dt == F64 else 8
-    w = workspace(nk * P * nb * esz + 256)
+    need = nk * P * nb * esz + 256
+    if dt == F64:   # packed operands of the tensor-core form (32 B per element), in pieces beyond 384 MB
+        need += min(384 << 20, 32 * nk * (P + 16) * (nG + nb + 256)) + 1024 + 4 * nk * (nG + nb)
+    w = workspace(need)
     check(LIB.addft_vnl_apply(dt, nk, nb, nG, P, _p(_c(proj, "proj")), _p(dion), _p(_c(becp_, "becp")),
                               _p(hpsi_inout), _p(w), w.numel(), _stream()), "vnl_apply")
     return hpsi_inout

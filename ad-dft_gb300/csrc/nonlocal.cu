@@ -5,6 +5,7 @@
 // Reference: src/addft/physics/nonlocal_op.py:25-82 (dion_full, projectors,
 // becp, vnl_apply, nonlocal_energy), ylm.py:8-26, psp.py:122-128, and
 // src/addft/ops/hpsi.py:35-50.
+#include "ozgemm.cuh"
 #include "radial.cuh"
 #include "transforms.cuh"
 
@@ -294,24 +295,50 @@ __global__ void __launch_bounds__(256) k_sum_splits2(const C *__restrict__ tmp, 
 inline int split_groups(int ns) { return (ns + kSplitGroup - 1) / kSplitGroup; }
 
 // DB[k][p][b] = sum_q D[p][q] becp[k][q][b]   (optionally scaled by wocc[k][b])
+// A CTA takes one row p of D (nonzero in one atom's block of nh^2 at most): it lists the row's
+// nonzeros in order, then its threads walk the bands over that list only.  Reading every D[p][q]
+// per output cost 113 us at P = 256, 160 bands (FP64).
+constexpr int kDList = 1024;
+
 template <typename R>
-__global__ void k_dbecp(const R *__restrict__ D, const typename Cx<R>::T *__restrict__ becp, int nk,
-                        int nproj, int nb, const double *__restrict__ wocc,
-                        typename Cx<R>::T *__restrict__ out) {
+__global__ void __launch_bounds__(128)
+k_dbecp(const R *__restrict__ D, const typename Cx<R>::T *__restrict__ becp, int nproj, int nb,
+        const double *__restrict__ wocc, typename Cx<R>::T *__restrict__ out) {
   using C = typename Cx<R>::T;
-  const size_t n = (size_t)nk * nproj * nb;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
-    const int b = (int)(t % nb);
-    const int p = (int)((t / nb) % nproj);
-    const int k = (int)(t / ((size_t)nb * nproj));
-    const C *Bk = becp + (size_t)k * nproj * nb;
-    C s = czero<C>();
-    for (int q = 0; q < nproj; ++q) {
-      const R d = D[(size_t)p * nproj + q];
-      if (d != (R)0) s = cadd(s, cscale(Bk[(size_t)q * nb + b], d));
+  __shared__ int qs[kDList];
+  __shared__ R ds[kDList];
+  __shared__ int wcnt[4];
+  const int p = blockIdx.x, k = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const C *Bk = becp + (size_t)k * nproj * nb;
+  C *o = out + ((size_t)k * nproj + p) * nb;
+  for (int q0 = 0; q0 < nproj; q0 += kDList) {
+    const int q1 = min(nproj, q0 + kDList);
+    int cnt = 0;
+    for (int c0 = q0; c0 < q1; c0 += 128) {
+      const int q = c0 + threadIdx.x;
+      const R d = q < q1 ? D[(size_t)p * nproj + q] : (R)0;
+      const bool nz = d != (R)0;
+      const unsigned m = __ballot_sync(0xffffffffu, nz);
+      if (lane == 0) wcnt[warp] = __popc(m);
+      __syncthreads();
+      int at = cnt;
+      for (int w = 0; w < warp; ++w) at += wcnt[w];
+      if (nz) {
+        const int i = at + __popc(m & ((1u << lane) - 1));
+        qs[i] = q;
+        ds[i] = d;
+      }
+      cnt += wcnt[0] + wcnt[1] + wcnt[2] + wcnt[3];
+      __syncthreads();
     }
-    if (wocc) s = cscale(s, (R)wocc[(size_t)k * nb + b]);
-    out[t] = s;
+    for (int b = threadIdx.x; b < nb; b += 128) {
+      C s = q0 ? o[b] : czero<C>();
+      for (int i = 0; i < cnt; ++i) s = cadd(s, cscale(Bk[(size_t)qs[i] * nb + b], ds[i]));
+      if (wocc && q1 == nproj) s = cscale(s, (R)wocc[(size_t)k * nb + b]);
+      o[b] = s;
+    }
+    __syncthreads();
   }
 }
 
@@ -578,18 +605,31 @@ static int becp_ctas_per_sm() {
   return m;
 }
 
+// The FP64 contractions run on the tensor cores (oz_gemm) from this many complex products per k
+// on; below, its five small kernels take longer than the FP64 SIMT kernel.
+constexpr double kOzMinWork = 3e5;
+inline bool on_tensor_cores(int m, int n, int kk) { return (double)m * n * kk >= kOzMinWork; }
+
 template <typename R>
 size_t becp_work_bytes(int nk, int nb, int nG, int nproj) {
   using C = typename Cx<R>::T;
   const int tiles = ((nproj + kBP - 1) / kBP) * ((nb + kBB - 1) / kBB) * nk;
   const int ns = pick_nsplit(tiles, nG);
-  return ns > 1 ? (size_t)(ns + split_groups(ns)) * nk * nproj * nb * sizeof(C) : 0;
+  const size_t simt = ns > 1 ? (size_t)(ns + split_groups(ns)) * nk * nproj * nb * sizeof(C) : 0;
+  if (sizeof(R) == 8 && on_tensor_cores(nproj, nb, nG)) return std::max(simt, oz_work_bytes(8, nproj, nb, nG, nk));
+  return simt;
 }
 
 template <typename R>
 addft_status becp_t(int nk, int nb, int nG, int nproj, const void *proj, const void *psi, void *becp,
                     void *work, size_t bytes, cudaStream_t st) {
   using C = typename Cx<R>::T;
+  if constexpr (sizeof(R) == 8) {
+    if (on_tensor_cores(nproj, nb, nG) && oz_fits(8, nproj, nb, nG, nk, work, bytes)) {
+      const OzMat b = {proj, nG, 1, (size_t)nproj * nG, 1}, x = {psi, nG, 1, (size_t)nb * nG, 0};
+      return oz_gemm(8, nproj, nb, nG, nk, b, x, becp, nb, 1, (size_t)nproj * nb, false, work, bytes, st);
+    }
+  }
   const int tiles = ((nproj + kBP - 1) / kBP) * ((nb + kBB - 1) / kBB) * nk;
   const int mode = sizeof(R) == 4 ? becp_mode() : 2;
   const bool tc = mode == 1;
@@ -643,9 +683,7 @@ template <typename R>
 addft_status dbecp_t(const void *D, const void *becp, int nk, int nproj, int nb, const double *wocc,
                      void *out, cudaStream_t st) {
   using C = typename Cx<R>::T;
-  const size_t n = (size_t)nk * nproj * nb;
-  k_dbecp<R><<<(int)std::min<size_t>((n + 255) / 256, 1024), 256, 0, st>>>(
-      (const R *)D, (const C *)becp, nk, nproj, nb, wocc, (C *)out);
+  k_dbecp<R><<<dim3(nproj, nk), 128, 0, st>>>((const R *)D, (const C *)becp, nproj, nb, wocc, (C *)out);
   return check_launch("k_dbecp");
 }
 
@@ -667,10 +705,23 @@ static int apply_mode() {
   return m;
 }
 
+// scratch (work, bytes) serves the FP64 tensor-core form; without enough of it the SIMT kernel runs
+template <typename R>
+size_t apply_work_bytes(int nk, int nj, int ni, int nG) {
+  return sizeof(R) == 8 && on_tensor_cores(ni, nj, nG) ? oz_work_bytes(8, ni, nG, nj, nk) : 0;
+}
+
 template <typename R, bool CONJ_A, bool ACCUM>
 addft_status apply_t(const void *X, int xs_j, int xs_i, size_t xs_k, const void *A, size_t as_k,
-                     int nk, int nj, int ni, int nG, void *out, size_t os_k, cudaStream_t st) {
+                     int nk, int nj, int ni, int nG, void *out, size_t os_k, void *work, size_t bytes,
+                     cudaStream_t st) {
   using C = typename Cx<R>::T;
+  if constexpr (sizeof(R) == 8) {
+    if (on_tensor_cores(ni, nj, nG) && oz_fits(8, ni, nG, nj, nk, work, bytes)) {
+      const OzMat x = {X, xs_i, xs_j, xs_k, 0}, a = {A, 1, nG, as_k, CONJ_A ? 1 : 0};
+      return oz_gemm(8, ni, nG, nj, nk, x, a, out, nG, 1, os_k, ACCUM, work, bytes, st);
+    }
+  }
   if constexpr (sizeof(R) == 4 && !CONJ_A) {
     if (apply_mode() == 1)
       return launch_apply_tc(ACCUM, (const float2 *)X, xs_j, xs_i, xs_k, (const float2 *)A, as_k, nk, nj, ni, nG,
@@ -697,11 +748,24 @@ addft_status apply_t(const void *X, int xs_j, int xs_i, size_t xs_k, const void 
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// one region serves becp's partials and, after it, the apply's operands
+template <typename R>
+size_t nl_split_bytes(int nk, int nb, int nG, int nproj) {
+  return std::max(becp_work_bytes<R>(nk, nb, nG, nproj), apply_work_bytes<R>(nk, nproj, nb, nG));
+}
+
 template <typename R>
 size_t nl_scratch(int nk, int nb, int nG, int nproj) {
   using C = typename Cx<R>::T;
   if (nproj == 0) return 0;
-  return align256(2 * (size_t)nk * nproj * nb * sizeof(C)) + align256(becp_work_bytes<R>(nk, nb, nG, nproj));
+  return align256(2 * (size_t)nk * nproj * nb * sizeof(C)) + align256(nl_split_bytes<R>(nk, nb, nG, nproj));
+}
+
+// the region shared by becp and the back-contraction Y of the gradients
+inline size_t nl_grad_scratch(addft_dtype dt, int nk, int nb, int nG, int nproj) {
+  return dt == ADDFT_F64
+             ? std::max(becp_work_bytes<double>(nk, nb, nG, nproj), apply_work_bytes<double>(nk, nb, nproj, nG))
+             : becp_work_bytes<float>(nk, nb, nG, nproj);
 }
 
 // H psi with the work buffer split as [becp | D becp | becp split-K partials | local FFT scratch].
@@ -753,7 +817,7 @@ addft_status hpsi_t(addft_plan plan, int nk, int nb, const void *psi, const void
   size_t split = 0;
   if (nproj > 0) {
     const size_t spare = (work_bytes - arrays - local_min) & ~size_t(255);
-    split = std::min(align256(becp_work_bytes<R>(nk, nb, pd.nG, nproj)), spare);
+    split = std::min(align256(nl_split_bytes<R>(nk, nb, pd.nG, nproj)), spare);
   }
   C *becp = (C *)work;
   C *db = becp + (size_t)nk * nproj * nb;
@@ -786,8 +850,9 @@ addft_status hpsi_t(addft_plan plan, int nk, int nb, const void *psi, const void
                                 : s;
     ADDFT_CUDA(cudaStreamWaitEvent(st, join, 0));
     ADDFT_TRY(sl);
+    // the becp partials and the FFT scratch are free by now
     return apply_t<R, false, true>(db, nb, 1, (size_t)nproj * nb, proj, (size_t)nproj * pd.nG, nk, nproj, nb,
-                                   pd.nG, hpsi, (size_t)nb * pd.nG, st);
+                                   pd.nG, hpsi, (size_t)nb * pd.nG, bw, work_bytes - arrays, st);
   }
   if (nproj > 0) {
     ADDFT_TRY(becp_t<R>(nk, nb, pd.nG, nproj, proj, psi, becp, split ? bw : nullptr, split, st));
@@ -796,7 +861,7 @@ addft_status hpsi_t(addft_plan plan, int nk, int nb, const void *psi, const void
   ADDFT_TRY(hpsi_local_t<R>(plan, nk, nb, psi, kin, v_r, hpsi, (char *)work + used, work_bytes - used, st));
   if (nproj > 0)
     ADDFT_TRY((apply_t<R, false, true>(db, nb, 1, (size_t)nproj * nb, proj, (size_t)nproj * pd.nG, nk, nproj, nb,
-                                       pd.nG, hpsi, (size_t)nb * pd.nG, st)));
+                                       pd.nG, hpsi, (size_t)nb * pd.nG, bw, work_bytes - arrays, st)));
   return ADDFT_OK;
 }
 
@@ -871,12 +936,16 @@ addft_status addft_vnl_apply(addft_dtype dt, int nk, int nb, int nG, int nproj, 
                 ADDFT_INVALID_ARG, "vnl_apply: null pointer or work < nk*nproj*nb complex");
   cudaStream_t st = as_stream(stream);
   const size_t Pk = (size_t)nproj * nG, Xk = (size_t)nproj * nb, Ok = (size_t)nb * nG;
+  // what the buffer holds beyond D becp (from a 256-byte boundary on) is the apply's scratch
+  const size_t db = (size_t)nk * nproj * nb * csz;
+  char *rest = (char *)(((uintptr_t)work + db + 255) & ~(uintptr_t)255);
+  const size_t off = (size_t)(rest - (char *)work), left = work_bytes > off ? work_bytes - off : 0;
   if (dt == ADDFT_F64) {
     ADDFT_TRY(dbecp_t<double>(dion, becp, nk, nproj, nb, nullptr, work, st));
-    return apply_t<double, false, true>(work, nb, 1, Xk, proj, Pk, nk, nproj, nb, nG, hpsi, Ok, st);
+    return apply_t<double, false, true>(work, nb, 1, Xk, proj, Pk, nk, nproj, nb, nG, hpsi, Ok, rest, left, st);
   }
   ADDFT_TRY(dbecp_t<float>(dion, becp, nk, nproj, nb, nullptr, work, st));
-  return apply_t<float, false, true>(work, nb, 1, Xk, proj, Pk, nk, nproj, nb, nG, hpsi, Ok, st);
+  return apply_t<float, false, true>(work, nb, 1, Xk, proj, Pk, nk, nproj, nb, nG, hpsi, Ok, rest, left, st);
 }
 
 addft_status addft_nonlocal_energy(addft_dtype dt, int nk, int nb, int nproj, const void *becp,
@@ -972,8 +1041,7 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
   const size_t o_y = take((size_t)nk * nproj * nG * csz);
   const size_t o_ep = take((size_t)nk * nb * sizeof(double));
   const size_t o_gp = take((size_t)nk * nproj * 12 * sizeof(double));
-  const size_t bwb = dt == ADDFT_F64 ? becp_work_bytes<double>(nk, nb, nG, nproj)
-                                     : becp_work_bytes<float>(nk, nb, nG, nproj);
+  const size_t bwb = nl_grad_scratch(dt, nk, nb, nG, nproj);   // becp's partials, then the operands of Y
   const size_t o_bw = take(bwb);
   ADDFT_REQUIRE(work_bytes >= off, ADDFT_INVALID_ARG, "nonlocal_gradients: work needs %zu B, got %zu B",
                 off, work_bytes);
@@ -984,7 +1052,7 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
     ADDFT_TRY(dbecp_t<double>(dion, w + o_becp, nk, nproj, nb, nullptr, w + o_db, st));
     ADDFT_TRY(dbecp_t<double>(dion, w + o_becp, nk, nproj, nb, wocc, w + o_mw, st));
     ADDFT_TRY((apply_t<double, true, false>(w + o_mw, 1, nb, (size_t)nproj * nb, psi, (size_t)nb * nG, nk, nb,
-                                            nproj, nG, w + o_y, (size_t)nproj * nG, st)));
+                                            nproj, nG, w + o_y, (size_t)nproj * nG, w + o_bw, bwb, st)));
     k_nl_energy<double><<<(nk * nb + 127) / 128, 128, 0, st>>>((const double2 *)(w + o_becp),
                                                               (const double2 *)(w + o_db), nk, nproj, nb,
                                                               wocc, (double *)(w + o_ep));
@@ -996,7 +1064,7 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
     ADDFT_TRY(dbecp_t<float>(dion, w + o_becp, nk, nproj, nb, nullptr, w + o_db, st));
     ADDFT_TRY(dbecp_t<float>(dion, w + o_becp, nk, nproj, nb, wocc, w + o_mw, st));
     ADDFT_TRY((apply_t<float, true, false>(w + o_mw, 1, nb, (size_t)nproj * nb, psi, (size_t)nb * nG, nk, nb,
-                                           nproj, nG, w + o_y, (size_t)nproj * nG, st)));
+                                           nproj, nG, w + o_y, (size_t)nproj * nG, w + o_bw, bwb, st)));
     k_nl_energy<float><<<(nk * nb + 127) / 128, 128, 0, st>>>((const float2 *)(w + o_becp),
                                                              (const float2 *)(w + o_db), nk, nproj, nb, wocc,
                                                              (double *)(w + o_ep));
@@ -1018,8 +1086,7 @@ size_t addft_nonlocal_gradients_work_bytes(addft_dtype dt, int nk, int nb, int n
   s += align256((size_t)nk * nproj * nb * csz) * 3;
   s += align256((size_t)nk * nb * sizeof(double));
   s += align256((size_t)nk * nproj * 12 * sizeof(double));
-  s += align256(dt == ADDFT_F64 ? becp_work_bytes<double>(nk, nb, nG, nproj)
-                                : becp_work_bytes<float>(nk, nb, nG, nproj));
+  s += align256(nl_grad_scratch(dt, nk, nb, nG, nproj));
   return s;
 }
 

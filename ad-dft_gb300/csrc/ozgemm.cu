@@ -1,0 +1,648 @@
+// Complex FP64 GEMM on the 5th-generation tensor cores (tcgen05.mma kind::f16) by exact
+// digit slicing (the Ozaki scheme), for the framework's FP64 contractions:
+//   becp = conj(beta) psi^T and V_NL psi = beta^T (D becp)   (nonlocal_op.py:67-82)
+//   the refinement's projections X^H Y and rotations U X      (solver/davidson.py:48-61)
+//
+//   C[i][j] = sum_k op(A)[i][k] op(B)[k][j],   complex128 in and out.
+//
+// GB300 runs FP64 FMA at 1.06 TFLOP/s (measured), 1/1800 of its FP16 tensor rate, so the
+// contraction is done on integers instead.  With E the binary exponent of the largest
+// |re|, |im| of a row of op(A) (a column of op(B)), every component x becomes the integer
+//   q = round(x 2^(B - E)),  |q| <= 2^B,  B = 62 (S = 8 digits) or 55 (S = 7 digits),
+// written in balanced base 256, q = sum_s d_s 256^(S-1-s), -128 <= d_s <= 128.  A digit is
+// exact in FP16 and a product of two is at most 2^14, so an FP32 accumulator adds 2^10 of them
+// without rounding.  The products d_s(a) d_t(b) of one level l = s + t share a weight and one
+// accumulator; levels 0 .. S-1 are kept (S (S + 1) / 2 digit products per real product), what
+// is dropped is below 2^-(8 S - 2) of the row's and the column's largest components.  Every 128 k
+// the accumulators are emptied into 64-bit integers, so nothing is rounded until the final
+// conversion to FP64: the error is that of the slicing, about 2^-62 (S = 8) or 2^-55 (S = 7)
+// relative to max|A_i.| max|B_.j| per term, against 2^-53 per operation of an FP64 sum.
+// Rows or columns that hold an infinity or a NaN are summed in plain FP64 at the end.
+//
+// Three kernels:
+//   k_oz_max   exponent of every row / column (one pass over each operand);
+//   k_oz_pack  digits into the operand layout of the MMA: per 16 k, real part then imaginary
+//              part, S slices each, a slice being 128 (A) or 32 (B) rows of 16 k in no-swizzle
+//              core matrices (8 rows x 16 bytes), so one stage of the GEMM is one contiguous block;
+//   k_oz_gemm  a CTA owns 128 x 32 complex outputs: the 512 columns of tensor memory hold S
+//              levels x 32 columns of the real and the imaginary accumulator.  The B slices
+//              lie side by side along N, so slice s of A times B slices 0 .. S-1-s is one MMA of
+//              N = 32 (S - s) columns that lands on levels s .. S-1: 8 MMAs per part pair
+//              instead of 36.  One thread copies stages (cp.async.bulk) and issues MMAs, sixteen
+//              warps empty the accumulators.  K is split across CTAs; the split sums are
+//              added in a fixed order.
+// MMA time bounds it: 32 MMAs per 16 k, about 2,500 cycles for 128 x 32 x 16 complex products
+// (the narrow ones wait for shared-memory operands, 4 KB per slice of A), a ceiling near
+// 64 TFLOP/s of complex FP64 work on 152 SMs.  Measured with the passes over the operands:
+//   becp, P 256, 160 bands, nG 23,847   14.34 ms (FP64 SIMT)        -> 0.43 ms
+//   apply of the same size              12.02 ms (FP64 SIMT)        -> 0.51 ms
+//   conj(X) Y^T, 168 x 336 x 23,847      3.33 ms (double-float SIMT) -> 0.61 ms
+#include <algorithm>
+
+#include "common.cuh"
+#include "ozgemm.cuh"
+
+namespace addft {
+
+namespace {
+
+__device__ unsigned g_oz_error = 0;   // bit 0: a bounded wait ran out
+
+constexpr int kRowsA = 128, kRowsB = 32;   // rows of an A / B tile
+constexpr int kStep = 16;                  // k per stage
+constexpr int kDrain = 8;                  // stages per accumulation block (128 k: sums stay exact)
+constexpr int kOzWait = 1 << 24;
+constexpr int kEpiWarps = 16;              // warps that empty the accumulators
+constexpr int kEpiCols = kRowsB / (kEpiWarps / 4);   // columns of each
+constexpr int kOzThreads = 32 * (kEpiWarps + 1);     // and one for copies and MMAs
+constexpr int kSms = 152;
+constexpr int kMinPieceK = 1024;           // K is not cut below this when scratch is short
+constexpr size_t kOzScratchCap = size_t(384) << 20;   // scratch asked for; more K, rows or batch go in pieces
+
+template <int S>
+struct Oz {
+  static constexpr int kBits = S == 8 ? 62 : 8 * S - 1;
+  static constexpr int kABytes = 2 * S * kRowsA * kStep * 2;   // one stage of A
+  static constexpr int kBBytes = 2 * S * kRowsB * kStep * 2;
+  static constexpr int kStages = 2;
+  static constexpr size_t kSmem = (size_t)kStages * (kABytes + kBBytes) + 1024;
+};
+
+__device__ __forceinline__ uint32_t sad(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity) {
+  for (int it = 0; it < kOzWait; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(sad(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void init_bar(uint64_t *bar, int n) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sad(bar)), "r"(n));
+}
+__device__ __forceinline__ void arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sad(bar)) : "memory");
+}
+__device__ __forceinline__ void commit_to(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sad(bar))
+               : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+      "r"(bytes), "r"(sad(bar))
+      : "memory");
+}
+// K-major operand without swizzle: 128 B between the two core matrices of 16 k, 256 B between row groups
+__device__ __forceinline__ uint64_t oz_desc(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
+         ((uint64_t)1 << 46);
+}
+// kind::f16, FP16 operands, FP32 accumulator, optionally negated A
+__device__ __forceinline__ uint32_t oz_idesc(int N, bool neg) {
+  return (1u << 4) | (neg ? 1u << 13 : 0u) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kRowsA >> 4) << 24);
+}
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc)
+      : "memory");
+}
+
+#define OZ_LD8(taddr, r)                                                                          \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"           \
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), \
+                 "=r"(r[7])                                                                      \
+               : "r"(taddr))
+
+// ---------------------------------------------------------------------------
+// exponents: ex[row] = largest exponent field of |re|, |im| over k (0x7ff: not finite)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int expo(double2 v) {
+  return max((__double2hiint(v.x) >> 20) & 0x7ff, (__double2hiint(v.y) >> 20) & 0x7ff);
+}
+
+// ROWMAJOR (k contiguous): a warp per row and k chunk; else a thread per row and k chunk
+template <bool ROWMAJOR>
+__global__ void __launch_bounds__(256)
+k_oz_max(const double2 *__restrict__ X, long s_row, long s_k, size_t s_batch, int rows, int K, int kchunk,
+         int *__restrict__ ex) {
+  const int k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
+  const double2 *Xb = X + blockIdx.z * s_batch;
+  int m = 0;
+  int row;
+  if (ROWMAJOR) {
+    row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row < rows)
+      for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) m = max(m, expo(Xb[row * s_row + k * s_k]));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (threadIdx.x & 31) return;
+  } else {
+    row = blockIdx.x * 256 + threadIdx.x;
+    if (row < rows)
+      for (int k = k0; k < k1; ++k) m = max(m, expo(Xb[row * s_row + k * s_k]));
+  }
+  if (row < rows && m > 0) atomicMax(ex + (size_t)blockIdx.z * rows + row, m);
+}
+
+// ---------------------------------------------------------------------------
+// digits
+// ---------------------------------------------------------------------------
+// x -> q = round(x 2^(bits - E)) of a row whose exponent field is em, plus 128 in every byte but
+// the top one: byte s of the result minus 128 is then the balanced digit.
+template <int S>
+__device__ __forceinline__ uint64_t oz_bytes(double x, int em) {
+  const uint64_t u = (uint64_t)__double_as_longlong(x);
+  const int e = (int)(u >> 52) & 0x7ff;
+  uint64_t m = u & 0xFFFFFFFFFFFFFull;
+  if (e) m |= 1ull << 52;
+  const int sh = Oz<S>::kBits - 53 - (max(em, 1) - max(e, 1));
+  uint64_t q;
+  if (sh >= 0) {
+    q = m << sh;
+  } else {
+    const int r = min(-sh, 63);
+    q = (m + (1ull << (r - 1))) >> r;
+  }
+  if ((int64_t)u < 0) q = 0 - q;
+  constexpr uint64_t kBias = S == 8 ? 0x0080808080808080ull : 0x0000808080808080ull;
+  return q + kBias;
+}
+
+// A CTA packs R rows x 2048 / R k: a coalesced read into shared memory, then a thread per row
+// and 8 k writes one 16-byte core-matrix row per part and slice.
+template <int S, int R>
+__global__ void __launch_bounds__(256)
+k_oz_pack(const double2 *__restrict__ X, long s_row, long s_k, size_t s_batch, int conj, int rows, int K, int nks,
+          const int *__restrict__ ex, unsigned char *__restrict__ out, size_t out_batch) {
+  constexpr int KT = 2048 / R;
+  constexpr int kSlice = R * kStep * 2;   // bytes of one slice
+  __shared__ double2 T[R * (KT + 1)];
+  const int r0 = blockIdx.y * R, k0 = blockIdx.x * KT;
+  const double2 *Xb = X + blockIdx.z * s_batch;
+  const bool kfast = s_k == 1;
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int i = threadIdx.x + 256 * t;
+    const int r = kfast ? i / KT : i % R, k = kfast ? i % KT : i / R;
+    double2 v = make_double2(0.0, 0.0);
+    if (r0 + r < rows && k0 + k < K) v = Xb[(r0 + r) * s_row + (k0 + k) * s_k];
+    T[r * (KT + 1) + k] = v;
+  }
+  __syncthreads();
+  const int r = threadIdx.x % R, oct = threadIdx.x / R;
+  const int step = k0 / kStep + oct / 2;
+  // rows of a tile beyond the operand's stay unwritten: each only reaches its own, unused, outputs
+  if (step >= nks || r0 + r >= rows) return;
+  const int em = ex[(size_t)blockIdx.z * rows + r0 + r];
+  unsigned char *dst = out + blockIdx.z * out_batch + ((size_t)blockIdx.y * nks + step) * (2 * S * kSlice) +
+                       (r >> 3) * 256 + (oct & 1) * 128 + (r & 7) * 16;
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    uint64_t q[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double2 v = T[r * (KT + 1) + oct * 8 + j];
+      // rows that are not finite are left to the FP64 sum of the GEMM's epilogue
+      const double x = em == 0x7ff ? 0.0 : (part ? (conj ? -v.y : v.y) : v.x);
+      q[j] = oz_bytes<S>(x, em);
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      uint32_t h[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t w;
+        if (s == 0) {   // top digit: signed, -128 .. 128
+          const int a = (int)((int64_t)q[2 * j] >> (8 * (S - 1))) + 128;
+          const int b = (int)((int64_t)q[2 * j + 1] >> (8 * (S - 1))) + 128;
+          w = (uint32_t)a | ((uint32_t)b << 16);
+        } else {
+          const uint32_t a = (uint32_t)(q[2 * j] >> (8 * (S - 1 - s))) & 0xff;
+          const uint32_t b = (uint32_t)(q[2 * j + 1] >> (8 * (S - 1 - s))) & 0xff;
+          w = a | (b << 16);
+        }
+        // 0x6400 + n is the FP16 number 1024 + n; minus 1152 leaves the digit, exactly
+        w += 0x64006400u;
+        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(h[j]) : "r"(w), "r"(0x64806480u));
+      }
+      *reinterpret_cast<uint4 *>(dst + (size_t)(part * S + s) * kSlice) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// GEMM
+// ---------------------------------------------------------------------------
+struct OzArgs {
+  const unsigned char *pa, *pb;   // packed operands
+  size_t pa_batch, pb_batch;
+  const int *ea, *eb;             // row exponents
+  int rows, cols, K, nks, nsplit, steps;   // steps: stages per split
+  // output element (i, j): out[b * s_batch + split * s_split + i * s_row + j * s_col]
+  double2 *out;
+  size_t s_batch, s_split;
+  long s_row, s_col;
+  int accum;
+  // the operands themselves, for rows and columns that are not finite
+  const double2 *A, *B;
+  long a_row, a_k, b_row, b_k;
+  size_t a_batch, b_batch;
+  int conj_a, conj_b;
+};
+
+// 2^n as a product of two factors in range
+__device__ __forceinline__ double scale2(double x, int n) {
+  const int a = n / 2, b = n - a;
+  auto p2 = [](int t) { return __hiloint2double((max(min(t, 1023), -1022) + 1023) << 20, 0); };
+  return x * p2(a) * p2(b);
+}
+
+// The FP64 sum of one output over k0 .. k1 - 1 (operands with infinities or NaNs).
+__device__ __noinline__ double2 oz_plain(const OzArgs &g, int bt, int i, int j, int k0, int k1) {
+  const double2 *a = g.A + bt * g.a_batch + i * g.a_row, *b = g.B + bt * g.b_batch + j * g.b_row;
+  double2 s = make_double2(0.0, 0.0);
+  for (int k = k0; k < k1; ++k) {
+    double2 x = a[k * g.a_k], y = b[k * g.b_k];
+    if (g.conj_a) x.y = -x.y;
+    if (g.conj_b) y.y = -y.y;
+    s.x += x.x * y.x - x.y * y.y;
+    s.y += x.x * y.y + x.y * y.x;
+  }
+  return s;
+}
+
+template <int S>
+__global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
+  using P = Oz<S>;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *smem = smem_raw + ((1024 - (sad(smem_raw) & 1023)) & 1023);
+  __shared__ __align__(8) uint64_t full[P::kStages], empty[P::kStages], accf, acce;
+  __shared__ uint32_t tslot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int bt = blockIdx.z / g.nsplit, sp = blockIdx.z - bt * g.nsplit;
+  const int s0 = sp * g.steps, s1 = min(g.nks, s0 + g.steps);
+  const int nst = max(0, s1 - s0);
+  const int nblk = (nst + kDrain - 1) / kDrain;
+  if (tid == 0) {
+    for (int i = 0; i < P::kStages; ++i) {
+      init_bar(&full[i], 1);
+      init_bar(&empty[i], 1);
+    }
+    init_bar(&accf, 1);
+    init_bar(&acce, kEpiWarps);
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sad(&tslot)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tslot;
+  const uint32_t sa = sad(smem), sb = sa + P::kStages * P::kABytes;
+  bool ok = true;
+
+  if (warp == kEpiWarps) {
+    if (lane == 0) {   // one thread copies stages and issues MMAs
+      const unsigned char *pa = g.pa + bt * g.pa_batch + ((size_t)blockIdx.x * g.nks + s0) * P::kABytes;
+      const unsigned char *pb = g.pb + bt * g.pb_batch + ((size_t)blockIdx.y * g.nks + s0) * P::kBBytes;
+      int issued = 0, landed = 0;
+      auto copy = [&](int s) {
+        const int st = s % P::kStages;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sad(&full[st])),
+                     "r"(P::kABytes + P::kBBytes)
+                     : "memory");
+        bulk_copy(sa + st * P::kABytes, pa + (size_t)s * P::kABytes, P::kABytes, &full[st]);
+        bulk_copy(sb + st * P::kBBytes, pb + (size_t)s * P::kBBytes, P::kBBytes, &full[st]);
+        issued = s + 1;
+      };
+      for (int s = 0; s < min(nst, P::kStages); ++s) copy(s);
+      for (int s = 0; s < nst; ++s) {
+        const int st = s % P::kStages, blk = s / kDrain;
+        const bool first = s % kDrain == 0;
+        if (first && blk > 0) ok = wait_bar(&acce, (blk - 1) & 1);   // the accumulators have been read
+        if (ok) ok = wait_bar(&full[st], (s / P::kStages) & 1);
+        if (!ok) break;
+        landed = s + 1;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a0 = sa + st * P::kABytes, b0 = sb + st * P::kBBytes;
+#pragma unroll
+        for (int pr = 0; pr < 4; ++pr) {
+          const int ra = pr >> 1, rb = pr & 1;               // part of A, part of B
+          const uint32_t d = tmem + ((ra ^ rb) ? 256 : 0);   // re: rr, ii; im: ri, ir
+          const uint64_t bd = oz_desc(b0 + rb * S * (kRowsB * kStep * 2));
+#pragma unroll
+          for (int i = 0; i < S; ++i) {
+            const uint64_t ad = oz_desc(a0 + (ra * S + i) * (kRowsA * kStep * 2));
+            mma_f16(d + 32 * i, ad, bd, oz_idesc(32 * (S - i), ra && rb), !(first && ra == 0 && i == 0));
+          }
+        }
+        commit_to(&empty[st]);
+        if (s % kDrain == kDrain - 1 || s == nst - 1) commit_to(&accf);
+        // the buffer of stage s - 1 is free once its MMAs are done, while those of s run
+        const int nx = s - 1 + P::kStages;
+        if (s >= 1 && nx < nst) {
+          ok = wait_bar(&empty[nx % P::kStages], ((s - 1) / P::kStages) & 1);
+          if (!ok) break;
+          copy(nx);
+        }
+      }
+      if (!ok) {
+        // neither a copy nor an MMA of this CTA may be in flight when it ends
+        atomicOr(&g_oz_error, 1u);
+        for (int s = landed; s < issued; ++s) wait_bar(&full[s % P::kStages], (s / P::kStages) & 1);
+        commit_to(&accf);
+        wait_bar(&accf, 0);
+        wait_bar(&accf, 1);
+      }
+    }
+  } else {
+    // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. and columns kEpiCols (w / 4) .. of
+    // each level
+    const int q = warp & 3, c0 = kEpiCols * (warp >> 2);
+    long long hi[2][kEpiCols], lo[2][kEpiCols];   // [re, im]
+#pragma unroll
+    for (int c = 0; c < kEpiCols; ++c) hi[0][c] = hi[1][c] = lo[0][c] = lo[1][c] = 0;
+    const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + c0;
+    for (int blk = 0; blk < nblk && ok; ++blk) {
+      ok = wait_bar(&accf, blk & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int l = 0; l < S; ++l) {
+        uint32_t v[2][kEpiCols];
+        OZ_LD8(base + 32 * l, v[0]);
+        OZ_LD8(base + 256 + 32 * l, v[1]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        const int w = l < 4 ? 1 << (8 * (3 - l)) : 1 << (8 * (S - 1 - l));
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+          for (int c = 0; c < kEpiCols; ++c) {
+            const long long x = (long long)__float2int_rn(__uint_as_float(v[p][c])) * w;
+            if (l < 4) hi[p][c] += x;
+            else lo[p][c] += x;
+          }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) arrive(&acce);
+    }
+    if (!ok && lane == 0) atomicOr(&g_oz_error, 1u);
+    const int row = blockIdx.x * kRowsA + 32 * q + lane;
+    if (ok && row < g.rows) {
+      const int em = g.ea[(size_t)bt * g.rows + row];
+      double2 *o = g.out + bt * g.s_batch + sp * g.s_split + row * g.s_row;
+      constexpr double kHi = S == 8 ? 4294967296.0 : 16777216.0;   // 256^(S - 4)
+      auto put = [&](int col, double2 v) {
+        double2 *p = o + col * g.s_col;
+        if (g.accum) {
+          const double2 w = *p;
+          v.x += w.x;
+          v.y += w.y;
+        }
+        *p = v;
+      };
+      unsigned plain = 0;   // columns left to the FP64 sum
+#pragma unroll
+      for (int c = 0; c < kEpiCols; ++c) {
+        const int col = blockIdx.y * kRowsB + c0 + c;
+        if (col >= g.cols) break;
+        const int en = g.eb[(size_t)bt * g.cols + col];
+        if (em == 0x7ff || en == 0x7ff) {
+          plain |= 1u << c;
+          continue;
+        }
+        // q_a q_b = 256^(S - 1) (hi 256^(S - 4) + lo), x = q 2^(E - bits), E = field - 1022
+        const int n = 8 * (S - 1) + max(em, 1) + max(en, 1) - 2 * 1022 - 2 * P::kBits;
+        put(col, make_double2(scale2(fma((double)hi[0][c], kHi, (double)lo[0][c]), n),
+                              scale2(fma((double)hi[1][c], kHi, (double)lo[1][c]), n)));
+      }
+      for (; plain; plain &= plain - 1) {
+        const int col = blockIdx.y * kRowsB + c0 + __ffs(plain) - 1;
+        put(col, oz_plain(g, bt, row, col, s0 * kStep, min(g.K, s1 * kStep)));
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+// C[i][j] (+)= sum_s part[s][j][i] in split order; part is column-major (rows fastest)
+__global__ void __launch_bounds__(256)
+k_oz_splits(const double2 *__restrict__ part, int nsplit, int rows, int cols, size_t part_batch, double2 *__restrict__ C,
+            long s_row, long s_col, size_t s_batch, int accum) {
+  const size_t n = (size_t)rows * cols;
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  // threads walk C along its contiguous index
+  const int i = s_row == 1 ? (int)(t % rows) : (int)(t / cols), j = s_row == 1 ? (int)(t / rows) : (int)(t % cols);
+  const double2 *p = part + blockIdx.y * part_batch + (size_t)j * rows + i;
+  double2 s = p[0];
+  for (int z = 1; z < nsplit; ++z) {
+    const double2 v = p[(size_t)z * n];
+    s.x += v.x;
+    s.y += v.y;
+  }
+  double2 *c = C + blockIdx.y * s_batch + i * s_row + j * s_col;
+  if (accum) {
+    s.x += c->x;
+    s.y += c->y;
+  }
+  *c = s;
+}
+
+inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
+
+struct OzLayout {
+  int ta, tb, nks, nsplit, steps;
+  size_t pa, pb;                       // packed bytes per batch entry
+  size_t o_ex, o_pa, o_pb, o_part, total;
+};
+
+// rows / cols as the kernel sees them (rows on the 128-row side)
+template <int S>
+OzLayout oz_layout(int rows, int cols, int K, int batch) {
+  OzLayout l;
+  l.ta = (rows + kRowsA - 1) / kRowsA;
+  l.tb = (cols + kRowsB - 1) / kRowsB;
+  l.nks = (K + kStep - 1) / kStep;
+  // A CTA fills an SM, so a split count costs waves x (accumulation blocks per CTA + about one
+  // block's time to start and to end a CTA); splits keep whole accumulation blocks.
+  const long tiles = (long)l.ta * l.tb * batch;
+  const int blocks = (l.nks + kDrain - 1) / kDrain;
+  int per = blocks;
+  long best = -1;
+  for (int ns = 1; ns <= std::min(blocks, 2 * kSms); ++ns) {
+    const int b = (blocks + ns - 1) / ns, used = (blocks + b - 1) / b;
+    const long cost = (tiles * used + kSms - 1) / kSms * (b + 1) + (used > 1 ? 1 : 0);
+    if (best < 0 || cost < best) {
+      best = cost;
+      per = b;
+    }
+    if (tiles >= 8 * kSms) break;   // many waves: nothing to fill
+  }
+  l.steps = per * kDrain;
+  l.nsplit = (l.nks + l.steps - 1) / l.steps;
+  l.pa = (size_t)l.ta * l.nks * Oz<S>::kABytes;
+  l.pb = (size_t)l.tb * l.nks * Oz<S>::kBBytes;
+  l.o_ex = 0;
+  l.o_pa = al256((size_t)batch * (rows + cols) * sizeof(int));
+  l.o_pb = l.o_pa + al256(l.pa * batch);
+  l.o_part = l.o_pb + al256(l.pb * batch);
+  l.total = l.o_part + (l.nsplit > 1 ? (size_t)l.nsplit * rows * cols * batch * sizeof(double2) : 0);
+  return l;
+}
+
+addft_status oz_max(const OzMat &m, int rows, int K, int batch, int *ex, cudaStream_t st) {
+  // enough blocks to stream the operand at memory rate
+  if (m.s_k == 1) {
+    const int rb = (rows + 7) / 8;
+    const int want = std::max(1, std::min((K + 255) / 256, (8 * 152 + rb * batch - 1) / (rb * batch)));
+    const int chunk = (K + want - 1) / want;
+    k_oz_max<true><<<dim3(rb, (K + chunk - 1) / chunk, batch), 256, 0, st>>>(
+        (const double2 *)m.p, m.s_row, m.s_k, m.s_batch, rows, K, chunk, ex);
+  } else {
+    const int rb = (rows + 255) / 256;
+    const int want = std::max(1, std::min((K + 7) / 8, (8 * 152 + rb * batch - 1) / (rb * batch)));
+    const int chunk = (K + want - 1) / want;
+    k_oz_max<false><<<dim3(rb, (K + chunk - 1) / chunk, batch), 256, 0, st>>>(
+        (const double2 *)m.p, m.s_row, m.s_k, m.s_batch, rows, K, chunk, ex);
+  }
+  return check_launch("k_oz_max");
+}
+
+template <int S, int R>
+addft_status oz_pack(const OzMat &m, int rows, int K, int nks, int batch, const int *ex, unsigned char *out,
+                     size_t out_batch, cudaStream_t st) {
+  constexpr int KT = 2048 / R;
+  k_oz_pack<S, R><<<dim3((nks * kStep + KT - 1) / KT, (rows + R - 1) / R, batch), 256, 0, st>>>(
+      (const double2 *)m.p, m.s_row, m.s_k, m.s_batch, m.conj, rows, K, nks, ex, out, out_batch);
+  return check_launch("k_oz_pack");
+}
+
+template <int S>
+addft_status oz_run(int rows, int cols, int K, int batch, const OzMat &A, const OzMat &B, double2 *C, long s_row,
+                    long s_col, size_t s_batch, bool accum, void *work, cudaStream_t st) {
+  const OzLayout l = oz_layout<S>(rows, cols, K, batch);
+  char *w = (char *)work;
+  int *ea = (int *)(w + l.o_ex), *eb = ea + (size_t)batch * rows;
+  unsigned char *pa = (unsigned char *)w + l.o_pa, *pb = (unsigned char *)w + l.o_pb;
+  ADDFT_CUDA(cudaMemsetAsync(ea, 0, (size_t)batch * (rows + cols) * sizeof(int), st));
+  ADDFT_TRY(oz_max(A, rows, K, batch, ea, st));
+  ADDFT_TRY(oz_max(B, cols, K, batch, eb, st));
+  ADDFT_TRY((oz_pack<S, kRowsA>(A, rows, K, l.nks, batch, ea, pa, l.pa, st)));
+  ADDFT_TRY((oz_pack<S, kRowsB>(B, cols, K, l.nks, batch, eb, pb, l.pb, st)));
+  OzArgs g;
+  g.pa = pa; g.pb = pb; g.pa_batch = l.pa; g.pb_batch = l.pb;
+  g.ea = ea; g.eb = eb;
+  g.rows = rows; g.cols = cols; g.K = K; g.nks = l.nks; g.nsplit = l.nsplit; g.steps = l.steps;
+  double2 *part = (double2 *)(w + l.o_part);
+  const size_t n = (size_t)rows * cols;
+  if (l.nsplit > 1) {
+    g.out = part; g.s_row = 1; g.s_col = rows; g.s_split = n; g.s_batch = n * l.nsplit; g.accum = 0;
+  } else {
+    g.out = C; g.s_row = s_row; g.s_col = s_col; g.s_split = 0; g.s_batch = s_batch; g.accum = accum ? 1 : 0;
+  }
+  g.A = (const double2 *)A.p; g.a_row = A.s_row; g.a_k = A.s_k; g.a_batch = A.s_batch; g.conj_a = A.conj;
+  g.B = (const double2 *)B.p; g.b_row = B.s_row; g.b_k = B.s_k; g.b_batch = B.s_batch; g.conj_b = B.conj;
+  ADDFT_TRY(smem_optin(k_oz_gemm<S>, Oz<S>::kSmem));
+  k_oz_gemm<S><<<dim3(l.ta, l.tb, batch * l.nsplit), kOzThreads, Oz<S>::kSmem, st>>>(g);
+  ADDFT_TRY(check_launch("k_oz_gemm"));
+  if (l.nsplit > 1) {
+    k_oz_splits<<<dim3((unsigned)((n + 255) / 256), batch), 256, 0, st>>>(part, l.nsplit, rows, cols, n * l.nsplit, C,
+                                                                         s_row, s_col, s_batch, accum ? 1 : 0);
+    ADDFT_TRY(check_launch("k_oz_splits"));
+  }
+  return ADDFT_OK;
+}
+
+// The 128-row side goes to the index that pads less, with 10 % in favour of the one C is
+// contiguous along, whose stores are then coalesced.
+bool oz_swap(int M, int N, bool m_contig, bool n_contig) {
+  auto pad = [](int a, int b) {
+    return (double)((a + kRowsA - 1) / kRowsA * kRowsA) * ((b + kRowsB - 1) / kRowsB * kRowsB);
+  };
+  return pad(N, M) * (n_contig ? 1.0 : 1.1) < pad(M, N) * (m_contig ? 1.0 : 1.1);
+}
+
+size_t oz_total(int digits, int r, int c, int K, int batch) {
+  return digits == 8 ? oz_layout<8>(r, c, K, batch).total : oz_layout<7>(r, c, K, batch).total;
+}
+
+// Pieces of a product that fit the scratch: batch entries at a time, then rows, columns or K cut
+// down, whichever packs largest.
+struct OzPieces { int batch, rows, cols, K; };
+bool oz_pieces(int digits, int r, int c, int K, int batch, size_t bytes, OzPieces &p) {
+  p = {batch, r, c, K};
+  while (oz_total(digits, p.rows, p.cols, p.K, p.batch) > bytes) {
+    auto half = [](int n, int unit) { return (n / 2 + unit - 1) / unit * unit; };
+    if (p.batch > 1) p.batch = (p.batch + 1) / 2;
+    else if (p.K > 2 * kMinPieceK) p.K = half(p.K, kDrain * kStep);
+    else if (p.rows >= p.cols && p.rows > 2 * kRowsA) p.rows = half(p.rows, kRowsA);
+    else if (p.cols > 2 * kRowsB) p.cols = half(p.cols, kRowsB);
+    else return false;
+  }
+  return (p.rows + kRowsA - 1) / kRowsA <= 65535 && (p.cols + kRowsB - 1) / kRowsB <= 65535;
+}
+
+}  // namespace
+
+size_t oz_work_bytes(int digits, int M, int N, int K, int batch) {
+  const size_t need = std::max(oz_total(digits, M, N, K, batch), oz_total(digits, N, M, K, batch));
+  return std::min(need, kOzScratchCap);
+}
+
+bool oz_fits(int digits, int M, int N, int K, int batch, const void *work, size_t bytes) {
+  OzPieces p;
+  return work && ((uintptr_t)work & 255) == 0 && oz_pieces(digits, M, N, K, batch, bytes, p) &&
+         oz_pieces(digits, N, M, K, batch, bytes, p);
+}
+
+addft_status oz_gemm(int digits, int M, int N, int K, int batch, const OzMat &A, const OzMat &B, void *C, long s_row,
+                     long s_col, size_t s_batch, bool accum, void *work, size_t work_bytes, cudaStream_t st) {
+  const bool sw = oz_swap(M, N, s_row == 1, s_col == 1);
+  const int r = sw ? N : M, c = sw ? M : N;
+  const OzMat &ma = sw ? B : A, &mb = sw ? A : B;
+  const long sr = sw ? s_col : s_row, sc = sw ? s_row : s_col;
+  OzPieces p;
+  ADDFT_REQUIRE(work && ((uintptr_t)work & 255) == 0 && oz_pieces(digits, r, c, K, batch, work_bytes, p),
+                ADDFT_INVALID_ARG, "oz_gemm: work buffer of %zu B too small or not 256-byte aligned", work_bytes);
+  auto at = [](const OzMat &m, int b, int row, int k) {
+    OzMat o = m;
+    o.p = (const double2 *)m.p + b * m.s_batch + row * m.s_row + k * m.s_k;
+    return o;
+  };
+  for (int b0 = 0; b0 < batch; b0 += p.batch)
+    for (int r0 = 0; r0 < r; r0 += p.rows)
+      for (int c0 = 0; c0 < c; c0 += p.cols)
+        for (int k0 = 0; k0 < K; k0 += p.K) {
+          const int nb = std::min(p.batch, batch - b0), nr = std::min(p.rows, r - r0), nc = std::min(p.cols, c - c0);
+          const int nk = std::min(p.K, K - k0);
+          const OzMat a = at(ma, b0, r0, k0), b = at(mb, b0, c0, k0);
+          double2 *o = (double2 *)C + b0 * s_batch + r0 * sr + c0 * sc;
+          ADDFT_TRY(digits == 8 ? oz_run<8>(nr, nc, nk, nb, a, b, o, sr, sc, s_batch, accum || k0 > 0, work, st)
+                                : oz_run<7>(nr, nc, nk, nb, a, b, o, sr, sc, s_batch, accum || k0 > 0, work, st));
+        }
+  return ADDFT_OK;
+}
+
+unsigned oz_status() {
+  unsigned v = 0, z = 0;
+  if (cudaMemcpyFromSymbol(&v, g_oz_error, sizeof(v)) != cudaSuccess) return 0xffffffffu;
+  cudaMemcpyToSymbol(g_oz_error, &z, sizeof(z));
+  return v;
+}
+
+}  // namespace addft

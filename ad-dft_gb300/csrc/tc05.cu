@@ -23,6 +23,7 @@
 // (read with addft_tc05_status), waits (bounded) for its own MMAs, frees its tensor
 // memory and returns.
 #include "common.cuh"
+#include "ozgemm.cuh"
 
 namespace addft {
 
@@ -526,7 +527,7 @@ unsigned addft_tc05_status(void) {
   unsigned v = 0, z = 0;
   if (cudaMemcpyFromSymbol(&v, addft::g_tc05_error, sizeof(v)) != cudaSuccess) return 0xffffffffu;
   cudaMemcpyToSymbol(addft::g_tc05_error, &z, sizeof(z));
-  return v;
+  return v | addft::oz_status();
 }
 
 }  // extern "C"

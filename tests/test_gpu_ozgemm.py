@@ -1,0 +1,111 @@
+"""The tensor-core form of the FP64 contractions (exact digit slices) against FP64 on the same
+operands: double-float entry point (7 digits), becp and the V_NL apply (8 digits), at the edges of
+its tiles (128 rows, 32 columns, 16 k per stage, 128 k per accumulation block)."""
+
+from __future__ import annotations
+
+import math
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+if torch.cuda.is_available():
+    from addft_gb300 import ops
+    from addft_gb300._lib import LIB
+
+U = 2.0 ** -53
+
+
+def rnd(seed, *s, spread=0.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.complex(torch.randn(*s, generator=g, device="cuda", dtype=torch.float64),
+                      torch.randn(*s, generator=g, device="cuda", dtype=torch.float64))
+    if spread:   # components over `spread` decades, as plane-wave coefficients have
+        x = x * 10.0 ** (-spread * torch.rand(*s, generator=g, device="cuda", dtype=torch.float64))
+    return x
+
+
+def bound(a, b, bits):
+    """Slicing (2^-bits of the row's and the column's largest components per term, on both operands
+    and for the dropped levels) plus the rounding of an FP64 sum of K terms in the reference."""
+    K = a.shape[1]
+    big = a.abs().amax(1)[:, None] * b.abs().amax(0)[None]
+    return 8.0 * K * big * 2.0 ** -bits + (math.sqrt(K) + 4.0) * 4 * U * (a.abs() @ b.abs())
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 32, 6000), (129, 33, 2049), (127, 31, 2047), (1, 70, 20000), (300, 5, 1111),
+                                   (64, 96, 1024), (65, 257, 4099), (37, 1700, 40), (200, 3000, 130)])
+@pytest.mark.parametrize("spread", [0.0, 9.0])
+def test_zgemm_df_tiles(M, N, K, spread):
+    a, b = rnd(M, M, K, spread=spread), rnd(N + 1, N, K, spread=spread)
+    out = ops.zgemm_df(a, b.transpose(0, 1), conj_a=True)
+    ref = a.conj() @ b.T
+    assert bool(((out - ref).abs() <= bound(a, b.T, 55)).all())
+    c = rnd(3, K, N)                       # rotation: the right operand's rows are contiguous along N
+    out = ops.zgemm_df(a, c)
+    assert bool(((out - a @ c).abs() <= bound(a, c, 55)).all())
+    out = ops.zgemm_df(a.T.contiguous().T, c.T.contiguous().T, conj_b=True)   # both operands transposed
+    assert bool(((out - a @ c.conj()).abs() <= bound(a, c, 55)).all())
+
+
+@pytest.mark.parametrize("nk,nb,P,nG", [(1, 64, 32, 1301), (2, 33, 129, 2050), (3, 31, 8, 4097), (1, 160, 64, 3001),
+                                        (1, 1, 260, 5000), (8, 4, 8, 20000)])
+def test_becp_and_apply_tiles(nk, nb, P, nG):
+    proj, psi = rnd(1, nk, P, nG, spread=6.0), rnd(2, nk, nb, nG)
+    b = ops.becp(proj, psi)
+    dion = torch.diag(torch.linspace(-2.0, 1.0, P, dtype=torch.float64, device="cuda"))
+    h0 = rnd(4, nk, nb, nG)
+    h = ops.vnl_apply(proj, dion, b, h0.clone())
+    for k in range(nk):
+        ref = proj[k].conj() @ psi[k].T
+        assert bool(((b[k] - ref).abs() <= bound(proj[k], psi[k].T, 60)).all())
+        db = dion.to(torch.complex128) @ b[k]
+        add = db.T @ proj[k]
+        assert bool(((h[k] - (h0[k] + add)).abs() <= bound(db.T, proj[k], 60) + 2 * U * h0[k].abs()).all())
+
+
+def test_scales_zeros_and_values_that_are_not_finite():
+    M, N, K = 40, 50, 3000
+    a, b = rnd(1, M, K), rnd(2, N, K)
+    a[0] *= 1e-290
+    a[1] *= 1e250
+    b[2] *= 1e-200
+    a[3] = 0
+    a[4, 1:] = 0
+    a[5] = 0.7                              # every digit of every term alike: the largest sums
+    b[5] = 0.9
+    a[6] = complex(5e-324, 0)               # subnormal
+    ref = a.conj() @ b.T
+    out = ops.zgemm_df(a, b.transpose(0, 1), conj_a=True)
+    rows = [i for i in range(M) if i != 6]
+    ok = (out - ref).abs() <= bound(a, b.T, 55) + 1e-323
+    assert bool(ok[rows].all())
+    a[7, 11] = complex(float("inf"), 0.0)
+    b[9, 13] = complex(0.0, float("nan"))
+    out2 = ops.zgemm_df(a, b.transpose(0, 1), conj_a=True)
+    bad = torch.zeros((M, N), dtype=torch.bool, device="cuda")
+    bad[7], bad[:, 9] = True, True
+    assert bool((~torch.isfinite(torch.view_as_real(out2)).all(-1) == bad).all())
+    assert torch.equal(out2[~bad], out[~bad])
+    assert LIB.addft_tc05_status() == 0
+
+
+def test_pieces_of_a_product_when_scratch_is_short():
+    """The same product with the scratch of the whole and with an eighth of it (K, rows in pieces)."""
+    import ctypes as C
+    M, N, K = 100, 90, 9000
+    a, b = rnd(1, M, K), rnd(2, N, K)
+    need = int(LIB.addft_zgemm_df_work_bytes(M, N, K))
+    outs = []
+    for nbytes in (need, need // 4):
+        w = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        out = torch.empty((M, N), dtype=torch.complex128, device="cuda")
+        st = LIB.addft_zgemm_df(M, N, K, C.c_void_p(a.data_ptr()), K, 1, 1, C.c_void_p(b.data_ptr()), 1, K, 0,
+                                C.c_void_p(out.data_ptr()), N, C.c_void_p(w.data_ptr()), nbytes,
+                                C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == 0
+        torch.cuda.synchronize()
+        outs.append(out)
+    for o in outs:
+        assert bool(((o - a.conj() @ b.T).abs() <= bound(a, b.T, 55)).all())
