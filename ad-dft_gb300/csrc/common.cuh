@@ -113,12 +113,17 @@ struct PlanDev {
   const int *row_i2;
   const int *plane_of_i1;  // n1 entries, -1 for empty planes
   const int *miller;       // nG*3 (original order), unwrapped integers
+  int mmax[3];             // largest |miller| per axis (sizes of the phase tables)
   // column pipeline: a column is an (i1, i2) pair holding sphere points; columns
   // are the rows above (row_i2, in plane order), ncols = nrows, padded to ncols_pad
   int ncols_pad;           // multiple of kColGroup
   const int *cgptr;        // ncols_pad / kColGroup + 1: first sorted point of each column group
   const int *pt_pos;       // nG: i3 * kColPitch + (column % kColGroup) of each sorted point
   const int *col_xy;       // ncols: i1 * (n2 | 1) + i2 of each column (xy tile position)
+  const int *pt_col;       // nG: column of each sorted point
+  const int *col_m;        // ncols * 2: unwrapped (m1, m2) of each column
+  int col_uniform;         // 1 when all points of every column share (m1, m2) (false only for Miller
+                           // indices that the box wraps onto one another's columns)
   // xy_direct = 1 when every active x-plane's columns are i2 = 0 .. nlo-1 and n2-nhi .. n2-1
   // (true for spheres around G = 0): row_lohi[p] = nlo | nhi << 16
   int xy_direct;
@@ -160,6 +165,32 @@ addft_status check_launch(const char *what);
     addft_status _s = (expr);            \
     if (_s != ADDFT_OK) return _s;       \
   } while (0)
+
+// b . R / 2 pi for a phase e^{-i m b.R}, less its nearest integer, as an unevaluated sum hi + lo
+// of two doubles: a phase then shows the coordinates it is given to their last bit (two atoms that
+// a symmetry maps onto one another up to rounding stay as unequal as they are).
+struct Turns { double hi, lo; };
+inline Turns phase_turns(const double *b, const double *r) {
+  double s = 0.0, e = 0.0;
+  for (int x = 0; x < 3; ++x) {
+    const double p = b[x] * r[x], pe = __builtin_fma(b[x], r[x], -p);
+    const double t = s + p, z = t - s;
+    e += (s - (t - z)) + (p - z) + pe;
+    s = t;
+  }
+  constexpr double hi = 6.283185307179586477, lo = 2.449293598294706414e-16;   // 2 pi
+  const double q = s / hi, rem = (__builtin_fma(-q, hi, s) - q * lo + e) / hi;
+  const double h = q - __builtin_rint(q), t = h + rem;
+  return {t, rem - (t - h)};
+}
+
+// e^{-2 pi i m f}: the rounding of m f.hi and m f.lo are put back as a rotation
+__device__ __forceinline__ double2 phase_exp(int m, Turns f) {
+  const double p = m * f.hi, d = (fma((double)m, f.hi, -p) + m * f.lo) * 6.283185307179586477;
+  double sn, cs;
+  sincospi(2.0 * p, &sn, &cs);
+  return make_double2(cs - sn * d, -(sn + cs * d));
+}
 
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 

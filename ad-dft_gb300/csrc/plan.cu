@@ -30,27 +30,20 @@ addft_status check_launch(const char *what) {
   return ADDFT_OK;
 }
 
-__global__ void k_finalize_sums(const double *partial, int nv, int nblk, double *out, int acc) {
-  __shared__ double red[32];
-  for (int j = 0; j < nv; ++j) {
+// A warp per value; with the values one after another in one block it took 17 us for ten.
+__global__ void __launch_bounds__(320) k_finalize_sums(const double *partial, int nv, int nblk, double *out, int acc) {
+  const int lane = threadIdx.x & 31;
+  for (int j = threadIdx.x >> 5; j < nv; j += blockDim.x >> 5) {
     double x = 0.0;
-    for (int i = threadIdx.x; i < nblk; i += blockDim.x) x += partial[(size_t)j * nblk + i];
+    for (int i = lane; i < nblk; i += 32) x += partial[(size_t)j * nblk + i];
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      const int nw = (blockDim.x + 31) >> 5;
-      double y = threadIdx.x < nw ? red[threadIdx.x] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
-      if (threadIdx.x == 0) out[j] = acc ? out[j] + y : y;
-    }
-    __syncthreads();
+    if (lane == 0) out[j] = acc ? out[j] + x : x;
   }
 }
 
 addft_status finalize_sums(const double *partial, int nv, int nblk, double *out, bool acc,
                            cudaStream_t st) {
-  k_finalize_sums<<<1, 256, 0, st>>>(partial, nv, nblk, out, acc ? 1 : 0);
+  k_finalize_sums<<<1, 32 * std::min(nv, 10), 0, st>>>(partial, nv, nblk, out, acc ? 1 : 0);
   return check_launch("finalize_sums");
 }
 
@@ -181,7 +174,8 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
   }
   // column pipeline tables: column c = c-th (i1, i2) row in sorted order
   const int ncols_pad = (nrows + kColGroup - 1) / kColGroup * kColGroup;
-  std::vector<int> cgptr(ncols_pad / kColGroup + 1, nG), pt_pos(nG), col_xy(nrows);
+  std::vector<int> cgptr(ncols_pad / kColGroup + 1, nG), pt_pos(nG), col_xy(nrows), pt_col(nG), col_m(2 * nrows);
+  bool col_uniform = true;
   {
     int c = -1;
     for (int k = 0; k < nG; ++k) {
@@ -190,7 +184,11 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
         ++c;
         col_xy[c] = i1[g] * (n2 | 1) + i2[g];
         if (c % kColGroup == 0) cgptr[c / kColGroup] = k;
+        col_m[2 * c] = miller[3 * (size_t)g];
+        col_m[2 * c + 1] = miller[3 * (size_t)g + 1];
       }
+      pt_col[k] = c;
+      if (col_m[2 * c] != miller[3 * (size_t)g] || col_m[2 * c + 1] != miller[3 * (size_t)g + 1]) col_uniform = false;
       pt_pos[k] = i3[g] * kColPitch + c % kColGroup;
     }
   }
@@ -229,7 +227,7 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
   const size_t o_spg = push(sp_g), o_spp = push(sp_pos), o_gptr = push(gptr),
                o_pi1 = push(plane_i1), o_rptr = push(rptr), o_row = push(row_i2),
                o_poi = push(plane_of_i1), o_mil = push(mil), o_cgp = push(cgptr), o_ptp = push(pt_pos),
-               o_cxy = push(col_xy), o_rlh = push(row_lohi);
+               o_cxy = push(col_xy), o_rlh = push(row_lohi), o_ptc = push(pt_col), o_cm = push(col_m);
   const size_t total = off_int + sizeof(int) * ints.size();
 
   auto *p = new addft_plan_s();
@@ -257,7 +255,15 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
   d.n1 = n1; d.n2 = n2; d.n3 = n3; d.nG = nG; d.np = np; d.nrows = nrows;
   d.sp_g = ib + o_spg; d.sp_pos = ib + o_spp; d.gptr = ib + o_gptr; d.plane_i1 = ib + o_pi1;
   d.rptr = ib + o_rptr; d.row_i2 = ib + o_row; d.plane_of_i1 = ib + o_poi; d.miller = ib + o_mil;
+  for (int a = 0; a < 3; ++a) {
+    d.mmax[a] = 0;
+    for (int g = 0; g < nG; ++g) {
+      const long m = miller[3 * (size_t)g + a];
+      d.mmax[a] = (int)std::max<long>(d.mmax[a], std::min<long>(m < 0 ? -m : m, 1 << 30));
+    }
+  }
   d.ncols_pad = ncols_pad; d.cgptr = ib + o_cgp; d.pt_pos = ib + o_ptp; d.col_xy = ib + o_cxy;
+  d.pt_col = ib + o_ptc; d.col_m = ib + o_cm; d.col_uniform = col_uniform ? 1 : 0;
   d.xy_direct = xy_direct ? 1 : 0; d.row_lohi = ib + o_rlh;
   d.tw_d = b + off_twd;
   d.tw_f = b + off_twf;
