@@ -179,12 +179,6 @@ static int df_nsplit(int M, int N, int K) {
   return std::max(ns, 1);
 }
 
-// From about 1e6 complex products on the product runs as exact digit slices on the tensor cores
-// (ozgemm.cu, 7 digits: 55 bits against the 48 of this file's splits; 168 x 336 x 23,847: 0.61 ms
-// against 3.33 ms here, error against FP64 1.9e-15 against 1.2e-13); smaller ones, and calls
-// without its scratch, stay here.
-static bool df_on_tensor_cores(int M, int N, int K) { return (double)M * N * K >= 1e6; }
-
 }  // namespace addft
 
 using namespace addft;
@@ -193,7 +187,7 @@ extern "C" size_t addft_zgemm_df_work_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const int ns = df_nsplit(M, N, K);
   const size_t df = ns > 1 ? (size_t)ns * M * N * sizeof(double2) : 0;
-  return df_on_tensor_cores(M, N, K) ? std::max(df, oz_work_bytes(7, M, N, K, 1)) : df;
+  return std::max(df, oz_work_bytes(7, M, N, K, 1));
 }
 
 extern "C" addft_status addft_zgemm_df(int M, int N, int K, const void *A, long sAi, long sAk, int conjA,
@@ -209,7 +203,7 @@ extern "C" addft_status addft_zgemm_df(int M, int N, int K, const void *A, long 
     return ADDFT_OK;
   }
   ADDFT_REQUIRE(A && B, ADDFT_INVALID_ARG, "zgemm_df: null operand");
-  if (df_on_tensor_cores(M, N, K) && oz_fits(7, M, N, K, 1, work, work_bytes)) {
+  if (oz_fits(7, M, N, K, 1, work, work_bytes)) {   // ozgemm.cu; without its scratch, this file's kernel
     const OzMat a = {A, sAi, sAk, 0, conjA}, b = {B, sBj, sBk, 0, conjB};
     return oz_gemm(7, M, N, K, 1, a, b, C, ldc, 1, 0, false, work, work_bytes, st);
   }

@@ -28,7 +28,7 @@
 //              levels x 32 columns of the real and the imaginary accumulator.  The B slices
 //              lie side by side along N, so slice s of A times B slices 0 .. S-1-s is one MMA of
 //              N = 32 (S - s) columns that lands on levels s .. S-1: 8 MMAs per part pair
-//              instead of 36.  One thread copies stages (cp.async.bulk) and issues MMAs, sixteen
+//              instead of 36.  One thread copies operands (cp.async.bulk), one issues MMAs, sixteen
 //              warps empty the accumulators.  K is split across CTAs; the split sums are
 //              added in a fixed order.
 // MMA time bounds it: 32 MMAs per 16 k, about 2,500 cycles for 128 x 32 x 16 complex products
@@ -54,7 +54,7 @@ constexpr int kDrain = 8;                  // stages per accumulation block (128
 constexpr int kOzWait = 1 << 24;
 constexpr int kEpiWarps = 16;              // warps that empty the accumulators
 constexpr int kEpiCols = kRowsB / (kEpiWarps / 4);   // columns of each
-constexpr int kOzThreads = 32 * (kEpiWarps + 1);     // and one for copies and MMAs
+constexpr int kOzThreads = 32 * (kEpiWarps + 2);     // one for copies, one for MMAs
 constexpr int kSms = 152;
 constexpr int kMinPieceK = 1024;           // K is not cut below this when scratch is short
 constexpr size_t kOzScratchCap = size_t(384) << 20;   // scratch asked for; more K, rows or batch go in pieces
@@ -64,8 +64,11 @@ struct Oz {
   static constexpr int kBits = S == 8 ? 62 : 8 * S - 1;
   static constexpr int kABytes = 2 * S * kRowsA * kStep * 2;   // one stage of A
   static constexpr int kBBytes = 2 * S * kRowsB * kStep * 2;
-  static constexpr int kStages = 2;
-  static constexpr size_t kSmem = (size_t)kStages * (kABytes + kBBytes) + 1024;
+  // A in a ring of parts (re, im of a stage are two items), B in a ring of stages: 208 KB (S = 8).
+  // Whole stages of both, twice buffered, left the copy of one stage to the MMAs of one: 2.6 us per
+  // stage where the MMAs take 1.25.
+  static constexpr int kAItem = kABytes / 2, kARing = 5, kBRing = 3;
+  static constexpr size_t kSmem = (size_t)kARing * kAItem + kBRing * kBBytes + 1024;
 };
 
 __device__ __forceinline__ uint32_t sad(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -245,7 +248,7 @@ struct OzArgs {
   const unsigned char *pa, *pb;   // packed operands
   size_t pa_batch, pb_batch;
   const int *ea, *eb;             // row exponents
-  int rows, cols, K, nks, nsplit, steps;   // steps: stages per split
+  int rows, cols, tb, K, nks, nsplit, steps;   // tb: column tiles; steps: stages per split
   // output element (i, j): out[b * s_batch + split * s_split + i * s_row + j * s_col]
   double2 *out;
   size_t s_batch, s_split;
@@ -258,11 +261,56 @@ struct OzArgs {
   int conj_a, conj_b;
 };
 
+// (hi 2^SH + lo) 2^n to nearest, ties to even, in integer arithmetic: on the FP64 pipe the
+// conversions and scalings of one 128 x 32 tile took 19 us, the MMAs of 16 k take 1.2 us.
+template <int SH>
+__device__ __forceinline__ double oz_value(long long hi, long long lo, int n);
+
 // 2^n as a product of two factors in range
 __device__ __forceinline__ double scale2(double x, int n) {
   const int a = n / 2, b = n - a;
   auto p2 = [](int t) { return __hiloint2double((max(min(t, 1023), -1022) + 1023) << 20, 0); };
   return x * p2(a) * p2(b);
+}
+
+template <int SH>
+__device__ __forceinline__ double oz_value(long long hi, long long lo, int n) {
+  uint64_t L = (uint64_t)hi << SH;
+  long long H = hi >> (64 - SH);
+  const uint64_t L2 = L + (uint64_t)lo;
+  H += (lo >> 63) + (L2 < L ? 1 : 0);
+  L = L2;
+  const bool neg = H < 0;
+  if (neg) {
+    L = 0 - L;
+    H = ~H + (L == 0 ? 1 : 0);
+  }
+  if ((H | (long long)L) == 0) return 0.0;
+  // top: the 64 bits from the leading one down, worth 2^(e - 63); rest: anything below
+  int e;
+  uint64_t top, rest;
+  if (H != 0) {
+    const int z = __clzll(H);
+    top = z ? ((uint64_t)H << z) | (L >> (64 - z)) : (uint64_t)H;
+    rest = L << z;
+    e = 127 - z;
+  } else {
+    const int z = __clzll((long long)L);
+    top = L << z;
+    rest = 0;
+    e = 63 - z;
+  }
+  const int be = e + n + 1023;
+  if (be <= 0 || be >= 2046) {   // subnormal, underflow or overflow
+    const double v = scale2((double)top * 5.42101086242752217e-20, 0);   // top 2^-64
+    const int m = e + n + 1;
+    const double r = scale2(scale2(v, m / 2), m - m / 2);
+    return neg ? -r : r;
+  }
+  uint64_t u = ((uint64_t)be << 52) + ((top >> 11) & 0xFFFFFFFFFFFFFull);
+  const uint64_t low = top & 0x7ff;
+  u += (low > 0x400 || (low == 0x400 && (rest || (u & 1)))) ? 1 : 0;
+  return __longlong_as_double((long long)(neg ? u | 0x8000000000000000ull : u));
 }
 
 // The FP64 sum of one output over k0 .. k1 - 1 (operands with infinities or NaNs).
@@ -284,17 +332,23 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
   using P = Oz<S>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = smem_raw + ((1024 - (sad(smem_raw) & 1023)) & 1023);
-  __shared__ __align__(8) uint64_t full[P::kStages], empty[P::kStages], accf, acce;
+  __shared__ __align__(8) uint64_t fa[P::kARing], ea[P::kARing], fb[P::kBRing], eb[P::kBRing], accf, acce;
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int bt = blockIdx.z / g.nsplit, sp = blockIdx.z - bt * g.nsplit;
+  // column tiles fastest: CTAs that run together share their rows' operand in L2
+  const int rt = blockIdx.x / g.tb, ct = blockIdx.x - rt * g.tb;
+  const int bt = blockIdx.y / g.nsplit, sp = blockIdx.y - bt * g.nsplit;
   const int s0 = sp * g.steps, s1 = min(g.nks, s0 + g.steps);
   const int nst = max(0, s1 - s0);
   const int nblk = (nst + kDrain - 1) / kDrain;
   if (tid == 0) {
-    for (int i = 0; i < P::kStages; ++i) {
-      init_bar(&full[i], 1);
-      init_bar(&empty[i], 1);
+    for (int i = 0; i < P::kARing; ++i) {
+      init_bar(&fa[i], 1);
+      init_bar(&ea[i], 1);
+    }
+    for (int i = 0; i < P::kBRing; ++i) {
+      init_bar(&fb[i], 1);
+      init_bar(&eb[i], 1);
     }
     init_bar(&accf, 1);
     init_bar(&acce, kEpiWarps);
@@ -308,58 +362,81 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
-  const uint32_t sa = sad(smem), sb = sa + P::kStages * P::kABytes;
+  const uint32_t sa = sad(smem), sb = sa + P::kARing * P::kAItem;
   bool ok = true;
 
   if (warp == kEpiWarps) {
-    if (lane == 0) {   // one thread copies stages and issues MMAs
-      const unsigned char *pa = g.pa + bt * g.pa_batch + ((size_t)blockIdx.x * g.nks + s0) * P::kABytes;
-      const unsigned char *pb = g.pb + bt * g.pb_batch + ((size_t)blockIdx.y * g.nks + s0) * P::kBBytes;
-      int issued = 0, landed = 0;
-      auto copy = [&](int s) {
-        const int st = s % P::kStages;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sad(&full[st])),
-                     "r"(P::kABytes + P::kBBytes)
-                     : "memory");
-        bulk_copy(sa + st * P::kABytes, pa + (size_t)s * P::kABytes, P::kABytes, &full[st]);
-        bulk_copy(sb + st * P::kBBytes, pb + (size_t)s * P::kBBytes, P::kBBytes, &full[st]);
-        issued = s + 1;
+    if (lane == 0) {   // copies
+      const unsigned char *pa = g.pa + bt * g.pa_batch + ((size_t)rt * g.nks + s0) * P::kABytes;
+      const unsigned char *pb = g.pb + bt * g.pb_batch + ((size_t)ct * g.nks + s0) * P::kBBytes;
+      // a tile with fewer rows copies only their core matrices, slice by slice
+      const int rows8 = (min(kRowsA, g.rows - rt * kRowsA) + 7) & ~7;
+      constexpr uint32_t kSlice = kRowsA * kStep * 2;
+      auto expect = [&](uint64_t *bar, uint32_t bytes) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sad(bar)), "r"(bytes) : "memory");
       };
-      for (int s = 0; s < min(nst, P::kStages); ++s) copy(s);
-      for (int s = 0; s < nst; ++s) {
-        const int st = s % P::kStages, blk = s / kDrain;
+      int na = 0, nb = 0;   // items under way
+      for (int a = 0; a < 2 * nst && ok; ++a) {
+        const int s = a >> 1;
+        if (!(a & 1)) {
+          const int j = s % P::kBRing;
+          if (s >= P::kBRing) ok = wait_bar(&eb[j], (s / P::kBRing - 1) & 1);
+          if (!ok) break;
+          expect(&fb[j], P::kBBytes);
+          bulk_copy(sb + j * P::kBBytes, pb + (size_t)s * P::kBBytes, P::kBBytes, &fb[j]);
+          nb = s + 1;
+        }
+        const int j = a % P::kARing;
+        if (a >= P::kARing) ok = wait_bar(&ea[j], (a / P::kARing - 1) & 1);
+        if (!ok) break;
+        const uint32_t dst = sa + j * P::kAItem;
+        const unsigned char *src = pa + (size_t)a * P::kAItem;
+        if (rows8 == kRowsA) {
+          expect(&fa[j], P::kAItem);
+          bulk_copy(dst, src, P::kAItem, &fa[j]);
+        } else {
+          expect(&fa[j], S * rows8 * kStep * 2);
+          for (int i = 0; i < S; ++i) bulk_copy(dst + i * kSlice, src + i * kSlice, rows8 * kStep * 2, &fa[j]);
+        }
+        na = a + 1;
+      }
+      // nothing may still be landing in shared memory when the CTA ends
+      for (int a = max(0, na - P::kARing); a < na; ++a) ok = wait_bar(&fa[a % P::kARing], (a / P::kARing) & 1) && ok;
+      for (int s = max(0, nb - P::kBRing); s < nb; ++s) ok = wait_bar(&fb[s % P::kBRing], (s / P::kBRing) & 1) && ok;
+      if (!ok) atomicOr(&g_oz_error, 1u);
+    }
+  } else if (warp == kEpiWarps + 1) {
+    if (lane == 0) {   // MMAs
+      for (int s = 0; s < nst && ok; ++s) {
+        const int jb = s % P::kBRing, blk = s / kDrain;
         const bool first = s % kDrain == 0;
         if (first && blk > 0) ok = wait_bar(&acce, (blk - 1) & 1);   // the accumulators have been read
-        if (ok) ok = wait_bar(&full[st], (s / P::kStages) & 1);
-        if (!ok) break;
-        landed = s + 1;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = sa + st * P::kABytes, b0 = sb + st * P::kBBytes;
+        if (ok) ok = wait_bar(&fb[jb], (s / P::kBRing) & 1);
+        const uint32_t b0 = sb + jb * P::kBBytes;
 #pragma unroll
-        for (int pr = 0; pr < 4; ++pr) {
-          const int ra = pr >> 1, rb = pr & 1;               // part of A, part of B
-          const uint32_t d = tmem + ((ra ^ rb) ? 256 : 0);   // re: rr, ii; im: ri, ir
-          const uint64_t bd = oz_desc(b0 + rb * S * (kRowsB * kStep * 2));
-#pragma unroll
-          for (int i = 0; i < S; ++i) {
-            const uint64_t ad = oz_desc(a0 + (ra * S + i) * (kRowsA * kStep * 2));
-            mma_f16(d + 32 * i, ad, bd, oz_idesc(32 * (S - i), ra && rb), !(first && ra == 0 && i == 0));
-          }
-        }
-        commit_to(&empty[st]);
-        if (s % kDrain == kDrain - 1 || s == nst - 1) commit_to(&accf);
-        // the buffer of stage s - 1 is free once its MMAs are done, while those of s run
-        const int nx = s - 1 + P::kStages;
-        if (s >= 1 && nx < nst) {
-          ok = wait_bar(&empty[nx % P::kStages], ((s - 1) / P::kStages) & 1);
+        for (int ra = 0; ra < 2; ++ra) {   // part of A
+          const int a = 2 * s + ra, ja = a % P::kARing;
+          if (ok) ok = wait_bar(&fa[ja], (a / P::kARing) & 1);
           if (!ok) break;
-          copy(nx);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a0 = sa + ja * P::kAItem;
+#pragma unroll
+          for (int rb = 0; rb < 2; ++rb) {   // part of B; re: rr, ii; im: ri, ir
+            const uint32_t d = tmem + ((ra ^ rb) ? 256 : 0);
+            const uint64_t bd = oz_desc(b0 + rb * S * (kRowsB * kStep * 2));
+#pragma unroll
+            for (int i = 0; i < S; ++i)
+              mma_f16(d + 32 * i, oz_desc(a0 + i * (kRowsA * kStep * 2)), bd, oz_idesc(32 * (S - i), ra && rb),
+                      !(first && ra == 0 && i == 0));
+          }
+          commit_to(&ea[ja]);
         }
+        if (!ok) break;
+        commit_to(&eb[jb]);
+        if (s % kDrain == kDrain - 1 || s == nst - 1) commit_to(&accf);
       }
-      if (!ok) {
-        // neither a copy nor an MMA of this CTA may be in flight when it ends
+      if (!ok) {   // every MMA issued has to be done before tensor memory is given back
         atomicOr(&g_oz_error, 1u);
-        for (int s = landed; s < issued; ++s) wait_bar(&full[s % P::kStages], (s / P::kStages) & 1);
         commit_to(&accf);
         wait_bar(&accf, 0);
         wait_bar(&accf, 1);
@@ -399,11 +476,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
       if (lane == 0) arrive(&acce);
     }
     if (!ok && lane == 0) atomicOr(&g_oz_error, 1u);
-    const int row = blockIdx.x * kRowsA + 32 * q + lane;
+    const int row = rt * kRowsA + 32 * q + lane;
     if (ok && row < g.rows) {
       const int em = g.ea[(size_t)bt * g.rows + row];
       double2 *o = g.out + bt * g.s_batch + sp * g.s_split + row * g.s_row;
-      constexpr double kHi = S == 8 ? 4294967296.0 : 16777216.0;   // 256^(S - 4)
       auto put = [&](int col, double2 v) {
         double2 *p = o + col * g.s_col;
         if (g.accum) {
@@ -416,7 +492,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
       unsigned plain = 0;   // columns left to the FP64 sum
 #pragma unroll
       for (int c = 0; c < kEpiCols; ++c) {
-        const int col = blockIdx.y * kRowsB + c0 + c;
+        const int col = ct * kRowsB + c0 + c;
         if (col >= g.cols) break;
         const int en = g.eb[(size_t)bt * g.cols + col];
         if (em == 0x7ff || en == 0x7ff) {
@@ -425,11 +501,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
         }
         // q_a q_b = 256^(S - 1) (hi 256^(S - 4) + lo), x = q 2^(E - bits), E = field - 1022
         const int n = 8 * (S - 1) + max(em, 1) + max(en, 1) - 2 * 1022 - 2 * P::kBits;
-        put(col, make_double2(scale2(fma((double)hi[0][c], kHi, (double)lo[0][c]), n),
-                              scale2(fma((double)hi[1][c], kHi, (double)lo[1][c]), n)));
+        put(col, make_double2(oz_value<8 * (S - 4)>(hi[0][c], lo[0][c], n), oz_value<8 * (S - 4)>(hi[1][c], lo[1][c], n)));
       }
       for (; plain; plain &= plain - 1) {
-        const int col = blockIdx.y * kRowsB + c0 + __ffs(plain) - 1;
+        const int col = ct * kRowsB + c0 + __ffs(plain) - 1;
         put(col, oz_plain(g, bt, row, col, s0 * kStep, min(g.K, s1 * kStep)));
       }
     }
@@ -461,6 +536,140 @@ k_oz_splits(const double2 *__restrict__ part, int nsplit, int rows, int cols, si
     s.y += c->y;
   }
   *c = s;
+}
+
+// ---------------------------------------------------------------------------
+// Small products in plain FP64, one launch
+// ---------------------------------------------------------------------------
+struct SmallArgs {
+  OzMat A, B;
+  double2 *C;
+  long s_row, s_col;
+  size_t s_batch;
+  int M, N, K, accum;
+};
+
+__device__ __forceinline__ void cfma(double2 &s, double2 x, double2 y) {
+  s.x += x.x * y.x - x.y * y.y;
+  s.y += x.x * y.y + x.y * y.x;
+}
+
+__device__ __forceinline__ void small_put(const SmallArgs &g, int b, int i, int j, double2 v) {
+  double2 *c = g.C + b * g.s_batch + i * g.s_row + j * g.s_col;
+  if (g.accum) {
+    v.x += c->x;
+    v.y += c->y;
+  }
+  *c = v;
+}
+
+// long K: a CTA sums 2 x 2 outputs over one of nsplit ranges of K
+__global__ void __launch_bounds__(128) k_small_dot(SmallArgs g, int nsplit, double2 *__restrict__ part) {
+  const int j0 = 2 * blockIdx.x, i0 = 2 * blockIdx.y, b = blockIdx.z / nsplit, sp = blockIdx.z % nsplit;
+  const int per = (g.K + nsplit - 1) / nsplit, k0 = sp * per, k1 = min(g.K, k0 + per);
+  const double2 *a = (const double2 *)g.A.p + b * g.A.s_batch, *x = (const double2 *)g.B.p + b * g.B.s_batch;
+  const double2 *ar[2], *xr[2];
+  for (int r = 0; r < 2; ++r) {
+    ar[r] = a + min(i0 + r, g.M - 1) * g.A.s_row;
+    xr[r] = x + min(j0 + r, g.N - 1) * g.B.s_row;
+  }
+  double2 s[2][2];
+  for (int r = 0; r < 2; ++r)
+    for (int c = 0; c < 2; ++c) s[r][c] = make_double2(0.0, 0.0);
+  const double ca = g.A.conj ? -1.0 : 1.0, cb = g.B.conj ? -1.0 : 1.0;
+#pragma unroll 2
+  for (int k = k0 + threadIdx.x; k < k1; k += 128) {
+    double2 u[2], v[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      u[r] = ar[r][k * g.A.s_k];
+      v[r] = xr[r][k * g.B.s_k];
+      u[r].y *= ca;
+      v[r].y *= cb;
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) cfma(s[r][c], u[r], v[c]);
+  }
+  __shared__ double red[4][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    double t = (q & 1) ? s[q >> 2][(q >> 1) & 1].y : s[q >> 2][(q >> 1) & 1].x;
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) red[warp][q] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    const int i = i0 + (threadIdx.x >> 1), j = j0 + (threadIdx.x & 1), q = 2 * threadIdx.x;
+    const double2 v = make_double2(red[0][q] + red[1][q] + red[2][q] + red[3][q],
+                                   red[0][q + 1] + red[1][q + 1] + red[2][q + 1] + red[3][q + 1]);
+    if (i < g.M && j < g.N) {
+      if (nsplit > 1) part[((size_t)b * nsplit + sp) * g.M * g.N + (size_t)j * g.M + i] = v;
+      else small_put(g, b, i, j, v);
+    }
+  }
+}
+
+// short K: a thread per output, lanes along the index C is contiguous in
+__global__ void __launch_bounds__(128) k_small_outer(SmallArgs g, int j_fast) {
+  const size_t n = (size_t)g.M * g.N;
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const int b = blockIdx.y;
+  if (t >= n) return;
+  const int i = j_fast ? (int)(t / g.N) : (int)(t % g.M), j = j_fast ? (int)(t % g.N) : (int)(t / g.M);
+  const double2 *a = (const double2 *)g.A.p + b * g.A.s_batch + i * g.A.s_row;
+  const double2 *x = (const double2 *)g.B.p + b * g.B.s_batch + j * g.B.s_row;
+  double2 s = make_double2(0.0, 0.0);
+#pragma unroll 4
+  for (int k = 0; k < g.K; ++k) {
+    double2 u = a[k * g.A.s_k], v = x[k * g.B.s_k];
+    if (g.A.conj) u.y = -u.y;
+    if (g.B.conj) v.y = -v.y;
+    cfma(s, u, v);
+  }
+  small_put(g, b, i, j, s);
+}
+
+// CTAs of k_small_dot per output group so that the chip has about four per SM
+int small_splits(int M, int N, int K, int batch) {
+  const long groups = (long)((M + 1) / 2) * ((N + 1) / 2) * batch;
+  return (int)std::max<long>(1, std::min<long>((K + 1023) / 1024, 4 * kSms / groups));
+}
+size_t small_bytes(int M, int N, int K, int batch) {
+  const int ns = small_splits(M, N, K, batch);
+  return ns > 1 ? (size_t)ns * M * N * batch * sizeof(double2) : 0;
+}
+
+// Estimated microseconds of the two forms (measured: plain FP64 16 us per 10^6 complex products
+// beyond its launch; the digit slices 25 us for their small kernels, then 1.3 us per tile and 16 k
+// over the SMs).
+bool small_product(int M, int N, int K, int batch) {
+  const double work = (double)M * N * K * batch;
+  if (work > 2e7) return false;
+  auto tiles = [](int r, int c) { return (double)((r + kRowsA - 1) / kRowsA) * ((c + kRowsB - 1) / kRowsB); };
+  const double t = std::min(tiles(M, N), tiles(N, M)) * batch * ((K + kStep - 1) / kStep);
+  return 5.0 + 16e-6 * work < 25.0 + 1.3 * t / kSms;
+}
+
+addft_status small_run(int M, int N, int K, int batch, const OzMat &A, const OzMat &B, double2 *C, long s_row, long s_col,
+                       size_t s_batch, bool accum, void *work, size_t bytes, cudaStream_t st) {
+  const SmallArgs g = {A, B, C, s_row, s_col, s_batch, M, N, K, accum ? 1 : 0};
+  const bool contig = A.s_k == 1 && B.s_k == 1;
+  const size_t n = (size_t)M * N;
+  if (K >= 64 && (contig || (double)M * N < 8192) && (M + 1) / 2 <= 65535) {
+    int ns = small_splits(M, N, K, batch);
+    if (!work || bytes < small_bytes(M, N, K, batch)) ns = 1;
+    k_small_dot<<<dim3((N + 1) / 2, (M + 1) / 2, batch * ns), 128, 0, st>>>(g, ns, (double2 *)work);
+    ADDFT_TRY(check_launch("k_small_dot"));
+    if (ns == 1) return ADDFT_OK;
+    k_oz_splits<<<dim3((unsigned)((n + 255) / 256), batch), 256, 0, st>>>((const double2 *)work, ns, M, N, n * ns, C, s_row,
+                                                                         s_col, s_batch, accum ? 1 : 0);
+    return check_launch("k_oz_splits");
+  }
+  k_small_outer<<<dim3((unsigned)((n + 127) / 128), batch), 128, 0, st>>>(g, s_col == 1 ? 1 : 0);
+  return check_launch("k_small_outer");
 }
 
 inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -547,7 +756,7 @@ addft_status oz_run(int rows, int cols, int K, int batch, const OzMat &A, const 
   OzArgs g;
   g.pa = pa; g.pb = pb; g.pa_batch = l.pa; g.pb_batch = l.pb;
   g.ea = ea; g.eb = eb;
-  g.rows = rows; g.cols = cols; g.K = K; g.nks = l.nks; g.nsplit = l.nsplit; g.steps = l.steps;
+  g.rows = rows; g.cols = cols; g.tb = l.tb; g.K = K; g.nks = l.nks; g.nsplit = l.nsplit; g.steps = l.steps;
   double2 *part = (double2 *)(w + l.o_part);
   const size_t n = (size_t)rows * cols;
   if (l.nsplit > 1) {
@@ -558,7 +767,7 @@ addft_status oz_run(int rows, int cols, int K, int batch, const OzMat &A, const 
   g.A = (const double2 *)A.p; g.a_row = A.s_row; g.a_k = A.s_k; g.a_batch = A.s_batch; g.conj_a = A.conj;
   g.B = (const double2 *)B.p; g.b_row = B.s_row; g.b_k = B.s_k; g.b_batch = B.s_batch; g.conj_b = B.conj;
   ADDFT_TRY(smem_optin(k_oz_gemm<S>, Oz<S>::kSmem));
-  k_oz_gemm<S><<<dim3(l.ta, l.tb, batch * l.nsplit), kOzThreads, Oz<S>::kSmem, st>>>(g);
+  k_oz_gemm<S><<<dim3(l.ta * l.tb, batch * l.nsplit), kOzThreads, Oz<S>::kSmem, st>>>(g);
   ADDFT_TRY(check_launch("k_oz_gemm"));
   if (l.nsplit > 1) {
     k_oz_splits<<<dim3((unsigned)((n + 255) / 256), batch), 256, 0, st>>>(part, l.nsplit, rows, cols, n * l.nsplit, C,
@@ -594,17 +803,19 @@ bool oz_pieces(int digits, int r, int c, int K, int batch, size_t bytes, OzPiece
     else if (p.cols > 2 * kRowsB) p.cols = half(p.cols, kRowsB);
     else return false;
   }
-  return (p.rows + kRowsA - 1) / kRowsA <= 65535 && (p.cols + kRowsB - 1) / kRowsB <= 65535;
+  return (p.rows + kRowsA - 1) / kRowsA <= 65535 && (p.cols + kRowsB - 1) / kRowsB <= 65535 && p.batch <= 200;
 }
 
 }  // namespace
 
 size_t oz_work_bytes(int digits, int M, int N, int K, int batch) {
+  if (small_product(M, N, K, batch)) return small_bytes(M, N, K, batch);
   const size_t need = std::max(oz_total(digits, M, N, K, batch), oz_total(digits, N, M, K, batch));
   return std::min(need, kOzScratchCap);
 }
 
 bool oz_fits(int digits, int M, int N, int K, int batch, const void *work, size_t bytes) {
+  if (small_product(M, N, K, batch)) return true;
   OzPieces p;
   return work && ((uintptr_t)work & 255) == 0 && oz_pieces(digits, M, N, K, batch, bytes, p) &&
          oz_pieces(digits, N, M, K, batch, bytes, p);
@@ -612,6 +823,8 @@ bool oz_fits(int digits, int M, int N, int K, int batch, const void *work, size_
 
 addft_status oz_gemm(int digits, int M, int N, int K, int batch, const OzMat &A, const OzMat &B, void *C, long s_row,
                      long s_col, size_t s_batch, bool accum, void *work, size_t work_bytes, cudaStream_t st) {
+  if (small_product(M, N, K, batch))
+    return small_run(M, N, K, batch, A, B, (double2 *)C, s_row, s_col, s_batch, accum, work, work_bytes, st);
   const bool sw = oz_swap(M, N, s_row == 1, s_col == 1);
   const int r = sw ? N : M, c = sw ? M : N;
   const OzMat &ma = sw ? B : A, &mb = sw ? A : B;
