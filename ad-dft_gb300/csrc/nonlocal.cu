@@ -21,6 +21,7 @@ struct GeoParams {
   double inv_sqrt_omega;
   int nat, nh, nk;
   double pos[kMaxAtoms * 3];
+  Turns frac[kMaxAtoms * 3];  // b_a . R / 2 pi: phases e^{-2 pi i m frac}
   double kpt[kMaxK * 3];
   // per projector channel c in [0, nh): radial index, l, m
   int ch_rad[kMaxNh], ch_l[kMaxNh], ch_m[kMaxNh];
@@ -40,6 +41,8 @@ inline addft_status make_geo(GeoParams &g, const double *bvec, double omega, int
   g.nat = nat;
   g.nk = nk;
   for (int i = 0; i < 3 * nat; ++i) g.pos[i] = pos[i];
+  for (int i = 0; i < nat; ++i)
+    for (int a = 0; a < 3; ++a) g.frac[3 * i + a] = phase_turns(bvec + 3 * a, pos + 3 * i);
   for (int i = 0; i < 3 * nk; ++i) g.kpt[i] = kpts ? kpts[i] : 0.0;
   g.nh = 0;
   if (psp) {
@@ -138,28 +141,129 @@ __device__ __forceinline__ ProjEval proj_eval(const GeoParams &gp, int c, double
   return out;
 }
 
-// proj[k][p][g], p = atom * nh + channel
-template <typename R>
-__global__ void k_projectors(PlanDev pd, GeoParams gp, typename Cx<R>::T *__restrict__ proj) {
-  using C = typename Cx<R>::T;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int p = blockIdx.y;
-  const int k = blockIdx.z;
-  if (g >= pd.nG) return;
-  const int i = p / gp.nh, c = p - i * gp.nh;
+__device__ __forceinline__ void kg_vec(const PlanDev &pd, const GeoParams &gp, int g, int k, double *G, double *v) {
   const double m1 = pd.miller[3 * g], m2 = pd.miller[3 * g + 1], m3 = pd.miller[3 * g + 2];
-  const double vx = m1 * gp.B[0] + m2 * gp.B[3] + m3 * gp.B[6] + gp.kpt[3 * k];
-  const double vy = m1 * gp.B[1] + m2 * gp.B[4] + m3 * gp.B[7] + gp.kpt[3 * k + 1];
-  const double vz = m1 * gp.B[2] + m2 * gp.B[5] + m3 * gp.B[8] + gp.kpt[3 * k + 2];
-  const ProjEval pe = proj_eval(gp, c, vx, vy, vz);
-  const double arg = vx * gp.pos[3 * i] + vy * gp.pos[3 * i + 1] + vz * gp.pos[3 * i + 2];
-  double sn, cs;
-  sincos(arg, &sn, &cs);
-  const double a = pe.beta * gp.inv_sqrt_omega;
-  C out;
-  out.x = (R)(a * cs);
-  out.y = (R)(-a * sn);   // e^{-i v.R}
-  proj[((size_t)k * gridDim.y + p) * pd.nG + g] = out;
+  for (int a = 0; a < 3; ++a) {
+    G[a] = m1 * gp.B[a] + m2 * gp.B[3 + a] + m3 * gp.B[6 + a];
+    v[a] = G[a] + gp.kpt[3 * k + a];
+  }
+}
+
+// The phases e^{-i(k+G).R} of one atom, from tables in shared memory: with G = sum_a m_a b_a they
+// are e12[m1, m2] e3[m3], e12 holding e^{-ik.R} too, so a phase costs one complex product where
+// its sincos costs some 60 FP64 instructions (GB300 issues under two per SM and cycle).
+// Entries e^{-2 pi i m f} come from sincospi, which reduces its argument exactly (phase_exp).
+struct PhaseTab {
+  double2 *e1, *e2, *e3, *e12;   // e12 == nullptr: no room for the products, e1 e2 instead
+  int M1, M2, M3;
+};
+
+__host__ __device__ inline size_t phase_small(const PlanDev &pd) {   // entries of e1, e2, e3
+  return 2 * ((size_t)pd.mmax[0] + pd.mmax[1] + pd.mmax[2]) + 3;
+}
+__host__ __device__ inline size_t phase_pairs(const PlanDev &pd) {
+  return (2 * (size_t)pd.mmax[0] + 1) * (2 * (size_t)pd.mmax[1] + 1);
+}
+// Shared-memory forms: 2 = with e12 (up to 64 KB, three CTAs per SM), 1 = e1, e2, e3 only,
+// 0 = a sincos per phase: shells with few G per table entry (building the tables then takes longer
+// than the phases; nG below about 800), and Miller indices far outside a box, which the plan wraps.
+constexpr size_t kPhaseBytes = 64 << 10;
+inline int phase_form(const PlanDev &pd, size_t &bytes) {
+  const size_t small = phase_small(pd) * sizeof(double2), all = small + phase_pairs(pd) * sizeof(double2);
+  if ((size_t)pd.nG < 16 * phase_small(pd)) { bytes = 0; return 0; }
+  if (all <= kPhaseBytes) { bytes = all; return 2; }
+  if (small <= kPhaseBytes) { bytes = small; return 1; }
+  bytes = 0;
+  return 0;
+}
+
+template <int FORM>
+__device__ __forceinline__ PhaseTab phase_build(const PlanDev &pd, const GeoParams &gp, int i, int k, double2 *sm) {
+  PhaseTab t;
+  t.M1 = pd.mmax[0];
+  t.M2 = pd.mmax[1];
+  t.M3 = pd.mmax[2];
+  t.e1 = sm;
+  t.e2 = t.e1 + 2 * t.M1 + 1;
+  t.e3 = t.e2 + 2 * t.M2 + 1;
+  t.e12 = FORM == 2 ? t.e3 + 2 * t.M3 + 1 : nullptr;
+  if (FORM == 0) return t;
+  const int n1 = 2 * t.M1 + 1, n2 = 2 * t.M2 + 1, n3 = 2 * t.M3 + 1;
+  const double kr = gp.kpt[3 * k] * gp.pos[3 * i] + gp.kpt[3 * k + 1] * gp.pos[3 * i + 1] +
+                    gp.kpt[3 * k + 2] * gp.pos[3 * i + 2];
+  for (int t0 = threadIdx.x; t0 < n1 + n2 + n3; t0 += blockDim.x) {
+    const int ax = t0 < n1 ? 0 : (t0 < n1 + n2 ? 1 : 2);
+    const int m = ax == 0 ? t0 - t.M1 : (ax == 1 ? t0 - n1 - t.M2 : t0 - n1 - n2 - t.M3);
+    double2 e = phase_exp(m, gp.frac[3 * i + ax]);
+    if (ax == 0 && kr != 0.0) {
+      double sn, cs;
+      sincos(kr, &sn, &cs);
+      e = cmul(e, make_double2(cs, -sn));
+    }
+    sm[t0] = e;
+  }
+  __syncthreads();
+  if (FORM == 2) {
+    for (int p = threadIdx.x; p < n1 * n2; p += blockDim.x) t.e12[p] = cmul(t.e1[p / n2], t.e2[p % n2]);
+    __syncthreads();
+  }
+  return t;
+}
+
+// e^{-i v.R_i} at G index g (v = k + G)
+template <int FORM>
+__device__ __forceinline__ double2 phase_at(const PlanDev &pd, const GeoParams &gp, const PhaseTab &t, int i, int k,
+                                            int g) {
+  if (FORM == 0) {
+    double G[3], v[3], sn, cs;
+    kg_vec(pd, gp, g, k, G, v);
+    sincos(v[0] * gp.pos[3 * i] + v[1] * gp.pos[3 * i + 1] + v[2] * gp.pos[3 * i + 2], &sn, &cs);
+    return make_double2(cs, -sn);
+  }
+  const int m1 = pd.miller[3 * g] + t.M1, m2 = pd.miller[3 * g + 1] + t.M2, m3 = pd.miller[3 * g + 2] + t.M3;
+  const double2 a = FORM == 2 ? t.e12[m1 * (2 * t.M2 + 1) + m2] : cmul(t.e1[m1], t.e2[m2]);
+  return cmul(a, t.e3[m3]);
+}
+
+// beta~_c(|k+G|) Y_lm(k+G) / sqrt(omega) of every channel, once per G instead of once per atom and
+// G: as doubles in the rows of the last atom of proj (8 or 16 bytes per element), which
+// k_projectors turns into that atom's projectors in its last launch.
+template <typename R>
+__global__ void __launch_bounds__(128)
+k_proj_forms(PlanDev pd, GeoParams gp, typename Cx<R>::T *__restrict__ proj) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+  if (g >= pd.nG) return;
+  double G[3], v[3];
+  kg_vec(pd, gp, g, k, G, v);
+  auto *last = proj + ((size_t)k * gp.nat + gp.nat - 1) * gp.nh * pd.nG;
+  for (int c = 0; c < gp.nh; ++c)
+    *reinterpret_cast<double *>(last + (size_t)c * pd.nG + g) = proj_eval(gp, c, v[0], v[1], v[2]).beta * gp.inv_sqrt_omega;
+}
+
+// proj[k][p][g], p = atom * nh + channel: the channels' form factors (k_proj_forms) times the
+// atom's phase.  A CTA takes one atom (i0 + blockIdx.y) and `per` G.  Bound by the FP64 pipe, 12
+// instructions per atom and G and the store of 16 nh bytes; evaluating form factor and sincos for
+// every (p, G) took 1,038 us for 256 projectors x 23,847 G, 70 us so.
+template <typename R, int FORM>
+__global__ void __launch_bounds__(256)
+k_projectors(PlanDev pd, GeoParams gp, int i0, int per, typename Cx<R>::T *__restrict__ proj) {
+  using C = typename Cx<R>::T;
+  extern __shared__ __align__(16) double2 ph_smem[];
+  const int i = i0 + blockIdx.y, k = blockIdx.z;
+  const PhaseTab t = phase_build<FORM>(pd, gp, i, k, ph_smem);
+  const C *form = proj + ((size_t)k * gp.nat + gp.nat - 1) * gp.nh * pd.nG;
+  C *out = proj + ((size_t)k * gp.nat + i) * gp.nh * pd.nG;
+  const int g1 = min(pd.nG, (int)(blockIdx.x + 1) * per);
+  for (int g = blockIdx.x * per + threadIdx.x; g < g1; g += 256) {
+    const double2 p = phase_at<FORM>(pd, gp, t, i, k, g);
+    for (int c = 0; c < gp.nh; ++c) {
+      const double f = *reinterpret_cast<const double *>(form + (size_t)c * pd.nG + g);
+      C o;
+      o.x = (R)(f * p.x);
+      o.y = (R)(f * p.y);
+      out[(size_t)c * pd.nG + g] = o;
+    }
+  }
 }
 
 // kinetic diagonal 1/2 |k+G|^2
@@ -424,62 +528,102 @@ k_apply(const typename Cx<R>::T *__restrict__ Xm, int xs_j, int xs_i, size_t xs_
   }
 }
 
-// E_NL partial per (k, b): wocc * Re(B^H D B); writes partial[k*nb + b]
+// E_NL partial per (k, b): wocc * Re(B^H D B); writes partial[k*nb + b].  32 bands per CTA, its
+// eight rows of threads share the projectors (one thread per band took 128 us at 160 x 256).
 template <typename R>
-__global__ void k_nl_energy(const typename Cx<R>::T *__restrict__ becp,
-                            const typename Cx<R>::T *__restrict__ dbecp, int nk, int nproj, int nb,
-                            const double *__restrict__ wocc, double *__restrict__ out) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nk * nb) return;
-  const int k = t / nb, b = t - k * nb;
+__global__ void __launch_bounds__(256)
+k_nl_energy(const typename Cx<R>::T *__restrict__ becp, const typename Cx<R>::T *__restrict__ dbecp, int nproj, int nb,
+            const double *__restrict__ wocc, double *__restrict__ out) {
+  __shared__ double red[8][33];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5, b = blockIdx.x * 32 + lane, k = blockIdx.y;
   double s = 0.0;
-  for (int p = 0; p < nproj; ++p) {
-    const auto x = becp[((size_t)k * nproj + p) * nb + b];
-    const auto y = dbecp[((size_t)k * nproj + p) * nb + b];
-    s += (double)x.x * (double)y.x + (double)x.y * (double)y.y;
+  if (b < nb)
+    for (int p = row; p < nproj; p += 8) {
+      const auto x = becp[((size_t)k * nproj + p) * nb + b];
+      const auto y = dbecp[((size_t)k * nproj + p) * nb + b];
+      s += (double)x.x * (double)y.x + (double)x.y * (double)y.y;
+    }
+  red[row][lane] = s;
+  __syncthreads();
+  if (row == 0 && b < nb) {
+    for (int r = 1; r < 8; ++r) s += red[r][lane];
+    out[(size_t)k * nb + b] = wocc[(size_t)k * nb + b] * s;
   }
-  out[t] = wocc[t] * s;
+}
+
+template <typename R>
+addft_status nl_energy_t(const void *becp, const void *dbecp, int nk, int nproj, int nb, const double *wocc, double *out,
+                         cudaStream_t st) {
+  using C = typename Cx<R>::T;
+  k_nl_energy<R><<<dim3((nb + 31) / 32, nk), 256, 0, st>>>((const C *)becp, (const C *)dbecp, nproj, nb, wocc, out);
+  return check_launch("k_nl_energy");
 }
 
 // Envelope gradients of E_NL from Y[k][p][g] = sum_b wocc (D B)[p][b] conj(psi_b(g)):
 //   dE/dR_{i,a} = sum_{p in i} sum_g 2 v_a Im(beta_p y)
 //   dE/deps_ab  = -2 sum_p sum_g Re(Q_pa y) G_b            (the -E_NL delta_ab term is added later)
-// one CTA per (k, p); partial[(k*P + p)*12 + j]
+// A CTA takes one atom, one k and one of nsplit ranges of g; partial[((k nat + i) nsplit + s) * 12 + j].
+// Channels are summed before the v and G factors are applied, and phases come from the tables above
+// (form[k][c][4][g]: beta and its gradient per channel, shared by the atoms, or nullptr: evaluated
+// here).  One CTA per (k, p) with a sincos and a form factor per (p, g) took 2,796 us on Si64, 190 us so.
 template <typename R>
-__global__ void __launch_bounds__(256)
-k_nl_grad(PlanDev pd, GeoParams gp, const typename Cx<R>::T *__restrict__ Y, int nproj,
-          double *__restrict__ partial) {
-  const int p = blockIdx.x, k = blockIdx.y;
-  const int i = p / gp.nh, c = p - i * gp.nh;
-  const auto *Yp = Y + ((size_t)k * nproj + p) * pd.nG;
+__global__ void __launch_bounds__(128)
+k_nl_forms(PlanDev pd, GeoParams gp, double *__restrict__ form) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+  if (g >= pd.nG) return;
+  double G[3], v[3];
+  kg_vec(pd, gp, g, k, G, v);
+  double *f = form + (size_t)k * gp.nh * 4 * pd.nG + g;
+  for (int c = 0; c < gp.nh; ++c) {
+    const ProjEval e = proj_eval(gp, c, v[0], v[1], v[2]);
+    f[(size_t)(4 * c) * pd.nG] = e.beta;
+    for (int a = 0; a < 3; ++a) f[(size_t)(4 * c + 1 + a) * pd.nG] = e.grad[a];
+  }
+}
+
+template <typename R, int FORM>
+__global__ void __launch_bounds__(256, 2)
+k_nl_grad(PlanDev pd, GeoParams gp, const typename Cx<R>::T *__restrict__ Y, const double *__restrict__ form,
+          int nsplit, double *__restrict__ partial) {
+  extern __shared__ __align__(16) double2 ph_smem[];
+  const int i = blockIdx.x, sp = blockIdx.y, k = blockIdx.z;
+  const PhaseTab t = phase_build<FORM>(pd, gp, i, k, ph_smem);
+  const auto *Yi = Y + ((size_t)k * gp.nat + i) * gp.nh * pd.nG;
+  const double *fk = form ? form + (size_t)k * gp.nh * 4 * pd.nG : nullptr;
+  const int per = (pd.nG + nsplit - 1) / nsplit;
+  const int ga = sp * per, gb = min(pd.nG, ga + per);
   double acc[12];
 #pragma unroll
   for (int j = 0; j < 12; ++j) acc[j] = 0.0;
-  for (int g = threadIdx.x; g < pd.nG; g += blockDim.x) {
-    const double m1 = pd.miller[3 * g], m2 = pd.miller[3 * g + 1], m3 = pd.miller[3 * g + 2];
-    const double Gx = m1 * gp.B[0] + m2 * gp.B[3] + m3 * gp.B[6];
-    const double Gy = m1 * gp.B[1] + m2 * gp.B[4] + m3 * gp.B[7];
-    const double Gz = m1 * gp.B[2] + m2 * gp.B[5] + m3 * gp.B[8];
-    const double v[3] = {Gx + gp.kpt[3 * k], Gy + gp.kpt[3 * k + 1], Gz + gp.kpt[3 * k + 2]};
-    const double G[3] = {Gx, Gy, Gz};
-    const ProjEval pe = proj_eval(gp, c, v[0], v[1], v[2]);
-    const double arg = v[0] * gp.pos[3 * i] + v[1] * gp.pos[3 * i + 1] + v[2] * gp.pos[3 * i + 2];
-    double sn, cs;
-    sincos(arg, &sn, &cs);
-    const auto yv = Yp[g];
-    const double yr = yv.x, yi = yv.y;
-    // phase * y = (cs - i sn)(yr + i yi)
-    const double pr = (cs * yr + sn * yi) * gp.inv_sqrt_omega;
-    const double pim = (cs * yi - sn * yr) * gp.inv_sqrt_omega;
-    // beta y = beta~ * (phase y)
-    const double im_by = pe.beta * pim;
+  for (int g = ga + threadIdx.x; g < gb; g += blockDim.x) {
+    double G[3], v[3];
+    kg_vec(pd, gp, g, k, G, v);
+    const double2 p = phase_at<FORM>(pd, gp, t, i, k, g);
+    double s = 0.0, r[3] = {0.0, 0.0, 0.0};
+    for (int c = 0; c < gp.nh; ++c) {
+      const auto yv = Yi[(size_t)c * pd.nG + g];
+      const double yr = yv.x, yi = yv.y;
+      const double pr = p.x * yr - p.y * yi, pim = p.x * yi + p.y * yr;   // phase * y
+      double b, gr[3];
+      if (fk) {
+        b = fk[(size_t)(4 * c) * pd.nG + g];
+        for (int a = 0; a < 3; ++a) gr[a] = fk[(size_t)(4 * c + 1 + a) * pd.nG + g];
+      } else {
+        const ProjEval e = proj_eval(gp, c, v[0], v[1], v[2]);
+        b = e.beta;
+        for (int a = 0; a < 3; ++a) gr[a] = e.grad[a];
+      }
+      s += b * pim;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) acc[a] += 2.0 * v[a] * im_by;
+      for (int a = 0; a < 3; ++a) r[a] += gr[a] * pr;
+    }
+    s *= 2.0 * gp.inv_sqrt_omega;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const double re_qy = pe.grad[a] * pr;
+      acc[a] += v[a] * s;
+      const double ra = -2.0 * gp.inv_sqrt_omega * r[a];
 #pragma unroll
-      for (int b = 0; b < 3; ++b) acc[3 + 3 * a + b] += -2.0 * re_qy * G[b];
+      for (int b = 0; b < 3; ++b) acc[3 + 3 * a + b] += ra * G[b];
     }
   }
   // block reduce 12 values
@@ -495,36 +639,41 @@ k_nl_grad(PlanDev pd, GeoParams gp, const typename Cx<R>::T *__restrict__ Y, int
   if (threadIdx.x < 12) {
     double s = 0.0;
     for (int w = 0; w < (blockDim.x >> 5); ++w) s += red[w][threadIdx.x];
-    partial[((size_t)k * nproj + p) * 12 + threadIdx.x] = s;
+    partial[(((size_t)k * gp.nat + i) * nsplit + sp) * 12 + threadIdx.x] = s;
   }
 }
 
-// out: [0] E_NL, [1..3nat] dE/dR, [1+3nat..] dE/deps (9)
-__global__ void k_nl_grad_final(const double *__restrict__ epart, int nkb,
-                                const double *__restrict__ gpart, int nk, int nproj, int nh,
-                                int nat, double *__restrict__ out) {
-  __shared__ double e_nl;
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int t = 0; t < nkb; ++t) s += epart[t];
-    e_nl = s;
-    out[0] = s;
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < 3 * nat + 9; t += blockDim.x) {
-    double s = 0.0;
-    if (t < 3 * nat) {
-      const int i = t / 3, a = t - 3 * i;
-      for (int k = 0; k < nk; ++k)
-        for (int c = 0; c < nh; ++c) s += gpart[((size_t)k * nproj + i * nh + c) * 12 + a];
+// out: [0] E_NL, [1..3nat] dE/dR, [1+3nat..] dE/deps (9); a warp per output
+__global__ void __launch_bounds__(128)
+k_nl_grad_final(const double *__restrict__ epart, int nkb, const double *__restrict__ gpart, int nk, int nat,
+                int nsplit, double *__restrict__ out) {
+  const int lane = threadIdx.x & 31, t = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (t >= 1 + 3 * nat + 9) return;
+  auto warp_sum = [&](double x) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+  double s = 0.0;
+  if (t >= 1 && t < 1 + 3 * nat) {
+    const int i = (t - 1) / 3, a = (t - 1) % 3;
+    for (int q = lane; q < nk * nsplit; q += 32)
+      s += gpart[(((size_t)(q / nsplit) * nat + i) * nsplit + q % nsplit) * 12 + a];
+    s = warp_sum(s);
+  } else {
+    const int ab = t - 1 - 3 * nat;
+    double e = 0.0;
+    if (t == 0 || ab % 4 == 0)
+      for (int q = lane; q < nkb; q += 32) e += epart[q];
+    e = warp_sum(e);
+    if (t > 0) {
+      for (int q = lane; q < nk * nat * nsplit; q += 32) s += gpart[(size_t)q * 12 + 3 + ab];
+      s = warp_sum(s);
+      if (ab % 4 == 0) s -= e;
     } else {
-      const int ab = t - 3 * nat;
-      for (int k = 0; k < nk; ++k)
-        for (int p = 0; p < nproj; ++p) s += gpart[((size_t)k * nproj + p) * 12 + 3 + ab];
-      if (ab == 0 || ab == 4 || ab == 8) s -= e_nl;
+      s = e;
     }
-    out[1 + t] = s;
   }
+  if (lane == 0) out[t] = s;
 }
 
 // kinetic stress partials: -sum wocc |psi|^2 (k+G)_a G_b
@@ -605,18 +754,13 @@ static int becp_ctas_per_sm() {
   return m;
 }
 
-// The FP64 contractions run on the tensor cores (oz_gemm) from this many complex products per k
-// on; below, its five small kernels take longer than the FP64 SIMT kernel.
-constexpr double kOzMinWork = 3e5;
-inline bool on_tensor_cores(int m, int n, int kk) { return (double)m * n * kk >= kOzMinWork; }
-
 template <typename R>
 size_t becp_work_bytes(int nk, int nb, int nG, int nproj) {
   using C = typename Cx<R>::T;
   const int tiles = ((nproj + kBP - 1) / kBP) * ((nb + kBB - 1) / kBB) * nk;
   const int ns = pick_nsplit(tiles, nG);
   const size_t simt = ns > 1 ? (size_t)(ns + split_groups(ns)) * nk * nproj * nb * sizeof(C) : 0;
-  if (sizeof(R) == 8 && on_tensor_cores(nproj, nb, nG)) return std::max(simt, oz_work_bytes(8, nproj, nb, nG, nk));
+  if (sizeof(R) == 8) return std::max(simt, oz_work_bytes(8, nproj, nb, nG, nk));
   return simt;
 }
 
@@ -625,7 +769,7 @@ addft_status becp_t(int nk, int nb, int nG, int nproj, const void *proj, const v
                     void *work, size_t bytes, cudaStream_t st) {
   using C = typename Cx<R>::T;
   if constexpr (sizeof(R) == 8) {
-    if (on_tensor_cores(nproj, nb, nG) && oz_fits(8, nproj, nb, nG, nk, work, bytes)) {
+    if (oz_fits(8, nproj, nb, nG, nk, work, bytes)) {
       const OzMat b = {proj, nG, 1, (size_t)nproj * nG, 1}, x = {psi, nG, 1, (size_t)nb * nG, 0};
       return oz_gemm(8, nproj, nb, nG, nk, b, x, becp, nb, 1, (size_t)nproj * nb, false, work, bytes, st);
     }
@@ -708,7 +852,7 @@ static int apply_mode() {
 // scratch (work, bytes) serves the FP64 tensor-core form; without enough of it the SIMT kernel runs
 template <typename R>
 size_t apply_work_bytes(int nk, int nj, int ni, int nG) {
-  return sizeof(R) == 8 && on_tensor_cores(ni, nj, nG) ? oz_work_bytes(8, ni, nG, nj, nk) : 0;
+  return sizeof(R) == 8 ? oz_work_bytes(8, ni, nG, nj, nk) : 0;
 }
 
 template <typename R, bool CONJ_A, bool ACCUM>
@@ -717,7 +861,7 @@ addft_status apply_t(const void *X, int xs_j, int xs_i, size_t xs_k, const void 
                      cudaStream_t st) {
   using C = typename Cx<R>::T;
   if constexpr (sizeof(R) == 8) {
-    if (on_tensor_cores(ni, nj, nG) && oz_fits(8, ni, nG, nj, nk, work, bytes)) {
+    if (oz_fits(8, ni, nG, nj, nk, work, bytes)) {
       const OzMat x = {X, xs_i, xs_j, xs_k, 0}, a = {A, 1, nG, as_k, CONJ_A ? 1 : 0};
       return oz_gemm(8, ni, nG, nj, nk, x, a, out, nG, 1, os_k, ACCUM, work, bytes, st);
     }
@@ -865,6 +1009,63 @@ addft_status hpsi_t(addft_plan plan, int nk, int nb, const void *psi, const void
   return ADDFT_OK;
 }
 
+template <typename R, int FORM>
+addft_status projectors_form(const PlanDev &pd, const GeoParams &gp, size_t smem, typename Cx<R>::T *proj,
+                             cudaStream_t st) {
+  ADDFT_TRY(smem_optin(k_projectors<R, FORM>, smem));
+  // about 4 CTAs per SM, each with enough G to pay for its phase tables
+  auto go = [&](int i0, int n) {
+    int chunks = (4 * 152 + n * gp.nk - 1) / (n * gp.nk);
+    chunks = std::max(1, std::min(chunks, (pd.nG + 1023) / 1024));
+    const int per = ((pd.nG + chunks - 1) / chunks + 255) / 256 * 256;
+    k_projectors<R, FORM><<<dim3((pd.nG + per - 1) / per, n, gp.nk), 256, smem, st>>>(pd, gp, i0, per, proj);
+    return check_launch("k_projectors");
+  };
+  if (gp.nat > 1) ADDFT_TRY(go(0, gp.nat - 1));
+  return go(gp.nat - 1, 1);   // in place, over the form factors
+}
+
+template <typename R>
+addft_status projectors_t(const PlanDev &pd, const GeoParams &gp, void *proj, cudaStream_t st) {
+  using C = typename Cx<R>::T;
+  k_proj_forms<R><<<dim3((pd.nG + 127) / 128, gp.nk), 128, 0, st>>>(pd, gp, (C *)proj);
+  ADDFT_TRY(check_launch("k_proj_forms"));
+  size_t smem = 0;
+  switch (phase_form(pd, smem)) {
+    case 2: return projectors_form<R, 2>(pd, gp, smem, (C *)proj, st);
+    case 1: return projectors_form<R, 1>(pd, gp, smem, (C *)proj, st);
+    default: return projectors_form<R, 0>(pd, gp, smem, (C *)proj, st);
+  }
+}
+
+// splits of the gradients' G range per atom: about four CTAs per SM, at least 256 G each
+inline int nl_grad_splits(int nk, int nat, int nG) {
+  return std::max(1, std::min((4 * 152 + nk * nat - 1) / (nk * nat), (nG + 255) / 256));
+}
+
+template <typename R>
+addft_status nl_grad_t(const PlanDev &pd, const GeoParams &gp, const void *Y, void *scratch, size_t scratch_bytes,
+                       double *part, cudaStream_t st) {
+  using C = typename Cx<R>::T;
+  // channel tables shared by the atoms, where there are several and the scratch holds them
+  double *form = nullptr;
+  if (gp.nat >= 4 && scratch_bytes >= (size_t)gp.nk * gp.nh * 4 * pd.nG * sizeof(double)) {
+    form = (double *)scratch;
+    k_nl_forms<R><<<dim3((pd.nG + 127) / 128, gp.nk), 128, 0, st>>>(pd, gp, form);
+    ADDFT_TRY(check_launch("k_nl_forms"));
+  }
+  size_t smem = 0;
+  const int f = phase_form(pd, smem);
+  const int nsplit = nl_grad_splits(gp.nk, gp.nat, pd.nG);
+  const dim3 grid(gp.nat, nsplit, gp.nk);
+  auto go = [&](auto kern) {
+    ADDFT_TRY(smem_optin(kern, smem));
+    kern<<<grid, 256, smem, st>>>(pd, gp, (const C *)Y, form, nsplit, part);
+    return check_launch("k_nl_grad");
+  };
+  return f == 2 ? go(k_nl_grad<R, 2>) : f == 1 ? go(k_nl_grad<R, 1>) : go(k_nl_grad<R, 0>);
+}
+
 // addft_hpsi on the caller's stream only (no second stream, no events): the form the
 // no-allocation entry point runs, which creates no CUDA objects per call.
 addft_status hpsi_one_stream(addft_plan plan, addft_dtype dt, int nk, int nb, const void *psi, const void *kin,
@@ -908,12 +1109,8 @@ addft_status addft_projectors(addft_plan plan, addft_dtype dt, const double *bve
   GeoParams gp;
   ADDFT_TRY(make_geo(gp, bvec, omega, nk, kpts, nat, pos, psp));
   if (nat * gp.nh == 0) return ADDFT_OK;
-  dim3 grid((plan->dev.nG + 127) / 128, nat * gp.nh, nk);
-  if (dt == ADDFT_F64)
-    k_projectors<double><<<grid, 128, 0, as_stream(stream)>>>(plan->dev, gp, (double2 *)proj);
-  else
-    k_projectors<float><<<grid, 128, 0, as_stream(stream)>>>(plan->dev, gp, (float2 *)proj);
-  return check_launch("k_projectors");
+  return dt == ADDFT_F64 ? projectors_t<double>(plan->dev, gp, proj, as_stream(stream))
+                         : projectors_t<float>(plan->dev, gp, proj, as_stream(stream));
 }
 
 addft_status addft_becp(addft_dtype dt, int nk, int nb, int nG, int nproj, const void *proj,
@@ -965,14 +1162,11 @@ addft_status addft_nonlocal_energy(addft_dtype dt, int nk, int nb, int nproj, co
   double *ep = (double *)(w + align256((size_t)nk * nproj * nb * csz));
   if (dt == ADDFT_F64) {
     ADDFT_TRY(dbecp_t<double>(dion, becp, nk, nproj, nb, nullptr, w, st));
-    k_nl_energy<double><<<(nk * nb + 127) / 128, 128, 0, st>>>((const double2 *)becp, (const double2 *)w,
-                                                              nk, nproj, nb, wocc, ep);
+    ADDFT_TRY(nl_energy_t<double>(becp, w, nk, nproj, nb, wocc, ep, st));
   } else {
     ADDFT_TRY(dbecp_t<float>(dion, becp, nk, nproj, nb, nullptr, w, st));
-    k_nl_energy<float><<<(nk * nb + 127) / 128, 128, 0, st>>>((const float2 *)becp, (const float2 *)w,
-                                                             nk, nproj, nb, wocc, ep);
+    ADDFT_TRY(nl_energy_t<float>(becp, w, nk, nproj, nb, wocc, ep, st));
   }
-  ADDFT_TRY(check_launch("k_nl_energy"));
   return finalize_sums(ep, 1, nk * nb, e_out, false, st);
 }
 
@@ -1040,7 +1234,8 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
   const size_t o_mw = take((size_t)nk * nproj * nb * csz);
   const size_t o_y = take((size_t)nk * nproj * nG * csz);
   const size_t o_ep = take((size_t)nk * nb * sizeof(double));
-  const size_t o_gp = take((size_t)nk * nproj * 12 * sizeof(double));
+  const int nsplit = nl_grad_splits(nk, nat, nG);
+  const size_t o_gp = take((size_t)nk * nat * nsplit * 12 * sizeof(double));
   const size_t bwb = nl_grad_scratch(dt, nk, nb, nG, nproj);   // becp's partials, then the operands of Y
   const size_t o_bw = take(bwb);
   ADDFT_REQUIRE(work_bytes >= off, ADDFT_INVALID_ARG, "nonlocal_gradients: work needs %zu B, got %zu B",
@@ -1053,28 +1248,22 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
     ADDFT_TRY(dbecp_t<double>(dion, w + o_becp, nk, nproj, nb, wocc, w + o_mw, st));
     ADDFT_TRY((apply_t<double, true, false>(w + o_mw, 1, nb, (size_t)nproj * nb, psi, (size_t)nb * nG, nk, nb,
                                             nproj, nG, w + o_y, (size_t)nproj * nG, w + o_bw, bwb, st)));
-    k_nl_energy<double><<<(nk * nb + 127) / 128, 128, 0, st>>>((const double2 *)(w + o_becp),
-                                                              (const double2 *)(w + o_db), nk, nproj, nb,
-                                                              wocc, (double *)(w + o_ep));
-    ADDFT_TRY(check_launch("k_nl_energy"));
-    k_nl_grad<double><<<dim3(nproj, nk), 256, 0, st>>>(plan->dev, gp, (const double2 *)(w + o_y), nproj,
-                                                      (double *)(w + o_gp));
+    ADDFT_TRY(nl_energy_t<double>(w + o_becp, w + o_db, nk, nproj, nb, wocc, (double *)(w + o_ep), st));
+    // the projector table has been used; its place takes the channel tables
+    ADDFT_TRY(nl_grad_t<double>(plan->dev, gp, w + o_y, w + o_proj, (size_t)nk * nproj * nG * csz,
+                                (double *)(w + o_gp), st));
   } else {
     ADDFT_TRY(becp_t<float>(nk, nb, nG, nproj, w + o_proj, psi, w + o_becp, w + o_bw, bwb, st));
     ADDFT_TRY(dbecp_t<float>(dion, w + o_becp, nk, nproj, nb, nullptr, w + o_db, st));
     ADDFT_TRY(dbecp_t<float>(dion, w + o_becp, nk, nproj, nb, wocc, w + o_mw, st));
     ADDFT_TRY((apply_t<float, true, false>(w + o_mw, 1, nb, (size_t)nproj * nb, psi, (size_t)nb * nG, nk, nb,
                                            nproj, nG, w + o_y, (size_t)nproj * nG, w + o_bw, bwb, st)));
-    k_nl_energy<float><<<(nk * nb + 127) / 128, 128, 0, st>>>((const float2 *)(w + o_becp),
-                                                             (const float2 *)(w + o_db), nk, nproj, nb, wocc,
-                                                             (double *)(w + o_ep));
-    ADDFT_TRY(check_launch("k_nl_energy"));
-    k_nl_grad<float><<<dim3(nproj, nk), 256, 0, st>>>(plan->dev, gp, (const float2 *)(w + o_y), nproj,
-                                                     (double *)(w + o_gp));
+    ADDFT_TRY(nl_energy_t<float>(w + o_becp, w + o_db, nk, nproj, nb, wocc, (double *)(w + o_ep), st));
+    ADDFT_TRY(nl_grad_t<float>(plan->dev, gp, w + o_y, w + o_proj, (size_t)nk * nproj * nG * csz,
+                               (double *)(w + o_gp), st));
   }
-  ADDFT_TRY(check_launch("k_nl_grad"));
-  k_nl_grad_final<<<1, 128, 0, st>>>((const double *)(w + o_ep), nk * nb, (const double *)(w + o_gp), nk,
-                                     nproj, gp.nh, nat, out);
+  k_nl_grad_final<<<(1 + 3 * nat + 9 + 3) / 4, 128, 0, st>>>((const double *)(w + o_ep), nk * nb,
+                                                            (const double *)(w + o_gp), nk, nat, nsplit, out);
   return check_launch("k_nl_grad_final");
 }
 
@@ -1085,7 +1274,7 @@ size_t addft_nonlocal_gradients_work_bytes(addft_dtype dt, int nk, int nb, int n
   s += align256((size_t)nk * nproj * nG * csz) * 2;
   s += align256((size_t)nk * nproj * nb * csz) * 3;
   s += align256((size_t)nk * nb * sizeof(double));
-  s += align256((size_t)nk * nproj * 12 * sizeof(double));
+  s += nat > 0 ? align256((size_t)nk * nat * nl_grad_splits(nk, nat, nG) * 12 * sizeof(double)) : 0;
   s += align256(nl_grad_scratch(dt, nk, nb, nG, nproj));
   return s;
 }
