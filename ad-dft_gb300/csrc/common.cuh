@@ -98,6 +98,13 @@ struct FftTuning {
                        // (0: only where the yz-plane tiles exceed a CTA's shared memory)
 };
 
+// Geometry of one axis' transform matrix as tensor-core digits (dft64.cu): K inputs in nks steps of 16,
+// `outs` outputs in `tiles` tiles of `per` (padded to R rows), tile_bytes each, from offset `off` on.
+struct D64Mat {
+  int K, outs, nks, R, per, tiles, tile_bytes;
+  long off;
+};
+
 // Device view of a plan: sphere-aware layout of one G-shell in one FFT box.
 //   planes p = 0..np-1 are the x-planes (fixed i1) that hold sphere points;
 //   each plane owns a contiguous range [gptr[p], gptr[p+1]) of the
@@ -128,6 +135,13 @@ struct PlanDev {
   // (true for spheres around G = 0): row_lohi[p] = nlo | nhi << 16
   int xy_direct;
   const int *row_lohi;
+  // FP64 transforms on the tensor cores: active y and z indices (in ascending order), and per column
+  int nq, nz;
+  const int *col_zg;       // ncols * nz: G index at each active z, -1 where the sphere has no point
+  const int *col_of;       // np * nq: column at (active plane, active y), -1 where there is none
+  const int *col_pq;       // ncols: plane * nq + y index
+  D64Mat d64[6];           // x, y, z inverse, then forward
+  const unsigned char *d64_F;
   const void *tw_d;        // double2 twiddles: n1 | n2 | n3, e^{-2 pi i t/n}
   const void *tw_f;        // float2 twiddles, same layout
   AxisPlan ax[3];

@@ -1,0 +1,838 @@
+// FP64 transforms between the G-sphere and the box as matrix products on the 5th-generation tensor
+// cores (tcgen05.mma kind::f16), FP64 accurate through exact digit slices (see ozgemm.cu).
+//
+// GB300 issues under two FP64 instructions per SM and cycle, so a 75-point FFT line costs about
+// 1,000 SM cycles however it is factored (1,700 instructions).  As a product with the DFT matrix
+// it needs 75 x 35 complex multiplications (35 = active indices of the sphere on that axis: only
+// those are read by an inverse and produced by a forward transform) and these run on the tensor
+// cores at 39 cycles per line, 16 inputs and 64 outputs: 234 and 195 cycles.
+//
+// A stage transforms one axis:   out[o][line] = sum_k F[o][k] in[k][line]
+//   z inverse: sphere columns -> Z[column][z];      y inverse: Z -> Y[plane][z][y];
+//   x inverse: Y -> times V into U[z][y][x], or |.|^2 summed over bands, or psi(r);
+//   x forward: U (or a real-space field) -> X[z][y][plane];  y forward: X -> W[z][plane][y index];
+//   z forward: W -> the sphere (scaled, plus kin psi for H psi).
+// Every stage writes its output index fastest and the next one takes neighbouring lines along that
+// index, so loads (lanes = lines) and stores (lanes = outputs) are both coalesced.
+//
+// k_d64: persistent, one CTA per SM, on blocks of 32 lines.  F stays in shared memory as digits: per 16 k
+// and slice the rows [-Im F | Re F | Im F] of R outputs, so that [Re; Im] and [-Im; Re] (2 R <= 128
+// rows) are the same bytes from two offsets and one accumulator row holds Re or Im of an output:
+//   D = [Re F; Im F] Re x + [-Im F; Re F] Im x.
+// Eight producer warps load 8 inputs of a line per lane, agree on the line's largest exponent and
+// write its 8 digits per component (62 bits below that exponent) into a ring of operand buffers;
+// one thread issues the MMAs (slice s of F against slices 0 .. 7 - s of the lines, side by side along
+// N = 32 (8 - s), landing on levels s .. 7); sixteen epilogue warps empty one of the two accumulators
+// (8 levels x 32 lines) while the other is filled, add the levels in 64-bit integers and round once
+// to FP64.  All waits are bounded (status as in ozgemm.cu).  The error is that of the slicing, 2^-62
+// of the line's largest input per term, and of one rounding: below an FP64 FFT's.
+#include <algorithm>
+#include <cmath>
+
+#include "dft64.cuh"
+#include "ozgemm.cuh"
+
+namespace addft {
+
+namespace {
+
+__device__ unsigned g_d64_error = 0;
+
+constexpr int kS = 8;            // digits
+constexpr int kBits = 62;
+constexpr int kLines = 32;       // lines per block
+constexpr int kStep = 16;        // k per MMA
+constexpr int kMaxK = 128;       // sums of 128 products per digit pair stay exact
+constexpr int kRing = 4;         // operand buffers (one kstep of 32 lines each)
+constexpr int kItem = 2 * kS * kLines * kStep * 2;   // 16 KB
+constexpr int kProd = 8, kEpi = 16;                  // warps
+constexpr int kEpiLines = 4 * kLines / kEpi;         // lines of an epilogue warp
+constexpr int kThreads = 32 * (kProd + kEpi + 1);
+constexpr int kWait = 1 << 20;
+constexpr size_t kMaxF = 154 << 10;   // bytes of F per CTA beside the ring
+constexpr int kSms = 152;
+
+__device__ __forceinline__ uint32_t sad(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity) {
+  for (int it = 0; it < kWait; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(sad(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void init_bar(uint64_t *bar, int n) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sad(bar)), "r"(n));
+}
+__device__ __forceinline__ void arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sad(bar)) : "memory");
+}
+__device__ __forceinline__ void commit_to(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sad(bar))
+               : "memory");
+}
+__device__ __forceinline__ uint64_t desc(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
+         ((uint64_t)1 << 46);
+}
+__device__ __forceinline__ uint32_t idesc(int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+      "l"(a), "l"(b), "r"(id), "r"(acc)
+      : "memory");
+}
+#define D64_LD8(taddr, r)                                                                         \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"           \
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), \
+                 "=r"(r[7])                                                                      \
+               : "r"(taddr))
+
+enum Stage { ZI, YI, XI_V, XI_R, XI_C, XI_D, XF, XR_R, XR_C, YF, ZF, ZF_H };
+
+struct Args {
+  PlanDev pd;
+  D64Mat m;
+  const unsigned char *F;
+  long lines;              // over all bands of the chunk (XI_D: per band)
+  int nb;                  // bands of the chunk
+  const double2 *in;
+  double2 *out;
+  const double *rin;       // XR_R
+  const double *V;         // XI_V: [z][y][x], scaled
+  double scale;
+  long sz, sy;             // YF: strides of z and y in X
+  const double2 *psi;      // ZF_H
+  const double *kin;
+  int nb_per_k, batch0;
+  const double *wocc;      // XI_D
+  double *part;            //   [group][z][y][x]
+  int groups, per;         //   band groups, bands per group
+};
+
+// where a line reads its inputs
+struct Line { long base; int aux; };
+
+template <int ST>
+__device__ __forceinline__ Line line_at(const Args &a, long l) {
+  const PlanDev &pd = a.pd;
+  Line r;
+  r.aux = 0;
+  if (ST == ZI) {
+    const long b = l / pd.nrows;
+    r.base = b * pd.nG;
+    r.aux = (int)(l - b * pd.nrows) * pd.nz;
+  } else if (ST == YI) {
+    const long t = l / pd.n3, b = t / pd.np;
+    r.base = b * pd.nrows * pd.n3 + (l - t * pd.n3);
+    r.aux = (int)(t - b * pd.np) * pd.nq;
+  } else if (ST == XI_V || ST == XI_R || ST == XI_C || ST == XI_D) {
+    const long n = (long)pd.n2 * pd.n3, b = l / n;
+    r.base = b * pd.np * n + (l - b * n);
+  } else if (ST == XF) {
+    r.base = l * pd.n1;
+  } else if (ST == XR_R || ST == XR_C) {   // lines (band, y, z)
+    const long n = (long)pd.n2 * pd.n3, b = l / n;
+    r.base = b * n * pd.n1 + (l - b * n);
+  } else if (ST == YF) {
+    const long t = l / pd.np, b = t / pd.n3;
+    r.base = b * pd.n2 * pd.n3 * pd.np + (t - b * pd.n3) * a.sz + (l - t * pd.np);
+  } else {
+    const long b = l / pd.nrows;
+    r.base = b * pd.n3 * pd.np * pd.nq + pd.col_pq[l - b * pd.nrows];
+  }
+  return r;
+}
+
+template <int ST>
+__device__ __forceinline__ double2 load_at(const Args &a, const Line &l, int k) {
+  const PlanDev &pd = a.pd;
+  const double2 z = make_double2(0.0, 0.0);
+  if (ST == ZI) {
+    const int g = pd.col_zg[l.aux + k];
+    return g >= 0 ? a.in[l.base + g] : z;
+  } else if (ST == YI) {
+    const int c = pd.col_of[l.aux + k];
+    return c >= 0 ? a.in[l.base + (long)c * pd.n3] : z;
+  } else if (ST == XI_V || ST == XI_R || ST == XI_C || ST == XI_D || ST == XR_C) {
+    return a.in[l.base + (long)k * pd.n2 * pd.n3];
+  } else if (ST == XR_R) {
+    return make_double2(a.rin[l.base + (long)k * pd.n2 * pd.n3], 0.0);
+  } else if (ST == XF) {
+    return a.in[l.base + k];
+  } else if (ST == YF) {
+    return a.in[l.base + k * a.sy];
+  } else {
+    return a.in[l.base + (long)k * pd.np * pd.nq];
+  }
+}
+
+// one component of output o of line l
+template <int ST>
+__device__ __forceinline__ void store_at(const Args &a, long l, int o, int comp, double v) {
+  const PlanDev &pd = a.pd;
+  double *out = reinterpret_cast<double *>(a.out);
+  if (ST == ZI) out[2 * (l * pd.n3 + o) + comp] = v;
+  else if (ST == YI) out[2 * (l * pd.n2 + o) + comp] = v;
+  else if (ST == XI_V) out[2 * (l * pd.n1 + o) + comp] = v * a.V[(l % ((long)pd.n2 * pd.n3)) * pd.n1 + o];
+  else if (ST == XI_C) out[2 * (l * pd.n1 + o) + comp] = v * a.scale;
+  else if (ST == XI_R) { if (!comp) out[l * pd.n1 + o] = v * a.scale; }
+  else if (ST == XF || ST == XR_R || ST == XR_C) out[2 * (l * pd.np + o) + comp] = v;
+  else if (ST == YF) out[2 * (l * pd.nq + o) + comp] = v;
+  else {
+    const long b = l / pd.nrows;
+    const int g = pd.col_zg[(l - b * pd.nrows) * pd.nz + o];
+    if (g < 0) return;
+    const long at = 2 * (b * pd.nG + g) + comp;
+    if (ST == ZF_H) v += a.kin[(a.batch0 + b) / a.nb_per_k * pd.nG + g] * reinterpret_cast<const double *>(a.psi)[at];
+    else v *= a.scale;
+    out[at] = v;
+  }
+}
+
+__device__ __forceinline__ double scale2(double x, int n) {
+  const int a = n / 2, b = n - a;
+  auto p2 = [](int t) { return __hiloint2double((max(min(t, 1023), -1022) + 1023) << 20, 0); };
+  return x * p2(a) * p2(b);
+}
+
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+}
+
+// T 2^n rounded to FP64, n in -1000 .. 900.  `scaled` takes one conversion on the FP64 pipe and an
+// exponent addition; to_double stays on the integer pipes (three times the instructions), for the
+// density stage, whose squares and sums fill the FP64 pipe already.
+__device__ __forceinline__ double scaled(long long T, int n) {
+  const double d = __ll2double_rn(T);
+  return T == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (n << 20), __double2loint(d));
+}
+__device__ __forceinline__ double to_double(long long T, int n) {
+  const unsigned long long u = T < 0 ? 0ull - (unsigned long long)T : (unsigned long long)T;
+  if (u == 0) return 0.0;
+  const int z = __clzll((long long)u);
+  const unsigned long long top = u << z, sign = (unsigned long long)T & 0x8000000000000000ull;
+  // the leading one of top >> 11 adds one to the exponent
+  const unsigned long long r = ((unsigned long long)(62 - z + n + 1023) << 52) + (top >> 11) + ((top >> 10) & 1);
+  return __longlong_as_double((long long)(r | sign));
+}
+
+// x as q = round(x 2^(62 - E)) of a line with exponent field em, 128 added to every byte but the top
+__device__ __forceinline__ uint64_t d64_bytes(double x, int em) {
+  const uint64_t u = (uint64_t)__double_as_longlong(x);
+  const int e = (int)(u >> 52) & 0x7ff;
+  uint64_t m = u & 0xFFFFFFFFFFFFFull;
+  if (e) m |= 1ull << 52;
+  const int sh = kBits - 53 - (max(em, 1) - max(e, 1));
+  uint64_t q;
+  if (sh >= 0) {
+    q = m << sh;
+  } else {
+    const int r = min(-sh, 63);
+    q = (m + (1ull << (r - 1))) >> r;
+  }
+  if ((int64_t)u < 0) q = 0 - q;
+  return q + 0x0080808080808080ull;
+}
+
+template <int ST>
+__global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *smem = smem_raw + ((1024 - (sad(smem_raw) & 1023)) & 1023);
+  __shared__ __align__(8) uint64_t fullB[kRing], emptyB[kRing], accf[2], acce[2], fbar;
+  __shared__ int pm[2][kProd][kLines];    // exponents found by each producer warp
+  __shared__ int lex[8][kLines];          // exponents of the lines of the last blocks
+  __shared__ uint32_t tslot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nks = a.m.nks, R = a.m.R, tile = blockIdx.y;
+  const long nblk = (a.lines + kLines - 1) / kLines;
+  const int inner_max = ST == XI_D ? a.per : 1;
+  const long units = ST == XI_D ? nblk * a.groups : nblk;
+  if (tid == 0) {
+    for (int i = 0; i < kRing; ++i) {
+      init_bar(&fullB[i], 2);
+      init_bar(&emptyB[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      init_bar(&accf[i], 1);
+      init_bar(&acce[i], kEpi);
+    }
+    init_bar(&fbar, 1);
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sad(&tslot)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tslot;
+  const uint32_t sring = sad(smem), sF = sring + kRing * kItem;   // F last: its 128-row reads may run past it
+  bool ok = true;
+
+  // a block: 32 lines starting at l0 (XI_D: of one band); `inner` blocks share a unit
+  auto unit_info = [&](long u, long &l0, int &b0, int &inner) {
+    if (ST == XI_D) {
+      const long lb = u / a.groups;
+      const int g = (int)(u - lb * a.groups);
+      l0 = lb * kLines;
+      b0 = g * a.per;
+      inner = max(0, min(a.per, a.nb - b0));
+    } else {
+      l0 = u * kLines;
+      b0 = 0;
+      inner = 1;
+    }
+  };
+
+  if (warp < kProd) {
+    // ---- producers: lane = line, warp = 8 inputs (and, above 64 inputs, 8 more)
+    const int noct = 2 * nks;
+    long blk = 0;
+    for (long u = blockIdx.x; u < units; u += gridDim.x) {
+      long l0;
+      int b0, inner;
+      unit_info(u, l0, b0, inner);
+      for (int it = 0; it < inner; ++it, ++blk) {
+        long l = l0 + lane;
+        const bool live = l < a.lines;
+        if (ST == XI_D) l += (long)(b0 + it) * a.lines;
+        const Line ln = line_at<ST>(a, live ? l : 0);
+        double2 x[8];
+        auto load = [&](int o) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int k = 8 * o + j;
+            x[j] = live && k < a.m.K ? load_at<ST>(a, ln, k) : make_double2(0.0, 0.0);
+          }
+        };
+        int em = 0;
+        // with more than 64 inputs a warp has two groups of 8; the first stays in registers
+#pragma unroll 1
+        for (int o = noct > kProd ? warp + kProd : warp; o >= 0; o -= kProd) {
+          load(o);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            em = max(em, max((__double2hiint(x[j].x) >> 20) & 0x7ff, (__double2hiint(x[j].y) >> 20) & 0x7ff));
+        }
+        int(*p)[kLines] = pm[blk & 1];
+        p[warp][lane] = em;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kProd) : "memory");   // every producer gets here, failed or not
+#pragma unroll
+        for (int w = 0; w < kProd; ++w) em = max(em, p[w][lane]);
+        if (warp == 0) lex[blk & 7][lane] = em;
+#pragma unroll 1
+        for (int o = warp; o < noct; o += kProd) {
+          if (o > warp) load(o);
+          const long t = blk * nks + (o >> 1);
+          const int slot = (int)(t % kRing);
+          const long round = t / kRing;
+          if (ok && round > 0) ok = __all_sync(0xffffffffu, wait_bar(&emptyB[slot], (uint32_t)(round - 1) & 1));
+          if (!ok) continue;
+          const uint32_t dst = sring + slot * kItem + (lane >> 3) * 256 + (o & 1) * 128 + (lane & 7) * 16;
+#pragma unroll
+          for (int part = 0; part < 2; ++part) {
+            uint64_t q[8];
+#pragma unroll
+            // a line that is not finite is all NaN in the epilogue, whatever its digits
+            for (int j = 0; j < 8; ++j) q[j] = d64_bytes(em == 0x7ff ? 0.0 : (part ? x[j].y : x[j].x), em);
+#pragma unroll
+            for (int s = 0; s < kS; ++s) {
+              uint32_t hh[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                uint32_t w;
+                if (s == 0) {
+                  w = ((uint32_t)((int)((int64_t)q[2 * j] >> 56) + 128) | ((uint32_t)((int)((int64_t)q[2 * j + 1] >> 56) + 128) << 16)) +
+                      0x64006400u;
+                } else {
+                  // byte 7 - s of both numbers into the low bytes of the halves
+                  const uint32_t lo = s < 4 ? (uint32_t)(q[2 * j] >> 32) : (uint32_t)q[2 * j];
+                  const uint32_t hi = s < 4 ? (uint32_t)(q[2 * j + 1] >> 32) : (uint32_t)q[2 * j + 1];
+                  const int y = s < 4 ? 3 - s : 7 - s;
+                  w = __byte_perm(__byte_perm(lo, hi, y | ((y + 4) << 4)), 0x64646464u, 0x4140);
+                }
+                // 0x6400 + n is the FP16 number 1024 + n; minus 1152 leaves the digit, exactly
+                asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(hh[j]) : "r"(w), "r"(0x64806480u));
+              }
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (part * kS + s) * (kLines * kStep * 2)),
+                           "r"(hh[0]), "r"(hh[1]), "r"(hh[2]), "r"(hh[3])
+                           : "memory");
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) arrive(&fullB[slot]);
+        }
+      }
+    }
+    if (!ok && lane == 0) atomicOr(&g_d64_error, 1u);
+  } else if (warp == kProd + kEpi) {
+    // ---- F, then MMAs
+    if (lane == 0) {
+      const uint32_t bytes = (uint32_t)a.m.tile_bytes;
+      const unsigned char *src = a.F + a.m.off + (size_t)tile * bytes;
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sad(&fbar)), "r"(bytes) : "memory");
+      for (uint32_t o = 0; o < bytes; o += 32768) {
+        const uint32_t n = min(32768u, bytes - o);
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sF + o),
+            "l"(src + o), "r"(n), "r"(sad(&fbar))
+            : "memory");
+      }
+      ok = wait_bar(&fbar, 0);
+      const uint32_t sl = 3 * R * 32;   // bytes of one slice of F
+      long blk = 0;
+      bool issued = false;
+      for (long u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        long l0;
+        int b0, inner;
+        unit_info(u, l0, b0, inner);
+        for (int it = 0; it < inner && ok; ++it, ++blk) {
+          const int buf = (int)(blk & 1);
+          if (blk >= 2) ok = wait_bar(&acce[buf], (uint32_t)(blk / 2 - 1) & 1);
+          for (int j = 0; j < nks && ok; ++j) {
+            const long t = blk * nks + j;
+            const int slot = (int)(t % kRing);
+            ok = wait_bar(&fullB[slot], (uint32_t)(t / kRing) & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            issued = true;
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {   // [Re; Im] Re x, then [-Im; Re] Im x
+              const uint32_t f0 = sF + j * kS * sl + (part ? 0 : R * 32);
+              const uint64_t bd = desc(sring + slot * kItem + part * kS * (kLines * kStep * 2));
+#pragma unroll
+              for (int i = 0; i < kS; ++i)
+                mma_f16(tmem + 256 * buf + 32 * i, desc(f0 + i * sl), bd, idesc(32 * (kS - i)), !(j == 0 && part == 0 && i == 0));
+            }
+            commit_to(&emptyB[slot]);
+          }
+          if (ok) commit_to(&accf[buf]);
+        }
+      }
+      if (!ok) {
+        atomicOr(&g_d64_error, 1u);
+        wait_bar(&fbar, 0);
+        if (issued) {   // no MMA may be in flight when tensor memory is given back
+          commit_to(&accf[0]);
+          wait_bar(&accf[0], 0);
+          wait_bar(&accf[0], 1);
+        }
+      }
+    }
+  } else {
+    // ---- epilogue: warp reads accumulator rows 32 (w % 4) .. of kEpiLines lines
+    const int w = warp - kProd, q = warp & 3, c0 = kEpiLines * (w >> 2);
+    const int row = 32 * q + lane, comp = row >= R ? 1 : 0, r = comp ? row - R : row;
+    const int o = tile * a.m.per + r;
+    const bool on = row < 2 * R && r < a.m.per && o < a.m.outs;
+    const bool any = 32 * q < 2 * R;
+    // the level sums as hi 2^32 + lo, hi <= 2^35 2 K: keep as many of lo's bits as 62 bits hold (18 to 21)
+    const int keep = 62 - 35 - (32 - __clz(2 * a.m.K));
+    const int w4 = 1 << (keep - 8), w5 = 1 << (keep - 16);
+    const float w67 = __int_as_float((127 - 32 + keep) << 23);
+    // q_F q_x = 256^7 (hi 2^32 + lo); F has exponent field 1023, x = q 2^(E - 62), E = field - 1022
+    const int nbase = 56 + 32 - keep + 1023 - 2 * 1022 - 2 * kBits;
+    double acc[kEpiLines];
+#pragma unroll
+    for (int c = 0; c < kEpiLines; ++c) acc[c] = 0.0;
+    long blk = 0;
+    for (long u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      long l0;
+      int b0, inner;
+      unit_info(u, l0, b0, inner);
+      for (int it = 0; it < inner && ok; ++it, ++blk) {
+        const int buf = (int)(blk & 1);
+        ok = __all_sync(0xffffffffu, wait_bar(&accf[buf], (uint32_t)(blk / 2) & 1));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t base = tmem + 256 * buf + ((uint32_t)(32 * q) << 16) + c0;
+        long long T[kEpiLines];
+        if (any) {
+          uint32_t v[2][kEpiLines];
+#pragma unroll
+          for (int l = 0; l < kS; l += 2) {
+            D64_LD8(base + 32 * l, v[0]);
+            D64_LD8(base + 32 * l + 32, v[1]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < kEpiLines; ++c) {
+              const float f0 = __uint_as_float(v[0][c]), f1 = __uint_as_float(v[1][c]);
+              if (l == 0) T[c] = mad_wide(__float2int_rn(f0), 1 << 24, mad_wide(__float2int_rn(f1), 1 << 16, 0));
+              else if (l == 2) T[c] = mad_wide(__float2int_rn(f0), 1 << 8, mad_wide(__float2int_rn(f1), 1, T[c])) << keep;
+              else if (l == 4) T[c] = mad_wide(__float2int_rn(f0), w4, mad_wide(__float2int_rn(f1), w5, T[c]));
+              else T[c] = mad_wide(__float2int_rn(fmaf(f0, 256.0f, f1) * w67), 1, T[c]);
+            }
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive(&acce[buf]);   // the accumulator has been read
+        if (!on) continue;
+        const double wb = ST == XI_D ? a.wocc[b0 + it] : 0.0;
+#pragma unroll
+        for (int c = 0; c < kEpiLines; ++c) {
+          const long l = l0 + c0 + c;
+          if (l >= a.lines) break;
+          const int em = lex[blk & 7][c0 + c], n = nbase + max(em, 1);
+          double v;
+          if (n >= -1000 && n <= 900) v = ST == XI_D ? to_double(T[c], n) : scaled(T[c], n);
+          else v = scale2(scale2((double)T[c], n / 2), n - n / 2);
+          if (em == 0x7ff) v = __longlong_as_double(0x7ff8000000000000ll);
+          if (ST == XI_D) acc[c] = fma(wb * v, v, acc[c]);
+          else store_at<ST>(a, l, o, comp, v);
+        }
+      }
+      if (ST == XI_D && ok) {   // Re^2 and Im^2 sit in different rows: [group][2][z][y][x]
+        const int g = b0 / a.per;
+        double *dst = a.part + ((size_t)g * 2 + comp) * a.lines * a.pd.n1;
+#pragma unroll
+        for (int c = 0; c < kEpiLines; ++c) {
+          const long l = l0 + c0 + c;
+          if (on && l < a.lines) dst[l * a.pd.n1 + o] = acc[c];
+          acc[c] = 0.0;
+        }
+      }
+    }
+    if (!ok && lane == 0) atomicOr(&g_d64_error, 1u);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+// Vt[z][y][x] = V[x][y][z] * s, through shared-memory tiles of 32 x 32 (x, z) per y
+__global__ void __launch_bounds__(256) k_d64_v(PlanDev pd, const double *__restrict__ V, double s, double *__restrict__ Vt) {
+  __shared__ double T[32][33];
+  const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32, y = blockIdx.z;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int x = w; x < 32; x += 8)
+    if (x0 + x < pd.n1 && z0 + lane < pd.n3) T[x][lane] = V[((long)(x0 + x) * pd.n2 + y) * pd.n3 + z0 + lane] * s;
+  __syncthreads();
+  for (int z = w; z < 32; z += 8)
+    if (z0 + z < pd.n3 && x0 + lane < pd.n1) Vt[((long)(z0 + z) * pd.n2 + y) * pd.n1 + x0 + lane] = T[lane][z];
+}
+
+// out[x][y][z] (+)= sum_j in[j][z][y][x], j < nsum slabs
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_d64_out(PlanDev pd, const T *__restrict__ in, int nsum, double scale, int acc, T *__restrict__ out);
+
+template <>
+__global__ void __launch_bounds__(256)
+k_d64_out<double>(PlanDev pd, const double *__restrict__ in, int nsum, double scale, int acc, double *__restrict__ out) {
+  __shared__ double T[32][33];
+  const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  const int nzt = (pd.n3 + 31) / 32;
+  const int x0 = blockIdx.x * 32, z0 = (blockIdx.y % nzt) * 32, b = blockIdx.y / nzt, y = blockIdx.z;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int z = w; z < 32; z += 8)
+    if (z0 + z < pd.n3 && x0 + lane < pd.n1) {
+      const double *p = in + (size_t)b * N + ((long)(z0 + z) * pd.n2 + y) * pd.n1 + x0 + lane;
+      double s = 0.0;
+      for (int j = 0; j < nsum; ++j) s += p[(size_t)j * N];
+      T[z][lane] = s * scale;
+    }
+  __syncthreads();
+  for (int x = w; x < 32; x += 8)
+    if (x0 + x < pd.n1 && z0 + lane < pd.n3) {
+      double *o = out + (size_t)b * N + ((long)(x0 + x) * pd.n2 + y) * pd.n3 + z0 + lane;
+      *o = acc ? *o + T[lane][x] : T[lane][x];
+    }
+}
+
+template <>
+__global__ void __launch_bounds__(256)
+k_d64_out<double2>(PlanDev pd, const double2 *__restrict__ in, int, double, int, double2 *__restrict__ out) {
+  __shared__ double2 T[32][33];
+  const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  const int nzt = (pd.n3 + 31) / 32;
+  const int x0 = blockIdx.x * 32, z0 = (blockIdx.y % nzt) * 32, b = blockIdx.y / nzt, y = blockIdx.z;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int z = w; z < 32; z += 8)
+    if (z0 + z < pd.n3 && x0 + lane < pd.n1) T[z][lane] = in[(size_t)b * N + ((long)(z0 + z) * pd.n2 + y) * pd.n1 + x0 + lane];
+  __syncthreads();
+  for (int x = w; x < 32; x += 8)
+    if (x0 + x < pd.n1 && z0 + lane < pd.n3) out[(size_t)b * N + ((long)(x0 + x) * pd.n2 + y) * pd.n3 + z0 + lane] = T[lane][x];
+}
+
+inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
+
+// The two scratch regions of a band: Z, U, W in the first, Y, X in the second.
+inline size_t region1(const PlanDev &pd) {
+  const size_t z = (size_t)pd.nrows * pd.n3, u = (size_t)pd.n1 * pd.n2 * pd.n3, w = (size_t)pd.n3 * pd.np * pd.nq;
+  return al256(std::max(std::max(z, u), w) * sizeof(double2));
+}
+inline size_t region2(const PlanDev &pd) { return al256((size_t)pd.np * pd.n2 * pd.n3 * sizeof(double2)); }
+
+template <int ST>
+addft_status stage(const PlanDev &pd, int axis, Args &a, long lines, cudaStream_t st) {
+  a.m = pd.d64[axis];
+  a.F = pd.d64_F;
+  a.lines = lines;
+  const size_t sm = (size_t)kRing * kItem + a.m.tile_bytes + 4096 + 1024;   // a 128-row read may pass F's end
+  ADDFT_TRY(smem_optin(k_d64<ST>, sm));
+  const long blocks = (lines + kLines - 1) / kLines * (ST == XI_D ? a.groups : 1);
+  const int gx = (int)std::max<long>(1, std::min<long>(blocks, kSms / a.m.tiles));
+  k_d64<ST><<<dim3(gx, a.m.tiles), kThreads, sm, st>>>(a);
+  return check_launch("k_d64");
+}
+
+inline Args base_args(const PlanDev &pd, int nb) {
+  Args a;
+  memset(&a, 0, sizeof(a));
+  a.pd = pd;
+  a.nb = nb;
+  a.scale = 1.0;
+  a.nb_per_k = 1;
+  return a;
+}
+
+// z and y inverse of nb bands: psi -> r1 (Z) -> r2 (Y)
+addft_status to_planes(const PlanDev &pd, int nb, const double2 *psi, double2 *r1, double2 *r2, cudaStream_t st) {
+  Args a = base_args(pd, nb);
+  a.in = psi;
+  a.out = r1;
+  ADDFT_TRY((stage<ZI>(pd, 2, a, (long)nb * pd.nrows, st)));
+  a.in = r1;
+  a.out = r2;
+  return stage<YI>(pd, 1, a, (long)nb * pd.np * pd.n3, st);
+}
+
+int chunk_bands(const PlanDev &pd, int nbatch, size_t bytes) {
+  const size_t per = d64_band_bytes(pd);
+  size_t fit = bytes / per, cap = std::max<size_t>(1, pd.tun.slab_chunk_bytes / per);
+  fit = std::min(std::min(fit, cap), (size_t)nbatch);
+  return (int)fit;
+}
+
+}  // namespace
+
+bool d64_handles(const PlanDev &pd, int nbatch) {
+  if (!pd.d64_F) return false;
+  for (int a = 0; a < 6; ++a)
+    if (pd.d64[a].tiles == 0) return false;
+  return (double)nbatch * pd.n1 * pd.n2 * pd.n3 >= 20000.0;
+}
+
+size_t d64_band_bytes(const PlanDev &pd) { return region1(pd) + region2(pd); }
+size_t d64_v_bytes(const PlanDev &pd) { return al256((size_t)pd.n1 * pd.n2 * pd.n3 * sizeof(double)); }
+
+addft_status d64_hpsi(const PlanDev &pd, int nbatch, const double2 *psi, const double *v_r, double2 *hpsi,
+                      const double *kin, int nb_per_k, void *work, size_t bytes, cudaStream_t st) {
+  const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  double *Vt = (double *)work;
+  char *w = (char *)work + d64_v_bytes(pd);
+  const int nc = chunk_bands(pd, nbatch, bytes - d64_v_bytes(pd));
+  k_d64_v<<<dim3((pd.n1 + 31) / 32, (pd.n3 + 31) / 32, pd.n2), 256, 0, st>>>(pd, v_r, 1.0 / (double)N, Vt);
+  ADDFT_TRY(check_launch("k_d64_v"));
+  double2 *r1 = (double2 *)w, *r2 = (double2 *)(w + (size_t)nc * region1(pd));
+  for (int b0 = 0; b0 < nbatch; b0 += nc) {
+    const int nb = std::min(nc, nbatch - b0);
+    const double2 *pin = psi + (size_t)b0 * pd.nG;
+    ADDFT_TRY(to_planes(pd, nb, pin, r1, r2, st));
+    Args a = base_args(pd, nb);
+    a.V = Vt;
+    a.in = r2;
+    a.out = r1;
+    ADDFT_TRY((stage<XI_V>(pd, 0, a, (long)nb * pd.n2 * pd.n3, st)));
+    a.in = r1;
+    a.out = r2;
+    ADDFT_TRY((stage<XF>(pd, 3, a, (long)nb * pd.n2 * pd.n3, st)));
+    a.in = r2;
+    a.out = r1;
+    a.sz = (long)pd.n2 * pd.np;
+    a.sy = pd.np;
+    ADDFT_TRY((stage<YF>(pd, 4, a, (long)nb * pd.n3 * pd.np, st)));
+    a.in = r1;
+    a.out = hpsi + (size_t)b0 * pd.nG;
+    a.psi = pin;
+    a.kin = kin;
+    a.nb_per_k = nb_per_k;
+    a.batch0 = b0;
+    ADDFT_TRY((stage<ZF_H>(pd, 5, a, (long)nb * pd.nrows, st)));
+  }
+  return ADDFT_OK;
+}
+
+addft_status d64_density(const PlanDev &pd, int nbatch, const double2 *psi, const double *wocc, double dscale, double *rho,
+                         void *work, size_t bytes, cudaStream_t st) {
+  const long N = (long)pd.n1 * pd.n2 * pd.n3, lines = (long)pd.n2 * pd.n3;
+  // band groups so that the CTAs of a tile share the (block, group) units evenly
+  const long blocks = (lines + kLines - 1) / kLines;
+  int groups = (int)std::max<long>(1, std::min<long>(4, (8 * kSms / pd.d64[0].tiles + blocks - 1) / blocks));
+  groups = std::min(groups, nbatch);
+  while (groups > 1 && bytes < (size_t)groups * 2 * N * sizeof(double) + d64_band_bytes(pd)) --groups;
+  const size_t pb = al256((size_t)groups * 2 * N * sizeof(double));
+  double *part = (double *)work;
+  char *w = (char *)work + pb;
+  const int nc = chunk_bands(pd, nbatch, bytes - pb);
+  double2 *r1 = (double2 *)w, *r2 = (double2 *)(w + (size_t)nc * region1(pd));
+  for (int b0 = 0; b0 < nbatch; b0 += nc) {
+    const int nb = std::min(nc, nbatch - b0);
+    ADDFT_TRY(to_planes(pd, nb, psi + (size_t)b0 * pd.nG, r1, r2, st));
+    Args a = base_args(pd, nb);
+    a.in = r2;
+    a.wocc = wocc + b0;
+    a.part = part;
+    a.per = (nb + groups - 1) / groups;
+    a.groups = (nb + a.per - 1) / a.per;
+    ADDFT_TRY((stage<XI_D>(pd, 0, a, lines, st)));
+    k_d64_out<double><<<dim3((pd.n1 + 31) / 32, (pd.n3 + 31) / 32, pd.n2), 256, 0, st>>>(pd, part, 2 * a.groups, dscale,
+                                                                                        b0 > 0 ? 1 : 0, rho);
+    ADDFT_TRY(check_launch("k_d64_out"));
+  }
+  return ADDFT_OK;
+}
+
+addft_status d64_to_real(const PlanDev &pd, int nbatch, const double2 *psi, double scale, void *out, bool real_part,
+                         void *work, size_t bytes, cudaStream_t st) {
+  const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  const int nc = chunk_bands(pd, nbatch, bytes);
+  double2 *r1 = (double2 *)work, *r2 = (double2 *)((char *)work + (size_t)nc * region1(pd));
+  for (int b0 = 0; b0 < nbatch; b0 += nc) {
+    const int nb = std::min(nc, nbatch - b0);
+    ADDFT_TRY(to_planes(pd, nb, psi + (size_t)b0 * pd.nG, r1, r2, st));
+    Args a = base_args(pd, nb);
+    a.in = r2;
+    a.out = r1;
+    a.scale = scale;
+    const dim3 grid((pd.n1 + 31) / 32, (pd.n3 + 31) / 32 * nb, pd.n2);
+    if (real_part) {
+      ADDFT_TRY((stage<XI_R>(pd, 0, a, (long)nb * pd.n2 * pd.n3, st)));
+      k_d64_out<double><<<grid, 256, 0, st>>>(pd, (const double *)r1, 1, 1.0, 0, (double *)out + (size_t)b0 * N);
+    } else {
+      ADDFT_TRY((stage<XI_C>(pd, 0, a, (long)nb * pd.n2 * pd.n3, st)));
+      k_d64_out<double2><<<grid, 256, 0, st>>>(pd, r1, 1, 1.0, 0, (double2 *)out + (size_t)b0 * N);
+    }
+    ADDFT_TRY(check_launch("k_d64_out"));
+  }
+  return ADDFT_OK;
+}
+
+addft_status d64_from_real(const PlanDev &pd, int nbatch, const void *in, bool in_real, double scale, double2 *psi,
+                           void *work, size_t bytes, cudaStream_t st) {
+  const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  const int nc = chunk_bands(pd, nbatch, bytes);
+  double2 *r1 = (double2 *)work, *r2 = (double2 *)((char *)work + (size_t)nc * region1(pd));
+  for (int b0 = 0; b0 < nbatch; b0 += nc) {
+    const int nb = std::min(nc, nbatch - b0);
+    Args a = base_args(pd, nb);
+    a.out = r2;
+    if (in_real) {
+      a.rin = (const double *)in + (size_t)b0 * N;
+      ADDFT_TRY((stage<XR_R>(pd, 3, a, (long)nb * pd.n2 * pd.n3, st)));
+    } else {
+      a.in = (const double2 *)in + (size_t)b0 * N;
+      ADDFT_TRY((stage<XR_C>(pd, 3, a, (long)nb * pd.n2 * pd.n3, st)));
+    }
+    a.in = r2;
+    a.out = r1;
+    a.sz = pd.np;                       // X[y][z][plane] here
+    a.sy = (long)pd.n3 * pd.np;
+    ADDFT_TRY((stage<YF>(pd, 4, a, (long)nb * pd.n3 * pd.np, st)));
+    a.in = r1;
+    a.out = psi + (size_t)b0 * pd.nG;
+    a.scale = scale;
+    ADDFT_TRY((stage<ZF>(pd, 5, a, (long)nb * pd.nrows, st)));
+  }
+  return ADDFT_OK;
+}
+
+unsigned d64_status() {
+  unsigned v = 0, z = 0;
+  if (cudaMemcpyFromSymbol(&v, g_d64_error, sizeof(v)) != cudaSuccess) return 0xffffffffu;
+  cudaMemcpyToSymbol(g_d64_error, &z, sizeof(z));
+  return v;
+}
+
+// ---------------------------------------------------------------------------
+// transform matrices
+// ---------------------------------------------------------------------------
+static uint16_t half_int(int d) {   // FP16 bits of an integer, |d| <= 128
+  if (d == 0) return 0;
+  const unsigned a = d < 0 ? -d : d;
+  int e = 0;
+  while ((a >> (e + 1)) != 0) ++e;
+  return (uint16_t)((d < 0 ? 0x8000u : 0u) | ((unsigned)(e + 15) << 10) | ((a << (10 - e)) & 0x3ffu));
+}
+
+static void digits_of(double x, uint16_t *h) {   // |x| <= 1, exponent field 1023
+  const int64_t q = (int64_t)std::llrint(std::ldexp(x, kBits - 1));
+  const uint64_t u = (uint64_t)q + 0x0080808080808080ull;
+  h[0] = half_int((int)((int64_t)u >> 56));
+  for (int s = 1; s < kS; ++s) h[s] = half_int((int)((u >> (56 - 8 * s)) & 0xff) - 128);
+}
+
+void d64_build(int n1, int n2, int n3, const std::vector<int> &xact, const std::vector<int> &yact,
+               const std::vector<int> &zact, D64Mat (&dm)[6], std::vector<unsigned char> &blob) {
+  const int n[3] = {n1, n2, n3};
+  const std::vector<int> *act[3] = {&xact, &yact, &zact};
+  for (int m = 0; m < 6; ++m) {
+    const int ax = m % 3;
+    const bool inv = m < 3;
+    D64Mat &d = dm[m];
+    memset(&d, 0, sizeof(d));
+    d.K = inv ? (int)act[ax]->size() : n[ax];
+    d.outs = inv ? n[ax] : (int)act[ax]->size();
+    d.nks = (d.K + kStep - 1) / kStep;
+    if (d.K > kMaxK) continue;
+    for (int t = 1; t <= 8; ++t) {
+      const int per = (d.outs + t - 1) / t, R = (per + 7) / 8 * 8;
+      const size_t bytes = (size_t)d.nks * kS * 3 * R * 32;
+      if (R > 64 || bytes > kMaxF) continue;
+      d.tiles = t;
+      d.per = per;
+      d.R = R;
+      d.tile_bytes = (int)bytes;
+      break;
+    }
+    if (d.tiles == 0) continue;
+    // digits of the n-th roots of unity: -Im, Re, Im of e^{+-2 pi i t / n}
+    std::vector<uint16_t> dig((size_t)n[ax] * 3 * kS);
+    for (int t = 0; t < n[ax]; ++t) {
+      const double ang = 2.0 * M_PI * (double)t / (double)n[ax];
+      const double re = std::cos(ang), im = inv ? std::sin(ang) : -std::sin(ang);
+      digits_of(-im, &dig[(size_t)(3 * t) * kS]);
+      digits_of(re, &dig[(size_t)(3 * t + 1) * kS]);
+      digits_of(im, &dig[(size_t)(3 * t + 2) * kS]);
+    }
+    while (blob.size() % 256) blob.push_back(0);
+    d.off = (long)blob.size();
+    blob.resize(blob.size() + (size_t)d.tiles * d.tile_bytes, 0);
+    for (int t = 0; t < d.tiles; ++t)
+      for (int r = 0; r < d.per; ++r) {
+        const int o = t * d.per + r;
+        if (o >= d.outs) break;
+        for (int k = 0; k < d.K; ++k) {
+          const long j = inv ? (long)o * (*act[ax])[k] : (long)(*act[ax])[o] * k;
+          const int i = (int)(j % n[ax]);
+          for (int b = 0; b < 3; ++b) {
+            const uint16_t *h = &dig[(size_t)(3 * i + b) * kS];
+            const int row = b * d.R + r;
+            for (int s = 0; s < kS; ++s) {
+              unsigned char *p = blob.data() + d.off + (size_t)t * d.tile_bytes +
+                                 (size_t)(k / kStep * kS + s) * (3 * d.R * 32) + (row >> 3) * 256 +
+                                 ((k % kStep) / 8) * 128 + (row & 7) * 16 + (k % 8) * 2;
+              p[0] = (unsigned char)(h[s] & 0xff);
+              p[1] = (unsigned char)(h[s] >> 8);
+            }
+          }
+        }
+      }
+  }
+}
+
+}  // namespace addft

@@ -35,7 +35,7 @@
 //     stream), processing as many bands per chunk as fit.
 #include <atomic>
 
-#include "common.cuh"
+#include "transforms.cuh"
 
 namespace {
 
@@ -87,7 +87,7 @@ addft_status addft_hpsi_noalloc(addft_plan plan, addft_dtype dt, int nk, int nb,
   // partials: with less room becp uses fewer splits, down to one)
   const size_t csz = dt == ADDFT_F64 ? 16 : 8;
   const size_t arrays = nproj > 0 ? ((2 * (size_t)nk * nproj * nb * csz + 255) & ~size_t(255)) : 0;
-  const size_t need = arrays + addft_work_bytes(plan, 1, dt);
+  const size_t need = arrays + addft::work_bytes_min(plan->dev, 1, dt == ADDFT_F64 ? 16 : 8);
   ADDFT_REQUIRE(need <= kNoAllocScratchBytes, ADDFT_UNSUPPORTED,
                 "hpsi_noalloc: this problem needs at least %zu B of scratch but the static scratch holds %zu B "
                 "(use addft_hpsi with a caller work buffer)",

@@ -955,7 +955,7 @@ addft_status hpsi_t(addft_plan plan, int nk, int nb, const void *psi, const void
   const PlanDev &pd = plan->dev;
   const addft_dtype dt = sizeof(R) == 8 ? ADDFT_F64 : ADDFT_F32;
   const size_t arrays = nproj > 0 ? align256(2 * (size_t)nk * nproj * nb * sizeof(C)) : 0;
-  const size_t local_min = addft_work_bytes(plan, 1, dt);
+  const size_t local_min = work_bytes_min(pd, 1, sizeof(C));
   ADDFT_REQUIRE(work && work_bytes >= arrays + local_min, ADDFT_INVALID_ARG,
                 "hpsi: work buffer of %zu B too small (need >= %zu B)", work_bytes, arrays + local_min);
   size_t split = 0;

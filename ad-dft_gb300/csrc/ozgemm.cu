@@ -226,14 +226,16 @@ k_oz_pack(const double2 *__restrict__ X, long s_row, long s_k, size_t s_batch, i
         if (s == 0) {   // top digit: signed, -128 .. 128
           const int a = (int)((int64_t)q[2 * j] >> (8 * (S - 1))) + 128;
           const int b = (int)((int64_t)q[2 * j + 1] >> (8 * (S - 1))) + 128;
-          w = (uint32_t)a | ((uint32_t)b << 16);
+          w = ((uint32_t)a | ((uint32_t)b << 16)) + 0x64006400u;
         } else {
-          const uint32_t a = (uint32_t)(q[2 * j] >> (8 * (S - 1 - s))) & 0xff;
-          const uint32_t b = (uint32_t)(q[2 * j + 1] >> (8 * (S - 1 - s))) & 0xff;
-          w = a | (b << 16);
+          // byte S - 1 - s of both numbers into the low bytes of the halves
+          constexpr int kTop = S - 1;
+          const int y = (kTop - s) & 3;
+          const uint32_t a = (uint32_t)(q[2 * j] >> (kTop - s >= 4 ? 32 : 0));
+          const uint32_t b = (uint32_t)(q[2 * j + 1] >> (kTop - s >= 4 ? 32 : 0));
+          w = __byte_perm(__byte_perm(a, b, y | ((y + 4) << 4)), 0x64646464u, 0x4140);
         }
         // 0x6400 + n is the FP16 number 1024 + n; minus 1152 leaves the digit, exactly
-        w += 0x64006400u;
         asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(h[j]) : "r"(w), "r"(0x64806480u));
       }
       *reinterpret_cast<uint4 *>(dst + (size_t)(part * S + s) * kSlice) = make_uint4(h[0], h[1], h[2], h[3]);

@@ -24,5 +24,6 @@ addft_status oz_gemm(int digits, int M, int N, int K, int batch, const OzMat &A,
 
 // Device-side error bits since the last call (bit 0: a bounded wait ran out), cleared by the read.
 unsigned oz_status();
+unsigned d64_status();   // the same for dft64.cu
 
 }  // namespace addft

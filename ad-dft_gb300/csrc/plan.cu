@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "dft64.cuh"
 #include "transforms.cuh"
 
 namespace addft {
@@ -82,6 +83,18 @@ static bool factorize(int n, AxisPlan &ap) {
   for (int r : best) ap.rad[ap.nst++] = r;
   if (n == 1) { ap.rad[0] = 1; ap.nst = 0; }
   return true;
+}
+
+// The least scratch of nbatch bands in flight: reduction partials (1 MB) + the potential in xy-plane
+// order (column pipeline, N reals) + per band the larger of the slab (np x n2 x n3) and the column
+// pipeline's buffers (n3 x ncols_pad columns + nG kinetic terms, with the kinetic diagonals of up to
+// one k point per band in flight, nG reals each).
+size_t work_bytes_min(const PlanDev &d, int nbatch, size_t csz) {
+  const size_t slab = (size_t)d.np * d.n2 * d.n3 * csz;
+  const size_t colb = (((size_t)d.n3 * d.ncols_pad * csz + 255) & ~size_t(255)) +
+                      (((size_t)d.nG * csz + 255) & ~size_t(255)) + (((size_t)d.nG * (csz / 2) + 255) & ~size_t(255));
+  const size_t vt = ((size_t)d.n1 * d.n2 * d.n3 * (csz / 2) + 255) & ~size_t(255);
+  return (size_t)nbatch * (slab > colb ? slab : colb) + (size_t(1) << 20) + vt;
 }
 
 }  // namespace addft
@@ -193,6 +206,28 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
     }
   }
 
+  // tables of the FP64 tensor-core transforms
+  std::vector<int> yact, zact, ypos(n2, -1), zpos(n3, -1);
+  for (int g = 0; g < nG; ++g) {
+    ypos[i2[g]] = 0;
+    zpos[i3[g]] = 0;
+  }
+  for (int y = 0; y < n2; ++y)
+    if (ypos[y] == 0) { ypos[y] = (int)yact.size(); yact.push_back(y); }
+  for (int z = 0; z < n3; ++z)
+    if (zpos[z] == 0) { zpos[z] = (int)zact.size(); zact.push_back(z); }
+  const int nq = (int)yact.size(), nz = (int)zact.size();
+  std::vector<int> col_zg((size_t)nrows * nz, -1), col_of((size_t)np * nq, -1), col_pq(nrows);
+  for (int k = 0; k < nG; ++k) {
+    const int g = order[k], c = pt_col[k], pq = plane_of_i1[i1[g]] * nq + ypos[i2[g]];
+    col_zg[(size_t)c * nz + zpos[i3[g]]] = g;
+    col_of[pq] = c;
+    col_pq[c] = pq;
+  }
+  D64Mat dm[6];
+  std::vector<unsigned char> dF;
+  d64_build(n1, n2, n3, plane_i1, yact, zact, dm, dF);
+
   // twiddles e^{-2 pi i t / n}
   const int ntw = n1 + n2 + n3;
   std::vector<double> twd(2 * ntw);
@@ -227,8 +262,9 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
   const size_t o_spg = push(sp_g), o_spp = push(sp_pos), o_gptr = push(gptr),
                o_pi1 = push(plane_i1), o_rptr = push(rptr), o_row = push(row_i2),
                o_poi = push(plane_of_i1), o_mil = push(mil), o_cgp = push(cgptr), o_ptp = push(pt_pos),
-               o_cxy = push(col_xy), o_rlh = push(row_lohi), o_ptc = push(pt_col), o_cm = push(col_m);
-  const size_t total = off_int + sizeof(int) * ints.size();
+               o_cxy = push(col_xy), o_rlh = push(row_lohi), o_ptc = push(pt_col), o_cm = push(col_m), o_zg = push(col_zg), o_cof = push(col_of), o_cpq = push(col_pq);
+  const size_t off_F = align(off_int + sizeof(int) * ints.size());
+  const size_t total = off_F + dF.size();
 
   auto *p = new addft_plan_s();
   if (cudaGetDevice(&p->device) != cudaSuccess) { delete p; set_error("cudaGetDevice failed"); return ADDFT_CUDA_ERROR; }
@@ -242,6 +278,7 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
   memcpy(host.data() + off_twd, twd.data(), sizeof(double) * twd.size());
   memcpy(host.data() + off_twf, twf.data(), sizeof(float) * twf.size());
   memcpy(host.data() + off_int, ints.data(), sizeof(int) * ints.size());
+  if (!dF.empty()) memcpy(host.data() + off_F, dF.data(), dF.size());
   e = cudaMemcpy(p->blob, host.data(), total, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(p->blob);
@@ -265,6 +302,10 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
   d.ncols_pad = ncols_pad; d.cgptr = ib + o_cgp; d.pt_pos = ib + o_ptp; d.col_xy = ib + o_cxy;
   d.pt_col = ib + o_ptc; d.col_m = ib + o_cm; d.col_uniform = col_uniform ? 1 : 0;
   d.xy_direct = xy_direct ? 1 : 0; d.row_lohi = ib + o_rlh;
+  d.nq = nq; d.nz = nz;
+  d.col_zg = ib + o_zg; d.col_of = ib + o_cof; d.col_pq = ib + o_cpq;
+  for (int a = 0; a < 6; ++a) d.d64[a] = dm[a];
+  d.d64_F = dF.empty() ? nullptr : (const unsigned char *)(b + off_F);
   d.tw_d = b + off_twd;
   d.tw_f = b + off_twf;
   for (int a = 0; a < 3; ++a) d.ax[a] = ax[a];
@@ -362,17 +403,10 @@ addft_status addft_plan_get_tuning(addft_plan plan, const char *key, long *value
 
 size_t addft_work_bytes(addft_plan plan, int nbatch, addft_dtype dt) {
   if (!plan || nbatch < 1) return 0;
-  const size_t csz = dt == ADDFT_F64 ? 16 : 8;
-  const PlanDev &d = plan->dev;
-  // reduction partials (1 MB) + the potential in xy-plane order (column pipeline, N reals)
-  // + nbatch bands of the larger of the slab (np x n2 x n3) and the column pipeline's per-band
-  // buffers (n3 x ncols_pad columns + nG kinetic terms)
-  const size_t slab = (size_t)d.np * d.n2 * d.n3 * csz;
-  // (the kinetic diagonals of up to one k point per band in flight, nG reals each, included)
-  const size_t colb = (((size_t)d.n3 * d.ncols_pad * csz + 255) & ~size_t(255)) +
-                      (((size_t)d.nG * csz + 255) & ~size_t(255)) + (((size_t)d.nG * (csz / 2) + 255) & ~size_t(255));
-  const size_t vt = ((size_t)d.n1 * d.n2 * d.n3 * (csz / 2) + 255) & ~size_t(255);
-  return (size_t)nbatch * (slab > colb ? slab : colb) + (size_t(1) << 20) + vt;
+  const size_t least = work_bytes_min(plan->dev, nbatch, dt == ADDFT_F64 ? 16 : 8);
+  if (dt != ADDFT_F64 || !d64_handles(plan->dev, nbatch)) return least;
+  // the FP64 tensor-core form keeps more of a band in flight; with less the FFT kernels run
+  return std::max(least, (size_t)nbatch * d64_band_bytes(plan->dev) + (size_t(1) << 20) + d64_v_bytes(plan->dev));
 }
 
 }  // extern "C"

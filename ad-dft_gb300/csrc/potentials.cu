@@ -7,6 +7,7 @@
 // physics/local.py:21-39, solver/scf.py:81-92 (effective_potential).
 #include <math.h>
 
+#include "dft64.cuh"
 #include "ozgemm.cuh"
 #include "radial.cuh"
 #include "transforms.cuh"
@@ -380,10 +381,16 @@ inline addft_status make_shell(ShellGeo &sg, const double *bvec, double omega, i
   return ADDFT_OK;
 }
 
+// scratch of one field's transform
+inline size_t slab_bytes(const PlanDev &pd) {
+  return d64_handles(pd, 1) ? d64_band_bytes(pd) : (size_t)pd.np * pd.n2 * pd.n3 * sizeof(double2);
+}
+
 // n(G) = fftn(rho)/N gathered on the plan's shell (f64), W = slab scratch
 inline addft_status density_to_shell(const PlanDev &pd, const double *rho, double2 *ng, void *W,
                                      cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  if (d64_handles(pd, 1)) return d64_from_real(pd, 1, rho, true, 1.0 / (double)N, ng, W, slab_bytes(pd), st);
   XArgs<double> a = xargs_default<double>(W);
   a.rin = rho;
   a.rin_is_real = 1;
@@ -397,6 +404,7 @@ inline addft_status density_to_shell(const PlanDev &pd, const double *rho, doubl
 // v(r) = Re(N ifftn(scatter(vg)))
 inline addft_status shell_to_real(const PlanDev &pd, const double2 *vg, double *v, void *W, cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  if (d64_handles(pd, 1)) return d64_to_real(pd, 1, vg, 1.0, v, true, W, slab_bytes(pd), st);
   ADDFT_TRY(launch_plane_inv<double>(pd, 1, vg, pd.nG, 1.0, (double2 *)W, st));
   XArgs<double> a = xargs_default<double>(W);
   a.rout = v;
@@ -464,7 +472,6 @@ inline addft_status phase_forces(const PlanDev &pd, const ShellGeo &sg, const Ph
   return check_launch("k_force_cols");
 }
 
-inline size_t slab_bytes(const PlanDev &pd) { return (size_t)pd.np * pd.n2 * pd.n3 * sizeof(double2); }
 
 }  // namespace addft
 

@@ -527,7 +527,7 @@ unsigned addft_tc05_status(void) {
   unsigned v = 0, z = 0;
   if (cudaMemcpyFromSymbol(&v, addft::g_tc05_error, sizeof(v)) != cudaSuccess) return 0xffffffffu;
   cudaMemcpyToSymbol(addft::g_tc05_error, &z, sizeof(z));
-  return v | addft::oz_status();
+  return v | addft::oz_status() | addft::d64_status();
 }
 
 }  // extern "C"

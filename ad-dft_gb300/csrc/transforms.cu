@@ -22,6 +22,7 @@
 #include <stdlib.h>
 
 #include "colfft.cuh"
+#include "dft64.cuh"
 #include "transforms.cuh"
 
 namespace addft {
@@ -588,11 +589,22 @@ XArgs<R> xargs_default(void *W) {
 // ---------------------------------------------------------------------------
 // entry-point bodies
 // ---------------------------------------------------------------------------
+// FP64 through the tensor-core form: a box and size it handles, and scratch for `extra` bytes and
+// one band; a plan whose tuning asks for the split stages or for other kernels than the defaults
+// keeps to the FFT kernels.
+static bool d64_runs(const PlanDev &pd, int nbatch, const void *work, size_t bytes, size_t extra) {
+  return pd.tun.colfft && !pd.tun.plane_split && d64_handles(pd, nbatch) && work && ((uintptr_t)work & 255) == 0 &&
+         bytes >= extra + 256 + d64_band_bytes(pd);
+}
+
 template <typename R>
 addft_status psi_to_real_t(addft_plan plan, int nbatch, double omega, const void *psi, void *psi_r,
                            void *work, size_t bytes, cudaStream_t st) {
   using C = typename Cx<R>::T;
   const PlanDev &pd = plan->dev;
+  if constexpr (sizeof(R) == 8)
+    if (d64_runs(pd, nbatch, work, bytes, 0))
+      return d64_to_real(pd, nbatch, (const double2 *)psi, 1.0 / sqrt(omega), psi_r, false, work, bytes, st);
   Work w;
   ADDFT_TRY(split_work(pd, sizeof(C), work, bytes, w));
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
@@ -614,9 +626,12 @@ addft_status real_to_psi_t(addft_plan plan, int nbatch, double omega, const void
                            void *work, size_t bytes, cudaStream_t st) {
   using C = typename Cx<R>::T;
   const PlanDev &pd = plan->dev;
+  const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  if constexpr (sizeof(R) == 8)
+    if (d64_runs(pd, nbatch, work, bytes, 0))
+      return d64_from_real(pd, nbatch, psi_r, false, sqrt(omega) / (double)N, (double2 *)psi, work, bytes, st);
   Work w;
   ADDFT_TRY(split_work(pd, sizeof(C), work, bytes, w));
-  const long N = (long)pd.n1 * pd.n2 * pd.n3;
   const R scale = (R)(sqrt(omega) / (double)N);
   for (int b0 = 0; b0 < nbatch; b0 += w.nbfit) {
     const int nbc = min(w.nbfit, nbatch - b0);
@@ -638,6 +653,10 @@ addft_status hpsi_local_t(addft_plan plan, int nk, int nb, const void *psi, cons
                           const void *v_r, void *hpsi, void *work, size_t bytes, cudaStream_t st) {
   using C = typename Cx<R>::T;
   const PlanDev &pd = plan->dev;
+  if constexpr (sizeof(R) == 8)
+    if (d64_runs(pd, nk * nb, work, bytes, d64_v_bytes(pd)))
+      return d64_hpsi(pd, nk * nb, (const double2 *)psi, (const double *)v_r, (double2 *)hpsi, (const double *)kin, nb,
+                      work, bytes, st);
   if (pd.tun.colfft && colfft_handles<R>(pd) && work != nullptr && ((uintptr_t)work & 255) == 0) {
     // column pipeline: [partials 1 MB | Vt (N reals) | column buffers, n3 x ncols_pad per band]
     const size_t red = size_t(1) << 20;
@@ -714,6 +733,9 @@ addft_status density_t(addft_plan plan, int nk, int nb, double omega, const void
     ADDFT_CUDA(cudaMemsetAsync(rho, 0, sizeof(double) * N, st));
     return ADDFT_OK;
   }
+  if constexpr (sizeof(R) == 8)
+    if (d64_runs(pd, nbatch, work, bytes, 2 * (size_t)N * sizeof(double)))
+      return d64_density(pd, nbatch, (const double2 *)psi, wocc, 1.0 / omega, rho, work, bytes, st);
   // split the bands across CTAs so the x-line stage has >= 4 CTAs per SM
   const int t3 = pick_t3<R>(pd, XM_DENSITY, nbatch);
   const int tiles = pd.n2 * ((pd.n3 + t3 - 1) / t3);

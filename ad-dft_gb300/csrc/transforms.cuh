@@ -41,6 +41,9 @@ struct XArgs {
   long N;                 // XM_DENSITY: points in the box
 };
 
+// least scratch of nbatch bands in flight (plan.cu); addft_work_bytes may ask for more
+size_t work_bytes_min(const PlanDev &pd, int nbatch, size_t csz);
+
 struct Work {
   double *partial;   // reduction partials (1 MB)
   void *W;           // slabs
