@@ -19,10 +19,10 @@
 // and slice the rows [-Im F | Re F | Im F] of R outputs, so that [Re; Im] and [-Im; Re] (2 R <= 128
 // rows) are the same bytes from two offsets and one accumulator row holds Re or Im of an output:
 //   D = [Re F; Im F] Re x + [-Im F; Re F] Im x.
-// Eight producer warps load 8 inputs of a line per lane, agree on the line's largest exponent and
-// write its 8 digits per component (62 bits below that exponent) into a ring of operand buffers;
+// Producer warps load 8 inputs of a line per lane, agree on the line's largest exponent and write
+// its 8 digits per component (62 bits below that exponent) into a ring of operand buffers;
 // one thread issues the MMAs (slice s of F against slices 0 .. 7 - s of the lines, side by side along
-// N = 32 (8 - s), landing on levels s .. 7); sixteen epilogue warps empty one of the two accumulators
+// N = 32 (8 - s), landing on levels s .. 7; F has 7 slices); twelve epilogue warps empty one of the two accumulators
 // (8 levels x 32 lines) while the other is filled, add the levels in 64-bit integers and round once
 // to FP64.  All waits are bounded (status as in ozgemm.cu).  The error is that of the slicing, 2^-62
 // of the line's largest input per term, and of one rounding: below an FP64 FFT's.
@@ -30,6 +30,7 @@
 #include <cmath>
 
 #include "dft64.cuh"
+#include "mma16.cuh"
 #include "ozgemm.cuh"
 
 namespace addft {
@@ -38,18 +39,26 @@ namespace {
 
 __device__ unsigned g_d64_error = 0;
 
-constexpr int kS = 8;            // digits
+constexpr int kS = 8;            // digits of a line's inputs
 constexpr int kBits = 62;
+constexpr int kSF = 7;           // digits of F: entries up to 1 to 2^-54, below their own rounding
+constexpr int kFBits = 54;
 constexpr int kLines = 32;       // lines per block
 constexpr int kStep = 16;        // k per MMA
 constexpr int kMaxK = 128;       // sums of 128 products per digit pair stay exact
-constexpr int kRing = 4;         // operand buffers (one kstep of 32 lines each)
+constexpr int kMaxRing = 8;      // operand buffers (one kstep of 32 lines each)
 constexpr int kItem = 2 * kS * kLines * kStep * 2;   // 16 KB
-constexpr int kProd = 8, kEpi = 16;                  // warps
-constexpr int kEpiLines = 4 * kLines / kEpi;         // lines of an epilogue warp
-constexpr int kThreads = 32 * (kProd + kEpi + 1);
+// Warps 0 .. 15 with warp % 4 < 3 empty the accumulator rows 32 (warp % 4) .. of 8 lines each (2 R <= 96
+// rows); warps 3, 7, 11 and those of 16 .. 26 with warp % 4 < 3 produce; warp 15 issues MMAs, on the
+// scheduler that has no epilogue warps.
+constexpr int kEpi = 12, kProd = 12, kEpiLines = 8;
+constexpr int kThreads = 32 * 27;
+constexpr int kMaxGroups = 4;    // groups of producers, each on blocks of its own
+constexpr int kLex = 32;         // blocks whose exponents are kept
 constexpr int kWait = 1 << 20;
-constexpr size_t kMaxF = 154 << 10;   // bytes of F per CTA beside the ring
+constexpr int kMaxR = 48;
+constexpr size_t kRoom = 221000;      // shared memory for F and the ring
+constexpr size_t kMaxF = kRoom - 4 * kItem;
 constexpr int kSms = 152;
 
 __device__ __forceinline__ uint32_t sad(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -75,20 +84,6 @@ __device__ __forceinline__ void arrive(uint64_t *bar) {
 __device__ __forceinline__ void commit_to(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sad(bar))
                : "memory");
-}
-__device__ __forceinline__ uint64_t desc(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
-         ((uint64_t)1 << 46);
-}
-__device__ __forceinline__ uint32_t idesc(int N) {
-  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-      "l"(a), "l"(b), "r"(id), "r"(acc)
-      : "memory");
 }
 #define D64_LD8(taddr, r)                                                                         \
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"           \
@@ -116,40 +111,47 @@ struct Args {
   const double *wocc;      // XI_D
   double *part;            //   [group][z][y][x]
   int groups, per;         //   band groups, bands per group
+  int ring, pw, ngrp, spg; // operand buffers; warps of a producer group, groups, buffers of each
 };
 
-// where a line reads its inputs
+// where a line reads its inputs (line numbers of a chunk stay below 2^30)
 struct Line { long base; int aux; };
 
 template <int ST>
-__device__ __forceinline__ Line line_at(const Args &a, long l) {
+__device__ __forceinline__ Line line_at(const Args &a, unsigned l) {
   const PlanDev &pd = a.pd;
   Line r;
   r.aux = 0;
   if (ST == ZI) {
-    const long b = l / pd.nrows;
-    r.base = b * pd.nG;
+    const unsigned b = l / (unsigned)pd.nrows;
+    r.base = (long)b * pd.nG;
     r.aux = (int)(l - b * pd.nrows) * pd.nz;
   } else if (ST == YI) {
-    const long t = l / pd.n3, b = t / pd.np;
-    r.base = b * pd.nrows * pd.n3 + (l - t * pd.n3);
+    const unsigned t = l / (unsigned)pd.n3, b = t / (unsigned)pd.np;
+    r.base = (long)b * pd.nrows * pd.n3 + (l - t * pd.n3);
     r.aux = (int)(t - b * pd.np) * pd.nq;
   } else if (ST == XI_V || ST == XI_R || ST == XI_C || ST == XI_D) {
-    const long n = (long)pd.n2 * pd.n3, b = l / n;
-    r.base = b * pd.np * n + (l - b * n);
+    const unsigned n = pd.n2 * pd.n3, b = l / n;
+    r.base = (long)b * pd.np * n + (l - b * n);
   } else if (ST == XF) {
-    r.base = l * pd.n1;
+    r.base = (long)l * pd.n1;
   } else if (ST == XR_R || ST == XR_C) {   // lines (band, y, z)
-    const long n = (long)pd.n2 * pd.n3, b = l / n;
-    r.base = b * n * pd.n1 + (l - b * n);
+    const unsigned n = pd.n2 * pd.n3, b = l / n;
+    r.base = (long)b * n * pd.n1 + (l - b * n);
   } else if (ST == YF) {
-    const long t = l / pd.np, b = t / pd.n3;
-    r.base = b * pd.n2 * pd.n3 * pd.np + (t - b * pd.n3) * a.sz + (l - t * pd.np);
+    const unsigned t = l / (unsigned)pd.np, b = t / (unsigned)pd.n3;
+    r.base = (long)b * pd.n2 * pd.n3 * pd.np + (t - b * pd.n3) * a.sz + (l - t * pd.np);
   } else {
-    const long b = l / pd.nrows;
-    r.base = b * pd.n3 * pd.np * pd.nq + pd.col_pq[l - b * pd.nrows];
+    const unsigned b = l / (unsigned)pd.nrows;
+    r.base = (long)b * pd.n3 * pd.np * pd.nq + pd.col_pq[l - b * pd.nrows];
   }
   return r;
+}
+
+// lines of one band in the stages whose stores need the band
+template <int ST>
+__device__ __forceinline__ unsigned period(const PlanDev &pd) {
+  return ST == XI_V ? pd.n2 * pd.n3 : (ST == ZF || ST == ZF_H ? pd.nrows : 0x7fffffff);
 }
 
 template <int ST>
@@ -175,24 +177,25 @@ __device__ __forceinline__ double2 load_at(const Args &a, const Line &l, int k) 
   }
 }
 
-// one component of output o of line l
+// one component of output o of line l = band * period + rem
 template <int ST>
-__device__ __forceinline__ void store_at(const Args &a, long l, int o, int comp, double v) {
+__device__ __forceinline__ void store_at(const Args &a, unsigned l, unsigned band, unsigned rem, int o, int comp,
+                                         double v) {
   const PlanDev &pd = a.pd;
   double *out = reinterpret_cast<double *>(a.out);
-  if (ST == ZI) out[2 * (l * pd.n3 + o) + comp] = v;
-  else if (ST == YI) out[2 * (l * pd.n2 + o) + comp] = v;
-  else if (ST == XI_V) out[2 * (l * pd.n1 + o) + comp] = v * a.V[(l % ((long)pd.n2 * pd.n3)) * pd.n1 + o];
-  else if (ST == XI_C) out[2 * (l * pd.n1 + o) + comp] = v * a.scale;
-  else if (ST == XI_R) { if (!comp) out[l * pd.n1 + o] = v * a.scale; }
-  else if (ST == XF || ST == XR_R || ST == XR_C) out[2 * (l * pd.np + o) + comp] = v;
-  else if (ST == YF) out[2 * (l * pd.nq + o) + comp] = v;
+  if (ST == ZI) out[2 * ((long)l * pd.n3 + o) + comp] = v;
+  else if (ST == YI) out[2 * ((long)l * pd.n2 + o) + comp] = v;
+  else if (ST == XI_V) out[2 * ((long)l * pd.n1 + o) + comp] = v * a.V[(long)rem * pd.n1 + o];
+  else if (ST == XI_C) out[2 * ((long)l * pd.n1 + o) + comp] = v * a.scale;
+  else if (ST == XI_R) { if (!comp) out[(long)l * pd.n1 + o] = v * a.scale; }
+  else if (ST == XF || ST == XR_R || ST == XR_C) out[2 * ((long)l * pd.np + o) + comp] = v;
+  else if (ST == YF) out[2 * ((long)l * pd.nq + o) + comp] = v;
   else {
-    const long b = l / pd.nrows;
-    const int g = pd.col_zg[(l - b * pd.nrows) * pd.nz + o];
+    const int g = pd.col_zg[rem * pd.nz + o];
     if (g < 0) return;
-    const long at = 2 * (b * pd.nG + g) + comp;
-    if (ST == ZF_H) v += a.kin[(a.batch0 + b) / a.nb_per_k * pd.nG + g] * reinterpret_cast<const double *>(a.psi)[at];
+    const long at = 2 * ((long)band * pd.nG + g) + comp;
+    if (ST == ZF_H)
+      v += a.kin[(long)((a.batch0 + (int)band) / a.nb_per_k) * pd.nG + g] * reinterpret_cast<const double *>(a.psi)[at];
     else v *= a.scale;
     out[at] = v;
   }
@@ -227,39 +230,40 @@ __device__ __forceinline__ double to_double(long long T, int n) {
   return __longlong_as_double((long long)(r | sign));
 }
 
-// x as q = round(x 2^(62 - E)) of a line with exponent field em, 128 added to every byte but the top
+// x as q = trunc(x 2^(62 - E)) of a line with exponent field em, 128 added to every byte but the top
 __device__ __forceinline__ uint64_t d64_bytes(double x, int em) {
-  const uint64_t u = (uint64_t)__double_as_longlong(x);
-  const int e = (int)(u >> 52) & 0x7ff;
-  uint64_t m = u & 0xFFFFFFFFFFFFFull;
-  if (e) m |= 1ull << 52;
-  const int sh = kBits - 53 - (max(em, 1) - max(e, 1));
-  uint64_t q;
-  if (sh >= 0) {
-    q = m << sh;
-  } else {
-    const int r = min(-sh, 63);
-    q = (m + (1ull << (r - 1))) >> r;
+  const uint32_t xh = (uint32_t)__double2hiint(x), xl = (uint32_t)__double2loint(x);
+  const int e = (int)(xh >> 20) & 0x7ff;
+  // 53 significand bits with the leading one at bit 61, then down by the exponents' difference
+  uint32_t h = (__funnelshift_l(xl, xh, 9) & 0x1fffffffu) | (e ? 0x20000000u : 0u), l = xl << 9;
+  int d = em - max(e, 1);
+  if (d >= 32) {
+    l = h;
+    h = 0;
+    d -= 32;
   }
-  if ((int64_t)u < 0) q = 0 - q;
-  return q + 0x0080808080808080ull;
+  l = __funnelshift_rc(l, h, d);
+  h = d < 32 ? h >> d : 0;
+  const uint32_t s = (uint32_t)((int)xh >> 31);
+  const uint64_t q = ((uint64_t)(h ^ s) << 32) | (l ^ s);
+  return q + (0x0080808080808080ull - (uint64_t)(int64_t)(int)s);
 }
 
 template <int ST>
 __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = smem_raw + ((1024 - (sad(smem_raw) & 1023)) & 1023);
-  __shared__ __align__(8) uint64_t fullB[kRing], emptyB[kRing], accf[2], acce[2], fbar;
-  __shared__ int pm[2][kProd][kLines];    // exponents found by each producer warp
-  __shared__ int lex[8][kLines];          // exponents of the lines of the last blocks
+  __shared__ __align__(8) uint64_t fullB[kMaxRing], emptyB[kMaxRing], accf[2], acce[2], fbar;
+  __shared__ uint16_t pm[2][kProd][kLines];   // exponents found by each producer warp
+  __shared__ uint16_t lex[kLex][kLines];      // exponents of the lines of the last blocks
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nks = a.m.nks, R = a.m.R, tile = blockIdx.y;
-  const long nblk = (a.lines + kLines - 1) / kLines;
-  const int inner_max = ST == XI_D ? a.per : 1;
-  const long units = ST == XI_D ? nblk * a.groups : nblk;
+  const int ngrp = a.ngrp, spg = a.spg;
+  const unsigned nblk = (unsigned)((a.lines + kLines - 1) / kLines);
+  const unsigned units = ST == XI_D ? nblk * a.groups : nblk;
   if (tid == 0) {
-    for (int i = 0; i < kRing; ++i) {
+    for (int i = 0; i < a.ring; ++i) {
       init_bar(&fullB[i], 2);
       init_bar(&emptyB[i], 1);
     }
@@ -278,13 +282,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
-  const uint32_t sring = sad(smem), sF = sring + kRing * kItem;   // F last: its 128-row reads may run past it
+  const uint32_t sring = sad(smem), sF = sring + a.ring * kItem;   // F last: its 128-row reads may run past it
   bool ok = true;
 
   // a block: 32 lines starting at l0 (XI_D: of one band); `inner` blocks share a unit
-  auto unit_info = [&](long u, long &l0, int &b0, int &inner) {
+  auto unit_info = [&](unsigned u, unsigned &l0, int &b0, int &inner) {
     if (ST == XI_D) {
-      const long lb = u / a.groups;
+      const unsigned lb = u / (unsigned)a.groups;
       const int g = (int)(u - lb * a.groups);
       l0 = lb * kLines;
       b0 = g * a.per;
@@ -296,18 +300,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
     }
   };
 
-  if (warp < kProd) {
-    // ---- producers: lane = line, warp = 8 inputs (and, above 64 inputs, 8 more)
+  const bool epi = warp < 16 && (warp & 3) < 3;
+  if (!epi && warp != 15) {
+    // ---- producers: lane = line, warp = 8 inputs (and 8 more where a group has fewer warps).  Groups
+    // take blocks in turn, so one loads while another converts; each has buffers of its own (at
+    // least a block's), or, alone, may share one between inputs of the same warps: the previous
+    // user of a buffer has then always been filled when its release is waited for.
+    const int pi = warp < 16 ? warp >> 2 : 3 * (warp >> 2) + (warp & 3) - 9, grp = pi / a.pw, me = pi - grp * a.pw;
     const int noct = 2 * nks;
-    long blk = 0;
-    for (long u = blockIdx.x; u < units; u += gridDim.x) {
-      long l0;
+    unsigned blk = 0;
+    if (grp < ngrp && (warp < 16 || (warp & 3) < 3))
+    for (unsigned u = blockIdx.x; u < units; u += gridDim.x) {
+      unsigned l0;
       int b0, inner;
       unit_info(u, l0, b0, inner);
       for (int it = 0; it < inner; ++it, ++blk) {
-        long l = l0 + lane;
+        const unsigned turn = blk / (unsigned)ngrp;
+        if ((int)(blk - turn * ngrp) != grp) continue;
+        unsigned l = l0 + lane;
         const bool live = l < a.lines;
-        if (ST == XI_D) l += (long)(b0 + it) * a.lines;
+        if (ST == XI_D) l += (unsigned)(b0 + it) * (unsigned)a.lines;
         const Line ln = line_at<ST>(a, live ? l : 0);
         double2 x[8];
         auto load = [&](int o) {
@@ -320,25 +332,24 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
         int em = 0;
         // with more than 64 inputs a warp has two groups of 8; the first stays in registers
 #pragma unroll 1
-        for (int o = noct > kProd ? warp + kProd : warp; o >= 0; o -= kProd) {
+        for (int o = noct > a.pw ? me + a.pw : me; o >= 0; o -= a.pw) {
           load(o);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             em = max(em, max((__double2hiint(x[j].x) >> 20) & 0x7ff, (__double2hiint(x[j].y) >> 20) & 0x7ff));
         }
-        int(*p)[kLines] = pm[blk & 1];
-        p[warp][lane] = em;
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * kProd) : "memory");   // every producer gets here, failed or not
-#pragma unroll
-        for (int w = 0; w < kProd; ++w) em = max(em, p[w][lane]);
-        if (warp == 0) lex[blk & 7][lane] = em;
+        uint16_t(*p)[kLines] = pm[turn & 1] + grp * a.pw;
+        p[me][lane] = (uint16_t)em;
+        // every warp of the group gets here, failed or not
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * a.pw) : "memory");
+        for (int w = 0; w < a.pw; ++w) em = max(em, (int)p[w][lane]);
+        if (me == 0) lex[blk % kLex][lane] = (uint16_t)em;
 #pragma unroll 1
-        for (int o = warp; o < noct; o += kProd) {
-          if (o > warp) load(o);
-          const long t = blk * nks + (o >> 1);
-          const int slot = (int)(t % kRing);
-          const long round = t / kRing;
-          if (ok && round > 0) ok = __all_sync(0xffffffffu, wait_bar(&emptyB[slot], (uint32_t)(round - 1) & 1));
+        for (int o = me; o < noct; o += a.pw) {
+          if (o > me) load(o);
+          const unsigned t = turn * nks + (o >> 1), round = t / (unsigned)spg;
+          const int slot = grp * spg + (int)(t - round * spg);
+          if (ok && round > 0) ok = __all_sync(0xffffffffu, wait_bar(&emptyB[slot], (round - 1) & 1));
           if (!ok) continue;
           const uint32_t dst = sring + slot * kItem + (lane >> 3) * 256 + (o & 1) * 128 + (lane & 7) * 16;
 #pragma unroll
@@ -346,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
             uint64_t q[8];
 #pragma unroll
             // a line that is not finite is all NaN in the epilogue, whatever its digits
-            for (int j = 0; j < 8; ++j) q[j] = d64_bytes(em == 0x7ff ? 0.0 : (part ? x[j].y : x[j].x), em);
+            for (int j = 0; j < 8; ++j) q[j] = d64_bytes(em == 0x7ff ? 0.0 : (part ? x[j].y : x[j].x), max(em, 1));
 #pragma unroll
             for (int s = 0; s < kS; ++s) {
               uint32_t hh[4];
@@ -378,9 +389,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
       }
     }
     if (!ok && lane == 0) atomicOr(&g_d64_error, 1u);
-  } else if (warp == kProd + kEpi) {
+  } else if (!epi) {
     // ---- F, then MMAs
-    if (lane == 0) {
+    const bool lead = elect_one();
+    if (lead) {
       const uint32_t bytes = (uint32_t)a.m.tile_bytes;
       const unsigned char *src = a.F + a.m.off + (size_t)tile * bytes;
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sad(&fbar)), "r"(bytes) : "memory");
@@ -391,66 +403,78 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
             "l"(src + o), "r"(n), "r"(sad(&fbar))
             : "memory");
       }
-      ok = wait_bar(&fbar, 0);
-      const uint32_t sl = 3 * R * 32;   // bytes of one slice of F
-      long blk = 0;
-      bool issued = false;
-      for (long u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        long l0;
-        int b0, inner;
-        unit_info(u, l0, b0, inner);
-        for (int it = 0; it < inner && ok; ++it, ++blk) {
-          const int buf = (int)(blk & 1);
-          if (blk >= 2) ok = wait_bar(&acce[buf], (uint32_t)(blk / 2 - 1) & 1);
-          for (int j = 0; j < nks && ok; ++j) {
-            const long t = blk * nks + j;
-            const int slot = (int)(t % kRing);
-            ok = wait_bar(&fullB[slot], (uint32_t)(t / kRing) & 1);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issued = true;
+    }
+    ok = wait_bar(&fbar, 0);
+    const uint32_t sl = (3 * R * 32) >> 4;   // one slice of F, in descriptor units
+    const uint32_t fre = desc_lo(sF + R * 32), fim = desc_lo(sF), ring0 = desc_lo(sring);
+    unsigned blk = 0, slot = 0, grp = 0;     // blk % ngrp; each group's buffers in turn
+    unsigned round = 0, pos = 0;             // of the current group's next buffer
+    bool issued = false;
+    for (unsigned u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      unsigned l0;
+      int b0, inner;
+      unit_info(u, l0, b0, inner);
+      for (int it = 0; it < inner && ok; ++it, ++blk) {
+        const unsigned buf = blk & 1;
+        if (blk >= 2) ok = wait_bar(&acce[buf], (blk / 2 - 1) & 1);
+        const unsigned turn = blk / (unsigned)ngrp;
+        grp = blk - turn * ngrp;
+        round = turn * nks / (unsigned)spg;
+        pos = turn * nks - round * spg;
+        for (int j = 0; j < nks && ok; ++j) {
+          slot = grp * spg + pos;
+          ok = wait_bar(&fullB[slot], round & 1);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          issued = true;
+          if (lead) {
+            const uint32_t d = tmem + 256 * buf, b = ring0 + slot * (kItem >> 4), f = j * kSF * sl;
 #pragma unroll
-            for (int part = 0; part < 2; ++part) {   // [Re; Im] Re x, then [-Im; Re] Im x
-              const uint32_t f0 = sF + j * kS * sl + (part ? 0 : R * 32);
-              const uint64_t bd = desc(sring + slot * kItem + part * kS * (kLines * kStep * 2));
+            for (int i = 0; i < kSF; ++i)   // [Re; Im] Re x
+              mma_f16(d + 32 * i, fre + f + i * sl, b, idesc_f16(32 * (kS - i), false), !(j == 0 && i == 0));
 #pragma unroll
-              for (int i = 0; i < kS; ++i)
-                mma_f16(tmem + 256 * buf + 32 * i, desc(f0 + i * sl), bd, idesc(32 * (kS - i)), !(j == 0 && part == 0 && i == 0));
-            }
+            for (int i = 0; i < kSF; ++i)   // [-Im; Re] Im x
+              mma_f16(d + 32 * i, fim + f + i * sl, b + ((kS * kLines * kStep * 2) >> 4), idesc_f16(32 * (kS - i), false), 1);
             commit_to(&emptyB[slot]);
+            if (j == nks - 1) commit_to(&accf[buf]);
           }
-          if (ok) commit_to(&accf[buf]);
+          __syncwarp();
+          if (++pos == (unsigned)spg) {
+            pos = 0;
+            ++round;
+          }
         }
       }
-      if (!ok) {
-        atomicOr(&g_d64_error, 1u);
-        wait_bar(&fbar, 0);
-        if (issued) {   // no MMA may be in flight when tensor memory is given back
-          commit_to(&accf[0]);
-          wait_bar(&accf[0], 0);
-          wait_bar(&accf[0], 1);
-        }
+    }
+    if (!ok) {
+      if (lead) atomicOr(&g_d64_error, 1u);
+      wait_bar(&fbar, 0);
+      if (issued) {   // no MMA may be in flight when tensor memory is given back
+        if (lead) commit_to(&accf[0]);
+        __syncwarp();
+        wait_bar(&accf[0], 0);
+        wait_bar(&accf[0], 1);
       }
     }
   } else {
     // ---- epilogue: warp reads accumulator rows 32 (w % 4) .. of kEpiLines lines
-    const int w = warp - kProd, q = warp & 3, c0 = kEpiLines * (w >> 2);
+    const int q = warp & 3, c0 = kEpiLines * (warp >> 2);
     const int row = 32 * q + lane, comp = row >= R ? 1 : 0, r = comp ? row - R : row;
     const int o = tile * a.m.per + r;
     const bool on = row < 2 * R && r < a.m.per && o < a.m.outs;
     const bool any = 32 * q < 2 * R;
-    // the level sums as hi 2^32 + lo, hi <= 2^35 2 K: keep as many of lo's bits as 62 bits hold (18 to 21)
-    const int keep = 62 - 35 - (32 - __clz(2 * a.m.K));
+    // the level sums as hi 2^32 + lo, hi <= 2^36 2 K: keep as many of lo's bits as 62 bits hold (17 to 20)
+    const int keep = 62 - 36 - (32 - __clz(2 * a.m.K));
     const int w4 = 1 << (keep - 8), w5 = 1 << (keep - 16);
     const float w67 = __int_as_float((127 - 32 + keep) << 23);
-    // q_F q_x = 256^7 (hi 2^32 + lo); F has exponent field 1023, x = q 2^(E - 62), E = field - 1022
-    const int nbase = 56 + 32 - keep + 1023 - 2 * 1022 - 2 * kBits;
+    // q_F q_x = 256^6 (hi 2^32 + lo); F = q 2^-54, x = q 2^(E - 62), E = field - 1022
+    const int nbase = 48 + 32 - keep - kFBits - 1022 - kBits;
     double acc[kEpiLines];
 #pragma unroll
     for (int c = 0; c < kEpiLines; ++c) acc[c] = 0.0;
-    long blk = 0;
-    for (long u = blockIdx.x; u < units && ok; u += gridDim.x) {
-      long l0;
+    unsigned blk = 0;
+    for (unsigned u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      unsigned l0;
       int b0, inner;
       unit_info(u, l0, b0, inner);
       for (int it = 0; it < inner && ok; ++it, ++blk) {
@@ -482,17 +506,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
         if (lane == 0) arrive(&acce[buf]);   // the accumulator has been read
         if (!on) continue;
         const double wb = ST == XI_D ? a.wocc[b0 + it] : 0.0;
+        const unsigned per = period<ST>(a.pd);
+        unsigned band = (l0 + c0) / per, rem = (l0 + c0) - band * per;
 #pragma unroll
         for (int c = 0; c < kEpiLines; ++c) {
-          const long l = l0 + c0 + c;
+          const unsigned l = l0 + c0 + c;
           if (l >= a.lines) break;
-          const int em = lex[blk & 7][c0 + c], n = nbase + max(em, 1);
+          if (c > 0 && ++rem == per) {
+            rem = 0;
+            ++band;
+          }
+          const int em = lex[blk % kLex][c0 + c], n = nbase + max(em, 1);
           double v;
           if (n >= -1000 && n <= 900) v = ST == XI_D ? to_double(T[c], n) : scaled(T[c], n);
           else v = scale2(scale2((double)T[c], n / 2), n - n / 2);
           if (em == 0x7ff) v = __longlong_as_double(0x7ff8000000000000ll);
           if (ST == XI_D) acc[c] = fma(wb * v, v, acc[c]);
-          else store_at<ST>(a, l, o, comp, v);
+          else store_at<ST>(a, l, band, rem, o, comp, v);
         }
       }
       if (ST == XI_D && ok) {   // Re^2 and Im^2 sit in different rows: [group][2][z][y][x]
@@ -500,8 +530,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
         double *dst = a.part + ((size_t)g * 2 + comp) * a.lines * a.pd.n1;
 #pragma unroll
         for (int c = 0; c < kEpiLines; ++c) {
-          const long l = l0 + c0 + c;
-          if (on && l < a.lines) dst[l * a.pd.n1 + o] = acc[c];
+          const unsigned l = l0 + c0 + c;
+          if (on && l < a.lines) dst[(long)l * a.pd.n1 + o] = acc[c];
           acc[c] = 0.0;
         }
       }
@@ -582,7 +612,12 @@ addft_status stage(const PlanDev &pd, int axis, Args &a, long lines, cudaStream_
   a.m = pd.d64[axis];
   a.F = pd.d64_F;
   a.lines = lines;
-  const size_t sm = (size_t)kRing * kItem + a.m.tile_bytes + 4096 + 1024;   // a 128-row read may pass F's end
+  a.ring = std::min<int>(kMaxRing, (int)((kRoom - a.m.tile_bytes) / kItem));
+  const int noct = 2 * a.m.nks;
+  a.pw = std::min(std::min(noct, kProd), 2 * a.ring);
+  a.ngrp = std::max(1, std::min(std::min(kMaxGroups, kProd / a.pw), a.ring / a.m.nks));
+  a.spg = a.ring / a.ngrp;
+  const size_t sm = (size_t)a.ring * kItem + a.m.tile_bytes + 4096 + 1024;   // a 128-row read may pass F's end
   ADDFT_TRY(smem_optin(k_d64<ST>, sm));
   const long blocks = (lines + kLines - 1) / kLines * (ST == XI_D ? a.groups : 1);
   const int gx = (int)std::max<long>(1, std::min<long>(blocks, kSms / a.m.tiles));
@@ -612,10 +647,13 @@ addft_status to_planes(const PlanDev &pd, int nb, const double2 *psi, double2 *r
 }
 
 int chunk_bands(const PlanDev &pd, int nbatch, size_t bytes) {
-  const size_t per = d64_band_bytes(pd);
-  size_t fit = bytes / per, cap = std::max<size_t>(1, pd.tun.slab_chunk_bytes / per);
-  fit = std::min(std::min(fit, cap), (size_t)nbatch);
-  return (int)fit;
+  // as many bands at once as the scratch holds, in equal chunks: every launch has the ramp of 152 CTAs
+  // that load F first (160 bands of Si64 in chunks of 10 / 20 / 40 / 80: 6.6 / 6.0 / 5.6 / 5.5 ms)
+  const size_t cap = (size_t(1) << 30) / ((size_t)pd.n2 * pd.n3);   // line numbers
+  const int fit = (int)std::min(std::min(bytes / d64_band_bytes(pd), cap), (size_t)nbatch);
+  if (fit < 1) return fit;
+  const int chunks = (nbatch + fit - 1) / fit;
+  return (nbatch + chunks - 1) / chunks;
 }
 
 }  // namespace
@@ -769,11 +807,11 @@ static uint16_t half_int(int d) {   // FP16 bits of an integer, |d| <= 128
   return (uint16_t)((d < 0 ? 0x8000u : 0u) | ((unsigned)(e + 15) << 10) | ((a << (10 - e)) & 0x3ffu));
 }
 
-static void digits_of(double x, uint16_t *h) {   // |x| <= 1, exponent field 1023
-  const int64_t q = (int64_t)std::llrint(std::ldexp(x, kBits - 1));
-  const uint64_t u = (uint64_t)q + 0x0080808080808080ull;
-  h[0] = half_int((int)((int64_t)u >> 56));
-  for (int s = 1; s < kS; ++s) h[s] = half_int((int)((u >> (56 - 8 * s)) & 0xff) - 128);
+static void digits_of(double x, uint16_t *h) {   // |x| <= 1
+  const int64_t q = (int64_t)std::llrint(std::ldexp(x, kFBits));
+  const uint64_t u = (uint64_t)q + 0x0000808080808080ull;
+  h[0] = half_int((int)((int64_t)u >> 48));
+  for (int s = 1; s < kSF; ++s) h[s] = half_int((int)((u >> (48 - 8 * s)) & 0xff) - 128);
 }
 
 void d64_build(int n1, int n2, int n3, const std::vector<int> &xact, const std::vector<int> &yact,
@@ -791,8 +829,8 @@ void d64_build(int n1, int n2, int n3, const std::vector<int> &xact, const std::
     if (d.K > kMaxK) continue;
     for (int t = 1; t <= 8; ++t) {
       const int per = (d.outs + t - 1) / t, R = (per + 7) / 8 * 8;
-      const size_t bytes = (size_t)d.nks * kS * 3 * R * 32;
-      if (R > 64 || bytes > kMaxF) continue;
+      const size_t bytes = (size_t)d.nks * kSF * 3 * R * 32;
+      if (R > kMaxR || bytes > kMaxF) continue;
       d.tiles = t;
       d.per = per;
       d.R = R;
@@ -801,13 +839,13 @@ void d64_build(int n1, int n2, int n3, const std::vector<int> &xact, const std::
     }
     if (d.tiles == 0) continue;
     // digits of the n-th roots of unity: -Im, Re, Im of e^{+-2 pi i t / n}
-    std::vector<uint16_t> dig((size_t)n[ax] * 3 * kS);
+    std::vector<uint16_t> dig((size_t)n[ax] * 3 * kSF);
     for (int t = 0; t < n[ax]; ++t) {
       const double ang = 2.0 * M_PI * (double)t / (double)n[ax];
       const double re = std::cos(ang), im = inv ? std::sin(ang) : -std::sin(ang);
-      digits_of(-im, &dig[(size_t)(3 * t) * kS]);
-      digits_of(re, &dig[(size_t)(3 * t + 1) * kS]);
-      digits_of(im, &dig[(size_t)(3 * t + 2) * kS]);
+      digits_of(-im, &dig[(size_t)(3 * t) * kSF]);
+      digits_of(re, &dig[(size_t)(3 * t + 1) * kSF]);
+      digits_of(im, &dig[(size_t)(3 * t + 2) * kSF]);
     }
     while (blob.size() % 256) blob.push_back(0);
     d.off = (long)blob.size();
@@ -820,11 +858,11 @@ void d64_build(int n1, int n2, int n3, const std::vector<int> &xact, const std::
           const long j = inv ? (long)o * (*act[ax])[k] : (long)(*act[ax])[o] * k;
           const int i = (int)(j % n[ax]);
           for (int b = 0; b < 3; ++b) {
-            const uint16_t *h = &dig[(size_t)(3 * i + b) * kS];
+            const uint16_t *h = &dig[(size_t)(3 * i + b) * kSF];
             const int row = b * d.R + r;
-            for (int s = 0; s < kS; ++s) {
+            for (int s = 0; s < kSF; ++s) {
               unsigned char *p = blob.data() + d.off + (size_t)t * d.tile_bytes +
-                                 (size_t)(k / kStep * kS + s) * (3 * d.R * 32) + (row >> 3) * 256 +
+                                 (size_t)(k / kStep * kSF + s) * (3 * d.R * 32) + (row >> 3) * 256 +
                                  ((k % kStep) / 8) * 128 + (row & 7) * 16 + (k % 8) * 2;
               p[0] = (unsigned char)(h[s] & 0xff);
               p[1] = (unsigned char)(h[s] >> 8);

@@ -40,6 +40,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "mma16.cuh"
 #include "ozgemm.cuh"
 
 namespace addft {
@@ -102,23 +103,6 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_
       "r"(bytes), "r"(sad(bar))
       : "memory");
 }
-// K-major operand without swizzle: 128 B between the two core matrices of 16 k, 256 B between row groups
-__device__ __forceinline__ uint64_t oz_desc(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
-         ((uint64_t)1 << 46);
-}
-// kind::f16, FP16 operands, FP32 accumulator, optionally negated A
-__device__ __forceinline__ uint32_t oz_idesc(int N, bool neg) {
-  return (1u << 4) | (neg ? 1u << 13 : 0u) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kRowsA >> 4) << 24);
-}
-__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc)
-      : "memory");
-}
-
 #define OZ_LD8(taddr, r)                                                                          \
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"           \
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), \
@@ -408,38 +392,57 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
       if (!ok) atomicOr(&g_oz_error, 1u);
     }
   } else if (warp == kEpiWarps + 1) {
-    if (lane == 0) {   // MMAs
-      for (int s = 0; s < nst && ok; ++s) {
-        const int jb = s % P::kBRing, blk = s / kDrain;
-        const bool first = s % kDrain == 0;
-        if (first && blk > 0) ok = wait_bar(&acce, (blk - 1) & 1);   // the accumulators have been read
-        if (ok) ok = wait_bar(&fb[jb], (s / P::kBRing) & 1);
-        const uint32_t b0 = sb + jb * P::kBBytes;
+    // MMAs
+    const bool lead = elect_one();
+    const uint32_t a_lo = desc_lo(sa), b_lo = desc_lo(sb);
+    int ja = 0, jb = 0;
+    uint32_t pa = 0, pb = 0;   // phases of the rings
+    bool issued = false;
+    for (int s = 0; s < nst && ok; ++s) {
+      const int blk = s / kDrain;
+      const bool first = s % kDrain == 0;
+      if (first && blk > 0) ok = wait_bar(&acce, (blk - 1) & 1);   // the accumulators have been read
+      if (ok) ok = wait_bar(&fb[jb], pb);
+      const uint32_t b0 = b_lo + jb * (P::kBBytes >> 4);
 #pragma unroll
-        for (int ra = 0; ra < 2; ++ra) {   // part of A
-          const int a = 2 * s + ra, ja = a % P::kARing;
-          if (ok) ok = wait_bar(&fa[ja], (a / P::kARing) & 1);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a0 = sa + ja * P::kAItem;
+      for (int ra = 0; ra < 2; ++ra) {   // part of A
+        if (ok) ok = wait_bar(&fa[ja], pa);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        issued = true;
+        if (lead) {
+          const uint32_t a0 = a_lo + ja * (P::kAItem >> 4);
 #pragma unroll
           for (int rb = 0; rb < 2; ++rb) {   // part of B; re: rr, ii; im: ri, ir
-            const uint32_t d = tmem + ((ra ^ rb) ? 256 : 0);
-            const uint64_t bd = oz_desc(b0 + rb * S * (kRowsB * kStep * 2));
+            const uint32_t d = tmem + ((ra ^ rb) ? 256 : 0), bd = b0 + ((rb * S * kRowsB * kStep * 2) >> 4);
 #pragma unroll
             for (int i = 0; i < S; ++i)
-              mma_f16(d + 32 * i, oz_desc(a0 + i * (kRowsA * kStep * 2)), bd, oz_idesc(32 * (S - i), ra && rb),
+              mma_f16(d + 32 * i, a0 + ((i * kRowsA * kStep * 2) >> 4), bd, idesc_f16(32 * (S - i), ra && rb),
                       !(first && ra == 0 && i == 0));
           }
           commit_to(&ea[ja]);
+          if (ra == 1) {
+            commit_to(&eb[jb]);
+            if (s % kDrain == kDrain - 1 || s == nst - 1) commit_to(&accf);
+          }
         }
-        if (!ok) break;
-        commit_to(&eb[jb]);
-        if (s % kDrain == kDrain - 1 || s == nst - 1) commit_to(&accf);
+        __syncwarp();
+        if (++ja == P::kARing) {
+          ja = 0;
+          pa ^= 1;
+        }
       }
-      if (!ok) {   // every MMA issued has to be done before tensor memory is given back
-        atomicOr(&g_oz_error, 1u);
-        commit_to(&accf);
+      if (!ok) break;
+      if (++jb == P::kBRing) {
+        jb = 0;
+        pb ^= 1;
+      }
+    }
+    if (!ok) {   // every MMA issued has to be done before tensor memory is given back
+      if (lead) atomicOr(&g_oz_error, 1u);
+      if (issued) {
+        if (lead) commit_to(&accf);
+        __syncwarp();
         wait_bar(&accf, 0);
         wait_bar(&accf, 1);
       }
