@@ -177,28 +177,35 @@ __device__ __forceinline__ double2 load_at(const Args &a, const Line &l, int k) 
   }
 }
 
-// one component of output o of line l = band * period + rem
+// What a store needs beside the value, read before the accumulator is waited for: V(r), or the sphere
+// point and kin psi there (reading it between the stores of a block cost a memory latency each).
 template <int ST>
-__device__ __forceinline__ void store_at(const Args &a, unsigned l, unsigned band, unsigned rem, int o, int comp,
-                                         double v) {
+__device__ __forceinline__ void pre_at(const Args &a, unsigned band, unsigned rem, int o, int comp, double &x, int &g) {
+  const PlanDev &pd = a.pd;
+  if (ST == XI_V) x = __ldg(a.V + (long)rem * pd.n1 + o);
+  if (ST == ZF || ST == ZF_H) g = __ldg(pd.col_zg + rem * pd.nz + o);
+  if (ST == ZF_H) {
+    x = 0.0;
+    if (g >= 0)
+      x = __ldg(a.kin + (long)((a.batch0 + (int)band) / a.nb_per_k) * pd.nG + g) *
+          __ldg(reinterpret_cast<const double *>(a.psi) + 2 * ((long)band * pd.nG + g) + comp);
+  }
+}
+
+// one component of output o of line l (of band `band`)
+template <int ST>
+__device__ __forceinline__ void store_at(const Args &a, unsigned l, unsigned band, int o, int comp, double v, double x,
+                                         int g) {
   const PlanDev &pd = a.pd;
   double *out = reinterpret_cast<double *>(a.out);
   if (ST == ZI) out[2 * ((long)l * pd.n3 + o) + comp] = v;
   else if (ST == YI) out[2 * ((long)l * pd.n2 + o) + comp] = v;
-  else if (ST == XI_V) out[2 * ((long)l * pd.n1 + o) + comp] = v * a.V[(long)rem * pd.n1 + o];
+  else if (ST == XI_V) out[2 * ((long)l * pd.n1 + o) + comp] = v * x;
   else if (ST == XI_C) out[2 * ((long)l * pd.n1 + o) + comp] = v * a.scale;
   else if (ST == XI_R) { if (!comp) out[(long)l * pd.n1 + o] = v * a.scale; }
   else if (ST == XF || ST == XR_R || ST == XR_C) out[2 * ((long)l * pd.np + o) + comp] = v;
   else if (ST == YF) out[2 * ((long)l * pd.nq + o) + comp] = v;
-  else {
-    const int g = pd.col_zg[rem * pd.nz + o];
-    if (g < 0) return;
-    const long at = 2 * ((long)band * pd.nG + g) + comp;
-    if (ST == ZF_H)
-      v += a.kin[(long)((a.batch0 + (int)band) / a.nb_per_k) * pd.nG + g] * reinterpret_cast<const double *>(a.psi)[at];
-    else v *= a.scale;
-    out[at] = v;
-  }
+  else if (g >= 0) out[2 * ((long)band * pd.nG + g) + comp] = ST == ZF_H ? v + x : v * a.scale;
 }
 
 __device__ __forceinline__ double scale2(double x, int n) {
@@ -215,7 +222,7 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
 
 // T 2^n rounded to FP64, n in -1000 .. 900.  `scaled` takes one conversion on the FP64 pipe and an
 // exponent addition; to_double stays on the integer pipes (three times the instructions), for the
-// density stage, whose squares and sums fill the FP64 pipe already.
+// x inverse, whose products with V or squares keep the FP64 pipe busy already.
 __device__ __forceinline__ double scaled(long long T, int n) {
   const double d = __ll2double_rn(T);
   return T == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (n << 20), __double2loint(d));
@@ -479,6 +486,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
       unit_info(u, l0, b0, inner);
       for (int it = 0; it < inner && ok; ++it, ++blk) {
         const int buf = (int)(blk & 1);
+        const unsigned per = period<ST>(a.pd);
+        double px[kEpiLines];
+        int pg[kEpiLines];
+        if ((ST == XI_V || ST == ZF || ST == ZF_H) && on) {
+          unsigned band = (l0 + c0) / per, rem = (l0 + c0) - band * per;
+#pragma unroll
+          for (int c = 0; c < kEpiLines; ++c) {
+            px[c] = 0.0;
+            pg[c] = -1;
+            if (l0 + c0 + c < a.lines) pre_at<ST>(a, band, rem, o, comp, px[c], pg[c]);
+            if (++rem == per) {
+              rem = 0;
+              ++band;
+            }
+          }
+        }
         ok = __all_sync(0xffffffffu, wait_bar(&accf[buf], (uint32_t)(blk / 2) & 1));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -506,7 +529,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
         if (lane == 0) arrive(&acce[buf]);   // the accumulator has been read
         if (!on) continue;
         const double wb = ST == XI_D ? a.wocc[b0 + it] : 0.0;
-        const unsigned per = period<ST>(a.pd);
         unsigned band = (l0 + c0) / per, rem = (l0 + c0) - band * per;
 #pragma unroll
         for (int c = 0; c < kEpiLines; ++c) {
@@ -518,11 +540,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
           }
           const int em = lex[blk % kLex][c0 + c], n = nbase + max(em, 1);
           double v;
-          if (n >= -1000 && n <= 900) v = ST == XI_D ? to_double(T[c], n) : scaled(T[c], n);
+          if (n >= -1000 && n <= 900) v = ST == XI_D || ST == XI_V ? to_double(T[c], n) : scaled(T[c], n);
           else v = scale2(scale2((double)T[c], n / 2), n - n / 2);
           if (em == 0x7ff) v = __longlong_as_double(0x7ff8000000000000ll);
           if (ST == XI_D) acc[c] = fma(wb * v, v, acc[c]);
-          else store_at<ST>(a, l, band, rem, o, comp, v);
+          else store_at<ST>(a, l, band, o, comp, v, px[c], pg[c]);
         }
       }
       if (ST == XI_D && ok) {   // Re^2 and Im^2 sit in different rows: [group][2][z][y][x]
