@@ -245,6 +245,8 @@ def vnl_apply(proj, dion, becp_, hpsi_inout):
     need = nk * P * nb * esz + 256
     if dt == F64:   # packed operands of the tensor-core form (32 B per element), in pieces beyond 384 MB
         need += min(384 << 20, 32 * nk * (P + 16) * (nG + nb + 256)) + 1024 + 4 * nk * (nG + nb)
+    elif P > 32:
+        need += 32 * nk * (P + 16) * (nb + nb // 2 + 96)
     w = workspace(need)
     check(LIB.addft_vnl_apply(dt, nk, nb, nG, P, _p(_c(proj, "proj")), _p(dion), _p(_c(becp_, "becp")),
                               _p(hpsi_inout), _p(w), w.numel(), _stream()), "vnl_apply")

@@ -723,24 +723,41 @@ addft_status launch_becp_tc(int nk, int nb, int nG, int nproj, int nsplit, int g
                             const float2 *psi, float2 *out, cudaStream_t st);
 addft_status launch_becp_f32(int nk, int nb, int nG, int nproj, int nsplit, int gchunk, const float2 *proj,
                              const float2 *psi, float2 *out, cudaStream_t st);
-// tc05.cu: split-TF32 becp on tcgen05 with a tensor-memory accumulator, same layout
-addft_status launch_becp_tc05(int nk, int nb, int nG, int nproj, int nsplit, int gchunk, const float2 *proj,
-                              const float2 *psi, float2 *out, cudaStream_t st);
+// tc05.cu: split-TF32 becp on tcgen05 with a tensor-memory accumulator, same partial layout, its tile
+void becp_tc05_tile(int nb, int nproj, int *pt, int *bt);
+addft_status launch_becp_tc05(int nk, int nb, int nG, int nproj, int nsplit, const float2 *proj, const float2 *psi,
+                              float2 *out, cudaStream_t st);
 
 // Kernel of the FP32 projector contractions, read once per process from ADDFT_BECP_TC /
 // ADDFT_APPLY_TC: 0 = register-tiled FP32 FMA, 1 = split-TF32 mma.sync tensor cores,
 // 2 = the generic SIMT kernels of this file, 3 = split-TF32 tcgen05 with a tensor-memory
-// accumulator.  Defaults (the fastest measured on the 72^3 microbench): becp 1 (the
-// tcgen05 becp has to transpose its operands through shared memory and is L1-bound),
-// apply 3.
+// accumulator (the default of both: the fastest and, its sums being taken out of the truncating
+// accumulators every 32 G, the most accurate.  becp, 1 against 3: 72^3 box, 64 bands x 32
+// projectors 60 -> 38 us, Si64 168 x 256 234 -> 84, 8 k points of Si2 8.2 -> 5.5; rms error 9.7e-7 -> 2.4e-7,
+// 3.3e-6 -> 2.6e-7, 3.0e-7 -> 1.9e-7).
 static int proj_mode(const char *var, int dflt) {
   const char *v = getenv(var);
   const int m = v ? atoi(v) : dflt;
   return m >= 0 && m <= 3 ? m : dflt;
 }
 static int becp_mode() {
-  static const int m = proj_mode("ADDFT_BECP_TC", 1);
+  static const int m = proj_mode("ADDFT_BECP_TC", 3);
   return m;
+}
+
+// K splits of the tcgen05 becp: the fewest waves of 32-G stages, each CTA about 6 stages' time on top
+static int becp_tc05_nsplit(int tiles, int nG) {
+  const int steps = (nG + 31) / 32;
+  int best = 1;
+  long least = 0;
+  for (int ns = 1; ns <= steps && (ns == 1 || (long)tiles * ns <= 2 * 152); ++ns) {
+    const long t = (((long)tiles * ns + 151) / 152) * ((steps + ns - 1) / ns + 6);
+    if (ns == 1 || t < least) {
+      least = t;
+      best = ns;
+    }
+  }
+  return best;
 }
 
 // CTAs per SM of split-K work for the tensor-core and register-tiled becp kernels
@@ -780,6 +797,11 @@ addft_status becp_t(int nk, int nb, int nG, int nproj, const void *proj, const v
   // the tensor-core and register-tiled forms hold 2 / 4 CTAs per SM: 4 per SM of work keeps
   // 1-2 waves of long K chunks
   int ns = pick_nsplit(tiles, nG, mode != 2 ? becp_ctas_per_sm() : 8);
+  if (mode == 3) {   // one CTA per SM
+    int pt, bt;
+    becp_tc05_tile(nb, nproj, &pt, &bt);
+    ns = std::min(ns, becp_tc05_nsplit(((nproj + pt - 1) / pt) * ((nb + bt - 1) / bt) * nk, nG));
+  }
   const size_t per = (size_t)nk * nproj * nb * sizeof(C);
   // partials (ns) + pass-1 group sums (ceil(ns / kSplitGroup)) must fit the work buffer
   while (ns > 1 && (work == nullptr || bytes < per * (size_t)(ns + split_groups(ns)))) --ns;
@@ -793,7 +815,7 @@ addft_status becp_t(int nk, int nb, int nG, int nproj, const void *proj, const v
   C *dst = ns > 1 ? (C *)work : (C *)becp;
   bool done = false;
   if constexpr (sizeof(R) == 4) {
-    if (tc) {
+    if (mode == 1) {
       ADDFT_TRY(launch_becp_tc(nk, nb, nG, nproj, ns, gchunk, (const float2 *)proj, (const float2 *)psi,
                                (float2 *)dst, st));
       done = true;
@@ -802,8 +824,7 @@ addft_status becp_t(int nk, int nb, int nG, int nproj, const void *proj, const v
                                 (float2 *)dst, st));
       done = true;
     } else if (mode == 3) {
-      ADDFT_TRY(launch_becp_tc05(nk, nb, nG, nproj, ns, gchunk, (const float2 *)proj, (const float2 *)psi,
-                                 (float2 *)dst, st));
+      ADDFT_TRY(launch_becp_tc05(nk, nb, nG, nproj, ns, (const float2 *)proj, (const float2 *)psi, (float2 *)dst, st));
       done = true;
     }
   }
@@ -839,20 +860,22 @@ addft_status launch_apply_tc(bool accum, const float2 *X, int xs_j, int xs_i, si
 addft_status launch_apply_f32(bool accum, const float2 *X, int xs_j, int xs_i, size_t xs_k, const float2 *A,
                               size_t as_k, int nk, int nj, int ni, int nG, float2 *out, size_t os_k,
                               cudaStream_t st);
-// tc05.cu: split-TF32 apply on tcgen05 with a tensor-memory accumulator
+// tc05.cu: split-TF32 apply on tcgen05 with a tensor-memory accumulator, the scratch it wants
 addft_status launch_apply_tc05(bool accum, const float2 *X, int xs_j, int xs_i, size_t xs_k, const float2 *A,
                                size_t as_k, int nk, int nj, int ni, int nG, float2 *out, size_t os_k,
-                               cudaStream_t st);
+                               void *work, size_t bytes, cudaStream_t st);
+size_t apply_tc05_bytes(int nk, int nj, int ni, int nG);
 
 static int apply_mode() {
   static const int m = proj_mode("ADDFT_APPLY_TC", 3);
   return m;
 }
 
-// scratch (work, bytes) serves the FP64 tensor-core form; without enough of it the SIMT kernel runs
+// scratch (work, bytes) serves the FP64 tensor-core form, without enough of it the SIMT kernel runs, and the
+// packed X of the FP32 one
 template <typename R>
 size_t apply_work_bytes(int nk, int nj, int ni, int nG) {
-  return sizeof(R) == 8 ? oz_work_bytes(8, ni, nG, nj, nk) : 0;
+  return sizeof(R) == 8 ? oz_work_bytes(8, ni, nG, nj, nk) : apply_tc05_bytes(nk, nj, ni, nG);
 }
 
 template <typename R, bool CONJ_A, bool ACCUM>
@@ -875,7 +898,7 @@ addft_status apply_t(const void *X, int xs_j, int xs_i, size_t xs_k, const void 
                               (float2 *)out, os_k, st);
     if (apply_mode() == 3)
       return launch_apply_tc05(ACCUM, (const float2 *)X, xs_j, xs_i, xs_k, (const float2 *)A, as_k, nk, nj, ni, nG,
-                               (float2 *)out, os_k, st);
+                               (float2 *)out, os_k, work, bytes, st);
   }
   const long ctas128 = (long)((nG + 127) / 128) * ((ni + kAI - 1) / kAI) * nk;
   if (ctas128 >= 4 * 152) {

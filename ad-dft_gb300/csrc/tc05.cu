@@ -5,10 +5,9 @@
 // 1e-6 relative, like the warp-MMA kernels.
 //
 //   becp[k][p][b] = sum_G conj(proj[k][p][G]) psi[k][b][G]          (nonlocal_op.py:67-70)
-//     D (128 x 32) = X (128 x K) P^T: rows of X are the 64 bands of a tile, then the
-//     same bands with each (re, im) pair replaced by (im, -re); columns of P are 32
-//     projectors; K runs over (G, re/im).  Row b of D is Re becp[.][b], row 64 + b
-//     is Im becp[.][b].  Split-K over G across CTAs, deterministic partials.
+//     D (128 x 2 NB) = P (128 x K) X^T: rows are hi and lo of 32 projectors and of the same
+//     with each (re, im) pair replaced by (-im, re), columns hi and lo of NB bands; K runs
+//     over (G, re/im).  Split-K over G across CTAs, deterministic partials.
 //   out[k][b][G] (+)= sum_p beta[k][p][G] DB[k][p][b]                 (nonlocal_op.py:73-76)
 //     D (128 x 128) = Bt (128 x K) Y^T: rows are 128 G of a tile, columns the real and
 //     imaginary parts of 64 bands; K runs over (projector, re/im).
@@ -22,7 +21,10 @@
 // Every mbarrier wait has an iteration limit: on expiry the kernel records an error
 // (read with addft_tc05_status), waits (bounded) for its own MMAs, frees its tensor
 // memory and returns.
+#include <algorithm>
+
 #include "common.cuh"
+#include "mma16.cuh"
 #include "ozgemm.cuh"
 
 namespace addft {
@@ -55,13 +57,23 @@ __device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t a, uint64_t b,
       : "memory");
 }
 
+// the same from the descriptors' lower words (start address, LBO), SBO = 128 B
+__device__ __forceinline__ void mma_tf32_lo(uint32_t dtmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
+  constexpr uint32_t hi = (128u >> 4) | (1u << 14);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %4};\n\tmov.b64 db, {%2, %4};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t}" ::"r"(dtmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "r"(acc)
+      : "memory");
+}
+
 __device__ __forceinline__ void commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar))
                : "memory");
 }
 
-__device__ __forceinline__ void bar_init(uint64_t *bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bar)));
+__device__ __forceinline__ void bar_init(uint64_t *bar, int count = 1) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(count));
 }
 
 // Bounded wait for the completion of the mbarrier phase with this parity; false on timeout.
@@ -100,6 +112,10 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
                : "memory");
 }
 
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+
 // byte offset of K-chunk kc (4 floats) of row r in a canonical tile of R rows, K = 8 per slice
 __device__ __forceinline__ uint32_t coff(int R, int r, int k4) {
   const int slice = k4 >> 1, kc = k4 & 1;
@@ -127,165 +143,239 @@ __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t ncols) {
 // ---------------------------------------------------------------------------
 // becp
 // ---------------------------------------------------------------------------
-constexpr int kBB = 64;            // bands per tile (rows 0..63 and 64..127 of X)
-constexpr int kBP = 32;            // projectors per tile (N)
-constexpr int kBGs = 16;           // G per stage (K = 32 floats = 4 MMA steps)
-constexpr int kXTile = 128 * 2 * kBGs * 4;   // bytes of one X tile (hi or lo): 16 KB
-constexpr int kPTile = kBP * 2 * kBGs * 4;   // bytes of one P tile: 4 KB
-constexpr int kStage = 2 * kXTile + 2 * kPTile;   // X hi, X lo, P hi, P lo
-constexpr size_t kBecpSmem = 2 * (size_t)kStage + 1024;   // two stages in shared memory, one in registers
-
+// A tile is 32 projectors x 16 RB bands over one chunk of G.  The M = 128 operand holds each
+// projector four times, as rows hi, lo, i hi, i lo (i x = (-Im x, Re x)), the N operand each band
+// twice, hi and lo; K is (G, re/im).  One MMA then gives every product of the split, lo lo included,
+// in accumulators of its own, and an element is split, exchanged and stored once per tile.
+//   Tensor memory adds with truncation, so an error grows with the number of MMAs in an accumulator (8:
+// 1.9e-7 rms of random becp, 16: 3.4e-7, 235: 4.5e-6).  Two sets of accumulators take turns, one
+// stage of 32 G (8 MMAs) each, and are added to FP32 sums in registers.
+//   A warp reads 256 contiguous bytes of a row; a lane splits its G and writes the halves of the
+// 16-byte chunks it shares with its neighbour.  The chunks of a row lie rows + 1 core-matrix rows
+// apart, so the 16 lanes of a shared-memory phase write 8 different bank groups.  16 warps convert and drain, one issues the MMAs; bounded waits.
+//   Bound by shared memory: the MMAs read A (4 KB) and B per K = 8 step at 90 to 110 B per cycle, beside the
+// operands' stores.
+constexpr int kBWarps = 16;
+constexpr int kBThreads = 32 * kBWarps + 32;
+template <int RB>
+struct BT {
+  static constexpr int NB = 16 * RB, N = 2 * NB;
+  static constexpr uint32_t kChunkA = 128 * 16 + 16, kChunkB = N * 16 + 16;   // bytes between 4-float K chunks
+  static constexpr uint32_t kA = 16 * kChunkA, kB = 16 * kChunkB, kStage = kA + kB;
+  static constexpr uint32_t kCols = 2 * N <= 64 ? 64 : 2 * N <= 128 ? 128 : 2 * N <= 256 ? 256 : 512;
+  static constexpr int kPitch = NB + 1;
+  static constexpr size_t kRed = (size_t)128 * kPitch * 4;
+  static constexpr size_t kSmem = 2 * kStage + 128;
+  static constexpr int kPre = RB <= 4 ? 2 : 1;          // stages of loads in registers
+  static constexpr int kQ = (NB / 8 + 3) / 4;           // 8-band groups per draining warp
+  static_assert(2 * N <= 512 && kSmem + 1024 <= 227 * 1024 && kRed <= kSmem, "tile");
+};
 }  // namespace
 
-__global__ void __launch_bounds__(128, 2)
+#define TC05_LD8(taddr, r)                                                                                   \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"                      \
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) \
+               : "r"(taddr))
+
+template <int RB>
+__global__ void __launch_bounds__(kBThreads, 1)
 k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int nb, int nG, int nproj, int nsplit,
-            int gchunk, float2 *__restrict__ out) {
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char *smem = smem_raw + ((1024 - (saddr(smem_raw) & 1023)) & 1023);
-  __shared__ __align__(8) uint64_t bars[2];
+            float2 *__restrict__ out) {
+  using T = BT<RB>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[2], accf[2], acce[2];   // operands written, MMAs done, sums taken
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int p0 = blockIdx.y * kBP, b0 = blockIdx.x * kBB;
+  const int p0 = blockIdx.y * 32, b0 = blockIdx.x * T::NB;
   const int nkz = gridDim.z / nsplit;
   const int k = blockIdx.z / nsplit, sp = blockIdx.z - k * nsplit;
-  const int ga = sp * gchunk, gb = min(nG, ga + gchunk);
-  const float2 *Pk = proj + (size_t)k * nproj * nG;
-  const float2 *Xk = psi + (size_t)k * nb * nG;
-  if (tid == 0) {
-    bar_init(&bars[0]);
-    bar_init(&bars[1]);
-  }
-  if (warp == 0) tmem_alloc(&tslot, 32);
+  // stages sp, sp + nsplit, ...: CTAs that run together read neighbouring G
+  const int nst = ((nG + 31) / 32 - sp + nsplit - 1) / nsplit;
+  if (tid == 0)
+    for (int i = 0; i < 2; ++i) {
+      bar_init(&full[i], kBWarps);
+      bar_init(&accf[i], 1);
+      bar_init(&acce[i], kBWarps);
+    }
+  if (warp == kBWarps) tmem_alloc(&tslot, T::kCols);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tslot;
-  const uint32_t idesc = idesc_tf32(128, kBP);
-  const int nst = (gb - ga + kBGs - 1) / kBGs;
-  // producer mapping: lane -> row rl = lane % 8 of an 8-row group and G quarter gq = lane / 8.
-  // A load instruction reads, per row, 4 consecutive G (32 B) from the 4 lanes rl, rl + 8,
-  // rl + 16, rl + 24: 8 rows x one sector.  The lanes of a pair (gq, gq ^ 1) swap their
-  // values, so both hold the two G of one 16-byte K chunk: the even lane writes the chunk,
-  // the odd lane its (im, -re) rotation (X) or its lo part (P).  Each group of 8
-  // consecutive lanes then writes 8 rows of one core matrix (128 contiguous bytes).
-  // X: row groups warp and warp + 4 (bands), P: warp.
-  const int rl = lane & 7, gq = lane >> 3, odd = gq & 1;
-  int xr[2];
-  bool xok[2];
-  const float2 *xs[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    xr[i] = 8 * (warp + 4 * i) + rl;
-    xok[i] = b0 + xr[i] < nb;
-    xs[i] = Xk + (size_t)(b0 + xr[i]) * nG;
-  }
-  const int pr = 8 * warp + rl;
-  const bool pok = p0 + pr < nproj;
-  const float2 *ps = Pk + (size_t)(p0 + pr) * nG;
-  float2 xv[2][4], pv[4];
-  auto load = [&](int s) {
-    const int g0 = ga + s * kBGs + gq;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const bool gin = g0 + 4 * j < gb;
-#pragma unroll
-      for (int i = 0; i < 2; ++i) xv[i][j] = (xok[i] && gin) ? xs[i][g0 + 4 * j] : make_float2(0.f, 0.f);
-      pv[j] = (pok && gin) ? ps[g0 + 4 * j] : make_float2(0.f, 0.f);
-    }
-  };
-  // (even, odd) G of this lane's pair
-  auto pair = [&](float2 v, float2 &e, float2 &o) {
-    float2 w;
-    w.x = __shfl_xor_sync(0xffffffffu, v.x, 8);
-    w.y = __shfl_xor_sync(0xffffffffu, v.y, 8);
-    e = odd ? w : v;
-    o = odd ? v : w;
-  };
+  const uint32_t tmem = tslot, sbase = saddr(smem);
   bool ok = true;
-  if (nst > 0) load(0);
-  for (int s = 0; s < nst && ok; ++s) {
-    const int buf = s & 1;
-    if (s >= 2) ok = __syncthreads_and(bar_wait(&bars[buf], ((s - 2) >> 1) & 1)) != 0;   // buffer free
-    if (!ok) break;
-    const uint32_t xhi = saddr(smem + buf * kStage), xlo = xhi + kXTile, phi = xhi + 2 * kXTile, plo = phi + kPTile;
+  float sum[T::kQ][8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {   // G 4 j .. 4 j + 3 of the stage: K chunks 2 j, 2 j + 1
-      const int k4 = 2 * j + (gq >> 1);
+  for (int c = 0; c < T::kQ; ++c)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        float2 e, o;
-        pair(xv[i][j], e, o);
-        float a[4];
-        if (odd) {   // (re, im) -> (im, -re), rows 64 + b
-          a[0] = e.y; a[1] = -e.x; a[2] = o.y; a[3] = -o.x;
-        } else {
-          a[0] = e.x; a[1] = e.y; a[2] = o.x; a[3] = o.y;
-        }
-        uint4 hi, lo;
-        split4(a, hi, lo);
-        const uint32_t off = coff(128, xr[i] + 64 * odd, k4);
-        sts128(xhi + off, hi);
-        sts128(xlo + off, lo);
+    for (int q = 0; q < 8; ++q) sum[c][q] = 0.f;
+
+  if (warp == kBWarps) {
+    const bool lead = elect_one();
+    constexpr uint32_t idesc = idesc_tf32(128, T::N);
+    const uint32_t a_lo = (sbase >> 4) | ((T::kChunkA >> 4) << 16);
+    const uint32_t b_lo = ((sbase + T::kA) >> 4) | ((T::kChunkB >> 4) << 16);
+    int s = 0;
+    for (; s < nst; ++s) {
+      const int j = s & 1;
+      ok = bar_wait(&full[j], (s >> 1) & 1);
+      if (ok && s >= 2) ok = bar_wait(&acce[j], ((s >> 1) - 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (lead) {
+        const uint32_t o = j * (T::kStage >> 4);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          mma_tf32_lo(tmem + j * T::N, a_lo + o + (2 * kk * T::kChunkA) / 16, b_lo + o + (2 * kk * T::kChunkB) / 16,
+                      idesc, kk > 0);
+        commit(&accf[j]);
       }
-      float2 e, o;
-      pair(pv[j], e, o);
-      float a[4] = {e.x, e.y, o.x, o.y};
-      uint4 hi, lo;
-      split4(a, hi, lo);
-      sts128((odd ? plo : phi) + coff(kBP, pr, k4), odd ? lo : hi);
+      __syncwarp();
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
+    if (!ok) {   // every MMA issued has to be done before tensor memory is given back
+      if (lead) atomicOr(&g_tc05_error, 1u);
+      for (int t = max(0, s - 2); t < s; ++t) bar_wait(&accf[t & 1], (t >> 1) & 1);
+    }
+  } else {
+    constexpr int NR = 2 + RB;   // rows of this warp: projectors warp, warp + 16, bands warp, warp + 16, ...
+    // rows past the end repeat the last one: they feed outputs that nobody stores
+    const float2 *Pk = proj + (size_t)k * nproj * nG, *Xk = psi + (size_t)k * nb * nG;
+    int row[NR];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) row[i] = min(p0 + warp + 16 * i, nproj - 1);
+#pragma unroll
+    for (int i = 0; i < RB; ++i) row[2 + i] = min(b0 + warp + 16 * i, nb - 1);
+    float2 v[T::kPre][NR];
+    auto load = [&](int s, float2 (&x)[NR]) {
+      // the last stage may be short: its lanes past the end read the last G and are cleared when written
+      const int g = min(32 * (sp + s * nsplit) + lane, nG - 1);
+#pragma unroll
+      for (int i = 0; i < NR; ++i) x[i] = (i < 2 ? Pk : Xk)[(long)row[i] * nG + g];
+    };
+    const uint32_t wa = sbase + (lane >> 1) * T::kChunkA + (lane & 1) * 8 + warp * 16;
+    const uint32_t wb = sbase + T::kA + (lane >> 1) * T::kChunkB + (lane & 1) * 8 + warp * 16;
+    // accumulators: part warp % 4 of the rows, 8-band groups warp / 4, warp / 4 + 4, ...
+    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 8 * (warp >> 2);
+    auto drain = [&](int j) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-      for (int kk = 0; kk < kBGs * 2 / 8; ++kk) {
-        const uint64_t xh_ = sdesc(xhi + kk * (128 / 8) * 256, 128, 256);
-        const uint64_t xl_ = sdesc(xlo + kk * (128 / 8) * 256, 128, 256);
-        const uint64_t ph_ = sdesc(phi + kk * (kBP / 8) * 256, 128, 256);
-        const uint64_t pl_ = sdesc(plo + kk * (kBP / 8) * 256, 128, 256);
-        mma_tf32(tmem, xh_, ph_, idesc, (s > 0 || kk > 0) ? 1u : 0u);
-        mma_tf32(tmem, xh_, pl_, idesc, 1u);
-        mma_tf32(tmem, xl_, ph_, idesc, 1u);
-      }
-      commit(&bars[buf]);
-    }
-    if (s + 1 < nst) load(s + 1);   // next stage's operands in flight while the MMAs run
-  }
-  // the commit of the last stage covers every MMA this CTA issued
-  bool fin = true;
-  if (nst > 0) fin = __syncthreads_and(bar_wait(&bars[(nst - 1) & 1], ((nst - 1) >> 1) & 1)) != 0;
-  const int row = 32 * warp + lane;
-  const int b = b0 + (row & 63);
-  float *o = reinterpret_cast<float *>(out + (((size_t)sp * nkz + k) * nproj + p0) * nb + b) + (row >> 6);
-  if (!ok || !fin) {
-    if (lane == 0) atomicOr(&g_tc05_error, 1u);
-  } else if (nst > 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    uint32_t rr[32];
-    TC05_LD32(tmem + ((uint32_t)(32 * warp) << 16), rr);
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    if (b < nb) {
+      for (int c = 0; c < T::kQ; ++c)
+        if (8 * (warp >> 2) + 32 * c < T::NB) {
+          uint32_t h[8], l[8];
+          TC05_LD8(tq + j * T::N + 32 * c, h);
+          TC05_LD8(tq + j * T::N + T::NB + 32 * c, l);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int j = 0; j < kBP; ++j)
-        if (p0 + j < nproj) o[(size_t)j * nb * 2] = __uint_as_float(rr[j]);
+          for (int q = 0; q < 8; ++q) sum[c][q] += __uint_as_float(h[q]) + __uint_as_float(l[q]);
+        }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&acce[j])) : "memory");
+    };
+    auto stage = [&](int s, float2 (&x)[NR]) {
+      const int j = s & 1;
+      if (s >= 2) {   // MMAs of stage s - 2: its operands' room and its accumulators
+        ok = bar_wait(&accf[j], ((s >> 1) - 1) & 1);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return;
+      }
+      const uint32_t o = j * T::kStage;
+      if (32 * (sp + s * nsplit) + lane >= nG) {
+#pragma unroll
+        for (int i = 0; i < NR; ++i) x[i] = make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < NR; ++i) {
+        const uint32_t hx = tf32_rna(x[i].x), hy = tf32_rna(x[i].y);
+        const uint32_t lx = tf32_rna(x[i].x - __uint_as_float(hx)), ly = tf32_rna(x[i].y - __uint_as_float(hy));
+        if (i < 2) {   // rows hi, lo, i hi, i lo of 32 each
+          const uint32_t d = wa + o + i * 256;
+          sts64(d, hx, hy);
+          sts64(d + 512, lx, ly);
+          sts64(d + 1024, hy ^ 0x80000000u, hx);
+          sts64(d + 1536, ly ^ 0x80000000u, lx);
+        } else {
+          const uint32_t d = wb + o + (i - 2) * 256;
+          sts64(d, hx, hy);
+          sts64(d + T::NB * 16, lx, ly);
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&full[j])) : "memory");
+      if (s + T::kPre < nst) load(s + T::kPre, x);
+      if (s >= 2) drain(j);
+    };
+#pragma unroll
+    for (int i = 0; i < T::kPre; ++i)
+      if (i < nst) load(i, v[i]);
+    for (int s = 0; s < nst && ok; s += T::kPre)
+#pragma unroll
+      for (int i = 0; i < T::kPre; ++i)
+        if (ok && s + i < nst) stage(s + i, v[i]);
+    for (int s = max(0, nst - 2); s < nst && ok; ++s) {
+      ok = bar_wait(&accf[s & 1], (s >> 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) drain(s & 1);
     }
-  } else if (b < nb) {
-    for (int j = 0; j < kBP; ++j)
-      if (p0 + j < nproj) o[(size_t)j * nb * 2] = 0.f;
+    if (!ok && lane == 0) atomicOr(&g_tc05_error, 1u);
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  ok = __syncthreads_and(ok) != 0;
+  float *red = reinterpret_cast<float *>(smem);   // [part][projector][band]
+  if (ok && warp < kBWarps) {
+    float *r = red + (32 * (warp & 3) + lane) * T::kPitch + 8 * (warp >> 2);
+#pragma unroll
+    for (int c = 0; c < T::kQ; ++c)
+      if (8 * (warp >> 2) + 32 * c < T::NB)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) r[32 * c + q] = sum[c][q];
+  }
   __syncthreads();
-  if (warp == 0) tmem_free(tmem, 32);
+  if (warp == kBWarps) {
+    tmem_free(tmem, T::kCols);
+    return;
+  }
+  if (!ok) return;
+  float2 *dst = out + ((size_t)sp * nkz + k) * nproj * nb;
+  for (int e = tid; e < 32 * T::NB; e += 32 * kBWarps) {
+    const int p = e / T::NB, b = e - p * T::NB;
+    if (p0 + p >= nproj || b0 + b >= nb) continue;
+    const float *r = red + p * T::kPitch + b;
+    constexpr int q = 32 * T::kPitch;
+    dst[(size_t)(p0 + p) * nb + b0 + b] = make_float2(r[0] + r[q], r[2 * q] + r[3 * q]);
+  }
 }
 
-addft_status launch_becp_tc05(int nk, int nb, int nG, int nproj, int nsplit, int gchunk, const float2 *proj,
-                              const float2 *psi, float2 *out, cudaStream_t st) {
-  ADDFT_TRY(smem_optin(k_becp_tc05, kBecpSmem));
-  dim3 grid((nb + kBB - 1) / kBB, (nproj + kBP - 1) / kBP, nk * nsplit);
-  k_becp_tc05<<<grid, 128, kBecpSmem, st>>>(proj, psi, nb, nG, nproj, nsplit, gchunk, out);
+// Tile of a problem: 32 projectors, equal tiles of up to kMost bands.
+void becp_tc05_tile(int nb, int nproj, int *pt, int *bt) {
+  constexpr int kMost = 96;
+  const int n = (nb + kMost - 1) / kMost;
+  *pt = 32;
+  *bt = ((nb + n - 1) / n + 15) / 16 * 16;
+  (void)nproj;
+}
+
+template <int RB>
+static addft_status becp_go(dim3 grid, int nb, int nG, int nproj, int nsplit, const float2 *proj, const float2 *psi,
+                            float2 *out, cudaStream_t st) {
+  ADDFT_TRY(smem_optin(k_becp_tc05<RB>, BT<RB>::kSmem));
+  k_becp_tc05<RB><<<grid, kBThreads, BT<RB>::kSmem, st>>>(proj, psi, nb, nG, nproj, nsplit, out);
   return check_launch("k_becp_tc05");
+}
+
+addft_status launch_becp_tc05(int nk, int nb, int nG, int nproj, int nsplit, const float2 *proj, const float2 *psi,
+                              float2 *out, cudaStream_t st) {
+  int pt, bt;
+  becp_tc05_tile(nb, nproj, &pt, &bt);
+  const dim3 grid((nb + bt - 1) / bt, (nproj + pt - 1) / pt, nk * nsplit);
+  switch (bt / 16) {
+#define BECP_CASE(rb) \
+  case rb: return becp_go<rb>(grid, nb, nG, nproj, nsplit, proj, psi, out, st);
+    BECP_CASE(1) BECP_CASE(2) BECP_CASE(3) BECP_CASE(4) BECP_CASE(5) BECP_CASE(6)
+#undef BECP_CASE
+  }
+  return ADDFT_INVALID_ARG;
 }
 
 // ---------------------------------------------------------------------------
@@ -433,13 +523,311 @@ k_apply_tc05(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, cons
   if (warp == 0) tmem_free(tmem, 128);
 }
 
+// ---------------------------------------------------------------------------
+// apply with more than one chunk of projectors
+// ---------------------------------------------------------------------------
+// k_deep_pack writes X, split and in operand layout, to scratch once.  A unit is 128 G x NB bands; K
+// runs over all projectors in stages of 16.  16 warps split A (a lane holds one G and two
+// projectors: coalesced loads, one 16-byte chunk, 8 lanes fill a core matrix), one lane copies X's
+// stages, one warp issues the MMAs (three of N = 2 NB per K = 8 step).  Two sets of accumulators take
+// turns, two stages each, and are added to FP32 sums in registers (tensor memory adds with
+// truncation); a unit's sums are added to `out` while the next unit's first stages run.  Bounded
+// waits.  Bound by shared memory (the MMAs' operands and the stores of them).
+namespace {
+constexpr int kDJ = 16;                                  // projectors per stage
+template <int NB>
+struct DT {
+  static constexpr int N = 2 * NB, kG = NB / 32;         // columns (re, im), band groups of 32 lanes
+  static constexpr uint32_t kChunkA = 128 * 16, kChunkB = N * 16, kA = kDJ / 2 * kChunkA, kB = kDJ / 2 * kChunkB;
+  static constexpr uint32_t kStage = 2 * kA + 2 * kB;    // A hi, A lo, B hi, B lo
+  static constexpr uint32_t kCols = 2 * N <= 128 ? 128 : 2 * N <= 256 ? 256 : 512;
+  static constexpr size_t kSmem = 2 * kStage + 128;
+};
+}  // namespace
+
+// X of (k, band tile, stage): B hi, then B lo; zeros past the last projector and band
+template <int NB>
+__global__ void k_deep_pack(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, int nj, int ni, int nst,
+                            int nbt, unsigned char *__restrict__ out) {
+  using T = DT<NB>;
+  const int b = threadIdx.x, q = blockIdx.x, bt = blockIdx.y, k = blockIdx.z;   // q: pair of projectors
+  const float2 *Xk = X + (size_t)k * xs_k + (size_t)(bt * NB + b) * xs_i;
+  float x[4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float2 v = 2 * q + h < nj && bt * NB + b < ni ? Xk[(size_t)(2 * q + h) * xs_j] : make_float2(0.f, 0.f);
+    x[2 * h] = v.x;
+    x[2 * h + 1] = v.y;
+  }
+  uint4 hi, lo;
+  split4(x, hi, lo);
+  constexpr uint32_t m = 0x80000000u;
+  const int s = q / (kDJ / 2), c = q - s * (kDJ / 2);
+  unsigned char *o = out + (((size_t)k * nbt + bt) * nst + s) * (2 * T::kB) + c * T::kChunkB + b * 16;
+  *(uint4 *)o = make_uint4(hi.x, hi.y ^ m, hi.z, hi.w ^ m);                     // re: (re, -im)
+  *(uint4 *)(o + T::kB) = make_uint4(lo.x, lo.y ^ m, lo.z, lo.w ^ m);
+  *(uint4 *)(o + NB * 16) = make_uint4(hi.y, hi.x, hi.w, hi.z);                 // im: (im, re)
+  *(uint4 *)(o + NB * 16 + T::kB) = make_uint4(lo.y, lo.x, lo.w, lo.z);
+}
+
+template <int NB, bool ACCUM>
+__global__ void __launch_bounds__(kBThreads + 32, 1)
+k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, size_t as_k, int nk, int nj, int ni, int nG, float2 *__restrict__ out, size_t os_k) {
+  using T = DT<NB>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[2], free_[2], accf[2], acce[2];
+  __shared__ uint32_t tslot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ntile = (nG + 127) / 128, nbt = (ni + NB - 1) / NB, units = ntile * nbt * nk;
+  const int nst = (nj + kDJ - 1) / kDJ;
+  if (tid == 0)
+    for (int i = 0; i < 2; ++i) {
+      bar_init(&full[i], kBWarps + 1);
+      bar_init(&free_[i], 1);
+      bar_init(&accf[i], 1);
+      bar_init(&acce[i], kBWarps);
+    }
+  if (warp == kBWarps) tmem_alloc(&tslot, T::kCols);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tslot, sbase = saddr(smem);
+  bool ok = true;
+
+  if (warp == kBWarps) {
+    const bool lead = elect_one();
+    constexpr uint32_t idesc = idesc_tf32(128, T::N);
+    const uint32_t a_lo = (sbase >> 4) | ((T::kChunkA >> 4) << 16);
+    const uint32_t b_lo = ((sbase + 2 * T::kA) >> 4) | ((T::kChunkB >> 4) << 16);
+    int it = 0, bl = 0;
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x)
+      for (int s = 0; s < nst && ok; ++s) {
+        const int j = it & 1, set = bl & 1;
+        const bool first = (s & 1) == 0, last = (s & 1) || s == nst - 1;
+        ok = bar_wait(&full[j], (it >> 1) & 1);
+        if (ok && first && bl >= 2) ok = bar_wait(&acce[set], ((bl >> 1) - 1) & 1);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (lead) {
+          const uint32_t ah = a_lo + j * (T::kStage >> 4), al = ah + (T::kA >> 4);
+          const uint32_t bh = b_lo + j * (T::kStage >> 4), bl_ = bh + (T::kB >> 4), d = tmem + set * T::N;
+#pragma unroll
+          for (int kk = 0; kk < kDJ / 4; ++kk) {
+            const uint32_t oa = 2 * kk * T::kChunkA / 16, ob = 2 * kk * T::kChunkB / 16;
+            mma_tf32_lo(d, ah + oa, bh + ob, idesc, !first || kk > 0);
+            mma_tf32_lo(d, ah + oa, bl_ + ob, idesc, 1u);
+            mma_tf32_lo(d, al + oa, bh + ob, idesc, 1u);
+          }
+          commit(&free_[j]);
+          if (last) commit(&accf[set]);
+        }
+        __syncwarp();
+        ++it;
+        if (last) ++bl;
+      }
+    if (!ok) {   // every MMA issued has to be done before tensor memory is given back
+      if (lead) atomicOr(&g_tc05_error, 1u);
+      for (int t = max(0, it - 2); t < it; ++t) bar_wait(&free_[t & 1], (t >> 1) & 1);
+    }
+  } else if (warp == kBWarps + 1) {
+    if (lane == 0) {   // X
+      int it = 0;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const int bt = u % nbt, k = u / nbt / ntile;
+        const unsigned char *src = X + ((size_t)k * nbt + bt) * nst * (2 * T::kB);
+        for (int s = 0; s < nst && ok; ++s, ++it) {
+          const int j = it & 1;
+          if (it >= 2) ok = bar_wait(&free_[j], ((it >> 1) - 1) & 1);
+          if (!ok) break;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(&full[j])), "r"(2 * T::kB)
+                       : "memory");
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                  sbase + j * T::kStage + 2 * T::kA),
+              "l"(src + (size_t)s * (2 * T::kB)), "r"(2 * T::kB), "r"(saddr(&full[j]))
+              : "memory");
+        }
+      }
+      // nothing may still be landing in shared memory when the CTA ends
+      for (int t = max(0, it - 2); t < it; ++t) ok = bar_wait(&full[t & 1], (t >> 1) & 1) && ok;
+      if (!ok) atomicOr(&g_tc05_error, 1u);
+    }
+  } else {
+    // two projectors of this lane's G, two stages ahead; tasks: pair t / 4, G group t % 4 of t = warp, warp + 16
+    float2 v0[2][2], v1[2][2];
+    int lu = blockIdx.x, ls = 0;   // unit and stage of the next load
+    const float2 *lp = nullptr;
+    auto load = [&](float2 (&x)[2][2]) __attribute__((always_inline)) {
+      if (lu >= units) return;
+      if (ls == 0) {
+        const int t = lu / nbt, k = t / ntile;
+        lp = A + (size_t)k * as_k + min((t - k * ntile) * 128 + 32 * (warp & 3) + lane, nG - 1);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int jj = ls * kDJ + 2 * ((warp + 16 * i) >> 2);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) x[i][h] = jj + h < nj ? lp[(size_t)(jj + h) * nG] : make_float2(0.f, 0.f);
+      }
+      if (++ls == nst) {
+        ls = 0;
+        lu += gridDim.x;
+      }
+    };
+    auto put = [&](int j, const float2 (&y)[2][2]) __attribute__((always_inline)) {
+      const uint32_t o = sbase + j * T::kStage;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float x[4] = {y[i][0].x, y[i][0].y, y[i][1].x, y[i][1].y};
+        uint4 hi, lo;
+        split4(x, hi, lo);
+        const uint32_t d = o + ((warp + 16 * i) >> 2) * T::kChunkA + (32 * (warp & 3) + lane) * 16;
+        sts128(d, hi);
+        sts128(d + T::kA, lo);
+      }
+    };
+    // sums: G rows 32 (warp % 4) + lane, bands 8 (warp / 4) + 32 c + q
+    float re[T::kG][8], im[T::kG][8];
+    auto clear = [&]() __attribute__((always_inline)) {
+#pragma unroll
+      for (int c = 0; c < T::kG; ++c)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) re[c][q] = im[c][q] = 0.f;
+    };
+    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 8 * (warp >> 2);
+    auto drain = [&](int b) __attribute__((always_inline)) {   // block b
+      const int set = b & 1;
+      ok = bar_wait(&accf[set], (b >> 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) return;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < T::kG; ++c) {
+        uint32_t x[8], y[8];
+        TC05_LD8(tq + set * T::N + 32 * c, x);
+        TC05_LD8(tq + set * T::N + NB + 32 * c, y);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          re[c][q] += __uint_as_float(x[q]);
+          im[c][q] += __uint_as_float(y[q]);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&acce[set])) : "memory");
+    };
+    auto finish = [&](int u) __attribute__((always_inline)) {
+      const int bt = u % nbt, t = u / nbt, k = t / ntile;
+      const int g = (t - k * ntile) * 128 + 32 * (warp & 3) + lane, b0 = bt * NB + 8 * (warp >> 2);
+      float2 *o = out + (size_t)k * os_k + g;
+#pragma unroll
+      for (int c = 0; c < T::kG; ++c)
+#pragma unroll
+        for (int r = 0; r < 8; r += 4) {
+          float2 w[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int b = b0 + 32 * c + r + q;
+            w[q] = ACCUM && g < nG && b < ni ? o[(size_t)b * nG] : make_float2(0.f, 0.f);
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int b = b0 + 32 * c + r + q;
+            if (g < nG && b < ni) o[(size_t)b * nG] = make_float2(re[c][r + q] + w[q].x, im[c][r + q] + w[q].y);
+          }
+        }
+      clear();
+    };
+    clear();
+    int it = 0, bl = 0, s = 0, u = blockIdx.x;
+    load(v0);
+    load(v1);
+    auto stage = [&](float2 (&x)[2][2]) __attribute__((always_inline)) {
+      const int j = it & 1;
+      if (it >= 2) ok = bar_wait(&free_[j], ((it >> 1) - 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) return;
+      put(j, x);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&full[j])) : "memory");
+      load(x);
+      ++it;
+      if ((s & 1) || s == nst - 1) {   // end of block bl: take the one before, a unit's last one with its store
+        if (bl > 0) drain(bl - 1);
+        if (ok && bl > 0 && s < 2) finish(u - gridDim.x);
+        ++bl;
+      }
+      if (++s == nst) {
+        s = 0;
+        u += gridDim.x;
+      }
+    };
+    while (ok && u < units) {
+      stage(v0);
+      if (ok && u < units) stage(v1);
+    }
+    if (ok && bl > 0) {
+      drain(bl - 1);
+      if (ok) finish(u - gridDim.x);
+    }
+    if (!ok && lane == 0) atomicOr(&g_tc05_error, 1u);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == kBWarps) tmem_free(tmem, T::kCols);
+}
+
+static int deep_nb(int ni) {   // equal tiles of up to 96 bands, in whole warps
+  const int nbt = (ni + 95) / 96;
+  return ((ni + nbt - 1) / nbt + 31) / 32 * 32;
+}
+
+// Scratch of the packed X; 0 where k_apply_tc05 runs.  That one keeps up to 32 projectors of X in shared
+// memory for all its G, and without packing it is quicker below about 3 stages per SM (ncu, one-chunk kernel
+// against packing + this one: 40 bands x 64 projectors x 6000 G, 188 stages: 11.2 / 12.8 us;
+// 64 x 36 x 20000, 471: 18.7 / 17.4; 80 x 128 x 12000, 752: 30.7 / 19.5; 64 x 64 x 142800: 68.5 / 60.3; 96 x 40 x
+// 190000: 152 / 95; Si64, 168 x 256 x 23847: 152 / 71; rms error there 3.7e-6 / 6.0e-7).
+size_t apply_tc05_bytes(int nk, int nj, int ni, int nG) {
+  if (nj <= kAJ) return 0;
+  const int nb = deep_nb(ni);
+  const long units = (long)((nG + 127) / 128) * ((ni + nb - 1) / nb) * nk;
+  if (units * ((nj + kDJ - 1) / kDJ) < 3 * 152) return 0;
+  return (size_t)nk * ((ni + nb - 1) / nb) * ((nj + kDJ - 1) / kDJ) * (32 * kDJ * nb);
+}
+
+template <int NB, bool ACCUM>
+static addft_status apply_deep_go(int nsm, const float2 *X, int xs_j, int xs_i, size_t xs_k, const float2 *A, size_t as_k,
+                                  int nk, int nj, int ni, int nG, float2 *out, size_t os_k, void *work, cudaStream_t st) {
+  const int nst = (nj + kDJ - 1) / kDJ, nbt = (ni + NB - 1) / NB;
+  k_deep_pack<NB><<<dim3(nst * kDJ / 2, nbt, nk), NB, 0, st>>>(X, xs_j, xs_i, xs_k, nj, ni, nst, nbt, (unsigned char *)work);
+  ADDFT_TRY(check_launch("k_deep_pack"));
+  const long units = (long)((nG + 127) / 128) * ((ni + NB - 1) / NB) * nk;
+  ADDFT_TRY(smem_optin(k_apply_deep<NB, ACCUM>, DT<NB>::kSmem));
+  k_apply_deep<NB, ACCUM><<<(int)std::min<long>(units, nsm), kBThreads + 32, DT<NB>::kSmem, st>>>(
+      (const unsigned char *)work, A, as_k, nk, nj, ni, nG, out, os_k);
+  return check_launch("k_apply_deep");
+}
+
 addft_status launch_apply_tc05(bool accum, const float2 *X, int xs_j, int xs_i, size_t xs_k, const float2 *A,
                                size_t as_k, int nk, int nj, int ni, int nG, float2 *out, size_t os_k,
-                               cudaStream_t st) {
-  ADDFT_TRY(smem_optin(accum ? k_apply_tc05<true> : k_apply_tc05<false>, kApplySmem));
+                               void *work, size_t bytes, cudaStream_t st) {
   int dev = 0, nsm = 0;
   ADDFT_CUDA(cudaGetDevice(&dev));
   ADDFT_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const size_t need = apply_tc05_bytes(nk, nj, ni, nG);
+  if (need > 0 && work && ((uintptr_t)work & 15) == 0 && bytes >= need) {
+    const int nb = deep_nb(ni) / 32;
+#define DEEP(c, a) \
+  if (nb == c && accum == a) \
+    return apply_deep_go<32 * c, a>(nsm, X, xs_j, xs_i, xs_k, A, as_k, nk, nj, ni, nG, out, os_k, work, st);
+    DEEP(1, true) DEEP(2, true) DEEP(3, true) DEEP(1, false) DEEP(2, false) DEEP(3, false)
+#undef DEEP
+  }
+  ADDFT_TRY(smem_optin(accum ? k_apply_tc05<true> : k_apply_tc05<false>, kApplySmem));
   const int nbt = (ni + kAB - 1) / kAB, ntile = (nG + kAG - 1) / kAG;
   int gx = (nsm + nbt * nk - 1) / (nbt * nk);   // about one CTA per SM over the whole grid
   if (gx > ntile) gx = ntile;
