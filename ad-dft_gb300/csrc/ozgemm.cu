@@ -34,9 +34,9 @@
 // MMA time bounds it: 32 MMAs per 16 k, about 2,500 cycles for 128 x 32 x 16 complex products
 // (the narrow ones wait for shared-memory operands, 4 KB per slice of A), a ceiling near
 // 64 TFLOP/s of complex FP64 work on 152 SMs.  Measured with the passes over the operands:
-//   becp, P 256, 160 bands, nG 23,847   14.34 ms (FP64 SIMT)        -> 0.43 ms
-//   apply of the same size              12.02 ms (FP64 SIMT)        -> 0.51 ms
-//   conj(X) Y^T, 168 x 336 x 23,847      3.33 ms (double-float SIMT) -> 0.61 ms
+//   becp, P 256, 160 bands, nG 23,847   14.34 ms (FP64 SIMT)        -> 0.37 ms
+//   apply of the same size              12.02 ms (FP64 SIMT)        -> 0.45 ms
+//   conj(X) Y^T, 168 x 336 x 23,847      3.33 ms (double-float SIMT) -> 0.45 ms
 #include <algorithm>
 
 #include "common.cuh"

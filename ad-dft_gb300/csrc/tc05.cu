@@ -1,8 +1,8 @@
 // FP32 projector contractions of V_NL psi on the 5th-generation tensor cores
 // (tcgen05.mma kind::tf32, accumulators in tensor memory), split-precision TF32:
-// every product a b is formed as hi(a) hi(b) + hi(a) lo(b) + lo(a) hi(b) with
-// FP32 accumulation (hi = round-to-nearest TF32 of x, lo = TF32 of x - hi), about
-// 1e-6 relative, like the warp-MMA kernels.
+// every product a b is formed as hi(a) hi(b) + hi(a) lo(b) + lo(a) hi(b) (becp: + lo(a) lo(b))
+// with FP32 accumulation (hi = round-to-nearest TF32 of x, lo = TF32 of x - hi); 2e-7 to
+// 6e-7 relative on random operands.
 //
 //   becp[k][p][b] = sum_G conj(proj[k][p][G]) psi[k][b][G]          (nonlocal_op.py:67-70)
 //     D (128 x 2 NB) = P (128 x K) X^T: rows are hi and lo of 32 projectors and of the same
@@ -13,9 +13,9 @@
 //     imaginary parts of 64 bands; K runs over (projector, re/im).
 //
 // Operands are written by the CTA's threads into shared memory in the canonical
-// no-swizzle K-major layout (8-row x 16-byte core matrices; LBO = 128 B between the
-// two core matrices of one K = 8 step, SBO = 256 B between 8-row groups), since the
-// hi/lo split has to happen in registers on the way.  One thread issues the MMAs; a
+// no-swizzle K-major layout (8-row x 16-byte core matrices; in the one-chunk apply
+// LBO = 128 B between the two core matrices of one K = 8 step, SBO = 256 B between 8-row
+// groups), since the hi/lo split has to happen in registers on the way.  One thread issues the MMAs; a
 // commit to an mbarrier tells the producers when the operand buffer is free again, and
 // the next step's global loads are in flight (in registers) while the MMAs run.
 // Every mbarrier wait has an iteration limit: on expiry the kernel records an error
@@ -153,8 +153,11 @@ __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t ncols) {
 //   A warp reads 256 contiguous bytes of a row; a lane splits its G and writes the halves of the
 // 16-byte chunks it shares with its neighbour.  The chunks of a row lie rows + 1 core-matrix rows
 // apart, so the 16 lanes of a shared-memory phase write 8 different bank groups.  16 warps convert and drain, one issues the MMAs; bounded waits.
-//   Bound by shared memory: the MMAs read A (4 KB) and B per K = 8 step at 90 to 110 B per cycle, beside the
-// operands' stores.
+//   Bound by shared memory (the MMAs read A, 4 KB, and B per K = 8 step at 90 to 110 B per cycle, beside the
+// operands' stores) with few projectors by the loads' latency: 168 bands x 256 projectors x 23,847 G 234
+// us (mma.sync) -> 84, 64 x 32 x 142,609 60 -> 38 (23 with the loads taken out).  Keeping 4 stages of
+// loads in flight, in registers or with cp.async, was no quicker (43, 39 us), nor were tiles of 64 projectors
+// with one set of accumulators (85 us with its sums, and 6e-6 rms).
 constexpr int kBWarps = 16;
 constexpr int kBThreads = 32 * kBWarps + 32;
 template <int RB>
@@ -532,7 +535,8 @@ k_apply_tc05(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, cons
 // stages, one warp issues the MMAs (three of N = 2 NB per K = 8 step).  Two sets of accumulators take
 // turns, two stages each, and are added to FP32 sums in registers (tensor memory adds with
 // truncation); a unit's sums are added to `out` while the next unit's first stages run.  Bounded
-// waits.  Bound by shared memory (the MMAs' operands and the stores of them).
+// waits.  Bound by shared memory (the MMAs' operands and the stores of them): 168 bands x 256
+// projectors x 23,847 G 152 -> 68 us; splitting X in every tile instead of once cost 140.
 namespace {
 constexpr int kDJ = 16;                                  // projectors per stage
 template <int NB>

@@ -112,11 +112,13 @@ addft_status addft_plan_info(addft_plan plan, int *nplanes, int *ncols, int *nG)
  *   "threads_plane", "threads_x"  threads per CTA of the generic plane / x-line
  *                                 kernels (multiple of 32 in [64, 512]);
  *   "xtile_kb"                    shared memory of a generic x-line tile [8, 200];
- *   "slab_mb"                     slab bytes per band chunk (bands in flight);
+ *   "slab_mb"                     slab bytes per band chunk (bands in flight) of the FFT kernels;
  *   "xline2", "plane2"            1: two-pass register kernels where instantiated;
  *   "threads_plane2"              threads per CTA of the two-pass plane kernels;
  *   "colfft"                      1: H psi through the column pipeline (z-column FFTs,
- *                                 fused xy-plane FFT with V(r)) where instantiated;
+ *                                 fused xy-plane FFT with V(r)) where instantiated, FP64
+ *                                 transforms as products on the tensor cores where the
+ *                                 scratch holds them (0, or plane_split: FFT kernels);
  *                                 2: the same pipeline as one persistent kernel whose
  *                                 CTAs take work items (z-column groups, xy-planes)
  *                                 band by band (FP32, cubic boxes; else as 1);
@@ -243,9 +245,9 @@ addft_status addft_kerker(addft_plan full_plan, const double *bvec_host, const d
 size_t addft_kerker_work_bytes(addft_plan full_plan);
 
 /* ---- a15: FP64 subspace products of the eigensolver (solver/davidson.py:48, :51-52, :59-61:
- * the projections q^H hq and the rotations q u, hq u), computed in double-float arithmetic on the
- * FP32 pipes (~1e-14 relative; operands split into FP32 hi/lo pairs, exact products,
- * compensated sums).  C (M x N, row stride ldc) = op(A) op(B) with
+ * the projections q^H hq and the rotations q u, hq u), to ~1e-15 relative as exact digit products
+ * on the tensor cores (55 bits below each row's and column's largest component), or, where work holds
+ * less than that wants, in double-float arithmetic on the FP32 pipes (~1e-14).  C (M x N, row stride ldc) = op(A) op(B) with
  *   op(A)[i][k] = A[i*sAi + k*sAk], conjugated when conjA != 0,
  *   op(B)[k][j] = B[k*sBk + j*sBj], conjugated when conjB != 0;
  * all complex128, strides in elements.  K is split across CTAs when work holds
@@ -302,7 +304,7 @@ size_t addft_ewald_work_bytes(int nat);
  * `stream`, and returns its rate (host *tflops) and CUDA-event time (host *ms).
  * sink: device scratch of >= 2 KB (never read).  Synchronises with the stream. */
 addft_status addft_peak_flops(int which, int iters, double *tflops, float *ms, void *sink, void *stream);
-/* Device-side error bits of the tcgen05 projector kernels since the last call (bit 0: a
+/* Device-side error bits of the tcgen05 kernels (projectors, FP64 products and transforms) since the last call (bit 0: a
  * bounded wait for tensor-core completion ran out; the kernel then returned without
  * results), cleared by the read; synchronises with the device.  Diagnostic, no
  * counterpart in the reference. */
