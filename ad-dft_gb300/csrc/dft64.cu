@@ -687,15 +687,17 @@ bool d64_handles(const PlanDev &pd, int nbatch) {
   for (int a = 0; a < 6; ++a)
     if (pd.d64[a].tiles == 0) return false;
   // Six launches of 11 to 14 us (H psi) that load F first, against 45 to 76 us of the FFT kernels in small
-  // calls, which cost 600 to 700 us per 10^6 band-points below 20 points an axis and 160 to 220 above,
-  // the products 200 and 90 to 180.  H psi, FFT / products, us: 12^3 x 16 bands 46 / 68, x 32 79 / 68; 15^3 x 8 76 /
-  // 68, x 64 222 / 102; 16^3 x 8 56 / 68, x 16 72 / 68; 24^3 x 16 70 / 97, x 32 109 / 126 (density 89 / 79), x 64 181
-  // / 187 (150 / 120); 30^3 x 8 81 / 88, x 16 134 / 107; 36^3 x 4 68 / 89, x 8 109 / 110 (93 / 66); 45^3 x 1 100 / 83,
-  // 48^3 x 1 99 / 83, x 32 726 / 381; 75^3 x 1 238 / 147, x 8 963 / 608.
+  // calls.  The FFT kernels' time follows the active planes (np n2 n3 points a band), below 20 points an axis
+  // at 600 to 700 us per 10^6 of them, above at 160 to 220; the products take 200 and 90 to 180.  H psi, FFT
+  // / products, us, spheres of 0.45 n: 12^3 x 16 bands 46 / 68, x 64 112 / 89; 15^3 x 8 76 / 68, x 64 222 /
+  // 102; 16^3 x 8 56 / 68, x 16 72 / 68, x 32 129 / 90; 24^3 x 16 70 / 97, x 32 109 / 126 (density 89 / 79), x
+  // 64 181 / 187 (150 / 120); 30^3 x 8 81 / 88, x 16 134 / 107; 36^3 x 4 68 / 89, x 8 109 / 110 (93 / 66); 45^3 x
+  // 1 100 / 83, 48^3 x 1 99 / 83, x 32 726 / 381; 75^3 x 1 238 / 147, x 8 963 / 608.  Density of Si2's 24 bands
+  // (18^3, a sphere of a quarter): 35 / 55.
   const int n = std::max(pd.n1, std::max(pd.n2, pd.n3));
-  const double points = (double)pd.n1 * pd.n2 * pd.n3;
-  const double least = n < 20 ? 50e3 : n < 32 ? 400e3 : points >= 90e3 ? 0.0 : 250e3;
-  return nbatch * points >= least;
+  const double plane = (double)pd.n2 * pd.n3, points = plane * pd.n1;
+  const double least = n < 20 ? 100e3 : n < 32 ? 360e3 : points >= 90e3 ? 60e3 : 300e3;
+  return nbatch * plane * pd.np >= least;
 }
 
 size_t d64_band_bytes(const PlanDev &pd) { return region1(pd) + region2(pd); }

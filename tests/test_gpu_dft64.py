@@ -42,8 +42,8 @@ def scatter(c, box, m):
 
 CASES = [((30, 32, 36), 0.45, 1), ((27, 30, 28 + 2), 0.25, 3), ((45, 45, 45), 0.45, 5), ((75, 72, 80), 0.24, 2),
          ((100, 96, 108), 0.3, 1), ((32, 32, 32), None, 1), ((128, 40, 9), 0.4, 2), ((64, 64, 64), 0.45, 33),
-         ((30, 32, 36), 0.45, 8), ((27, 30, 30), 0.25, 17), ((128, 40, 9), 0.4, 6), ((15, 12, 16), 0.45, 20),
-         ((32, 32, 32), None, 9), ((9, 9, 9), 0.45, 80)]
+         ((30, 32, 36), 0.45, 11), ((27, 30, 30), 0.25, 40), ((128, 40, 9), 0.4, 10), ((15, 12, 16), 0.45, 45),
+         ((32, 32, 32), None, 10), ((9, 9, 9), 0.45, 160)]
 
 
 @pytest.mark.parametrize("box,frac,nb", CASES)
@@ -75,7 +75,7 @@ def test_transforms_hpsi_and_density(box, frac, nb):
     assert LIB.addft_tc05_status() == 0
 
 
-@pytest.mark.parametrize("nb", [3, 9])
+@pytest.mark.parametrize("nb", [3, 13])
 def test_lines_that_are_not_finite_stay_with_their_band(nb):
     box = (32, 32, 32)
     m = sphere(box, 0.4)
