@@ -1,4 +1,6 @@
-// Complex FP64 GEMM in double-float arithmetic on the FP32 pipes.
+// Complex FP64 GEMM of the subspace products: exact digit products on the tensor cores (ozgemm.cu, 168 x
+// 336 x 23,847: 0.45 ms) where the scratch holds their operands, else double-float arithmetic on the FP32
+// pipes (3.3 ms), described here.
 //
 //   C (M x N) = op(A) op(B),  op(A)[i][k] = A[i sAi + k sAk] (conjugated if conjA),
 //                             op(B)[k][j] = B[k sBk + j sBj] (conjugated if conjB),

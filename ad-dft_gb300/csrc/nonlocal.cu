@@ -944,7 +944,8 @@ inline size_t nl_grad_scratch(addft_dtype dt, int nk, int nb, int nG, int nproj)
 // ADDFT_HPSI_OVERLAP (read once per process): 0 = one stream; 1 (default) = the chain on a
 // second stream of the calling thread, forked from and joined back into the caller's stream
 // with events (also inside a stream capture); 2 = the same with that stream at the highest
-// priority.  72^3 microbench, 64 bands: 0.428 ms (0), 0.399 ms (1), 0.400 ms (2).
+// priority.  72^3 microbench, 64 bands, with becp on mma.sync: 0.428 ms (0), 0.399 ms (1), 0.400 ms
+// (2); with it on tcgen05 0.388 ms (1).
 static int overlap_mode() {
   static const int m = [] {
     const char *v = getenv("ADDFT_HPSI_OVERLAP");
