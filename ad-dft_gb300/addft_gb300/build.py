@@ -35,7 +35,7 @@ def nvcc() -> str:
 
 
 def _newest_header() -> float:
-    hs = list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
+    hs = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.hpp")) + list(INCLUDE.glob("*.h"))
     return max((h.stat().st_mtime for h in hs), default=0.0)
 
 

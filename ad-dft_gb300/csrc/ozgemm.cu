@@ -42,6 +42,7 @@
 #include "common.cuh"
 #include "mma16.cuh"
 #include "ozgemm.cuh"
+#include "ozlayout.hpp"
 
 namespace addft {
 
@@ -49,15 +50,12 @@ namespace {
 
 __device__ unsigned g_oz_error = 0;   // bit 0: a bounded wait ran out
 
-constexpr int kRowsA = 128, kRowsB = 32;   // rows of an A / B tile
-constexpr int kStep = 16;                  // k per stage
-constexpr int kDrain = 8;                  // stages per accumulation block (128 k: sums stay exact)
+constexpr int kRowsA = kOzRowsA, kRowsB = kOzRowsB, kStep = kOzStep, kDrain = kOzDrain;
 constexpr int kOzWait = 1 << 24;
 constexpr int kEpiWarps = 16;              // warps that empty the accumulators
 constexpr int kEpiCols = kRowsB / (kEpiWarps / 4);   // columns of each
 constexpr int kOzThreads = 32 * (kEpiWarps + 2);     // one for copies, one for MMAs
-constexpr int kSms = 152;
-constexpr int kMinPieceK = 1024;           // K is not cut below this when scratch is short
+constexpr int kSms = kOzSms;
 constexpr size_t kOzScratchCap = size_t(384) << 20;   // scratch asked for; more K, rows or batch go in pieces
 
 template <int S>
@@ -677,48 +675,6 @@ addft_status small_run(int M, int N, int K, int batch, const OzMat &A, const OzM
   return check_launch("k_small_outer");
 }
 
-inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
-
-struct OzLayout {
-  int ta, tb, nks, nsplit, steps;
-  size_t pa, pb;                       // packed bytes per batch entry
-  size_t o_ex, o_pa, o_pb, o_part, total;
-};
-
-// rows / cols as the kernel sees them (rows on the 128-row side)
-template <int S>
-OzLayout oz_layout(int rows, int cols, int K, int batch) {
-  OzLayout l;
-  l.ta = (rows + kRowsA - 1) / kRowsA;
-  l.tb = (cols + kRowsB - 1) / kRowsB;
-  l.nks = (K + kStep - 1) / kStep;
-  // A CTA fills an SM, so a split count costs waves x (accumulation blocks per CTA + about one
-  // block's time to start and to end a CTA); splits keep whole accumulation blocks.
-  const long tiles = (long)l.ta * l.tb * batch;
-  const int blocks = (l.nks + kDrain - 1) / kDrain;
-  int per = blocks;
-  long best = -1;
-  for (int ns = 1; ns <= std::min(blocks, 2 * kSms); ++ns) {
-    const int b = (blocks + ns - 1) / ns, used = (blocks + b - 1) / b;
-    const long cost = (tiles * used + kSms - 1) / kSms * (b + 1) + (used > 1 ? 1 : 0);
-    if (best < 0 || cost < best) {
-      best = cost;
-      per = b;
-    }
-    if (tiles >= 8 * kSms) break;   // many waves: nothing to fill
-  }
-  l.steps = per * kDrain;
-  l.nsplit = (l.nks + l.steps - 1) / l.steps;
-  l.pa = (size_t)l.ta * l.nks * Oz<S>::kABytes;
-  l.pb = (size_t)l.tb * l.nks * Oz<S>::kBBytes;
-  l.o_ex = 0;
-  l.o_pa = al256((size_t)batch * (rows + cols) * sizeof(int));
-  l.o_pb = l.o_pa + al256(l.pa * batch);
-  l.o_part = l.o_pb + al256(l.pb * batch);
-  l.total = l.o_part + (l.nsplit > 1 ? (size_t)l.nsplit * rows * cols * batch * sizeof(double2) : 0);
-  return l;
-}
-
 addft_status oz_max(const OzMat &m, int rows, int K, int batch, int *ex, cudaStream_t st) {
   // enough blocks to stream the operand at memory rate
   if (m.s_k == 1) {
@@ -748,8 +704,10 @@ addft_status oz_pack(const OzMat &m, int rows, int K, int nks, int batch, const 
 
 template <int S>
 addft_status oz_run(int rows, int cols, int K, int batch, const OzMat &A, const OzMat &B, double2 *C, long s_row,
-                    long s_col, size_t s_batch, bool accum, void *work, cudaStream_t st) {
-  const OzLayout l = oz_layout<S>(rows, cols, K, batch);
+                    long s_col, size_t s_batch, bool accum, int max_split, void *work, size_t bytes, cudaStream_t st) {
+  const OzLayout l = oz_layout(S, rows, cols, K, batch, max_split);
+  ADDFT_REQUIRE(l.total <= bytes, ADDFT_INVALID_ARG, "oz_gemm: a piece of %d x %d x %d wants %zu B of %zu", rows, cols, K,
+                l.total, bytes);
   char *w = (char *)work;
   int *ea = (int *)(w + l.o_ex), *eb = ea + (size_t)batch * rows;
   unsigned char *pa = (unsigned char *)w + l.o_pa, *pb = (unsigned char *)w + l.o_pb;
@@ -791,31 +749,11 @@ bool oz_swap(int M, int N, bool m_contig, bool n_contig) {
   return pad(N, M) * (n_contig ? 1.0 : 1.1) < pad(M, N) * (m_contig ? 1.0 : 1.1);
 }
 
-size_t oz_total(int digits, int r, int c, int K, int batch) {
-  return digits == 8 ? oz_layout<8>(r, c, K, batch).total : oz_layout<7>(r, c, K, batch).total;
-}
-
-// Pieces of a product that fit the scratch: batch entries at a time, then rows, columns or K cut
-// down, whichever packs largest.
-struct OzPieces { int batch, rows, cols, K; };
-bool oz_pieces(int digits, int r, int c, int K, int batch, size_t bytes, OzPieces &p) {
-  p = {batch, r, c, K};
-  while (oz_total(digits, p.rows, p.cols, p.K, p.batch) > bytes) {
-    auto half = [](int n, int unit) { return (n / 2 + unit - 1) / unit * unit; };
-    if (p.batch > 1) p.batch = (p.batch + 1) / 2;
-    else if (p.K > 2 * kMinPieceK) p.K = half(p.K, kDrain * kStep);
-    else if (p.rows >= p.cols && p.rows > 2 * kRowsA) p.rows = half(p.rows, kRowsA);
-    else if (p.cols > 2 * kRowsB) p.cols = half(p.cols, kRowsB);
-    else return false;
-  }
-  return (p.rows + kRowsA - 1) / kRowsA <= 65535 && (p.cols + kRowsB - 1) / kRowsB <= 65535 && p.batch <= 200;
-}
-
 }  // namespace
 
 size_t oz_work_bytes(int digits, int M, int N, int K, int batch) {
   if (small_product(M, N, K, batch)) return small_bytes(M, N, K, batch);
-  const size_t need = std::max(oz_total(digits, M, N, K, batch), oz_total(digits, N, M, K, batch));
+  const size_t need = std::max(oz_layout(digits, M, N, K, batch).total, oz_layout(digits, N, M, K, batch).total);
   return std::min(need, kOzScratchCap);
 }
 
@@ -842,18 +780,12 @@ addft_status oz_gemm(int digits, int M, int N, int K, int batch, const OzMat &A,
     o.p = (const double2 *)m.p + b * m.s_batch + row * m.s_row + k * m.s_k;
     return o;
   };
-  for (int b0 = 0; b0 < batch; b0 += p.batch)
-    for (int r0 = 0; r0 < r; r0 += p.rows)
-      for (int c0 = 0; c0 < c; c0 += p.cols)
-        for (int k0 = 0; k0 < K; k0 += p.K) {
-          const int nb = std::min(p.batch, batch - b0), nr = std::min(p.rows, r - r0), nc = std::min(p.cols, c - c0);
-          const int nk = std::min(p.K, K - k0);
-          const OzMat a = at(ma, b0, r0, k0), b = at(mb, b0, c0, k0);
-          double2 *o = (double2 *)C + b0 * s_batch + r0 * sr + c0 * sc;
-          ADDFT_TRY(digits == 8 ? oz_run<8>(nr, nc, nk, nb, a, b, o, sr, sc, s_batch, accum || k0 > 0, work, st)
-                                : oz_run<7>(nr, nc, nk, nb, a, b, o, sr, sc, s_batch, accum || k0 > 0, work, st));
-        }
-  return ADDFT_OK;
+  return (addft_status)oz_each_piece(r, c, K, batch, p, [&](int b0, int r0, int c0, int k0, int nb, int nr, int nc, int nk) {
+    const OzMat a = at(ma, b0, r0, k0), b = at(mb, b0, c0, k0);
+    double2 *o = (double2 *)C + b0 * s_batch + r0 * sr + c0 * sc;
+    return (int)(digits == 8 ? oz_run<8>(nr, nc, nk, nb, a, b, o, sr, sc, s_batch, accum || k0 > 0, p.nsplit, work, work_bytes, st)
+                             : oz_run<7>(nr, nc, nk, nb, a, b, o, sr, sc, s_batch, accum || k0 > 0, p.nsplit, work, work_bytes, st));
+  });
 }
 
 unsigned oz_status() {

@@ -109,3 +109,42 @@ def test_pieces_of_a_product_when_scratch_is_short():
         outs.append(out)
     for o in outs:
         assert bool(((o - a.conj() @ b.T).abs() <= bound(a, b.T, 55)).all())
+
+
+def guarded(nbytes):
+    """A work buffer of `nbytes` before 32 MB of a pattern."""
+    w = torch.full((nbytes + (32 << 20),), 0xA5, dtype=torch.uint8, device="cuda")
+    return w, lambda: bool((w[nbytes:] == 0xA5).all())
+
+
+@pytest.mark.parametrize("M,N,K,mb", [(1280, 320, 2432, 70),    # cut along K: the last piece would take more splits
+                                      (591, 1316, 3000, 40),    # K, then rows and columns
+                                      (1500, 700, 200, 3),      # rows and columns
+                                      (40, 3000, 130, 2)])
+def test_pieces_stay_within_the_scratch(M, N, K, mb):
+    import ctypes as C
+    a, b = rnd(1, M, K, spread=3.0), rnd(2, N, K)
+    nbytes = mb << 20
+    assert nbytes < int(LIB.addft_zgemm_df_work_bytes(M, N, K))
+    w, clean = guarded(nbytes)
+    out = torch.empty((M, N), dtype=torch.complex128, device="cuda")
+    st = LIB.addft_zgemm_df(M, N, K, C.c_void_p(a.data_ptr()), K, 1, 1, C.c_void_p(b.data_ptr()), 1, K, 0,
+                            C.c_void_p(out.data_ptr()), N, C.c_void_p(w.data_ptr()), nbytes,
+                            C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0
+    assert bool(((out - a.conj() @ b.T).abs() <= bound(a, b.T, 55)).all()) and clean()
+
+
+@pytest.mark.parametrize("nk,nb,P,nG,mb", [(5, 40, 72, 3001, 40), (3, 70, 130, 2200, 24)])
+def test_pieces_of_a_batch_stay_within_the_scratch(nk, nb, P, nG, mb):
+    import ctypes as C
+    proj, psi = rnd(1, nk, P, nG), rnd(2, nk, nb, nG)
+    w, clean = guarded(mb << 20)
+    out = torch.empty((nk, P, nb), dtype=torch.complex128, device="cuda")
+    st = LIB.addft_becp(1, nk, nb, nG, P, C.c_void_p(proj.data_ptr()), C.c_void_p(psi.data_ptr()),
+                        C.c_void_p(out.data_ptr()), C.c_void_p(w.data_ptr()), mb << 20,
+                        C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0
+    for k in range(nk):
+        assert bool(((out[k] - proj[k].conj() @ psi[k].T).abs() <= bound(proj[k], psi[k].T, 60)).all())
+    assert clean()
