@@ -674,10 +674,16 @@ int chunk_bands(const PlanDev &pd, int nbatch, size_t bytes) {
   // as many bands at once as the scratch holds, in equal chunks: every launch has the ramp of 152 CTAs
   // that load F first (160 bands of Si64 in chunks of 10 / 20 / 40 / 80: 6.6 / 6.0 / 5.6 / 5.5 ms)
   const size_t cap = (size_t(1) << 30) / ((size_t)pd.n2 * pd.n3);   // line numbers
-  const int fit = (int)std::min(std::min(bytes / d64_band_bytes(pd), cap), (size_t)nbatch);
-  if (fit < 1) return fit;
+  const int fit = (int)std::max<size_t>(1, std::min(std::min(bytes / d64_band_bytes(pd), cap), (size_t)nbatch));
   const int chunks = (nbatch + fit - 1) / fit;
   return (nbatch + chunks - 1) / chunks;
+}
+
+// Every entry needs `fixed` bytes and a band's: callers ask for that (d64_runs), and with less nothing runs.
+addft_status room(const PlanDev &pd, size_t bytes, size_t fixed) {
+  ADDFT_REQUIRE(bytes >= fixed + d64_band_bytes(pd), ADDFT_INVALID_ARG, "dft64: work needs %zu B, got %zu",
+                fixed + d64_band_bytes(pd), bytes);
+  return ADDFT_OK;
 }
 
 }  // namespace
@@ -706,6 +712,7 @@ size_t d64_v_bytes(const PlanDev &pd) { return al256((size_t)pd.n1 * pd.n2 * pd.
 addft_status d64_hpsi(const PlanDev &pd, int nbatch, const double2 *psi, const double *v_r, double2 *hpsi,
                       const double *kin, int nb_per_k, void *work, size_t bytes, cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  ADDFT_TRY(room(pd, bytes, d64_v_bytes(pd)));
   double *Vt = (double *)work;
   char *w = (char *)work + d64_v_bytes(pd);
   const int nc = chunk_bands(pd, nbatch, bytes - d64_v_bytes(pd));
@@ -747,8 +754,10 @@ addft_status d64_density(const PlanDev &pd, int nbatch, const double2 *psi, cons
   const long blocks = (lines + kLines - 1) / kLines;
   int groups = (int)std::max<long>(1, std::min<long>(4, (8 * kSms / pd.d64[0].tiles + blocks - 1) / blocks));
   groups = std::min(groups, nbatch);
-  while (groups > 1 && bytes < (size_t)groups * 2 * N * sizeof(double) + d64_band_bytes(pd)) --groups;
-  const size_t pb = al256((size_t)groups * 2 * N * sizeof(double));
+  auto part_bytes = [N](int g) { return al256((size_t)g * 2 * N * sizeof(double)); };
+  while (groups > 1 && bytes < part_bytes(groups) + d64_band_bytes(pd)) --groups;
+  const size_t pb = part_bytes(groups);
+  ADDFT_TRY(room(pd, bytes, pb));
   double *part = (double *)work;
   char *w = (char *)work + pb;
   const int nc = chunk_bands(pd, nbatch, bytes - pb);
@@ -773,6 +782,7 @@ addft_status d64_density(const PlanDev &pd, int nbatch, const double2 *psi, cons
 addft_status d64_to_real(const PlanDev &pd, int nbatch, const double2 *psi, double scale, void *out, bool real_part,
                          void *work, size_t bytes, cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  ADDFT_TRY(room(pd, bytes, 0));
   const int nc = chunk_bands(pd, nbatch, bytes);
   double2 *r1 = (double2 *)work, *r2 = (double2 *)((char *)work + (size_t)nc * region1(pd));
   for (int b0 = 0; b0 < nbatch; b0 += nc) {
@@ -798,6 +808,7 @@ addft_status d64_to_real(const PlanDev &pd, int nbatch, const double2 *psi, doub
 addft_status d64_from_real(const PlanDev &pd, int nbatch, const void *in, bool in_real, double scale, double2 *psi,
                            void *work, size_t bytes, cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
+  ADDFT_TRY(room(pd, bytes, 0));
   const int nc = chunk_bands(pd, nbatch, bytes);
   double2 *r1 = (double2 *)work, *r2 = (double2 *)((char *)work + (size_t)nc * region1(pd));
   for (int b0 = 0; b0 < nbatch; b0 += nc) {

@@ -88,3 +88,34 @@ def test_lines_that_are_not_finite_stay_with_their_band(nb):
     rest = [0] + list(range(2, nb))
     assert torch.equal(out[rest], good[rest])
     assert bool(torch.isnan(torch.view_as_real(out[1])).all())
+
+
+@pytest.mark.parametrize("box,nb", [((45, 45, 45), 5), ((25, 27, 45), 9)])
+def test_density_in_scratch_of_every_size_around_its_groups(box, nb):
+    """Scratch of g slabs of partial sums and one band, and up to 300 bytes more or less: one chunk of bands
+    at a time, in as many groups as fit; nothing is written past the buffer's end."""
+    import ctypes as C
+    m = sphere(box, 0.45)
+    plan = ops.Plan(box, m)
+    g = torch.Generator(device="cuda").manual_seed(nb)
+    c = torch.randn((1, nb, plan.nG), dtype=C128, device="cuda", generator=g)
+    w = torch.rand((1, nb), dtype=F64, device="cuda", generator=g)
+    x, _ = scatter(c[0], box, m)
+    r = torch.fft.ifftn(x, dim=(1, 2, 3), norm="forward").reshape(nb, plan.N)
+    ref = (w[0][:, None] * (r.real ** 2 + r.imag ** 2)).sum(0) / 2.5
+    l1 = c[0].abs().sum(1, keepdim=True)
+    tol = (w[0][:, None] * (16 * U * l1 * r.abs() + 8 * U * (r.abs() ** 2))).sum(0) / 2.5 + nb * 4 * U * ref
+    band = plan.work_bytes(nb, 1) - plan.work_bytes(nb - 1, 1)
+    for groups in (1, 2, 3, 4):
+        for more in (-256, -1, 0, 1, 100, 191, 192, 255, 256, 300):
+            nbytes = groups * 16 * plan.N + band + more
+            work = torch.full((nbytes + 4096,), 0xA5, dtype=torch.uint8, device="cuda")
+            rho = torch.full((plan.N,), float("nan"), dtype=F64, device="cuda")
+            st = LIB.addft_density(plan.handle, 1, 1, nb, 2.5, C.c_void_p(c.data_ptr()), C.c_void_p(w.data_ptr()),
+                                   C.c_void_p(rho.data_ptr()), C.c_void_p(work.data_ptr()), nbytes,
+                                   C.c_void_p(torch.cuda.current_stream().cuda_stream))
+            if st != 0:        # refused only below the least scratch of one band
+                assert st == 1 and nbytes < plan.work_bytes(1, 1), (groups, more)
+                continue
+            assert bool(((rho - ref).abs() <= tol).all()), (groups, more)
+            assert bool((work[nbytes:] == 0xA5).all()), (groups, more)
