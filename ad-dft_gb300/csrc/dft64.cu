@@ -673,7 +673,8 @@ addft_status to_planes(const PlanDev &pd, int nb, const double2 *psi, double2 *r
 int chunk_bands(const PlanDev &pd, int nbatch, size_t bytes) {
   // as many bands at once as the scratch holds, in equal chunks: every launch has the ramp of 152 CTAs
   // that load F first (160 bands of Si64 in chunks of 10 / 20 / 40 / 80: 6.6 / 6.0 / 5.6 / 5.5 ms)
-  const size_t cap = (size_t(1) << 30) / ((size_t)pd.n2 * pd.n3);   // line numbers
+  const size_t lines = (size_t(1) << 30) / ((size_t)pd.n2 * pd.n3), grid = 65535 / ((pd.n3 + 31) / 32);   // k_d64_out's y
+  const size_t cap = std::min(lines, grid);
   const int fit = (int)std::max<size_t>(1, std::min(std::min(bytes / d64_band_bytes(pd), cap), (size_t)nbatch));
   const int chunks = (nbatch + fit - 1) / fit;
   return (nbatch + chunks - 1) / chunks;

@@ -119,3 +119,16 @@ def test_density_in_scratch_of_every_size_around_its_groups(box, nb):
                 continue
             assert bool(((rho - ref).abs() <= tol).all()), (groups, more)
             assert bool((work[nbytes:] == 0xA5).all()), (groups, more)
+
+
+def test_more_bands_than_a_grid_has_rows():
+    """Small boxes in large batches: the reordering kernel's grid holds 65,535 bands of one z tile."""
+    box, nb = (4, 4, 5), 66000
+    m = sphere(box, 0.45)
+    plan = ops.Plan(box, m)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    c = torch.randn((nb, plan.nG), dtype=C128, device="cuda", generator=g)
+    out = ops.psi_to_real(plan, c, 1.0)
+    x, _ = scatter(c, box, m)
+    ref = torch.fft.ifftn(x, dim=(1, 2, 3), norm="forward").reshape(nb, plan.N)
+    assert bool(((out - ref).abs() <= 8 * U * c.abs().sum(1, keepdim=True)).all())
