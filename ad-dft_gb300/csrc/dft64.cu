@@ -690,7 +690,8 @@ addft_status room(const PlanDev &pd, size_t bytes, size_t fixed) {
 }  // namespace
 
 bool d64_handles(const PlanDev &pd, int nbatch) {
-  if (!pd.d64_F) return false;
+  // tuning that asks for the split stages or for other kernels than the defaults keeps to the FFT kernels
+  if (!pd.d64_F || !pd.tun.colfft || pd.tun.plane_split) return false;
   for (int a = 0; a < 6; ++a)
     if (pd.d64[a].tiles == 0) return false;
   // Six launches of 11 to 14 us (H psi) that load F first, against 45 to 76 us of the FFT kernels in small

@@ -11,7 +11,7 @@ namespace addft {
 void d64_build(int n1, int n2, int n3, const std::vector<int> &xact, const std::vector<int> &yact,
                const std::vector<int> &zact, D64Mat (&dm)[6], std::vector<unsigned char> &blob);
 
-// Whether the FP64 transforms of nbatch bands on this plan go through dft64 (box and size).
+// Whether the FP64 transforms of nbatch bands on this plan go through dft64 (box, size and tuning).
 bool d64_handles(const PlanDev &pd, int nbatch);
 
 // Scratch bytes per band in flight, and of the potential in the order the x stage reads it.

@@ -16,7 +16,7 @@
 namespace addft {
 
 constexpr int kMaxAtomsP = 256;
-constexpr int kForceSplits = 64;   // ranges of G (columns) per atom in the local forces
+constexpr int kForceSplits = 64, kForceSplitsLeast = 16;   // ranges of G (columns) per atom in the local forces
 
 inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
@@ -381,16 +381,18 @@ inline addft_status make_shell(ShellGeo &sg, const double *bvec, double omega, i
   return ADDFT_OK;
 }
 
-// scratch of one field's transform
+// Scratch of one field's transform: what it needs (FFT kernels), and what the tensor-core form wants.
+inline size_t slab_least(const PlanDev &pd) { return (size_t)pd.np * pd.n2 * pd.n3 * sizeof(double2); }
 inline size_t slab_bytes(const PlanDev &pd) {
-  return d64_handles(pd, 1) ? d64_band_bytes(pd) : (size_t)pd.np * pd.n2 * pd.n3 * sizeof(double2);
+  return d64_handles(pd, 1) ? std::max(d64_band_bytes(pd), slab_least(pd)) : slab_least(pd);
 }
+inline bool slab_d64(const PlanDev &pd, size_t bytes) { return d64_handles(pd, 1) && bytes >= d64_band_bytes(pd); }
 
-// n(G) = fftn(rho)/N gathered on the plan's shell (f64), W = slab scratch
-inline addft_status density_to_shell(const PlanDev &pd, const double *rho, double2 *ng, void *W,
+// n(G) = fftn(rho)/N gathered on the plan's shell (f64), W = slab scratch of `bytes`
+inline addft_status density_to_shell(const PlanDev &pd, const double *rho, double2 *ng, void *W, size_t bytes,
                                      cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
-  if (d64_handles(pd, 1)) return d64_from_real(pd, 1, rho, true, 1.0 / (double)N, ng, W, slab_bytes(pd), st);
+  if (slab_d64(pd, bytes)) return d64_from_real(pd, 1, rho, true, 1.0 / (double)N, ng, W, bytes, st);
   XArgs<double> a = xargs_default<double>(W);
   a.rin = rho;
   a.rin_is_real = 1;
@@ -402,9 +404,10 @@ inline addft_status density_to_shell(const PlanDev &pd, const double *rho, doubl
 }
 
 // v(r) = Re(N ifftn(scatter(vg)))
-inline addft_status shell_to_real(const PlanDev &pd, const double2 *vg, double *v, void *W, cudaStream_t st) {
+inline addft_status shell_to_real(const PlanDev &pd, const double2 *vg, double *v, void *W, size_t bytes,
+                                  cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
-  if (d64_handles(pd, 1)) return d64_to_real(pd, 1, vg, 1.0, v, true, W, slab_bytes(pd), st);
+  if (slab_d64(pd, bytes)) return d64_to_real(pd, 1, vg, 1.0, v, true, W, bytes, st);
   ADDFT_TRY(launch_plane_inv<double>(pd, 1, vg, pd.nG, 1.0, (double2 *)W, st));
   XArgs<double> a = xargs_default<double>(W);
   a.rout = v;
@@ -509,17 +512,17 @@ addft_status addft_hartree(addft_plan plan, const double *bvec, double omega, co
   const size_t o_ng = o_sum + al256(16 * sizeof(double));
   const size_t o_vg = o_ng + al256(pd.nG * sizeof(double2));
   const size_t o_w = o_vg + al256(pd.nG * sizeof(double2));
-  ADDFT_REQUIRE(work && work_bytes >= o_w + slab_bytes(pd), ADDFT_INVALID_ARG,
-                "hartree: work needs %zu B", o_w + slab_bytes(pd));
+  ADDFT_REQUIRE(work && work_bytes >= o_w + slab_least(pd), ADDFT_INVALID_ARG,
+                "hartree: work needs %zu B", o_w + slab_least(pd));
   char *w = (char *)work;
   double2 *ng = (double2 *)(w + o_ng), *vg = (double2 *)(w + o_vg);
-  ADDFT_TRY(density_to_shell(pd, rho, ng, w + o_w, st));
+  ADDFT_TRY(density_to_shell(pd, rho, ng, w + o_w, work_bytes - o_w, st));
   k_hartree_g<<<kRedBlocks, kRedThreads, 0, st>>>(pd, sg, ng, vg, (double *)(w + o_part));
   ADDFT_TRY(check_launch("k_hartree_g"));
   ADDFT_TRY(finalize_sums((double *)(w + o_part), 10, kRedBlocks, (double *)(w + o_sum), false, st));
   k_hartree_final<<<1, 32, 0, st>>>((double *)(w + o_sum), omega, e_h, nullptr);
   ADDFT_TRY(check_launch("k_hartree_final"));
-  if (v_h) ADDFT_TRY(shell_to_real(pd, vg, v_h, w + o_w, st));
+  if (v_h) ADDFT_TRY(shell_to_real(pd, vg, v_h, w + o_w, work_bytes - o_w, st));
   return ADDFT_OK;
 }
 
@@ -540,8 +543,8 @@ addft_status addft_local_potential(addft_plan rho_plan, const double *bvec, doub
   ShellGeo sg;
   ADDFT_TRY(make_shell(sg, bvec, omega, nat, pos, psp));
   const size_t o_vg = 0, o_w = al256(pd.nG * sizeof(double2));
-  ADDFT_REQUIRE(work && work_bytes >= o_w + slab_bytes(pd), ADDFT_INVALID_ARG,
-                "local_potential: work needs %zu B", o_w + slab_bytes(pd));
+  ADDFT_REQUIRE(work && work_bytes >= o_w + slab_least(pd), ADDFT_INVALID_ARG,
+                "local_potential: work needs %zu B", o_w + slab_least(pd));
   char *w = (char *)work;
   PhaseMats pm;
   bool phases = false;
@@ -550,7 +553,7 @@ addft_status addft_local_potential(addft_plan rho_plan, const double *bvec, doub
   if (phases) ADDFT_TRY(phase_struct(pd, sg, pm, vg, st));
   k_vloc_g<<<(pd.nG + 255) / 256, 256, 0, st>>>(pd, sg, phases ? vg : nullptr, vg);
   ADDFT_TRY(check_launch("k_vloc_g"));
-  return shell_to_real(pd, (const double2 *)(w + o_vg), v_loc, w + o_w, st);
+  return shell_to_real(pd, (const double2 *)(w + o_vg), v_loc, w + o_w, work_bytes - o_w, st);
 }
 
 addft_status addft_kerker(addft_plan full_plan, const double *bvec, const double *in, double alpha, double gg0,
@@ -563,13 +566,13 @@ addft_status addft_kerker(addft_plan full_plan, const double *bvec, const double
   ShellGeo sg;
   ADDFT_TRY(make_shell(sg, bvec, 1.0, 0, nullptr, nullptr));
   const size_t o_g = 0, o_w = al256(pd.nG * sizeof(double2));
-  ADDFT_REQUIRE(work && work_bytes >= o_w + slab_bytes(pd), ADDFT_INVALID_ARG, "kerker: work needs %zu B",
-                o_w + slab_bytes(pd));
+  ADDFT_REQUIRE(work && work_bytes >= o_w + slab_least(pd), ADDFT_INVALID_ARG, "kerker: work needs %zu B",
+                o_w + slab_least(pd));
   char *w = (char *)work;
-  ADDFT_TRY(density_to_shell(pd, in, (double2 *)(w + o_g), w + o_w, st));
+  ADDFT_TRY(density_to_shell(pd, in, (double2 *)(w + o_g), w + o_w, work_bytes - o_w, st));
   k_kerker_g<<<(pd.nG + 255) / 256, 256, 0, st>>>(pd, sg, alpha, gg0, (double2 *)(w + o_g));
   ADDFT_TRY(check_launch("k_kerker_g"));
-  return shell_to_real(pd, (const double2 *)(w + o_g), out, w + o_w, st);
+  return shell_to_real(pd, (const double2 *)(w + o_g), out, w + o_w, work_bytes - o_w, st);
 }
 
 size_t addft_kerker_work_bytes(addft_plan full_plan) {
@@ -595,23 +598,30 @@ addft_status addft_density_gradients(addft_plan wfc_plan, addft_plan rho_plan, c
   cudaStream_t st = as_stream(stream);
   ShellGeo sg;
   ADDFT_TRY(make_shell(sg, bvec, omega, nat, pos, psp));
-  const int nsplit = kForceSplits;
-  size_t off = 0;
-  auto take = [&](size_t b) { size_t o = off; off += al256(b); return o; };
-  const size_t o_hp = take(10 * kRedBlocks * sizeof(double));
-  const size_t o_lp = take(10 * kRedBlocks * sizeof(double));
-  const size_t o_hs = take(10 * sizeof(double));
-  const size_t o_ls = take(10 * sizeof(double));
-  const size_t o_fp = take((size_t)(nat > 0 ? nat : 1) * nsplit * 3 * sizeof(double));
-  const size_t o_nw = take(pw.nG * sizeof(double2));
-  const size_t o_nr = take(pr.nG * sizeof(double2));
-  const size_t o_w = take(std::max(slab_bytes(pw), slab_bytes(pr)));
+  // the layout up to the transforms' scratch, with as many column ranges per atom as the buffer has room for
+  size_t o_hp, o_lp, o_hs, o_ls, o_fp, o_nw, o_nr, o_w;
+  auto layout = [&](int splits) {
+    size_t off = 0;
+    auto take = [&](size_t b) { size_t o = off; off += al256(b); return o; };
+    o_hp = take(10 * kRedBlocks * sizeof(double));
+    o_lp = take(10 * kRedBlocks * sizeof(double));
+    o_hs = take(10 * sizeof(double));
+    o_ls = take(10 * sizeof(double));
+    o_fp = take((size_t)(nat > 0 ? nat : 1) * splits * 3 * sizeof(double));
+    o_nw = take(pw.nG * sizeof(double2));
+    o_nr = take(pr.nG * sizeof(double2));
+    o_w = off;
+    return off + al256(std::max(slab_least(pw), slab_least(pr)));
+  };
+  int nsplit = kForceSplits;
+  if (layout(nsplit) > work_bytes) nsplit = kForceSplitsLeast;
+  const size_t off = layout(nsplit);
   ADDFT_REQUIRE(work && work_bytes >= off, ADDFT_INVALID_ARG, "density_gradients: work needs %zu B", off);
   char *w = (char *)work;
   const size_t s_bytes = al256(pr.nG * sizeof(double2));   // S(G), then the phase tables, after the slabs' use
   double2 *S = (double2 *)(w + o_w);
-  ADDFT_TRY(density_to_shell(pw, rho, (double2 *)(w + o_nw), w + o_w, st));
-  ADDFT_TRY(density_to_shell(pr, rho, (double2 *)(w + o_nr), w + o_w, st));
+  ADDFT_TRY(density_to_shell(pw, rho, (double2 *)(w + o_nw), w + o_w, work_bytes - o_w, st));
+  ADDFT_TRY(density_to_shell(pr, rho, (double2 *)(w + o_nr), w + o_w, work_bytes - o_w, st));
   k_hartree_g<<<kRedBlocks, kRedThreads, 0, st>>>(pw, sg, (const double2 *)(w + o_nw), nullptr,
                                                  (double *)(w + o_hp));
   ADDFT_TRY(check_launch("k_hartree_g"));

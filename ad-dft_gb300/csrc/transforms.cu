@@ -589,11 +589,10 @@ XArgs<R> xargs_default(void *W) {
 // ---------------------------------------------------------------------------
 // entry-point bodies
 // ---------------------------------------------------------------------------
-// FP64 through the tensor-core form: a box and size it handles, and scratch for `extra` bytes and
-// one band; a plan whose tuning asks for the split stages or for other kernels than the defaults
-// keeps to the FFT kernels.
+// FP64 through the tensor-core form: a box, size and tuning it handles, and scratch for `extra` bytes and
+// one band.
 static bool d64_runs(const PlanDev &pd, int nbatch, const void *work, size_t bytes, size_t extra) {
-  return pd.tun.colfft && !pd.tun.plane_split && d64_handles(pd, nbatch) && work && ((uintptr_t)work & 255) == 0 &&
+  return d64_handles(pd, nbatch) && work && ((uintptr_t)work & 255) == 0 &&
          bytes >= extra + 256 + d64_band_bytes(pd);
 }
 
