@@ -670,16 +670,6 @@ addft_status to_planes(const PlanDev &pd, int nb, const double2 *psi, double2 *r
   return stage<YI>(pd, 1, a, (long)nb * pd.np * pd.n3, st);
 }
 
-int chunk_bands(const PlanDev &pd, int nbatch, size_t bytes) {
-  // as many bands at once as the scratch holds, in equal chunks: every launch has the ramp of 152 CTAs
-  // that load F first (160 bands of Si64 in chunks of 10 / 20 / 40 / 80: 6.6 / 6.0 / 5.6 / 5.5 ms)
-  const size_t lines = (size_t(1) << 30) / ((size_t)pd.n2 * pd.n3), grid = 65535 / ((pd.n3 + 31) / 32);   // k_d64_out's y
-  const size_t cap = std::min(lines, grid);
-  const int fit = (int)std::max<size_t>(1, std::min(std::min(bytes / d64_band_bytes(pd), cap), (size_t)nbatch));
-  const int chunks = (nbatch + fit - 1) / fit;
-  return (nbatch + chunks - 1) / chunks;
-}
-
 // Every entry needs `fixed` bytes and a band's: callers ask for that (d64_runs), and with less nothing runs.
 addft_status room(const PlanDev &pd, size_t bytes, size_t fixed) {
   ADDFT_REQUIRE(bytes >= fixed + d64_band_bytes(pd), ADDFT_INVALID_ARG, "dft64: work needs %zu B, got %zu",
@@ -689,23 +679,48 @@ addft_status room(const PlanDev &pd, size_t bytes, size_t fixed) {
 
 }  // namespace
 
-bool d64_handles(const PlanDev &pd, int nbatch) {
+int d64_chunk(const PlanDev &pd, int nbatch, size_t bytes) {
+  // as many bands at once as the scratch holds, in equal chunks: every launch has the ramp of 152 CTAs
+  // that load F first (160 bands of Si64 in chunks of 10 / 20 / 40 / 80: 6.6 / 6.0 / 5.6 / 5.5 ms)
+  const size_t lines = (size_t(1) << 30) / ((size_t)pd.n2 * pd.n3), grid = 65535 / ((pd.n3 + 31) / 32);   // k_d64_out's y
+  const int fit = (int)std::min(std::min(bytes / d64_band_bytes(pd), std::min(lines, grid)), (size_t)nbatch);
+  if (fit < 1) return 0;
+  const int chunks = (nbatch + fit - 1) / fit;
+  return (nbatch + chunks - 1) / chunks;
+}
+
+bool d64_handles(const PlanDev &pd, D64Op op, int bands) {
   // tuning that asks for the split stages or for other kernels than the defaults keeps to the FFT kernels
   if (!pd.d64_F || !pd.tun.colfft || pd.tun.plane_split) return false;
   for (int a = 0; a < 6; ++a)
     if (pd.d64[a].tiles == 0) return false;
-  // Six launches of 11 to 14 us (H psi) that load F first, against 45 to 76 us of the FFT kernels in small
-  // calls.  The FFT kernels' time follows the active planes (np n2 n3 points a band), below 20 points an axis
-  // at 600 to 700 us per 10^6 of them, above at 160 to 220; the products take 200 and 90 to 180.  H psi, FFT
-  // / products, us, spheres of 0.45 n: 12^3 x 16 bands 46 / 68, x 64 112 / 89; 15^3 x 8 76 / 68, x 64 222 /
-  // 102; 16^3 x 8 56 / 68, x 16 72 / 68, x 32 129 / 90; 24^3 x 16 70 / 97, x 32 109 / 126 (density 89 / 79), x
-  // 64 181 / 187 (150 / 120); 30^3 x 8 81 / 88, x 16 134 / 107; 36^3 x 4 68 / 89, x 8 109 / 110 (93 / 66); 45^3 x
-  // 1 100 / 83, 48^3 x 1 99 / 83, x 32 726 / 381; 75^3 x 1 238 / 147, x 8 963 / 608.  Density of Si2's 24 bands
-  // (18^3, a sphere of a quarter): 35 / 55.
-  const int n = std::max(pd.n1, std::max(pd.n2, pd.n3));
-  const double plane = (double)pd.n2 * pd.n3, points = plane * pd.n1;
-  const double least = n < 20 ? 100e3 : n < 32 ? 360e3 : points >= 90e3 ? 60e3 : 300e3;
-  return nbatch * plane * pd.np >= least;
+  // Where the products start, in box points x bands at once, by (n1 n2 n3)^(1/3).  They take 65 to 80 (H psi) or
+  // 36 to 48 us (density, one way) before the work shows, launches that load F first; the FFT kernels 40 to 60 and
+  // 20 to 35, growing with the box.  Measured on 39 boxes from 9^3 to 80^3, cubes and 1 : 1 : 1.25 to 2, 1 to
+  // 64 bands, spheres of 0.45 and 0.25 n; FFT / products in us, spheres of 0.45:
+  //   H psi    18^3 x 64 bands 97 / 132, 20^3 x 64 130 / 152, 24^3 x 32 109 / 125, x 64 181 / 185, 25^3 x 16 89 / 101,
+  //            x 32 144 / 132, 30^3 x 8 80 / 88, x 16 134 / 107, 32^3 x 16 125 / 125, x 32 196 / 180, 36^3 x 8 109 / 109,
+  //            32 x 32 x 64 x 4 82 / 103, x 8 142 / 136, 40^3 x 4 116 / 92, 45^3 x 1 98 / 79, 75^3 x 1 239 / 146
+  //   density  18^3 x 64 87 / 107, 20^3 x 64 120 / 109, 24^3 x 16 58 / 60, x 32 89 / 79, 30^3 x 8 48 / 53, x 16 74 / 63,
+  //            32^3 x 16 72 / 66, 36^3 x 4 54 / 51, x 8 93 / 66, 40^3 x 8 95 / 70, 45^3 x 1 54 / 48
+  //   one way  18^3 x 32 46 / 53, x 64 81 / 67, 24^3 x 16 53 / 49, 30^3 x 8 46 / 48, x 16 72 / 55, 32^3 x 16 68 / 62,
+  //            36^3 x 1 49 / 43, 45^3 x 1 60 / 44
+  struct Row { double size, from[3]; };
+  static const Row rows[] = {{22.0, {1300e3, 600e3, 260e3}}, {26.5, {800e3, 400e3, 380e3}}, {31.9, {430e3, 320e3, 320e3}},
+                             {33.0, {500e3, 600e3, 520e3}},  {36.5, {400e3, 370e3, 290e3}}, {42.0, {300e3, 430e3, 0}},
+                             {1e9, {0, 0, 0}}};
+  const double points = (double)pd.n1 * pd.n2 * pd.n3, work = points * bands;
+  // Axes of one pass (up to 16 points) give the FFT kernels a CTA per plane and band with one line per thread: their time
+  // follows planes x bands and starts early (H psi 12^3 x 32 78 / 68, 15^3 x 32 132 / 80, 16^3 x 32 129 / 89, x 16
+  // 72 / 68, 12 x 12 x 24 x 32 78 / 83; density 16^3 x 32 74 / 66, 12^3 x 64 93 / 91; one way 16^3 x 32 50 / 45).
+  if (pd.ax[0].nst == 1 && pd.ax[1].nst == 1) {
+    const double planes = (double)pd.np * bands;
+    return op == D64Op::kHpsi ? planes >= 300 && work >= 55e3 : planes >= 450 && work >= (op == D64Op::kDensity ? 100e3 : 55e3);
+  }
+  const double size = std::cbrt(points);
+  for (const Row &r : rows)
+    if (size < r.size) return work >= r.from[(int)op];
+  return true;
 }
 
 size_t d64_band_bytes(const PlanDev &pd) { return region1(pd) + region2(pd); }
@@ -717,7 +732,7 @@ addft_status d64_hpsi(const PlanDev &pd, int nbatch, const double2 *psi, const d
   ADDFT_TRY(room(pd, bytes, d64_v_bytes(pd)));
   double *Vt = (double *)work;
   char *w = (char *)work + d64_v_bytes(pd);
-  const int nc = chunk_bands(pd, nbatch, bytes - d64_v_bytes(pd));
+  const int nc = d64_chunk(pd, nbatch, bytes - d64_v_bytes(pd));
   k_d64_v<<<dim3((pd.n1 + 31) / 32, (pd.n3 + 31) / 32, pd.n2), 256, 0, st>>>(pd, v_r, 1.0 / (double)N, Vt);
   ADDFT_TRY(check_launch("k_d64_v"));
   double2 *r1 = (double2 *)w, *r2 = (double2 *)(w + (size_t)nc * region1(pd));
@@ -762,7 +777,7 @@ addft_status d64_density(const PlanDev &pd, int nbatch, const double2 *psi, cons
   ADDFT_TRY(room(pd, bytes, pb));
   double *part = (double *)work;
   char *w = (char *)work + pb;
-  const int nc = chunk_bands(pd, nbatch, bytes - pb);
+  const int nc = d64_chunk(pd, nbatch, bytes - pb);
   double2 *r1 = (double2 *)w, *r2 = (double2 *)(w + (size_t)nc * region1(pd));
   for (int b0 = 0; b0 < nbatch; b0 += nc) {
     const int nb = std::min(nc, nbatch - b0);
@@ -785,7 +800,7 @@ addft_status d64_to_real(const PlanDev &pd, int nbatch, const double2 *psi, doub
                          void *work, size_t bytes, cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
   ADDFT_TRY(room(pd, bytes, 0));
-  const int nc = chunk_bands(pd, nbatch, bytes);
+  const int nc = d64_chunk(pd, nbatch, bytes);
   double2 *r1 = (double2 *)work, *r2 = (double2 *)((char *)work + (size_t)nc * region1(pd));
   for (int b0 = 0; b0 < nbatch; b0 += nc) {
     const int nb = std::min(nc, nbatch - b0);
@@ -811,7 +826,7 @@ addft_status d64_from_real(const PlanDev &pd, int nbatch, const void *in, bool i
                            void *work, size_t bytes, cudaStream_t st) {
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
   ADDFT_TRY(room(pd, bytes, 0));
-  const int nc = chunk_bands(pd, nbatch, bytes);
+  const int nc = d64_chunk(pd, nbatch, bytes);
   double2 *r1 = (double2 *)work, *r2 = (double2 *)((char *)work + (size_t)nc * region1(pd));
   for (int b0 = 0; b0 < nbatch; b0 += nc) {
     const int nb = std::min(nc, nbatch - b0);

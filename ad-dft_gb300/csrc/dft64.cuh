@@ -11,8 +11,13 @@ namespace addft {
 void d64_build(int n1, int n2, int n3, const std::vector<int> &xact, const std::vector<int> &yact,
                const std::vector<int> &zact, D64Mat (&dm)[6], std::vector<unsigned char> &blob);
 
-// Whether the FP64 transforms of nbatch bands on this plan go through dft64 (box, size and tuning).
-bool d64_handles(const PlanDev &pd, int nbatch);
+// Whether FP64 transforms of `bands` bands at once go through dft64 (box, size and tuning): local H psi, a
+// band density, or a transform one way.
+enum class D64Op { kHpsi, kDensity, kField };
+bool d64_handles(const PlanDev &pd, D64Op op, int bands);
+
+// Bands at once of a call over nbatch with `bytes` of scratch for them; 0: not one.
+int d64_chunk(const PlanDev &pd, int nbatch, size_t bytes);
 
 // Scratch bytes per band in flight, and of the potential in the order the x stage reads it.
 size_t d64_band_bytes(const PlanDev &pd);

@@ -404,7 +404,10 @@ addft_status addft_plan_get_tuning(addft_plan plan, const char *key, long *value
 size_t addft_work_bytes(addft_plan plan, int nbatch, addft_dtype dt) {
   if (!plan || nbatch < 1) return 0;
   const size_t least = work_bytes_min(plan->dev, nbatch, dt == ADDFT_F64 ? 16 : 8);
-  if (dt != ADDFT_F64 || !d64_handles(plan->dev, nbatch)) return least;
+  const PlanDev &d = plan->dev;
+  if (dt != ADDFT_F64 || !(d64_handles(d, D64Op::kHpsi, nbatch) || d64_handles(d, D64Op::kDensity, nbatch) ||
+                           d64_handles(d, D64Op::kField, nbatch)))
+    return least;
   // the FP64 tensor-core form keeps more of a band in flight; with less the FFT kernels run
   return std::max(least, (size_t)nbatch * d64_band_bytes(plan->dev) + (size_t(1) << 20) + d64_v_bytes(plan->dev));
 }

@@ -384,9 +384,9 @@ inline addft_status make_shell(ShellGeo &sg, const double *bvec, double omega, i
 // Scratch of one field's transform: what it needs (FFT kernels), and what the tensor-core form wants.
 inline size_t slab_least(const PlanDev &pd) { return (size_t)pd.np * pd.n2 * pd.n3 * sizeof(double2); }
 inline size_t slab_bytes(const PlanDev &pd) {
-  return d64_handles(pd, 1) ? std::max(d64_band_bytes(pd), slab_least(pd)) : slab_least(pd);
+  return d64_handles(pd, D64Op::kField, 1) ? std::max(d64_band_bytes(pd), slab_least(pd)) : slab_least(pd);
 }
-inline bool slab_d64(const PlanDev &pd, size_t bytes) { return d64_handles(pd, 1) && bytes >= d64_band_bytes(pd); }
+inline bool slab_d64(const PlanDev &pd, size_t bytes) { return d64_handles(pd, D64Op::kField, 1) && bytes >= d64_band_bytes(pd); }
 
 // n(G) = fftn(rho)/N gathered on the plan's shell (f64), W = slab scratch of `bytes`
 inline addft_status density_to_shell(const PlanDev &pd, const double *rho, double2 *ng, void *W, size_t bytes,

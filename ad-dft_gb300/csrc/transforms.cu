@@ -589,11 +589,11 @@ XArgs<R> xargs_default(void *W) {
 // ---------------------------------------------------------------------------
 // entry-point bodies
 // ---------------------------------------------------------------------------
-// FP64 through the tensor-core form: a box, size and tuning it handles, and scratch for `extra` bytes and
-// one band.
-static bool d64_runs(const PlanDev &pd, int nbatch, const void *work, size_t bytes, size_t extra) {
-  return d64_handles(pd, nbatch) && work && ((uintptr_t)work & 255) == 0 &&
-         bytes >= extra + 256 + d64_band_bytes(pd);
+// FP64 through the tensor-core form: scratch for `extra` bytes and some bands, as many of them at once as make it
+// the quicker one.
+static bool d64_runs(const PlanDev &pd, D64Op op, int nbatch, const void *work, size_t bytes, size_t extra) {
+  if (!work || ((uintptr_t)work & 255) != 0 || bytes < extra + 256 + d64_band_bytes(pd)) return false;
+  return d64_handles(pd, op, d64_chunk(pd, nbatch, bytes - extra - 256));
 }
 
 template <typename R>
@@ -602,7 +602,7 @@ addft_status psi_to_real_t(addft_plan plan, int nbatch, double omega, const void
   using C = typename Cx<R>::T;
   const PlanDev &pd = plan->dev;
   if constexpr (sizeof(R) == 8)
-    if (d64_runs(pd, nbatch, work, bytes, 0))
+    if (d64_runs(pd, D64Op::kField, nbatch, work, bytes, 0))
       return d64_to_real(pd, nbatch, (const double2 *)psi, 1.0 / sqrt(omega), psi_r, false, work, bytes, st);
   Work w;
   ADDFT_TRY(split_work(pd, sizeof(C), work, bytes, w));
@@ -627,7 +627,7 @@ addft_status real_to_psi_t(addft_plan plan, int nbatch, double omega, const void
   const PlanDev &pd = plan->dev;
   const long N = (long)pd.n1 * pd.n2 * pd.n3;
   if constexpr (sizeof(R) == 8)
-    if (d64_runs(pd, nbatch, work, bytes, 0))
+    if (d64_runs(pd, D64Op::kField, nbatch, work, bytes, 0))
       return d64_from_real(pd, nbatch, psi_r, false, sqrt(omega) / (double)N, (double2 *)psi, work, bytes, st);
   Work w;
   ADDFT_TRY(split_work(pd, sizeof(C), work, bytes, w));
@@ -653,7 +653,7 @@ addft_status hpsi_local_t(addft_plan plan, int nk, int nb, const void *psi, cons
   using C = typename Cx<R>::T;
   const PlanDev &pd = plan->dev;
   if constexpr (sizeof(R) == 8)
-    if (d64_runs(pd, nk * nb, work, bytes, d64_v_bytes(pd)))
+    if (d64_runs(pd, D64Op::kHpsi, nk * nb, work, bytes, d64_v_bytes(pd)))
       return d64_hpsi(pd, nk * nb, (const double2 *)psi, (const double *)v_r, (double2 *)hpsi, (const double *)kin, nb,
                       work, bytes, st);
   if (pd.tun.colfft && colfft_handles<R>(pd) && work != nullptr && ((uintptr_t)work & 255) == 0) {
@@ -733,7 +733,7 @@ addft_status density_t(addft_plan plan, int nk, int nb, double omega, const void
     return ADDFT_OK;
   }
   if constexpr (sizeof(R) == 8)
-    if (d64_runs(pd, nbatch, work, bytes, 2 * (size_t)N * sizeof(double)))
+    if (d64_runs(pd, D64Op::kDensity, nbatch, work, bytes, 2 * (size_t)N * sizeof(double)))
       return d64_density(pd, nbatch, (const double2 *)psi, wocc, 1.0 / omega, rho, work, bytes, st);
   // split the bands across CTAs so the x-line stage has >= 4 CTAs per SM
   const int t3 = pick_t3<R>(pd, XM_DENSITY, nbatch);

@@ -132,3 +132,33 @@ def test_more_bands_than_a_grid_has_rows():
     x, _ = scatter(c, box, m)
     ref = torch.fft.ifftn(x, dim=(1, 2, 3), norm="forward").reshape(nb, plan.N)
     assert bool(((out - ref).abs() <= 8 * U * c.abs().sum(1, keepdim=True)).all())
+
+
+# boxes of every size class from where the products start, and one band below
+@pytest.mark.parametrize("box,frac,nb", [((12, 12, 12), 0.45, 46), ((9, 10, 15), 0.45, 60), ((20, 20, 20), 0.25, 165),
+                                         ((24, 24, 24), 0.45, 58), ((25, 25, 50), 0.25, 14), ((32, 32, 32), None, 19),
+                                         ((30, 32, 36), 0.45, 30), ((36, 36, 36), 0.25, 9), ((32, 32, 64), 0.45, 7)])
+def test_where_the_products_start(box, frac, nb):
+    for n in (nb, nb - 1):
+        test_transforms_hpsi_and_density(box, frac, n)
+
+
+def test_many_bands_in_scratch_for_a_few_run_the_ffts():
+    """24^3 x 64 bands in 8 MB: the products would go in four chunks of six launches."""
+    import ctypes as C
+    box = (24, 24, 24)
+    m = sphere(box, 0.45)
+    plan = ops.Plan(box, m)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    c = torch.randn((1, 64, plan.nG), dtype=C128, device="cuda", generator=g)
+    v = torch.randn(plan.N, dtype=F64, device="cuda", generator=g)
+    kin = torch.rand((1, plan.nG), dtype=F64, device="cuda", generator=g)
+    whole = ops.hpsi(plan, c, kin, v)
+    out = torch.empty_like(c)
+    n = LIB.addft_launch_count()
+    st = LIB.addft_hpsi_noalloc(plan.handle, 1, 1, 64, C.c_void_p(c.data_ptr()), C.c_void_p(kin.data_ptr()),
+                                C.c_void_p(v.data_ptr()), 0, C.c_void_p(0), C.c_void_p(0), C.c_void_p(out.data_ptr()),
+                                C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0 and LIB.addft_launch_count() - n <= 12
+    l1 = c[0].abs().sum(1, keepdim=True)
+    assert bool(((out - whole).abs() <= 16 * U * l1 * v.abs().max() + 4 * U * (kin[:, None] * c).abs()).all())
