@@ -771,14 +771,19 @@ static int becp_ctas_per_sm() {
   return m;
 }
 
+// partial sums of the split-K kernels at their default number of splits
 template <typename R>
-size_t becp_work_bytes(int nk, int nb, int nG, int nproj) {
+size_t becp_partial_bytes(int nk, int nb, int nG, int nproj) {
   using C = typename Cx<R>::T;
   const int tiles = ((nproj + kBP - 1) / kBP) * ((nb + kBB - 1) / kBB) * nk;
   const int ns = pick_nsplit(tiles, nG);
-  const size_t simt = ns > 1 ? (size_t)(ns + split_groups(ns)) * nk * nproj * nb * sizeof(C) : 0;
-  if (sizeof(R) == 8) return std::max(simt, oz_work_bytes(8, nproj, nb, nG, nk));
-  return simt;
+  return ns > 1 ? (size_t)(ns + split_groups(ns)) * nk * nproj * nb * sizeof(C) : 0;
+}
+
+template <typename R>
+size_t becp_work_bytes(int nk, int nb, int nG, int nproj) {
+  const size_t least = becp_partial_bytes<R>(nk, nb, nG, nproj);
+  return sizeof(R) == 8 ? std::max(least, oz_work_bytes(8, nproj, nb, nG, nk)) : least;
 }
 
 template <typename R>
@@ -936,9 +941,9 @@ inline size_t nl_grad_scratch(addft_dtype dt, int nk, int nb, int nG, int nproj)
 }
 
 // H psi with the work buffer split as [becp | D becp | becp split-K partials | local FFT scratch].
-// The local part needs at least one band of FFT scratch (addft_work_bytes(plan, 1)); the split-K
-// partials get what remains beyond that, up to what the default number of splits uses, and becp_t
-// lowers the number of splits to fit (down to one, which needs no partials).
+// The local part needs at least one band of FFT scratch (addft_work_bytes(plan, 1)); becp gets what
+// remains beyond that, up to what it asks for, and lowers the number of splits to fit (down to one, which
+// needs no partials).
 // The projector chain (becp, split sums, D becp) only reads psi and the beta tables and
 // writes its own part of the work buffer, so it can run beside the local FFT pipeline.
 // ADDFT_HPSI_OVERLAP (read once per process): 0 = one stream; 1 (default) = the chain on a
@@ -985,7 +990,14 @@ addft_status hpsi_t(addft_plan plan, int nk, int nb, const void *psi, const void
   size_t split = 0;
   if (nproj > 0) {
     const size_t spare = (work_bytes - arrays - local_min) & ~size_t(255);
-    split = std::min(align256(nl_split_bytes<R>(nk, nb, pd.nG, nproj)), spare);
+    split = align256(nl_split_bytes<R>(nk, nb, pd.nG, nproj));
+    if (split > spare) {
+      // Short of that: up to half of what is spare where the products of FP64 go in pieces of it, else the split
+      // partials.  What a form would leave unused belongs to the transforms: their bands at once decide their time.
+      const size_t half = std::min(align256(oz_work_bytes(8, nproj, nb, pd.nG, nk)), (spare / 2) & ~size_t(255));
+      split = std::min(align256(becp_partial_bytes<R>(nk, nb, pd.nG, nproj)), spare);
+      if (sizeof(R) == 8 && oz_fits(8, nproj, nb, pd.nG, nk, (char *)work + arrays, half)) split = std::max(split, half);
+    }
   }
   C *becp = (C *)work;
   C *db = becp + (size_t)nk * nproj * nb;

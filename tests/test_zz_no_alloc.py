@@ -159,3 +159,23 @@ def test_noalloc_call_leaves_free_device_memory_unchanged():
     torch.cuda.synchronize()
     free1, _ = torch.cuda.mem_get_info()
     assert free0 == free1
+
+
+def test_noalloc_fp64_with_projectors_leaves_the_transforms_their_scratch():
+    """24^3, 64 projectors, 48 bands in FP64: the packed operands of the projector products (32 MB) do not
+    go into the static scratch, and then they may not take it from the bands of the local part (16 chunks of
+    three bands before; six chunks of three or four launches beside becp's partials)."""
+    plan, nG = _sphere_plan(24)
+    nb, P = 48, 64
+    g = torch.Generator(device="cuda").manual_seed(12)
+    psi = torch.randn((1, nb, nG), dtype=torch.complex128, device="cuda", generator=g)
+    proj = torch.randn((1, P, nG), dtype=torch.complex128, device="cuda", generator=g)
+    kin = torch.rand((1, nG), dtype=torch.float64, device="cuda", generator=g)
+    v = torch.rand(24 ** 3, dtype=torch.float64, device="cuda", generator=g) - 0.5
+    dion = torch.diag(torch.linspace(-1.0, 1.0, P, dtype=torch.float64, device="cuda"))
+    ref = ops.hpsi(plan, psi, kin, v, proj, dion)
+    out = torch.full_like(psi, float("nan"))
+    n = LIB.addft_launch_count()
+    assert _noalloc(plan, 1, psi, kin, v, proj, dion, out) == 0, LIB.addft_last_error()
+    assert LIB.addft_launch_count() - n <= 48
+    assert float((out - ref).abs().max() / ref.abs().max()) < 1e-10
