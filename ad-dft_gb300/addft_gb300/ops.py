@@ -118,9 +118,20 @@ class Plan:
             self.handle = None
 
 
+def _bands_that_fit(nbytes, limit: int, nbatch: int) -> int:
+    """Largest number of bands up to nbatch (one at least) whose scratch nbytes(bands) stays within the
+    limit; nbytes grows with the bands, in steps where another form of the transforms starts."""
+    if nbytes(nbatch) <= limit:
+        return nbatch
+    lo, hi = 1, nbatch
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (mid, hi) if nbytes(mid) <= limit else (lo, mid)
+    return lo
+
+
 def _chunk_work(plan: Plan, dtype: int, nbatch: int, extra: int = 0, max_bytes: int = 1 << 30) -> torch.Tensor:
-    per = plan.work_bytes(1, dtype) - (1 << 20)
-    nfit = max(1, min(nbatch, (max_bytes - extra - (1 << 20)) // max(per, 1)))
+    nfit = _bands_that_fit(lambda n: plan.work_bytes(n, dtype), max_bytes - extra, max(nbatch, 1))
     return workspace(extra + plan.work_bytes(nfit, dtype))
 
 
@@ -188,9 +199,7 @@ def hpsi(plan: Plan, psi: torch.Tensor, kin: torch.Tensor, v_r: torch.Tensor, pr
         dion = _c(torch.as_tensor(dion, device=psi.device).to(rdt), "dion")
     if out is None:
         out = torch.empty_like(psi)
-    per = plan.work_bytes(2, dt) - plan.work_bytes(1, dt)   # slab bytes per extra band in flight
-    base = hpsi_work_bytes(plan, dt, nk, nb, nproj, 1)
-    chunk = max(1, min(nk * nb, 1 + (max_work - base) // max(per, 1)))
+    chunk = _bands_that_fit(lambda c: hpsi_work_bytes(plan, dt, nk, nb, nproj, c), max_work, max(nk * nb, 1))
     wb = hpsi_work_bytes(plan, dt, nk, nb, nproj, chunk)
     w = workspace(wb)
     check(LIB.addft_hpsi(plan.handle, dt, nk, nb, _p(psi), _p(kin), _p(v_r), nproj, _p(proj),
@@ -314,7 +323,9 @@ def hartree(plan: Plan, bvec, omega, rho: torch.Tensor, want_potential=True):
 def local_potential(rho_plan: Plan, bvec, omega, pos, psp) -> torch.Tensor:
     pos = np.asarray(pos, dtype=np.float64).reshape(-1, 3)
     out = torch.empty(rho_plan.N, dtype=torch.float64, device="cuda")
-    w = workspace(int(LIB.addft_local_potential_work_bytes(rho_plan.handle)))
+    # enough for the phase tables of any number of atoms, or (forces included) for those of this one
+    w = workspace(min(int(LIB.addft_local_potential_work_bytes(rho_plan.handle)),
+                      int(LIB.addft_density_gradients_work_bytes(rho_plan.handle, rho_plan.handle, pos.shape[0]))))
     cs = psp.c_struct()
     check(LIB.addft_local_potential(rho_plan.handle, _d3(bvec), float(omega), pos.shape[0], _d3(pos),
                                     C.byref(cs), _p(out), _p(w), w.numel(), _stream()), "local_potential")

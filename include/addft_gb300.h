@@ -291,6 +291,7 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
 size_t addft_hpsi_work_bytes(addft_plan plan, addft_dtype dt, int nk, int nb, int nproj,
                              int nbatch_chunk);
 size_t addft_hartree_work_bytes(addft_plan plan);
+/* tables for as many atoms as there can be; fewer need less, and without them one kernel per atom and G runs */
 size_t addft_local_potential_work_bytes(addft_plan rho_plan);
 size_t addft_density_gradients_work_bytes(addft_plan wfc_plan, addft_plan rho_plan, int nat);
 size_t addft_nonlocal_gradients_work_bytes(addft_dtype dt, int nk, int nb, int nG, int nat, int nh);

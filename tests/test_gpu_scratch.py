@@ -117,3 +117,47 @@ def test_tuning_for_the_fft_kernels_reaches_every_potential(key):
         ffts = call(torch.empty(least, dtype=torch.uint8, device="cuda"), least)[cut]   # holds no other form
         assert torch.equal(call(room, room.numel())[cut], ffts), name
         assert not torch.equal(potentials(*plain, 2)[name][0](room, room.numel())[cut], ffts), name
+
+
+def test_scratch_limits_hold_where_the_products_start(monkeypatch):
+    """The wrappers' byte limits where more bands at once bring a form with larger bands."""
+    sizes = []
+    keep = ops.workspace
+    monkeypatch.setattr(ops, "workspace", lambda n: (sizes.append(n), keep(n))[1])
+    for box, nb in (((24, 24, 24), 200), ((30, 30, 32), 64), ((45, 45, 45), 20)):
+        r = [int(0.45 * n) for n in box]
+        m = np.stack(np.meshgrid(*(np.arange(-k, k + 1) for k in r), indexing="ij"), -1).reshape(-1, 3)
+        plan = ops.Plan(box, m[np.sum((m / (np.asarray(box) * 0.45)) ** 2, axis=1) <= 1.0].astype(np.int32))
+        psi = torch.zeros((1, nb, plan.nG), dtype=torch.complex128, device="cuda")
+        kin = torch.zeros((1, plan.nG), dtype=F64, device="cuda")
+        v = torch.zeros(plan.N, dtype=F64, device="cuda")
+        for limit in (12 << 20, 24 << 20, 48 << 20, 96 << 20):
+            sizes.clear()
+            ops.hpsi(plan, psi, kin, v, max_work=limit)
+            ops._chunk_work(plan, 1, nb, extra=1000, max_bytes=limit)
+            for n in sizes:
+                assert n <= limit
+            assert all(n >= limit // 4 or n >= plan.work_bytes(nb, 1) for n in sizes)
+
+
+def test_local_potential_of_few_atoms_asks_for_little():
+    """Phase tables are sized for the atoms of the call, not for the most that there can be."""
+    plan = plans()[0]
+    cell = LIB.addft_local_potential_work_bytes(plan.handle)
+    seen = []
+    keep = ops.workspace
+    ops.workspace = lambda n: (seen.append(n), keep(n))[1]
+    try:
+        ops.local_potential(plan, B, OMEGA, atoms(2), synthetic())
+    finally:
+        ops.workspace = keep
+    assert seen[0] < cell / 2
+    big = atoms(40)                                  # 40 atoms x 4e4 G: the products
+    assert 40 * plan.nG > 5e5
+    v = ops.local_potential(plan, B, OMEGA, big, synthetic())
+    w = torch.empty(al256(plan.nG * 16) + plan.nplanes * BOX[1] * BOX[2] * 16, dtype=torch.uint8, device="cuda")
+    ref = torch.empty_like(v)                        # scratch of one slab: a sincos per atom and G
+    psp = synthetic().c_struct()
+    assert LIB.addft_local_potential(plan.handle, dbl_array(B.reshape(-1)), OMEGA, 40, dbl_array(big.reshape(-1)),
+                                     C.byref(psp), p(ref), p(w), w.numel(), stream()) == 0
+    assert bool(((v - ref).abs() <= 1e-12 * ref.abs().max()).all())
