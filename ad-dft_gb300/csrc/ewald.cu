@@ -227,8 +227,9 @@ addft_status addft_ewald(const double *lattice, int nat, const double *pos, cons
   ADDFT_REQUIRE(lattice && out && nat >= 1 && pos && charges && eta > 0 && nmax >= 0, ADDFT_INVALID_ARG,
                 "ewald: bad arguments");
   ADDFT_REQUIRE(nat <= kMaxAtomsE, ADDFT_UNSUPPORTED, "ewald: nat = %d exceeds %d", nat, kMaxAtomsE);
-  ADDFT_REQUIRE(work && work_bytes >= addft_ewald_work_bytes(nat), ADDFT_INVALID_ARG,
-                "ewald: work needs %zu B", addft_ewald_work_bytes(nat));
+  // partial sums of the pairs, then of the reciprocal CTAs: as many of those as the buffer holds, four at least
+  const size_t pairs = (((size_t)nat * nat * 13 * sizeof(double)) + 255) & ~size_t(255), per = (10 + 3 * nat) * sizeof(double);
+  ADDFT_REQUIRE(work && work_bytes >= pairs + 4 * per, ADDFT_INVALID_ARG, "ewald: work needs %zu B", pairs + 4 * per);
   EwaldParams ep;
   memset(&ep, 0, sizeof(ep));
   for (int i = 0; i < 9; ++i) ep.L[i] = lattice[i];
@@ -256,10 +257,8 @@ addft_status addft_ewald(const double *lattice, int nat, const double *pos, cons
   for (int i = 0; i < 3 * nat; ++i) ep.pos[i] = pos[i];
   for (int i = 0; i < nat; ++i) ep.z[i] = charges[i];
   cudaStream_t st = as_stream(stream);
-  auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
   char *w = (char *)work;
-  double *real_part = (double *)w;
-  double *recip = (double *)(w + al((size_t)nat * nat * 13 * sizeof(double)));
+  double *real_part = (double *)w, *recip = (double *)(w + pairs);
   // translations within the cut: |a + f_i - f_j| h <= cut on every axis, h = 2 pi / |b_a|
   for (int a = 0; a < 3; ++a) {
     double lo = 0.0, hi = 0.0;
@@ -279,7 +278,7 @@ addft_status addft_ewald(const double *lattice, int nat, const double *pos, cons
   const int ns = (int)std::max<long>(1, std::min<long>(std::min<long>(nat, (terms + 255) / 256), (304 + nat - 1) / nat));
   k_ewald_real<<<dim3(nat, ns), 256, 0, st>>>(ep, real_part);
   ADDFT_TRY(check_launch("k_ewald_real"));
-  const int side = 2 * (nmax + 2) + 1, nctas = std::min(kRecipCtas, side * side);
+  const int side = 2 * (nmax + 2) + 1, nctas = (int)std::min<size_t>(std::min(kRecipCtas, side * side), (work_bytes - pairs) / per);
   const size_t sm = 2 * (size_t)kRecipChunk * nat * sizeof(double2);
   ADDFT_TRY(smem_optin(k_ewald_recip, sm));
   const int natp = (nat + 31) / 32 * 32;

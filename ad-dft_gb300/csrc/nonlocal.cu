@@ -1081,7 +1081,7 @@ inline int nl_grad_splits(int nk, int nat, int nG) {
 
 template <typename R>
 addft_status nl_grad_t(const PlanDev &pd, const GeoParams &gp, const void *Y, void *scratch, size_t scratch_bytes,
-                       double *part, cudaStream_t st) {
+                       int nsplit, double *part, cudaStream_t st) {
   using C = typename Cx<R>::T;
   // channel tables shared by the atoms, where there are several and the scratch holds them
   double *form = nullptr;
@@ -1092,7 +1092,6 @@ addft_status nl_grad_t(const PlanDev &pd, const GeoParams &gp, const void *Y, vo
   }
   size_t smem = 0;
   const int f = phase_form(pd, smem);
-  const int nsplit = nl_grad_splits(gp.nk, gp.nat, pd.nG);
   const dim3 grid(gp.nat, nsplit, gp.nk);
   auto go = [&](auto kern) {
     ADDFT_TRY(smem_optin(kern, smem));
@@ -1270,12 +1269,17 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
   const size_t o_mw = take((size_t)nk * nproj * nb * csz);
   const size_t o_y = take((size_t)nk * nproj * nG * csz);
   const size_t o_ep = take((size_t)nk * nb * sizeof(double));
-  const int nsplit = nl_grad_splits(nk, nat, nG);
-  const size_t o_gp = take((size_t)nk * nat * nsplit * 12 * sizeof(double));
-  const size_t bwb = nl_grad_scratch(dt, nk, nb, nG, nproj);   // becp's partials, then the operands of Y
-  const size_t o_bw = take(bwb);
+  // fewer splits of the G range and less scratch for the contractions, where the buffer is short of what is asked for
+  const size_t partials = align256(dt == ADDFT_F64 ? becp_partial_bytes<double>(nk, nb, nG, nproj)
+                                                   : becp_partial_bytes<float>(nk, nb, nG, nproj));
+  auto sums = [&](int n) { return (size_t)nk * nat * n * 12 * sizeof(double); };
+  int nsplit = nl_grad_splits(nk, nat, nG);
+  while (nsplit > 1 && off + align256(sums(nsplit)) + partials > work_bytes) --nsplit;
+  const size_t o_gp = take(sums(nsplit)), o_bw = off;
+  off += partials;
   ADDFT_REQUIRE(work_bytes >= off, ADDFT_INVALID_ARG, "nonlocal_gradients: work needs %zu B, got %zu B",
                 off, work_bytes);
+  const size_t bwb = work_bytes - o_bw;   // becp's partials or operands, then the operands of Y
   char *w = (char *)work;
   ADDFT_TRY(addft_projectors(plan, dt, bvec, omega, nk, kpts, nat, pos, psp, w + o_proj, stream));
   if (dt == ADDFT_F64) {
@@ -1286,7 +1290,7 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
                                             nproj, nG, w + o_y, (size_t)nproj * nG, w + o_bw, bwb, st)));
     ADDFT_TRY(nl_energy_t<double>(w + o_becp, w + o_db, nk, nproj, nb, wocc, (double *)(w + o_ep), st));
     // the projector table has been used; its place takes the channel tables
-    ADDFT_TRY(nl_grad_t<double>(plan->dev, gp, w + o_y, w + o_proj, (size_t)nk * nproj * nG * csz,
+    ADDFT_TRY(nl_grad_t<double>(plan->dev, gp, w + o_y, w + o_proj, (size_t)nk * nproj * nG * csz, nsplit,
                                 (double *)(w + o_gp), st));
   } else {
     ADDFT_TRY(becp_t<float>(nk, nb, nG, nproj, w + o_proj, psi, w + o_becp, w + o_bw, bwb, st));
@@ -1295,7 +1299,7 @@ addft_status addft_nonlocal_gradients(addft_plan plan, addft_dtype dt, const dou
     ADDFT_TRY((apply_t<float, true, false>(w + o_mw, 1, nb, (size_t)nproj * nb, psi, (size_t)nb * nG, nk, nb,
                                            nproj, nG, w + o_y, (size_t)nproj * nG, w + o_bw, bwb, st)));
     ADDFT_TRY(nl_energy_t<float>(w + o_becp, w + o_db, nk, nproj, nb, wocc, (double *)(w + o_ep), st));
-    ADDFT_TRY(nl_grad_t<float>(plan->dev, gp, w + o_y, w + o_proj, (size_t)nk * nproj * nG * csz,
+    ADDFT_TRY(nl_grad_t<float>(plan->dev, gp, w + o_y, w + o_proj, (size_t)nk * nproj * nG * csz, nsplit,
                                (double *)(w + o_gp), st));
   }
   k_nl_grad_final<<<(1 + 3 * nat + 9 + 3) / 4, 128, 0, st>>>((const double *)(w + o_ep), nk * nb,

@@ -161,3 +161,61 @@ def test_local_potential_of_few_atoms_asks_for_little():
     assert LIB.addft_local_potential(plan.handle, dbl_array(B.reshape(-1)), OMEGA, 40, dbl_array(big.reshape(-1)),
                                      C.byref(psp), p(ref), p(w), w.numel(), stream()) == 0
     assert bool(((v - ref).abs() <= 1e-12 * ref.abs().max()).all())
+
+
+@pytest.mark.parametrize("nat", [1, 2, 33, 70, 256])
+def test_ewald_takes_less_scratch(nat):
+    """From the scratch that the sums over pairs and a few reciprocal CTAs need (what was enough before the
+    reciprocal sum kept partial sums per CTA) up to what the size query returns."""
+    pos, z = atoms(nat), np.random.default_rng(5).uniform(0.5, 4.0, nat)
+    nmax = 3
+    whole = ops.ewald(LAT, pos, z, nmax=nmax)
+    asked = LIB.addft_ewald_work_bytes(nat)
+    pairs = al256(nat * nat * 13 * 8)
+    for nbytes in (pairs + 24320 + 256 + al256(nat * 24), pairs + 4 * (10 + 3 * nat) * 8, (pairs + asked) // 2):
+        w = torch.full((nbytes + 4096,), 0xA5, dtype=torch.uint8, device="cuda")
+        out = torch.empty_like(whole)
+        assert LIB.addft_ewald(dbl_array(LAT.reshape(-1)), nat, dbl_array(pos.reshape(-1)), dbl_array(z), 0.9, nmax,
+                               p(out), p(w), nbytes, stream()) == 0
+        # sums in another order: a few hundred roundings of the largest output
+        assert bool(((out - whole).abs() <= 1e-12 * whole.abs().max()).all()), nbytes
+        assert bool((w[nbytes:] == 0xA5).all())
+
+
+@pytest.mark.parametrize("dt", [1, 0])
+@pytest.mark.parametrize("nat,nb", [(1, 3), (6, 40), (40, 20)])
+def test_nonlocal_gradients_take_less_scratch(dt, nat, nb):
+    plan = ops.Plan(BOX, sphere(0.24))
+    psp = synthetic()
+    nh, nG, nk, csz = psp.nh, plan.nG, 1, 16 if dt else 8
+    P = nat * nh
+    pos = atoms(nat)
+    g = torch.Generator(device="cuda").manual_seed(nat)
+    psi = torch.randn((nk, nb, nG), dtype=torch.complex128, device="cuda", generator=g) / nG ** 0.5
+    w_occ = torch.rand((nk, nb), dtype=F64, device="cuda", generator=g)
+    dion = torch.diag(torch.linspace(-1.0, 1.0, P, dtype=F64, device="cuda"))
+    if not dt:
+        psi = psi.to(torch.complex64)
+    whole = ops.nonlocal_gradients(plan, B, OMEGA, np.zeros((1, 3)), pos, psp, psi, w_occ, dion)
+    asked = LIB.addft_nonlocal_gradients_work_bytes(dt, nk, nb, nG, nat, nh)
+    # the same split-K partial sums as the size query's least (becp's default splits), one range of G
+    tiles = -(-P // 32) * -(-nb // 64) * nk
+    ns = max(1, min(-(-8 * 152 // tiles), -(-nG // 64)))
+    partials = al256((ns + -(-ns // 8)) * nk * P * nb * csz) if ns > 1 else 0
+    least = 2 * al256(nk * P * nG * csz) + 3 * al256(nk * P * nb * csz) + al256(nk * nb * 8) + al256(nk * P * 12 * 8)
+    d = dion.to(F64 if dt else torch.float32).contiguous()
+    cs = psp.c_struct()
+    tol = 1e-12 if dt else 2e-6
+    taken = 0
+    for nbytes in sorted({least + partials, least + 4 * partials, (least + partials + asked) // 2, asked}):
+        w = torch.full((nbytes + 4096,), 0xA5, dtype=torch.uint8, device="cuda")
+        out = torch.empty_like(whole)
+        st = LIB.addft_nonlocal_gradients(plan.handle, dt, dbl_array(B.reshape(-1)), OMEGA, nk, dbl_array([0.0] * 3), nb,
+                                          nat, dbl_array(pos.reshape(-1)), C.byref(cs), p(psi), p(w_occ), p(d), p(out),
+                                          p(w), nbytes, stream())
+        assert st == 0 or (st == 1 and nbytes == least + partials)   # the test's guess of the least partials
+        if st == 0:
+            taken += nbytes < asked
+            assert bool(((out - whole).abs() <= tol * whole.abs().max()).all()), nbytes
+            assert bool((w[nbytes:] == 0xA5).all())
+    assert taken >= 1 or asked <= least + 4 * partials
