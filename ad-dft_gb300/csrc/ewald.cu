@@ -36,13 +36,15 @@ constexpr double kRealCut = 10.0;
 __global__ void __launch_bounds__(256) k_ewald_real(EwaldParams ep, double *__restrict__ partial) {
   const int i = blockIdx.x, ns = gridDim.y;
   const int s1 = 2 * ep.nr[0] + 1, s2 = 2 * ep.nr[1] + 1, s3 = 2 * ep.nr[2] + 1, nt = s1 * s2 * s3;
+  // translations of one pair fit 32 bits, pairs times translations need not (a small eta reaches far)
+  const long total = (long)ep.nat * nt, stride = (long)ns * blockDim.x;
   const double rp = 1.1283791670955125739 * ep.eta;   // 2 eta / sqrt(pi)
   const double cut2 = (kRealCut / ep.eta) * (kRealCut / ep.eta);
   double acc[13];
 #pragma unroll
   for (int t = 0; t < 13; ++t) acc[t] = 0.0;
-  for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < ep.nat * nt; q += ns * blockDim.x) {
-    const int j = q / nt, t = q - j * nt;
+  for (long q = blockIdx.y * blockDim.x + threadIdx.x; q < total; q += stride) {
+    const int j = total <= 0x7fffffff ? (int)q / nt : (int)(q / nt), t = (int)(q - (long)j * nt);
     const int a = t / (s2 * s3) - ep.nr[0], b = (t / s3) % s2 - ep.nr[1], c = t % s3 - ep.nr[2];
     if (i == j && a == 0 && b == 0 && c == 0) continue;
     double d[3];
@@ -274,7 +276,9 @@ addft_status addft_ewald(const double *lattice, int nat, const double *pos, cons
     ep.nr[a] = reach < nmax ? (int)reach : nmax;
   }
   // splits of an atom's sum: about 2 CTAs per SM, at least 256 terms each; the buffer holds nat
-  const long terms = (long)nat * (2 * ep.nr[0] + 1) * (2 * ep.nr[1] + 1) * (2 * ep.nr[2] + 1);
+  const double cells = (2.0 * ep.nr[0] + 1) * (2.0 * ep.nr[1] + 1) * (2.0 * ep.nr[2] + 1);
+  ADDFT_REQUIRE(cells <= 2147483647.0, ADDFT_UNSUPPORTED, "ewald: %.0f translations within reach", cells);
+  const long terms = (long)nat * (long)cells;
   const int ns = (int)std::max<long>(1, std::min<long>(std::min<long>(nat, (terms + 255) / 256), (304 + nat - 1) / nat));
   k_ewald_real<<<dim3(nat, ns), 256, 0, st>>>(ep, real_part);
   ADDFT_TRY(check_launch("k_ewald_real"));

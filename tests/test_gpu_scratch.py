@@ -92,7 +92,7 @@ def plans():
     return ops.Plan(BOX, sphere(0.45)), ops.Plan(BOX, sphere(0.24)), ops.Plan(BOX, full())
 
 
-@pytest.mark.parametrize("nat", [1, 5])
+@pytest.mark.parametrize("nat", [1, 5, 40])   # 40 atoms x 4e4 G: phases as products, with less scratch directly
 @pytest.mark.parametrize("name", ["hartree", "vloc", "kerker", "grads"])
 def test_potentials_take_the_scratch_of_one_slab(name, nat):
     call, least, asked = potentials(*plans(), nat)[name]
