@@ -323,9 +323,11 @@ def hartree(plan: Plan, bvec, omega, rho: torch.Tensor, want_potential=True):
 def local_potential(rho_plan: Plan, bvec, omega, pos, psp) -> torch.Tensor:
     pos = np.asarray(pos, dtype=np.float64).reshape(-1, 3)
     out = torch.empty(rho_plan.N, dtype=torch.float64, device="cuda")
-    # enough for the phase tables of any number of atoms, or (forces included) for those of this one
-    w = workspace(min(int(LIB.addft_local_potential_work_bytes(rho_plan.handle)),
-                      int(LIB.addft_density_gradients_work_bytes(rho_plan.handle, rho_plan.handle, pos.shape[0]))))
+    # the phase tables of these atoms (forces included), or, where that is less, of as many as there can be
+    need = int(LIB.addft_density_gradients_work_bytes(rho_plan.handle, rho_plan.handle, pos.shape[0]))
+    if pos.shape[0] > 8:
+        need = min(need, int(LIB.addft_local_potential_work_bytes(rho_plan.handle)))
+    w = workspace(need)
     cs = psp.c_struct()
     check(LIB.addft_local_potential(rho_plan.handle, _d3(bvec), float(omega), pos.shape[0], _d3(pos),
                                     C.byref(cs), _p(out), _p(w), w.numel(), _stream()), "local_potential")

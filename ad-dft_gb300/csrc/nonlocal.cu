@@ -21,7 +21,6 @@ struct GeoParams {
   double inv_sqrt_omega;
   int nat, nh, nk;
   double pos[kMaxAtoms * 3];
-  Turns frac[kMaxAtoms * 3];  // b_a . R / 2 pi: phases e^{-2 pi i m frac}
   double kpt[kMaxK * 3];
   // per projector channel c in [0, nh): radial index, l, m
   int ch_rad[kMaxNh], ch_l[kMaxNh], ch_m[kMaxNh];
@@ -41,8 +40,6 @@ inline addft_status make_geo(GeoParams &g, const double *bvec, double omega, int
   g.nat = nat;
   g.nk = nk;
   for (int i = 0; i < 3 * nat; ++i) g.pos[i] = pos[i];
-  for (int i = 0; i < nat; ++i)
-    for (int a = 0; a < 3; ++a) g.frac[3 * i + a] = phase_turns(bvec + 3 * a, pos + 3 * i);
   for (int i = 0; i < 3 * nk; ++i) g.kpt[i] = kpts ? kpts[i] : 0.0;
   g.nh = 0;
   if (psp) {
@@ -149,6 +146,24 @@ __device__ __forceinline__ void kg_vec(const PlanDev &pd, const GeoParams &gp, i
   }
 }
 
+// b_a . R / 2 pi of the atoms, for phases e^{-2 pi i m frac}: a parameter of its own (12 KB) that only the kernels
+// with tables take
+struct Fracs { Turns f[kMaxAtoms * 3]; };
+struct NoFracs {};
+template <int FORM>
+using FracsOf = std::conditional_t<FORM == 0, NoFracs, Fracs>;
+
+template <int FORM>
+FracsOf<FORM> make_fracs(const GeoParams &gp) {
+  FracsOf<FORM> fr;
+  if constexpr (FORM != 0) {
+    memset(&fr, 0, sizeof(fr));
+    for (int i = 0; i < gp.nat; ++i)
+      for (int a = 0; a < 3; ++a) fr.f[3 * i + a] = phase_turns(gp.B + 3 * a, gp.pos + 3 * i);
+  }
+  return fr;
+}
+
 // The phases e^{-i(k+G).R} of one atom, from tables in shared memory: with G = sum_a m_a b_a they
 // are e12[m1, m2] e3[m3], e12 holding e^{-ik.R} too, so a phase costs one complex product where
 // its sincos costs some 60 FP64 instructions (GB300 issues under two per SM and cycle).
@@ -178,34 +193,36 @@ inline int phase_form(const PlanDev &pd, size_t &bytes) {
 }
 
 template <int FORM>
-__device__ __forceinline__ PhaseTab phase_build(const PlanDev &pd, const GeoParams &gp, int i, int k, double2 *sm) {
+__device__ __forceinline__ PhaseTab phase_build(const PlanDev &pd, const GeoParams &gp, const FracsOf<FORM> &fr, int i,
+                                                int k, double2 *sm) {
   PhaseTab t;
-  t.M1 = pd.mmax[0];
-  t.M2 = pd.mmax[1];
-  t.M3 = pd.mmax[2];
-  t.e1 = sm;
-  t.e2 = t.e1 + 2 * t.M1 + 1;
-  t.e3 = t.e2 + 2 * t.M2 + 1;
-  t.e12 = FORM == 2 ? t.e3 + 2 * t.M3 + 1 : nullptr;
-  if (FORM == 0) return t;
-  const int n1 = 2 * t.M1 + 1, n2 = 2 * t.M2 + 1, n3 = 2 * t.M3 + 1;
-  const double kr = gp.kpt[3 * k] * gp.pos[3 * i] + gp.kpt[3 * k + 1] * gp.pos[3 * i + 1] +
-                    gp.kpt[3 * k + 2] * gp.pos[3 * i + 2];
-  for (int t0 = threadIdx.x; t0 < n1 + n2 + n3; t0 += blockDim.x) {
-    const int ax = t0 < n1 ? 0 : (t0 < n1 + n2 ? 1 : 2);
-    const int m = ax == 0 ? t0 - t.M1 : (ax == 1 ? t0 - n1 - t.M2 : t0 - n1 - n2 - t.M3);
-    double2 e = phase_exp(m, gp.frac[3 * i + ax]);
-    if (ax == 0 && kr != 0.0) {
-      double sn, cs;
-      sincos(kr, &sn, &cs);
-      e = cmul(e, make_double2(cs, -sn));
+  if constexpr (FORM != 0) {
+    t.M1 = pd.mmax[0];
+    t.M2 = pd.mmax[1];
+    t.M3 = pd.mmax[2];
+    t.e1 = sm;
+    t.e2 = t.e1 + 2 * t.M1 + 1;
+    t.e3 = t.e2 + 2 * t.M2 + 1;
+    t.e12 = FORM == 2 ? t.e3 + 2 * t.M3 + 1 : nullptr;
+    const int n1 = 2 * t.M1 + 1, n2 = 2 * t.M2 + 1, n3 = 2 * t.M3 + 1;
+    const double kr = gp.kpt[3 * k] * gp.pos[3 * i] + gp.kpt[3 * k + 1] * gp.pos[3 * i + 1] +
+                      gp.kpt[3 * k + 2] * gp.pos[3 * i + 2];
+    for (int t0 = threadIdx.x; t0 < n1 + n2 + n3; t0 += blockDim.x) {
+      const int ax = t0 < n1 ? 0 : (t0 < n1 + n2 ? 1 : 2);
+      const int m = ax == 0 ? t0 - t.M1 : (ax == 1 ? t0 - n1 - t.M2 : t0 - n1 - n2 - t.M3);
+      double2 e = phase_exp(m, fr.f[3 * i + ax]);
+      if (ax == 0 && kr != 0.0) {
+        double sn, cs;
+        sincos(kr, &sn, &cs);
+        e = cmul(e, make_double2(cs, -sn));
+      }
+      sm[t0] = e;
     }
-    sm[t0] = e;
-  }
-  __syncthreads();
-  if (FORM == 2) {
-    for (int p = threadIdx.x; p < n1 * n2; p += blockDim.x) t.e12[p] = cmul(t.e1[p / n2], t.e2[p % n2]);
     __syncthreads();
+    if (FORM == 2) {
+      for (int p = threadIdx.x; p < n1 * n2; p += blockDim.x) t.e12[p] = cmul(t.e1[p / n2], t.e2[p % n2]);
+      __syncthreads();
+    }
   }
   return t;
 }
@@ -224,6 +241,27 @@ __device__ __forceinline__ double2 phase_at(const PlanDev &pd, const GeoParams &
   const double2 a = FORM == 2 ? t.e12[m1 * (2 * t.M2 + 1) + m2] : cmul(t.e1[m1], t.e2[m2]);
   return cmul(a, t.e3[m3]);
 }
+
+// Projectors of few atoms, in one launch: a thread evaluates form factor and phase of its (p, g).  Up to
+// kDirectProj of them (k points x projectors x G), 35 to 50 us a call from Python against 45 to 58 for the three
+// launches with tables: 8 k points of 2 atoms, 925 G, 39 / 55; one of 16 atoms, 3,071 G, 43 / 59; 236,800
+// 49 / 57; beyond, 263,000 52 / 50 to 55, 393,000 72 / 56 to 66, 786,000 136 / 58.
+template <typename R>
+__global__ void __launch_bounds__(128) k_proj_direct(PlanDev pd, GeoParams gp, typename Cx<R>::T *__restrict__ proj) {
+  using C = typename Cx<R>::T;
+  const int g = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.y, k = blockIdx.z;
+  if (g >= pd.nG) return;
+  const int i = p / gp.nh, c = p - i * gp.nh;
+  double G[3], v[3], sn, cs;
+  kg_vec(pd, gp, g, k, G, v);
+  const double a = proj_eval(gp, c, v[0], v[1], v[2]).beta * gp.inv_sqrt_omega;
+  sincos(v[0] * gp.pos[3 * i] + v[1] * gp.pos[3 * i + 1] + v[2] * gp.pos[3 * i + 2], &sn, &cs);
+  C o;
+  o.x = (R)(a * cs);
+  o.y = (R)(-a * sn);   // e^{-i v.R}
+  proj[((size_t)k * gridDim.y + p) * pd.nG + g] = o;
+}
+constexpr double kDirectProj = 3e5;
 
 // beta~_c(|k+G|) Y_lm(k+G) / sqrt(omega) of every channel, once per G instead of once per atom and
 // G: as doubles in the rows of the last atom of proj (8 or 16 bytes per element), which
@@ -246,11 +284,11 @@ k_proj_forms(PlanDev pd, GeoParams gp, typename Cx<R>::T *__restrict__ proj) {
 // every (p, G) took 1,038 us for 256 projectors x 23,847 G, 70 us so.
 template <typename R, int FORM>
 __global__ void __launch_bounds__(256)
-k_projectors(PlanDev pd, GeoParams gp, int i0, int per, typename Cx<R>::T *__restrict__ proj) {
+k_projectors(PlanDev pd, GeoParams gp, FracsOf<FORM> fr, int i0, int per, typename Cx<R>::T *__restrict__ proj) {
   using C = typename Cx<R>::T;
   extern __shared__ __align__(16) double2 ph_smem[];
   const int i = i0 + blockIdx.y, k = blockIdx.z;
-  const PhaseTab t = phase_build<FORM>(pd, gp, i, k, ph_smem);
+  const PhaseTab t = phase_build<FORM>(pd, gp, fr, i, k, ph_smem);
   const C *form = proj + ((size_t)k * gp.nat + gp.nat - 1) * gp.nh * pd.nG;
   C *out = proj + ((size_t)k * gp.nat + i) * gp.nh * pd.nG;
   const int g1 = min(pd.nG, (int)(blockIdx.x + 1) * per);
@@ -583,11 +621,11 @@ k_nl_forms(PlanDev pd, GeoParams gp, double *__restrict__ form) {
 
 template <typename R, int FORM>
 __global__ void __launch_bounds__(256, 2)
-k_nl_grad(PlanDev pd, GeoParams gp, const typename Cx<R>::T *__restrict__ Y, const double *__restrict__ form,
+k_nl_grad(PlanDev pd, GeoParams gp, FracsOf<FORM> fr, const typename Cx<R>::T *__restrict__ Y, const double *__restrict__ form,
           int nsplit, double *__restrict__ partial) {
   extern __shared__ __align__(16) double2 ph_smem[];
   const int i = blockIdx.x, sp = blockIdx.y, k = blockIdx.z;
-  const PhaseTab t = phase_build<FORM>(pd, gp, i, k, ph_smem);
+  const PhaseTab t = phase_build<FORM>(pd, gp, fr, i, k, ph_smem);
   const auto *Yi = Y + ((size_t)k * gp.nat + i) * gp.nh * pd.nG;
   const double *fk = form ? form + (size_t)k * gp.nh * 4 * pd.nG : nullptr;
   const int per = (pd.nG + nsplit - 1) / nsplit;
@@ -1049,12 +1087,13 @@ template <typename R, int FORM>
 addft_status projectors_form(const PlanDev &pd, const GeoParams &gp, size_t smem, typename Cx<R>::T *proj,
                              cudaStream_t st) {
   ADDFT_TRY(smem_optin(k_projectors<R, FORM>, smem));
+  const auto fr = make_fracs<FORM>(gp);
   // about 4 CTAs per SM, each with enough G to pay for its phase tables
   auto go = [&](int i0, int n) {
     int chunks = (4 * 152 + n * gp.nk - 1) / (n * gp.nk);
     chunks = std::max(1, std::min(chunks, (pd.nG + 1023) / 1024));
     const int per = ((pd.nG + chunks - 1) / chunks + 255) / 256 * 256;
-    k_projectors<R, FORM><<<dim3((pd.nG + per - 1) / per, n, gp.nk), 256, smem, st>>>(pd, gp, i0, per, proj);
+    k_projectors<R, FORM><<<dim3((pd.nG + per - 1) / per, n, gp.nk), 256, smem, st>>>(pd, gp, fr, i0, per, proj);
     return check_launch("k_projectors");
   };
   if (gp.nat > 1) ADDFT_TRY(go(0, gp.nat - 1));
@@ -1064,14 +1103,15 @@ addft_status projectors_form(const PlanDev &pd, const GeoParams &gp, size_t smem
 template <typename R>
 addft_status projectors_t(const PlanDev &pd, const GeoParams &gp, void *proj, cudaStream_t st) {
   using C = typename Cx<R>::T;
+  size_t smem = 0;
+  const int form = phase_form(pd, smem);
+  if (form == 0 || (double)gp.nk * gp.nat * gp.nh * pd.nG < kDirectProj) {
+    k_proj_direct<R><<<dim3((pd.nG + 127) / 128, gp.nat * gp.nh, gp.nk), 128, 0, st>>>(pd, gp, (C *)proj);
+    return check_launch("k_proj_direct");
+  }
   k_proj_forms<R><<<dim3((pd.nG + 127) / 128, gp.nk), 128, 0, st>>>(pd, gp, (C *)proj);
   ADDFT_TRY(check_launch("k_proj_forms"));
-  size_t smem = 0;
-  switch (phase_form(pd, smem)) {
-    case 2: return projectors_form<R, 2>(pd, gp, smem, (C *)proj, st);
-    case 1: return projectors_form<R, 1>(pd, gp, smem, (C *)proj, st);
-    default: return projectors_form<R, 0>(pd, gp, smem, (C *)proj, st);
-  }
+  return form == 2 ? projectors_form<R, 2>(pd, gp, smem, (C *)proj, st) : projectors_form<R, 1>(pd, gp, smem, (C *)proj, st);
 }
 
 // splits of the gradients' G range per atom: about four CTAs per SM, at least 256 G each
@@ -1093,12 +1133,14 @@ addft_status nl_grad_t(const PlanDev &pd, const GeoParams &gp, const void *Y, vo
   size_t smem = 0;
   const int f = phase_form(pd, smem);
   const dim3 grid(gp.nat, nsplit, gp.nk);
-  auto go = [&](auto kern) {
+  auto go = [&](auto kern, const auto &fr) {
     ADDFT_TRY(smem_optin(kern, smem));
-    kern<<<grid, 256, smem, st>>>(pd, gp, (const C *)Y, form, nsplit, part);
+    kern<<<grid, 256, smem, st>>>(pd, gp, fr, (const C *)Y, form, nsplit, part);
     return check_launch("k_nl_grad");
   };
-  return f == 2 ? go(k_nl_grad<R, 2>) : f == 1 ? go(k_nl_grad<R, 1>) : go(k_nl_grad<R, 0>);
+  return f == 2   ? go(k_nl_grad<R, 2>, make_fracs<2>(gp))
+         : f == 1 ? go(k_nl_grad<R, 1>, make_fracs<1>(gp))
+                  : go(k_nl_grad<R, 0>, make_fracs<0>(gp));
 }
 
 // addft_hpsi on the caller's stream only (no second stream, no events): the form the

@@ -53,7 +53,6 @@ struct ShellGeo {
   double omega;
   int nat;
   double pos[kMaxAtomsP * 3];
-  Turns frac[kMaxAtomsP * 3];   // b_a . R / 2 pi
   double vamp, vsig;
   int kind, nrad;      // kind 1: tabulated smooth part (function nrad of rt) + Coulomb tail
   RadialTab rt;
@@ -161,12 +160,15 @@ struct PhaseMats {
   int n1, n2, n3, nax;
 };
 
-__global__ void k_axis_phases(ShellGeo sg, PhaseMats pm) {
+// b_a . R / 2 pi of the atoms, a parameter of the one kernel that reads them
+struct ShellFracs { Turns f[kMaxAtomsP * 3]; };
+
+__global__ void k_axis_phases(ShellFracs fr, PhaseMats pm) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
   if (t >= pm.nax) return;
   const int a = t < pm.n1 ? 0 : (t < pm.n1 + pm.n2 ? 1 : 2);
   const int m = a == 0 ? t - pm.n1 / 2 : (a == 1 ? t - pm.n1 - pm.n2 / 2 : t - pm.n1 - pm.n2 - pm.n3 / 2);
-  pm.ax[(size_t)i * pm.nax + t] = phase_exp(m, sg.frac[3 * i + a]);
+  pm.ax[(size_t)i * pm.nax + t] = phase_exp(m, fr.f[3 * i + a]);
 }
 
 __global__ void k_col_phases(PlanDev pd, int nat, PhaseMats pm) {
@@ -363,8 +365,6 @@ inline addft_status make_shell(ShellGeo &sg, const double *bvec, double omega, i
   sg.omega = omega;
   sg.nat = nat;
   for (int i = 0; i < 3 * nat; ++i) sg.pos[i] = pos[i];
-  for (int i = 0; i < nat; ++i)
-    for (int a = 0; a < 3; ++a) sg.frac[3 * i + a] = phase_turns(bvec + 3 * a, pos + 3 * i);
   if (psp) {
     ADDFT_REQUIRE(psp->kind == 0 || (psp->kind == 1 && psp->tab && psp->nq >= 2 && psp->dq > 0),
                   ADDFT_INVALID_ARG, "psp: kind 0, or kind 1 with tab, nq >= 2, dq > 0");
@@ -450,7 +450,11 @@ inline addft_status phase_setup(const PlanDev &pd, const ShellGeo &sg, bool forc
   pm.c = (double2 *)take(std::max((size_t)pd.nrows * pm.n3, forces ? 2 * (size_t)pd.nrows * sg.nat : 0) * sizeof(double2));
   pm.oz = w;
   pm.oz_bytes = (char *)work + need - w;
-  k_axis_phases<<<dim3((pm.nax + 127) / 128, sg.nat), 128, 0, st>>>(sg, pm);
+  ShellFracs fr;
+  memset(&fr, 0, sizeof(fr));
+  for (int i = 0; i < sg.nat; ++i)
+    for (int a = 0; a < 3; ++a) fr.f[3 * i + a] = phase_turns(sg.B + 3 * a, sg.pos + 3 * i);
+  k_axis_phases<<<dim3((pm.nax + 127) / 128, sg.nat), 128, 0, st>>>(fr, pm);
   ADDFT_TRY(check_launch("k_axis_phases"));
   const size_t n = (size_t)pd.nrows * sg.nat;
   k_col_phases<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(pd, sg.nat, pm);
