@@ -65,7 +65,9 @@ def energy_terms(geo: Cell, static: Static, state: SCFState, active=ALL_TAGS, ca
         out["nonlocal"] = ops.nonlocal_energy(b, cache.dion, wocc_of(static, state.occ))[0]
     if "ewald" in active:
         out["ewald"] = _ewald(static, geo, cache)[0]
-    return {k: float(v) for k, v in out.items()}
+    out = {k: float(v) for k, v in out.items()}
+    ops.raise_on_device_errors()
+    return out
 
 
 def total_energy(geo, static, state, active=ALL_TAGS):
@@ -84,7 +86,9 @@ def energy_variational(geo: Cell, static: Static, state: SCFState, cache: Geomet
     e_xc = scale * (sums[0] + sums[1])
     e_dc = scale * sums[2]
     e_ii = _ewald(static, geo, cache)[0]
-    return float(e_band - parts["e_h"][0] + e_xc - e_dc + e_ii)
+    e = float(e_band - parts["e_h"][0] + e_xc - e_dc + e_ii)
+    ops.raise_on_device_errors()
+    return e
 
 
 def entropy(occ: torch.Tensor, kweights: torch.Tensor) -> torch.Tensor:
@@ -127,7 +131,9 @@ def envelope_gradients(geo: Cell, static: Static, state: SCFState, cache: Geomet
     ew = _ewald(static, geo, cache)
     dR = dR + ew[1:1 + 3 * nat].reshape(nat, 3)
     deps = deps + ew[1 + 3 * nat:].reshape(3, 3)
-    return dR.cpu().numpy(), deps.cpu().numpy()
+    dR, deps = dR.cpu().numpy(), deps.cpu().numpy()
+    ops.raise_on_device_errors()
+    return dR, deps
 
 
 def forces_from_dR(dR) -> np.ndarray:

@@ -24,6 +24,16 @@ def require_cuda():
         raise RuntimeError("addft_gb300 needs a CUDA device (GB300, sm_103a); there is no CPU path")
 
 
+def raise_on_device_errors() -> None:
+    """Raises AddftError when a bounded wait of a tensor-core kernel ran out since the last look: the kernel
+    then returned without results, and its launch had reported none.  Synchronises; the solvers look where they have
+    just read a result."""
+    bits = int(LIB.addft_tc05_status())
+    if bits:
+        raise _lib.AddftError(f"a tensor-core kernel gave up waiting (status 0x{bits:x}): results since the last "
+                              "check are not valid")
+
+
 def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 

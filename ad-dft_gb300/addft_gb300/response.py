@@ -358,6 +358,7 @@ def implicit_grad(geo: Cell, static: Static, state: SCFState, g_n: torch.Tensor,
     dR, deps = _map_theta_vjp(resp, lam)
     dR = dR.cpu().numpy()
     deps = deps.cpu().numpy()
+    ops.raise_on_device_errors()
     if dL_dR is not None:
         dR = dR + np.asarray(dL_dR)
     if dL_deps is not None:

@@ -814,6 +814,7 @@ def solve_scf(geo: Cell, static: Static, alpha=0.9, gg0=0.5, tol=1e-10, max_iter
     v_eff, _ = effective_potential(static, cache, rho)
     eig, psi, eres = eigs.solve(v_eff, 1e-11, refine=fp32, final=True)
     occ, mu = occupations(static, eig)
+    ops.raise_on_device_errors()
     if stats is not None:
         stats.update(napply64=eigs.napply64, napply32=eigs.napply32, iters=it, eig_resid=eres)
     return SCFState(psi=psi, eig=eig, occ=occ, mu=mu, rho_r=rho, n_iter=it, residual=res)

@@ -855,7 +855,7 @@ addft_status d64_from_real(const PlanDev &pd, int nbatch, const void *in, bool i
 unsigned d64_status() {
   unsigned v = 0, z = 0;
   if (cudaMemcpyFromSymbol(&v, g_d64_error, sizeof(v)) != cudaSuccess) return 0xffffffffu;
-  cudaMemcpyToSymbol(g_d64_error, &z, sizeof(z));
+  if (v) cudaMemcpyToSymbol(g_d64_error, &z, sizeof(z));
   return v;
 }
 

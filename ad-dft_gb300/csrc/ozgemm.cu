@@ -791,7 +791,7 @@ addft_status oz_gemm(int digits, int M, int N, int K, int batch, const OzMat &A,
 unsigned oz_status() {
   unsigned v = 0, z = 0;
   if (cudaMemcpyFromSymbol(&v, g_oz_error, sizeof(v)) != cudaSuccess) return 0xffffffffu;
-  cudaMemcpyToSymbol(g_oz_error, &z, sizeof(z));
+  if (v) cudaMemcpyToSymbol(g_oz_error, &z, sizeof(z));
   return v;
 }
 

@@ -918,7 +918,7 @@ extern "C" {
 unsigned addft_tc05_status(void) {
   unsigned v = 0, z = 0;
   if (cudaMemcpyFromSymbol(&v, addft::g_tc05_error, sizeof(v)) != cudaSuccess) return 0xffffffffu;
-  cudaMemcpyToSymbol(addft::g_tc05_error, &z, sizeof(z));
+  if (v) cudaMemcpyToSymbol(addft::g_tc05_error, &z, sizeof(z));
   return v | addft::oz_status() | addft::d64_status();
 }
 
