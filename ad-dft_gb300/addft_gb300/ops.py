@@ -356,9 +356,10 @@ def kerker(full_plan: Plan, bvec, x: torch.Tensor, alpha: float, gg0: float) -> 
 
 def zgemm_df(a: torch.Tensor, b: torch.Tensor, conj_a: bool = False, conj_b: bool = False,
              out: torch.Tensor = None) -> torch.Tensor:
-    """op(a) @ op(b) for complex128 matrices (any strides; op = conjugate when asked) in
-    double-float arithmetic on the FP32 pipes, ~1e-14 relative: the subspace products of
-    the refinement (solver/davidson.py:48, :51-52, :59-61).  conj(x) @ y.T is
+    """op(a) @ op(b) for complex128 matrices (any strides; op = conjugate when asked) as digit products
+    on the tensor cores, 55 bits below the largest component of each row of a and column of b: errors are about
+    sqrt(K) 2^-54 of the product of those two, whatever the size of the output.  The subspace products
+    of the refinement (solver/davidson.py:48, :51-52, :59-61).  conj(x) @ y.T is
     zgemm_df(x, y.transpose(0, 1), conj_a=True) without a copy."""
     if a.dtype != torch.complex128 or b.dtype != torch.complex128 or not (a.is_cuda and b.is_cuda):
         raise TypeError("zgemm_df: complex128 CUDA tensors expected")

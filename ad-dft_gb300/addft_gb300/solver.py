@@ -315,16 +315,17 @@ def _ritz_fp64(X, HX):
 FP32_APPLY_ERR = 8 * 6e-8
 
 # The refinement's FP64 subspace products (projections off X, Rayleigh-Ritz at the
-# anchors, rotations of X and H X) run in double-float arithmetic on the FP32 pipes
-# (ops.zgemm_df, ~1e-14 relative) unless ADDFT_DF_GEMM=0 (cuBLAS ZGEMM, ~1 TFLOP/s on
-# GB300).  DF_ERR bounds the relative error one such rotation adds to H X.
+# anchors, rotations of X and H X) run as digit products on the tensor cores (ops.zgemm_df,
+# 55 bits below the largest components of a row and a column) unless ADDFT_DF_GEMM=0 (cuBLAS ZGEMM, ~1 TFLOP/s on
+# GB300).  DF_ERR bounds the error one such rotation adds to H X, relative to its largest row: rows of unitary
+# matrices have components up to 1, so sqrt(K) 2^-54 of a column's largest component, 1e-15 for K = 336.
 DF_GEMM = os.environ.get("ADDFT_DF_GEMM", "1") != "0"
 DF_ERR = 3e-14
 
 
 def _mm64(a, b, conj_a=False, conj_b=False):
-    """op(a) @ op(b) for complex128 matrices, to ~1e-14 relative (host tensors, which
-    only the host-logic tests with a dense stand-in H use, go through torch)."""
+    """op(a) @ op(b) for complex128 matrices, to sqrt(K) 2^-54 of the largest components of a row and a column
+    (host tensors, which only the host-logic tests with a dense stand-in H use, go through torch)."""
     if DF_GEMM and a.is_cuda:
         return ops.zgemm_df(a, b, conj_a, conj_b)
     return (a.conj() if conj_a else a) @ (b.conj() if conj_b else b)
@@ -503,7 +504,7 @@ def refine_lowest(H: HApply, k: int, X: torch.Tensor, nband: int, diag: torch.Te
             # FP32 error of H B is ~e |H| per unit block row; U_B weighs it in
             drift += (FP32_APPLY_ERR * float(torch.max(torch.sum(torch.abs(UB32), dim=1)))
                       * float(torch.max(torch.linalg.vector_norm(HB, dim=1))))
-            if DF_GEMM and HX.is_cuda:   # the double-float rotation of H X
+            if DF_GEMM and HX.is_cuda:   # the rotation of H X in digit products
                 drift += DF_ERR * float(torch.max(torch.linalg.vector_norm(HX, dim=1)))
             R = HX - lam[:, None] * X
             rn = wnorm(R)

@@ -24,8 +24,11 @@
 // one thread issues the MMAs (slice s of F against slices 0 .. 7 - s of the lines, side by side along
 // N = 32 (8 - s), landing on levels s .. 7; F has 7 slices); twelve epilogue warps empty one of the two accumulators
 // (8 levels x 32 lines) while the other is filled, add the levels in 64-bit integers and round once
-// to FP64.  All waits are bounded (status as in ozgemm.cu).  The error is that of the slicing, 2^-62
-// of the line's largest input and 2^-55 of F per term, and of one rounding: as an FP64 FFT's or below.
+// to FP64.  All waits are bounded (status as in ozgemm.cu).  The error of an output is that of the slicing, 2^-62
+// of the line's largest component and 2^-55 of F per term, of the level sums (2^-55 of that component), and of one
+// rounding: like an FFT's it is relative to the line, and against 80-bit transforms it is at or below the FFT kernels'
+// (densities, rms: 32 x 32 x 60 1.3e-16 both, 27 x 27 x 54 3.8e-16 -> 1.4e-16, 36^3 2.1e-16 -> 1.3e-16).  A line with an
+// infinity or a NaN is NaN as a whole, where an FFT leaves infinities in some components.
 //   Si64, 75^3, 160 bands: local H psi 11.5 -> 3.9 ms, density 9.2 -> 2.3 ms; 15^3, 64 bands, H psi with its
 // projectors 328 -> 160 us (six launches of 13 to 21 us: filling F and the first lines, not rates).
 #include <algorithm>
@@ -47,7 +50,7 @@ constexpr int kSF = 7;           // digits of F: entries up to 1 to 2^-54, below
 constexpr int kFBits = 54;
 constexpr int kLines = 32;       // lines per block
 constexpr int kStep = 16;        // k per MMA
-constexpr int kMaxK = 128;       // sums of 128 products per digit pair stay exact
+constexpr int kMaxK = 128;       // a level's 256 (l + 1) products of 2^14: exact below 2^24, 2^25 with aligned digits at most
 constexpr int kMaxRing = 8;      // operand buffers (one kstep of 32 lines each)
 constexpr int kItem = 2 * kS * kLines * kStep * 2;   // 16 KB
 // Warps 0 .. 15 with warp % 4 < 3 empty the accumulator rows 32 (warp % 4) .. of 8 lines each (2 R <= 96

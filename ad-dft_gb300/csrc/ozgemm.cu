@@ -9,14 +9,22 @@
 // contraction is done on integers instead.  With E the binary exponent of the largest
 // |re|, |im| of a row of op(A) (a column of op(B)), every component x becomes the integer
 //   q = round(x 2^(B - E)),  |q| <= 2^B,  B = 62 (S = 8 digits) or 55 (S = 7 digits),
-// written in balanced base 256, q = sum_s d_s 256^(S-1-s), -128 <= d_s <= 128.  A digit is
-// exact in FP16 and a product of two is at most 2^14, so an FP32 accumulator adds 2^10 of them
-// without rounding.  The products d_s(a) d_t(b) of one level l = s + t share a weight and one
-// accumulator; levels 0 .. S-1 are kept (S (S + 1) / 2 digit products per real product), what
-// is dropped is below 2^-(8 S - 2) of the row's and the column's largest components.  Every 128 k
-// the accumulators are emptied into 64-bit integers, so nothing is rounded until the final
-// conversion to FP64: the error is that of the slicing, about 2^-62 (S = 8) or 2^-55 (S = 7)
-// relative to max|A_i.| max|B_.j| per term, against 2^-53 per operation of an FP64 sum.
+// written in balanced base 256, q = sum_s d_s 256^(S-1-s), -128 <= d_s <= 128.  A digit is exact in
+// FP16 and a product of two is at most 2^14.  The products d_s(a) d_t(b) of one level l = s + t share a
+// weight and one FP32 accumulator in tensor memory; levels 0 .. S-1 are kept (S (S + 1) / 2 digit products per real
+// product).  Every 128 k the accumulators are emptied into 64-bit integers, and the only rounding after that is
+// the conversion to FP64.
+//   Accuracy is that of fixed point, relative to max|A_i.| max|B_j.| of an output's row and column and not to the
+// output or to its terms: where a large component of one meets a zero or a small one of the other, and only small
+// ones meet, the result has fewer correct digits than an FP64 sum (K = 512, a 1 against a zero, the rest 10^-6
+// against 1: 1e-13 of sum|a b| with 8 digits, 7e-12 with 7; 10^-3: 2e-16, 1e-14).  In units of the two maxima:
+//   slicing, per term: 2^-61 (S = 8), 2^-54 (S = 7); what the dropped levels hold at most, digits aligned: 2^-56, 2^-50
+//     per term, on data whose digits are not about sqrt(K) 2^-60, sqrt(K) 2^-54 in all;
+//   accumulators: a level's sum over 128 k is below 2^24 and exact up to level 3, and beyond it unless digits are aligned
+//     (256 (l + 1) products of 2^14 are 2^25 at most); then each MMA may drop units of that level, 2^-52 and
+//     smaller ones (l >= 5) against a sum of at least 2^6.
+// That is within the normwise error of an FP64 sum, 2^-53 |A_i.| |B_j.|, for S = 8 up to K of 10^5, and of the
+// double-float form (2^-48) for S = 7.
 // Rows or columns that hold an infinity or a NaN are summed in plain FP64 at the end.
 //
 // Three kernels:

@@ -141,7 +141,9 @@ addft_status addft_plan_get_tuning(addft_plan plan, const char *key, long *value
 
 /* Scratch bytes that lets one call process `nbatch` bands at once.  Every
  * transform entry point accepts any work size >= addft_work_bytes(plan, 1,
- * dtype) and loops over band chunks that fit. */
+ * dtype) and loops over band chunks that fit.
+ * FP64 transforms run on the FFT kernels or as digit products on the tensor cores, whichever is quicker for the box
+ * and the bands at once; in the latter a line (x, y or z) that holds an infinity or a NaN is NaN as a whole. */
 size_t addft_work_bytes(addft_plan plan, int nbatch, addft_dtype dtype);
 
 /* ---- a5/a4: G-sphere <-> box transforms (basis.py:237-254) ---------- */
@@ -171,7 +173,11 @@ addft_status addft_hpsi(addft_plan plan, addft_dtype dt, int nk, int nb, const v
                         void *stream);
 
 /* ---- a9: nonlocal projector contractions (nonlocal_op.py:67-82) ------
- * becp[k, p, b] = sum_G conj(proj[k, p, G]) psi[k, b, G]   (nk, nproj, nb) complex. */
+ * becp[k, p, b] = sum_G conj(proj[k, p, G]) psi[k, b, G]   (nk, nproj, nb) complex.
+ * In FP64 these contractions (H psi's and the gradients' too, and the structure factors of addft_local_potential and
+ * addft_density_gradients) run as digit products of 62 bits where the size pays: like an FP64 sum their error is within
+ * 2^-53 of the norms of the two operand rows, but it is relative to the rows' largest components (about sqrt(K) 2^-60
+ * of their product, at most K 2^-56), not to the terms of each sum. */
 addft_status addft_becp(addft_dtype dt, int nk, int nb, int nG, int nproj, const void *proj,
                         const void *psi, void *becp, void *work, size_t work_bytes,
                         void *stream);
@@ -245,9 +251,13 @@ addft_status addft_kerker(addft_plan full_plan, const double *bvec_host, const d
 size_t addft_kerker_work_bytes(addft_plan full_plan);
 
 /* ---- a15: FP64 subspace products of the eigensolver (solver/davidson.py:48, :51-52, :59-61:
- * the projections q^H hq and the rotations q u, hq u), to ~1e-15 relative as exact digit products
- * on the tensor cores (55 bits below each row's and column's largest component), or, where work holds
- * less than that wants, in double-float arithmetic on the FP32 pipes (~1e-14).  C (M x N, row stride ldc) = op(A) op(B) with
+ * the projections q^H hq and the rotations q u, hq u), as digit products on the tensor cores, 55 bits below the
+ * largest component of each row of op(A) and column of op(B).  The error of C[i][j] is relative to those two
+ * components, not to C[i][j] or its terms: about sqrt(K) 2^-54 of their product and at most K 2^-50, so an output whose
+ * row and column meet only in components far below their largest ones has fewer digits (an entry of 1 against
+ * zero, 511 pairs of 1e-6 against 1: 7e-12 of the terms' sum).  Small products (plain FP64) and calls whose work holds
+ * less than the digit form wants (double-float on the FP32 pipes, ~1e-14) are accurate to sum |a b|.
+ * C (M x N, row stride ldc) = op(A) op(B) with
  *   op(A)[i][k] = A[i*sAi + k*sAk], conjugated when conjA != 0,
  *   op(B)[k][j] = B[k*sBk + j*sBj], conjugated when conjB != 0;
  * all complex128, strides in elements.  K is split across CTAs when work holds

@@ -148,3 +148,35 @@ def test_pieces_of_a_batch_stay_within_the_scratch(nk, nb, P, nG, mb):
     for k in range(nk):
         assert bool(((out[k] - proj[k].conj() @ psi[k].T).abs() <= bound(proj[k], psi[k].T, 60)).all())
     assert clean()
+
+
+@pytest.mark.parametrize("K", [128, 384, 1024])
+def test_aligned_digits(K):
+    """Equal components whose digits are all next to the largest: the sums of a level pass 2^24 in its FP32
+    accumulator.  What it drops, and what the dropped levels hold, stays below four roundings of the result (in
+    products that are not split along K: the split sums are added in FP64)."""
+    from fractions import Fraction
+    x = float(Fraction(63, 64) + sum(Fraction(127, 64 * 256 ** i) for i in range(1, 6)))
+    M, N = 400, 200
+    a = torch.full((M, K), complex(x, x), dtype=torch.complex128, device="cuda")
+    b = torch.full((N, K), complex(x, -x), dtype=torch.complex128, device="cuda")
+    want = float(2 * K * Fraction(x) ** 2)
+    for out in (ops.zgemm_df(a, b.transpose(0, 1)), ops.becp(a.conj().resolve_conj()[None], b[None])[0]):
+        assert bool(((out.real - want).abs() <= 4 * U * want).all())
+        assert bool((out.imag.abs() <= 4 * U * want).all())
+
+
+@pytest.mark.parametrize("decades", [3, 6, 9, 12])
+@pytest.mark.parametrize("K", [40, 512, 6000])
+def test_graded_rows_meet_the_stated_bound(decades, K):
+    """A large component against a zero, the rest far below it: errors are relative to the largest components
+    of row and column (2^-50 K with 7 digits, 2^-56 K with 8), as stated, not to the result."""
+    M, N = 130, 70
+    a, b = rnd(1, M, K) * 10.0 ** -decades, rnd(2, N, K)
+    a[:, 3] = 1.0
+    b[:, 3] = 0.0
+    ref = a.conj() @ b.T
+    big = a.abs().amax(1)[:, None] * b.abs().amax(1)[None]
+    fp64 = (math.sqrt(K) + 4.0) * 4 * U * (a.abs() @ b.abs().T)
+    assert bool(((ops.zgemm_df(a, b.transpose(0, 1), conj_a=True) - ref).abs() <= K * 2.0 ** -50 * big + fp64).all())
+    assert bool(((ops.becp(a[None], b[None])[0] - ref).abs() <= K * 2.0 ** -56 * big + fp64).all())
