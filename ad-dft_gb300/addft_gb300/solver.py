@@ -77,19 +77,11 @@ class HApply:
         self.kin0 = None
 
     def _apply64(self, k: int, Q: torch.Tensor) -> torch.Tensor:
-        """FP64-accurate H Q.  The plain FP64 kernel form (precision "fp64") runs every term in
-        FP64.  The FP32 arm's anchors take the local part from the FP64 kernels and the two
-        projector contractions (becp = conj(beta) Q^T, H Q += (D becp)^T beta) from the
-        double-float GEMM (~1e-14 relative, 3-4x the FP64 rate), like its subspace products."""
+        """H Q in FP64."""
         c = self.cache
-        Q = Q.contiguous()
-        if self.precision != "fp32" or not DF_GEMM or c.proj.shape[1] == 0:
-            return ops.hpsi(self.plan, Q.unsqueeze(0), c.kin[k:k + 1], self.v64, c.proj[k:k + 1], c.dion)[0]
-        out = ops.hpsi(self.plan, Q.unsqueeze(0), c.kin[k:k + 1], self.v64)[0]
-        beta = c.proj[k]                                            # (P, nG)
-        becp = ops.zgemm_df(beta, Q.transpose(0, 1), conj_a=True)   # (P, m)
-        db = c.dion.to(torch.complex128) @ becp                     # (P, m), P x P x m
-        return out + ops.zgemm_df(db.transpose(0, 1), beta)         # (m, nG)
+        P = c.proj.shape[1]
+        return ops.hpsi(self.plan, Q.contiguous().unsqueeze(0), c.kin[k:k + 1], self.v64, c.proj[k:k + 1] if P else None,
+                        c.dion if P else None)[0]
 
     def apply_native(self, k: int, Q: torch.Tensor) -> torch.Tensor:
         """H Q in the precision of Q (complex64 -> FP32 kernels, complex128 -> FP64-accurate)."""
