@@ -299,7 +299,7 @@ def si64_kernel_breakdown(top=30):
 
 def subspace_gemm_block(reps=10):
     """The refinement's FP64 subspace products on the Si64 shapes (168 bands + blocks,
-    nG 23,847): double-float GEMM on the FP32 pipes against cuBLAS FP64 ZGEMM (CUDA
+    nG 23,847): digit products on the tensor cores (zgemm_df) against cuBLAS FP64 ZGEMM (CUDA
     events; max error relative to |op(a)| |op(b)|)."""
     import torch
     from addft_gb300 import ops
@@ -332,7 +332,7 @@ def subspace_gemm_block(reps=10):
         td = timed_ms(lambda: ops.zgemm_df(a, b, ca, cb))
         tc = timed_ms(lambda: (a.conj() if ca else a) @ (b.conj() if cb else b))
         fl = 8.0 * M * N * K
-        out[name] = {"double_float_ms": td, "double_float_tflops": fl / td / 1e9, "zgemm_fp64_ms": tc,
+        out[name] = {"zgemm_df_ms": td, "zgemm_df_tflops": fl / td / 1e9, "zgemm_fp64_ms": tc,
                      "zgemm_fp64_tflops": fl / tc / 1e9, "rel_err": err}
     return out
 
@@ -526,8 +526,8 @@ def run_gpu(args, rank, world):
     byts, fft_f, proj_f = model(nG, N, nb, P)
     achieved = byts / t_launch / 1e9
     # arithmetic roof: FFT flops at the FP32 FMA rate plus projector flops at the rates of the
-    # kernels that run them -- half the projector flops are becp (split-TF32 mma.sync), half
-    # the V_NL apply (split-TF32 tcgen05), three MMAs per product -- all measured on this GPU
+    # kernels that run them -- half the projector flops are becp, half the V_NL apply, by default both
+    # split-TF32 on tcgen05 with four and three MMAs per product -- all measured on this GPU
     # by measure_peaks (nominal rates if --peaks 0)
     fp32_peak = 152 * 128 * 2 * float(peaks.get("sm_max_mhz", 2070.0)) * 1e6 / 1e12
     tf32_peak, tc05_peak = 1100.0, 1100.0
@@ -537,8 +537,9 @@ def run_gpu(args, rank, world):
         tf32_peak = mpeaks["tf32_mma_sync"]["tflops"]
         tc05_peak = mpeaks["tf32_tcgen05"]["tflops"]
         peak_kind = "measured (addft_peak_flops on this GPU)"
-    becp_rate = tf32_peak / 3.0 if os.environ.get("ADDFT_BECP_TC", "1") == "1" else fp32_peak
-    apply_rate = tc05_peak / 3.0 if os.environ.get("ADDFT_APPLY_TC", "3") == "3" else tf32_peak / 3.0
+    rates = {"1": (tf32_peak / 3.0, tf32_peak / 3.0), "3": (tc05_peak / 4.0, tc05_peak / 3.0)}
+    becp_rate = rates.get(os.environ.get("ADDFT_BECP_TC", "3"), (fp32_peak, 0.0))[0]
+    apply_rate = rates.get(os.environ.get("ADDFT_APPLY_TC", "3"), (0.0, fp32_peak))[1]
     t_hbm, t_fp32 = byts / (hbm * 1e9), fft_f / (fp32_peak * 1e12)
     t_tc = 0.5 * proj_f / (becp_rate * 1e12) + 0.5 * proj_f / (apply_rate * 1e12)
     proj_peak = proj_f / t_tc / 1e12
