@@ -53,7 +53,16 @@ def _dt(t: torch.Tensor) -> int:
 def _c(t: torch.Tensor, what: str) -> torch.Tensor:
     if not t.is_cuda:
         raise ValueError(f"{what} must be a CUDA tensor")
-    return t.contiguous()
+    return _plain(t)
+
+
+def _plain(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous memory that holds the tensor's values: x.conj() and x.conj().imag are views with a pending
+    conjugation or sign, which contiguous() keeps."""
+    t = t.contiguous()
+    if t.is_conj() or t.is_neg():
+        t = t.resolve_conj().resolve_neg()
+    return t
 
 
 def _d3(x):
@@ -224,7 +233,7 @@ def hpsi_host(plan: Plan, psi_h: torch.Tensor, kin: torch.Tensor, v_r: torch.Ten
     Returns the host result; the current stream is joined with the last download."""
     if psi_h.is_cuda:
         raise ValueError("psi_h must be a host tensor (pinned for overlapped copies)")
-    psi_h = psi_h.contiguous()
+    psi_h = _plain(psi_h)
     nk, nb, nG = psi_h.shape
     dt = _dt(psi_h)
     rdt = torch.float64 if dt == F64 else torch.float32
@@ -363,6 +372,10 @@ def zgemm_df(a: torch.Tensor, b: torch.Tensor, conj_a: bool = False, conj_b: boo
     zgemm_df(x, y.transpose(0, 1), conj_a=True) without a copy."""
     if a.dtype != torch.complex128 or b.dtype != torch.complex128 or not (a.is_cuda and b.is_cuda):
         raise TypeError("zgemm_df: complex128 CUDA tensors expected")
+    if a.is_conj():
+        a, conj_a = a.conj(), not conj_a
+    if b.is_conj():
+        b, conj_b = b.conj(), not conj_b
     M, K = a.shape
     K2, N = b.shape
     if K != K2:
