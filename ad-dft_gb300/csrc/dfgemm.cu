@@ -1,4 +1,4 @@
-// Complex FP64 GEMM of the subspace products: exact digit products on the tensor cores (ozgemm.cu, 168 x
+// Complex FP64 GEMM of the subspace products: digit products on the tensor cores (ozgemm.cu, 168 x
 // 336 x 23,847: 0.45 ms) where the scratch holds their operands, else double-float arithmetic on the FP32
 // pipes (3.3 ms), described here.
 //

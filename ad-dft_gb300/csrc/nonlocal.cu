@@ -762,7 +762,7 @@ addft_status launch_becp_tc(int nk, int nb, int nG, int nproj, int nsplit, int g
 addft_status launch_becp_f32(int nk, int nb, int nG, int nproj, int nsplit, int gchunk, const float2 *proj,
                              const float2 *psi, float2 *out, cudaStream_t st);
 // tc05.cu: split-TF32 becp on tcgen05 with a tensor-memory accumulator, same partial layout, its tile
-void becp_tc05_tile(int nb, int nproj, int *pt, int *bt);
+void becp_tc05_tile(int nb, int *pt, int *bt);
 addft_status launch_becp_tc05(int nk, int nb, int nG, int nproj, int nsplit, const float2 *proj, const float2 *psi,
                               float2 *out, cudaStream_t st);
 
@@ -842,7 +842,7 @@ addft_status becp_t(int nk, int nb, int nG, int nproj, const void *proj, const v
   int ns = pick_nsplit(tiles, nG, mode != 2 ? becp_ctas_per_sm() : 8);
   if (mode == 3) {   // one CTA per SM
     int pt, bt;
-    becp_tc05_tile(nb, nproj, &pt, &bt);
+    becp_tc05_tile(nb, &pt, &bt);
     ns = std::min(ns, becp_tc05_nsplit(((nproj + pt - 1) / pt) * ((nb + bt - 1) / bt) * nk, nG));
   }
   const size_t per = (size_t)nk * nproj * nb * sizeof(C);

@@ -1,4 +1,4 @@
-// Complex FP64 GEMM on the tensor cores by exact digit slicing (ozgemm.cu).
+// Complex FP64 GEMM on the tensor cores by digit slicing (ozgemm.cu).
 #pragma once
 #include "common.cuh"
 
@@ -13,7 +13,7 @@ struct OzMat {
   int conj;
 };
 
-// Scratch that oz_gemm wants with 8 (FP64-accurate) or 7 (about 2^-55) digits, 256-byte aligned; it
+// Scratch that oz_gemm wants with 8 (62 bits) or 7 (55 bits) digits, 256-byte aligned; it
 // works in pieces with less, and oz_fits tells whether a buffer is enough for that.
 size_t oz_work_bytes(int digits, int M, int N, int K, int batch);
 bool oz_fits(int digits, int M, int N, int K, int batch, const void *work, size_t bytes);

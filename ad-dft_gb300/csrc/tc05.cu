@@ -351,12 +351,11 @@ k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int
 }
 
 // Tile of a problem: 32 projectors, equal tiles of up to kMost bands.
-void becp_tc05_tile(int nb, int nproj, int *pt, int *bt) {
+void becp_tc05_tile(int nb, int *pt, int *bt) {
   constexpr int kMost = 96;
   const int n = (nb + kMost - 1) / kMost;
   *pt = 32;
   *bt = ((nb + n - 1) / n + 15) / 16 * 16;
-  (void)nproj;
 }
 
 template <int RB>
@@ -370,7 +369,7 @@ static addft_status becp_go(dim3 grid, int nb, int nG, int nproj, int nsplit, co
 addft_status launch_becp_tc05(int nk, int nb, int nG, int nproj, int nsplit, const float2 *proj, const float2 *psi,
                               float2 *out, cudaStream_t st) {
   int pt, bt;
-  becp_tc05_tile(nb, nproj, &pt, &bt);
+  becp_tc05_tile(nb, &pt, &bt);
   const dim3 grid((nb + bt - 1) / bt, (nproj + pt - 1) / pt, nk * nsplit);
   switch (bt / 16) {
 #define BECP_CASE(rb) \
