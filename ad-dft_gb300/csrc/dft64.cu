@@ -67,36 +67,6 @@ constexpr size_t kRoom = 221000;      // shared memory for F and the ring
 constexpr size_t kMaxF = kRoom - 4 * kItem;
 constexpr int kSms = 152;
 
-__device__ __forceinline__ uint32_t sad(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity) {
-  for (int it = 0; it < kWait; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(sad(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void init_bar(uint64_t *bar, int n) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sad(bar)), "r"(n));
-}
-__device__ __forceinline__ void arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sad(bar)) : "memory");
-}
-__device__ __forceinline__ void commit_to(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sad(bar))
-               : "memory");
-}
-#define D64_LD8(taddr, r)                                                                         \
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"           \
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), \
-                 "=r"(r[7])                                                                      \
-               : "r"(taddr))
-
 enum Stage { ZI, YI, XI_V, XI_R, XI_C, XI_D, XF, XR_R, XR_C, YF, ZF, ZF_H };
 
 struct Args {
@@ -214,12 +184,6 @@ __device__ __forceinline__ void store_at(const Args &a, unsigned l, unsigned ban
   else if (g >= 0) out[2 * ((long)band * pd.nG + g) + comp] = ST == ZF_H ? v + x : v * a.scale;
 }
 
-__device__ __forceinline__ double scale2(double x, int n) {
-  const int a = n / 2, b = n - a;
-  auto p2 = [](int t) { return __hiloint2double((max(min(t, 1023), -1022) + 1023) << 20, 0); };
-  return x * p2(a) * p2(b);
-}
-
 __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
   long long r;
   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
@@ -265,7 +229,7 @@ __device__ __forceinline__ uint64_t d64_bytes(double x, int em) {
 template <int ST>
 __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char *smem = smem_raw + ((1024 - (sad(smem_raw) & 1023)) & 1023);
+  unsigned char *smem = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
   __shared__ __align__(8) uint64_t fullB[kMaxRing], emptyB[kMaxRing], accf[2], acce[2], fbar;
   __shared__ uint16_t pm[2][kProd][kLines];   // exponents found by each producer warp
   __shared__ uint16_t lex[kLex][kLines];      // exponents of the lines of the last blocks
@@ -277,25 +241,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
   const unsigned units = ST == XI_D ? nblk * a.groups : nblk;
   if (tid == 0) {
     for (int i = 0; i < a.ring; ++i) {
-      init_bar(&fullB[i], 2);
-      init_bar(&emptyB[i], 1);
+      bar_init(&fullB[i], 2);
+      bar_init(&emptyB[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
-      init_bar(&accf[i], 1);
-      init_bar(&acce[i], kEpi);
+      bar_init(&accf[i], 1);
+      bar_init(&acce[i], kEpi);
     }
-    init_bar(&fbar, 1);
+    bar_init(&fbar, 1);
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sad(&tslot)), "r"(512));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  if (warp == 0) tmem_alloc(&tslot, 512);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
-  const uint32_t sring = sad(smem), sF = sring + a.ring * kItem;   // F last: its 128-row reads may run past it
+  const uint32_t sring = smem_addr(smem), sF = sring + a.ring * kItem;   // F last: its 128-row reads may run past it
   bool ok = true;
 
   // a block: 32 lines starting at l0 (XI_D: of one band); `inner` blocks share a unit
@@ -362,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
           if (o > me) load(o);
           const unsigned t = turn * nks + (o >> 1), round = t / (unsigned)spg;
           const int slot = grp * spg + (int)(t - round * spg);
-          if (ok && round > 0) ok = __all_sync(0xffffffffu, wait_bar(&emptyB[slot], (round - 1) & 1));
+          if (ok && round > 0) ok = __all_sync(0xffffffffu, bar_wait<kWait>(&emptyB[slot], (round - 1) & 1));
           if (!ok) continue;
           const uint32_t dst = sring + slot * kItem + (lane >> 3) * 256 + (o & 1) * 128 + (lane & 7) * 16;
 #pragma unroll
@@ -375,21 +336,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
             for (int s = 0; s < kS; ++s) {
               uint32_t hh[4];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                uint32_t w;
-                if (s == 0) {
-                  w = ((uint32_t)((int)((int64_t)q[2 * j] >> 56) + 128) | ((uint32_t)((int)((int64_t)q[2 * j + 1] >> 56) + 128) << 16)) +
-                      0x64006400u;
-                } else {
-                  // byte 7 - s of both numbers into the low bytes of the halves
-                  const uint32_t lo = s < 4 ? (uint32_t)(q[2 * j] >> 32) : (uint32_t)q[2 * j];
-                  const uint32_t hi = s < 4 ? (uint32_t)(q[2 * j + 1] >> 32) : (uint32_t)q[2 * j + 1];
-                  const int y = s < 4 ? 3 - s : 7 - s;
-                  w = __byte_perm(__byte_perm(lo, hi, y | ((y + 4) << 4)), 0x64646464u, 0x4140);
-                }
-                // 0x6400 + n is the FP16 number 1024 + n; minus 1152 leaves the digit, exactly
-                asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(hh[j]) : "r"(w), "r"(0x64806480u));
-              }
+              for (int j = 0; j < 4; ++j) hh[j] = digit_pair<kS>(q[2 * j], q[2 * j + 1], s);
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (part * kS + s) * (kLines * kStep * 2)),
                            "r"(hh[0]), "r"(hh[1]), "r"(hh[2]), "r"(hh[3])
                            : "memory");
@@ -397,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
-          if (lane == 0) arrive(&fullB[slot]);
+          if (lane == 0) bar_arrive(&fullB[slot]);
         }
       }
     }
@@ -408,16 +355,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
     if (lead) {
       const uint32_t bytes = (uint32_t)a.m.tile_bytes;
       const unsigned char *src = a.F + a.m.off + (size_t)tile * bytes;
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sad(&fbar)), "r"(bytes) : "memory");
-      for (uint32_t o = 0; o < bytes; o += 32768) {
-        const uint32_t n = min(32768u, bytes - o);
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sF + o),
-            "l"(src + o), "r"(n), "r"(sad(&fbar))
-            : "memory");
-      }
+      bar_expect(&fbar, bytes);
+      for (uint32_t o = 0; o < bytes; o += 32768) bulk_copy(sF + o, src + o, min(32768u, bytes - o), &fbar);
     }
-    ok = wait_bar(&fbar, 0);
+    ok = bar_wait<kWait>(&fbar, 0);
     const uint32_t sl = (3 * R * 32) >> 4;   // one slice of F, in descriptor units
     const uint32_t fre = desc_lo(sF + R * 32), fim = desc_lo(sF), ring0 = desc_lo(sring);
     unsigned blk = 0, slot = 0, grp = 0;     // blk % ngrp; each group's buffers in turn
@@ -429,14 +370,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
       unit_info(u, l0, b0, inner);
       for (int it = 0; it < inner && ok; ++it, ++blk) {
         const unsigned buf = blk & 1;
-        if (blk >= 2) ok = wait_bar(&acce[buf], (blk / 2 - 1) & 1);
+        if (blk >= 2) ok = bar_wait<kWait>(&acce[buf], (blk / 2 - 1) & 1);
         const unsigned turn = blk / (unsigned)ngrp;
         grp = blk - turn * ngrp;
         round = turn * nks / (unsigned)spg;
         pos = turn * nks - round * spg;
         for (int j = 0; j < nks && ok; ++j) {
           slot = grp * spg + pos;
-          ok = wait_bar(&fullB[slot], round & 1);
+          ok = bar_wait<kWait>(&fullB[slot], round & 1);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           issued = true;
@@ -448,8 +389,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
 #pragma unroll
             for (int i = 0; i < kSF; ++i)   // [-Im; Re] Im x
               mma_f16(d + 32 * i, fim + f + i * sl, b + ((kS * kLines * kStep * 2) >> 4), idesc_f16(32 * (kS - i), false), 1);
-            commit_to(&emptyB[slot]);
-            if (j == nks - 1) commit_to(&accf[buf]);
+            mma_commit(&emptyB[slot]);
+            if (j == nks - 1) mma_commit(&accf[buf]);
           }
           __syncwarp();
           if (++pos == (unsigned)spg) {
@@ -461,12 +402,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
     }
     if (!ok) {
       if (lead) atomicOr(&g_d64_error, 1u);
-      wait_bar(&fbar, 0);
+      bar_wait<kWait>(&fbar, 0);
       if (issued) {   // no MMA may be in flight when tensor memory is given back
-        if (lead) commit_to(&accf[0]);
+        if (lead) mma_commit(&accf[0]);
         __syncwarp();
-        wait_bar(&accf[0], 0);
-        wait_bar(&accf[0], 1);
+        bar_wait<kWait>(&accf[0], 0);
+        bar_wait<kWait>(&accf[0], 1);
       }
     }
   } else {
@@ -508,7 +449,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
             }
           }
         }
-        ok = __all_sync(0xffffffffu, wait_bar(&accf[buf], (uint32_t)(blk / 2) & 1));
+        ok = __all_sync(0xffffffffu, bar_wait<kWait>(&accf[buf], (uint32_t)(blk / 2) & 1));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t base = tmem + 256 * buf + ((uint32_t)(32 * q) << 16) + c0;
@@ -517,8 +458,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
           uint32_t v[2][kEpiLines];
 #pragma unroll
           for (int l = 0; l < kS; l += 2) {
-            D64_LD8(base + 32 * l, v[0]);
-            D64_LD8(base + 32 * l + 32, v[1]);
+            TMEM_LD8(base + 32 * l, v[0]);
+            TMEM_LD8(base + 32 * l + 32, v[1]);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int c = 0; c < kEpiLines; ++c) {
@@ -532,7 +473,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) arrive(&acce[buf]);   // the accumulator has been read
+        if (lane == 0) bar_arrive(&acce[buf]);   // the accumulator has been read
         if (!on) continue;
         const double wb = ST == XI_D ? a.wocc[b0 + it] : 0.0;
         unsigned band = (l0 + c0) / per, rem = (l0 + c0) - band * per;
@@ -568,7 +509,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_d64(Args a) {
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  if (warp == 0) tmem_free(tmem, 512);
 }
 
 // Vt[z][y][x] = V[x][y][z] * s, through shared-memory tiles of 32 x 32 (x, z) per y

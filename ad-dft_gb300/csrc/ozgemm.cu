@@ -78,43 +78,6 @@ struct Oz {
   static constexpr size_t kSmem = (size_t)kARing * kAItem + kBRing * kBBytes + 1024;
 };
 
-__device__ __forceinline__ uint32_t sad(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity) {
-  for (int it = 0; it < kOzWait; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(sad(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void init_bar(uint64_t *bar, int n) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sad(bar)), "r"(n));
-}
-__device__ __forceinline__ void arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sad(bar)) : "memory");
-}
-__device__ __forceinline__ void commit_to(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sad(bar))
-               : "memory");
-}
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
-      "r"(bytes), "r"(sad(bar))
-      : "memory");
-}
-#define OZ_LD8(taddr, r)                                                                          \
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"           \
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), \
-                 "=r"(r[7])                                                                      \
-               : "r"(taddr))
-
 // ---------------------------------------------------------------------------
 // exponents: ex[row] = largest exponent field of |re|, |im| over k (0x7ff: not finite)
 // ---------------------------------------------------------------------------
@@ -211,23 +174,7 @@ k_oz_pack(const double2 *__restrict__ X, long s_row, long s_k, size_t s_batch, i
     for (int s = 0; s < S; ++s) {
       uint32_t h[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint32_t w;
-        if (s == 0) {   // top digit: signed, -128 .. 128
-          const int a = (int)((int64_t)q[2 * j] >> (8 * (S - 1))) + 128;
-          const int b = (int)((int64_t)q[2 * j + 1] >> (8 * (S - 1))) + 128;
-          w = ((uint32_t)a | ((uint32_t)b << 16)) + 0x64006400u;
-        } else {
-          // byte S - 1 - s of both numbers into the low bytes of the halves
-          constexpr int kTop = S - 1;
-          const int y = (kTop - s) & 3;
-          const uint32_t a = (uint32_t)(q[2 * j] >> (kTop - s >= 4 ? 32 : 0));
-          const uint32_t b = (uint32_t)(q[2 * j + 1] >> (kTop - s >= 4 ? 32 : 0));
-          w = __byte_perm(__byte_perm(a, b, y | ((y + 4) << 4)), 0x64646464u, 0x4140);
-        }
-        // 0x6400 + n is the FP16 number 1024 + n; minus 1152 leaves the digit, exactly
-        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(h[j]) : "r"(w), "r"(0x64806480u));
-      }
+      for (int j = 0; j < 4; ++j) h[j] = digit_pair<S>(q[2 * j], q[2 * j + 1], s);
       *reinterpret_cast<uint4 *>(dst + (size_t)(part * S + s) * kSlice) = make_uint4(h[0], h[1], h[2], h[3]);
     }
   }
@@ -257,13 +204,6 @@ struct OzArgs {
 // conversions and scalings of one 128 x 32 tile took 19 us, the MMAs of 16 k take 1.2 us.
 template <int SH>
 __device__ __forceinline__ double oz_value(long long hi, long long lo, int n);
-
-// 2^n as a product of two factors in range
-__device__ __forceinline__ double scale2(double x, int n) {
-  const int a = n / 2, b = n - a;
-  auto p2 = [](int t) { return __hiloint2double((max(min(t, 1023), -1022) + 1023) << 20, 0); };
-  return x * p2(a) * p2(b);
-}
 
 template <int SH>
 __device__ __forceinline__ double oz_value(long long hi, long long lo, int n) {
@@ -323,7 +263,7 @@ template <int S>
 __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
   using P = Oz<S>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char *smem = smem_raw + ((1024 - (sad(smem_raw) & 1023)) & 1023);
+  unsigned char *smem = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
   __shared__ __align__(8) uint64_t fa[P::kARing], ea[P::kARing], fb[P::kBRing], eb[P::kBRing], accf, acce;
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -335,26 +275,23 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
   const int nblk = (nst + kDrain - 1) / kDrain;
   if (tid == 0) {
     for (int i = 0; i < P::kARing; ++i) {
-      init_bar(&fa[i], 1);
-      init_bar(&ea[i], 1);
+      bar_init(&fa[i], 1);
+      bar_init(&ea[i], 1);
     }
     for (int i = 0; i < P::kBRing; ++i) {
-      init_bar(&fb[i], 1);
-      init_bar(&eb[i], 1);
+      bar_init(&fb[i], 1);
+      bar_init(&eb[i], 1);
     }
-    init_bar(&accf, 1);
-    init_bar(&acce, kEpiWarps);
+    bar_init(&accf, 1);
+    bar_init(&acce, kEpiWarps);
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sad(&tslot)), "r"(512));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  if (warp == 0) tmem_alloc(&tslot, 512);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
-  const uint32_t sa = sad(smem), sb = sa + P::kARing * P::kAItem;
+  const uint32_t sa = smem_addr(smem), sb = sa + P::kARing * P::kAItem;
   bool ok = true;
 
   if (warp == kEpiWarps) {
@@ -364,37 +301,34 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
       // a tile with fewer rows copies only their core matrices, slice by slice
       const int rows8 = (min(kRowsA, g.rows - rt * kRowsA) + 7) & ~7;
       constexpr uint32_t kSlice = kRowsA * kStep * 2;
-      auto expect = [&](uint64_t *bar, uint32_t bytes) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sad(bar)), "r"(bytes) : "memory");
-      };
       int na = 0, nb = 0;   // items under way
       for (int a = 0; a < 2 * nst && ok; ++a) {
         const int s = a >> 1;
         if (!(a & 1)) {
           const int j = s % P::kBRing;
-          if (s >= P::kBRing) ok = wait_bar(&eb[j], (s / P::kBRing - 1) & 1);
+          if (s >= P::kBRing) ok = bar_wait<kOzWait>(&eb[j], (s / P::kBRing - 1) & 1);
           if (!ok) break;
-          expect(&fb[j], P::kBBytes);
+          bar_expect(&fb[j], P::kBBytes);
           bulk_copy(sb + j * P::kBBytes, pb + (size_t)s * P::kBBytes, P::kBBytes, &fb[j]);
           nb = s + 1;
         }
         const int j = a % P::kARing;
-        if (a >= P::kARing) ok = wait_bar(&ea[j], (a / P::kARing - 1) & 1);
+        if (a >= P::kARing) ok = bar_wait<kOzWait>(&ea[j], (a / P::kARing - 1) & 1);
         if (!ok) break;
         const uint32_t dst = sa + j * P::kAItem;
         const unsigned char *src = pa + (size_t)a * P::kAItem;
         if (rows8 == kRowsA) {
-          expect(&fa[j], P::kAItem);
+          bar_expect(&fa[j], P::kAItem);
           bulk_copy(dst, src, P::kAItem, &fa[j]);
         } else {
-          expect(&fa[j], S * rows8 * kStep * 2);
+          bar_expect(&fa[j], S * rows8 * kStep * 2);
           for (int i = 0; i < S; ++i) bulk_copy(dst + i * kSlice, src + i * kSlice, rows8 * kStep * 2, &fa[j]);
         }
         na = a + 1;
       }
       // nothing may still be landing in shared memory when the CTA ends
-      for (int a = max(0, na - P::kARing); a < na; ++a) ok = wait_bar(&fa[a % P::kARing], (a / P::kARing) & 1) && ok;
-      for (int s = max(0, nb - P::kBRing); s < nb; ++s) ok = wait_bar(&fb[s % P::kBRing], (s / P::kBRing) & 1) && ok;
+      for (int a = max(0, na - P::kARing); a < na; ++a) ok = bar_wait<kOzWait>(&fa[a % P::kARing], (a / P::kARing) & 1) && ok;
+      for (int s = max(0, nb - P::kBRing); s < nb; ++s) ok = bar_wait<kOzWait>(&fb[s % P::kBRing], (s / P::kBRing) & 1) && ok;
       if (!ok) atomicOr(&g_oz_error, 1u);
     }
   } else if (warp == kEpiWarps + 1) {
@@ -407,12 +341,12 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
     for (int s = 0; s < nst && ok; ++s) {
       const int blk = s / kDrain;
       const bool first = s % kDrain == 0;
-      if (first && blk > 0) ok = wait_bar(&acce, (blk - 1) & 1);   // the accumulators have been read
-      if (ok) ok = wait_bar(&fb[jb], pb);
+      if (first && blk > 0) ok = bar_wait<kOzWait>(&acce, (blk - 1) & 1);   // the accumulators have been read
+      if (ok) ok = bar_wait<kOzWait>(&fb[jb], pb);
       const uint32_t b0 = b_lo + jb * (P::kBBytes >> 4);
 #pragma unroll
       for (int ra = 0; ra < 2; ++ra) {   // part of A
-        if (ok) ok = wait_bar(&fa[ja], pa);
+        if (ok) ok = bar_wait<kOzWait>(&fa[ja], pa);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         issued = true;
@@ -426,10 +360,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
               mma_f16(d + 32 * i, a0 + ((i * kRowsA * kStep * 2) >> 4), bd, idesc_f16(32 * (S - i), ra && rb),
                       !(first && ra == 0 && i == 0));
           }
-          commit_to(&ea[ja]);
+          mma_commit(&ea[ja]);
           if (ra == 1) {
-            commit_to(&eb[jb]);
-            if (s % kDrain == kDrain - 1 || s == nst - 1) commit_to(&accf);
+            mma_commit(&eb[jb]);
+            if (s % kDrain == kDrain - 1 || s == nst - 1) mma_commit(&accf);
           }
         }
         __syncwarp();
@@ -447,10 +381,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
     if (!ok) {   // every MMA issued has to be done before tensor memory is given back
       if (lead) atomicOr(&g_oz_error, 1u);
       if (issued) {
-        if (lead) commit_to(&accf);
+        if (lead) mma_commit(&accf);
         __syncwarp();
-        wait_bar(&accf, 0);
-        wait_bar(&accf, 1);
+        bar_wait<kOzWait>(&accf, 0);
+        bar_wait<kOzWait>(&accf, 1);
       }
     }
   } else {
@@ -462,15 +396,15 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
     for (int c = 0; c < kEpiCols; ++c) hi[0][c] = hi[1][c] = lo[0][c] = lo[1][c] = 0;
     const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + c0;
     for (int blk = 0; blk < nblk && ok; ++blk) {
-      ok = wait_bar(&accf, blk & 1);
+      ok = bar_wait<kOzWait>(&accf, blk & 1);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int l = 0; l < S; ++l) {
         uint32_t v[2][kEpiCols];
-        OZ_LD8(base + 32 * l, v[0]);
-        OZ_LD8(base + 256 + 32 * l, v[1]);
+        TMEM_LD8(base + 32 * l, v[0]);
+        TMEM_LD8(base + 256 + 32 * l, v[1]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         const int w = l < 4 ? 1 << (8 * (3 - l)) : 1 << (8 * (S - 1 - l));
 #pragma unroll
@@ -484,7 +418,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) arrive(&acce);
+      if (lane == 0) bar_arrive(&acce);
     }
     if (!ok && lane == 0) atomicOr(&g_oz_error, 1u);
     const int row = rt * kRowsA + 32 * q + lane;
@@ -522,7 +456,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(OzArgs g) {
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  if (warp == 0) tmem_free(tmem, 512);
 }
 
 // C[i][j] (+)= sum_s part[s][j][i] in split order; part is column-major (rows fastest)

@@ -35,8 +35,6 @@ __device__ unsigned g_tc05_error = 0;   // bit 0: an mbarrier wait ran out
 
 constexpr int kWaitLimit = 1 << 24;
 
-__device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
 // tcgen05 shared-memory matrix descriptor: start address, LBO, SBO (bytes >> 4), the
 // fixed 0b001 at bits 46-48, base offset 0, no swizzle.
 __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
@@ -65,30 +63,6 @@ __device__ __forceinline__ void mma_tf32_lo(uint32_t dtmem, uint32_t a_lo, uint3
       "setp.ne.b32 p, %5, 0;\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t}" ::"r"(dtmem),
       "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(hi), "r"(acc)
       : "memory");
-}
-
-__device__ __forceinline__ void commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void bar_init(uint64_t *bar, int count = 1) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(count));
-}
-
-// Bounded wait for the completion of the mbarrier phase with this parity; false on timeout.
-__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
-  for (int it = 0; it < kWaitLimit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(saddr(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
 }
 
 __device__ __forceinline__ uint32_t tf32_rna(float x) {
@@ -120,14 +94,6 @@ __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
 __device__ __forceinline__ uint32_t coff(int R, int r, int k4) {
   const int slice = k4 >> 1, kc = k4 & 1;
   return (uint32_t)(slice * (R / 8) * 256 + (r >> 3) * 256 + kc * 128 + (r & 7) * 16);
-}
-
-__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(slot)), "r"(ncols));
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-}
-__device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
 }
 
 #define TC05_LD32(taddr, r)                                                                                      \
@@ -175,11 +141,6 @@ struct BT {
 };
 }  // namespace
 
-#define TC05_LD8(taddr, r)                                                                                   \
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"                      \
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) \
-               : "r"(taddr))
-
 template <int RB>
 __global__ void __launch_bounds__(kBThreads, 1)
 k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int nb, int nG, int nproj, int nsplit,
@@ -205,7 +166,7 @@ k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tslot, sbase = saddr(smem);
+  const uint32_t tmem = tslot, sbase = smem_addr(smem);
   bool ok = true;
   float sum[T::kQ][8];
 #pragma unroll
@@ -221,8 +182,8 @@ k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int
     int s = 0;
     for (; s < nst; ++s) {
       const int j = s & 1;
-      ok = bar_wait(&full[j], (s >> 1) & 1);
-      if (ok && s >= 2) ok = bar_wait(&acce[j], ((s >> 1) - 1) & 1);
+      ok = bar_wait<kWaitLimit>(&full[j], (s >> 1) & 1);
+      if (ok && s >= 2) ok = bar_wait<kWaitLimit>(&acce[j], ((s >> 1) - 1) & 1);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -232,13 +193,13 @@ k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int
         for (int kk = 0; kk < 8; ++kk)
           mma_tf32_lo(tmem + j * T::N, a_lo + o + (2 * kk * T::kChunkA) / 16, b_lo + o + (2 * kk * T::kChunkB) / 16,
                       idesc, kk > 0);
-        commit(&accf[j]);
+        mma_commit(&accf[j]);
       }
       __syncwarp();
     }
     if (!ok) {   // every MMA issued has to be done before tensor memory is given back
       if (lead) atomicOr(&g_tc05_error, 1u);
-      for (int t = max(0, s - 2); t < s; ++t) bar_wait(&accf[t & 1], (t >> 1) & 1);
+      for (int t = max(0, s - 2); t < s; ++t) bar_wait<kWaitLimit>(&accf[t & 1], (t >> 1) & 1);
     }
   } else {
     constexpr int NR = 2 + RB;   // rows of this warp: projectors warp, warp + 16, bands warp, warp + 16, ...
@@ -266,20 +227,20 @@ k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int
       for (int c = 0; c < T::kQ; ++c)
         if (8 * (warp >> 2) + 32 * c < T::NB) {
           uint32_t h[8], l[8];
-          TC05_LD8(tq + j * T::N + 32 * c, h);
-          TC05_LD8(tq + j * T::N + T::NB + 32 * c, l);
+          TMEM_LD8(tq + j * T::N + 32 * c, h);
+          TMEM_LD8(tq + j * T::N + T::NB + 32 * c, l);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int q = 0; q < 8; ++q) sum[c][q] += __uint_as_float(h[q]) + __uint_as_float(l[q]);
         }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&acce[j])) : "memory");
+      if (lane == 0) bar_arrive(&acce[j]);
     };
     auto stage = [&](int s, float2 (&x)[NR]) {
       const int j = s & 1;
       if (s >= 2) {   // MMAs of stage s - 2: its operands' room and its accumulators
-        ok = bar_wait(&accf[j], ((s >> 1) - 1) & 1);
+        ok = bar_wait<kWaitLimit>(&accf[j], ((s >> 1) - 1) & 1);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) return;
       }
@@ -306,7 +267,7 @@ k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&full[j])) : "memory");
+      if (lane == 0) bar_arrive(&full[j]);
       if (s + T::kPre < nst) load(s + T::kPre, x);
       if (s >= 2) drain(j);
     };
@@ -318,7 +279,7 @@ k_becp_tc05(const float2 *__restrict__ proj, const float2 *__restrict__ psi, int
       for (int i = 0; i < T::kPre; ++i)
         if (ok && s + i < nst) stage(s + i, v[i]);
     for (int s = max(0, nst - 2); s < nst && ok; ++s) {
-      ok = bar_wait(&accf[s & 1], (s >> 1) & 1);
+      ok = bar_wait<kWaitLimit>(&accf[s & 1], (s >> 1) & 1);
       ok = __all_sync(0xffffffffu, ok);
       if (ok) drain(s & 1);
     }
@@ -396,7 +357,7 @@ __global__ void __launch_bounds__(256, 1)
 k_apply_tc05(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, const float2 *__restrict__ A,
              size_t as_k, int nj, int ni, int nG, float2 *__restrict__ out, size_t os_k) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char *smem = smem_raw + ((1024 - (saddr(smem_raw) & 1023)) & 1023);
+  unsigned char *smem = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -412,7 +373,7 @@ k_apply_tc05(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, cons
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
   const uint32_t idesc = idesc_tf32(128, 128);
-  const uint32_t ahi = saddr(smem), alo = ahi + kATile, bhi = alo + kATile, blo = bhi + kATile;
+  const uint32_t ahi = smem_addr(smem), alo = ahi + kATile, bhi = alo + kATile, blo = bhi + kATile;
   const int nchunk = (nj + kAJ - 1) / kAJ;
   const int ntile = (nG + kAG - 1) / kAG;
   // operand rows: row r = tid % 128 of A (G) and B (band part), projector half ph = tid / 128
@@ -460,7 +421,7 @@ k_apply_tc05(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, cons
   const int bh = warp >> 2;
   for (int t = blockIdx.x; t < ntile && ok; t += gridDim.x) {
     for (int c = 0; c < nchunk && ok; ++c) {
-      if (ncommit > 0) ok = __syncthreads_and(bar_wait(&bar, (ncommit - 1) & 1)) != 0;   // operands free
+      if (ncommit > 0) ok = __syncthreads_and(bar_wait<kWaitLimit>(&bar, (ncommit - 1) & 1)) != 0;   // operands free
       if (!ok) break;
       if (nchunk > 1) build_b(c);
 #pragma unroll
@@ -483,7 +444,7 @@ k_apply_tc05(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, cons
           mma_tf32(tmem, ah, bl, idesc, 1u);
           mma_tf32(tmem, al, bh_, idesc, 1u);
         }
-        commit(&bar);
+        mma_commit(&bar);
       }
       ++ncommit;
       // next operands in flight while the MMAs run
@@ -498,7 +459,7 @@ k_apply_tc05(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, cons
       const int b = b0 + 32 * bh + j;
       w[j] = (ACCUM && b < ni && row < nG) ? ok_[(size_t)b * nG + row] : make_float2(0.f, 0.f);
     }
-    ok = __syncthreads_and(bar_wait(&bar, (ncommit - 1) & 1)) != 0;   // accumulator complete
+    ok = __syncthreads_and(bar_wait<kWaitLimit>(&bar, (ncommit - 1) & 1)) != 0;   // accumulator complete
     if (!ok) break;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t re[32], im[32];
@@ -516,8 +477,8 @@ k_apply_tc05(const float2 *__restrict__ X, int xs_j, int xs_i, size_t xs_k, cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
   if (!ok) {
-    if (tid == 0 && ncommit > 0) commit(&bar);   // one more commit tracks every MMA issued
-    bar_wait(&bar, ncommit & 1);
+    if (tid == 0 && ncommit > 0) mma_commit(&bar);   // one more commit tracks every MMA issued
+    bar_wait<kWaitLimit>(&bar, ncommit & 1);
     if (lane == 0) atomicOr(&g_tc05_error, 1u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -595,7 +556,7 @@ k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tslot, sbase = saddr(smem);
+  const uint32_t tmem = tslot, sbase = smem_addr(smem);
   bool ok = true;
 
   if (warp == kBWarps) {
@@ -608,8 +569,8 @@ k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, 
       for (int s = 0; s < nst && ok; ++s) {
         const int j = it & 1, set = bl & 1;
         const bool first = (s & 1) == 0, last = (s & 1) || s == nst - 1;
-        ok = bar_wait(&full[j], (it >> 1) & 1);
-        if (ok && first && bl >= 2) ok = bar_wait(&acce[set], ((bl >> 1) - 1) & 1);
+        ok = bar_wait<kWaitLimit>(&full[j], (it >> 1) & 1);
+        if (ok && first && bl >= 2) ok = bar_wait<kWaitLimit>(&acce[set], ((bl >> 1) - 1) & 1);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -623,8 +584,8 @@ k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, 
             mma_tf32_lo(d, ah + oa, bl_ + ob, idesc, 1u);
             mma_tf32_lo(d, al + oa, bh + ob, idesc, 1u);
           }
-          commit(&free_[j]);
-          if (last) commit(&accf[set]);
+          mma_commit(&free_[j]);
+          if (last) mma_commit(&accf[set]);
         }
         __syncwarp();
         ++it;
@@ -632,7 +593,7 @@ k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, 
       }
     if (!ok) {   // every MMA issued has to be done before tensor memory is given back
       if (lead) atomicOr(&g_tc05_error, 1u);
-      for (int t = max(0, it - 2); t < it; ++t) bar_wait(&free_[t & 1], (t >> 1) & 1);
+      for (int t = max(0, it - 2); t < it; ++t) bar_wait<kWaitLimit>(&free_[t & 1], (t >> 1) & 1);
     }
   } else if (warp == kBWarps + 1) {
     if (lane == 0) {   // X
@@ -642,19 +603,14 @@ k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, 
         const unsigned char *src = X + ((size_t)k * nbt + bt) * nst * (2 * T::kB);
         for (int s = 0; s < nst && ok; ++s, ++it) {
           const int j = it & 1;
-          if (it >= 2) ok = bar_wait(&free_[j], ((it >> 1) - 1) & 1);
+          if (it >= 2) ok = bar_wait<kWaitLimit>(&free_[j], ((it >> 1) - 1) & 1);
           if (!ok) break;
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(&full[j])), "r"(2 * T::kB)
-                       : "memory");
-          asm volatile(
-              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                  sbase + j * T::kStage + 2 * T::kA),
-              "l"(src + (size_t)s * (2 * T::kB)), "r"(2 * T::kB), "r"(saddr(&full[j]))
-              : "memory");
+          bar_expect(&full[j], 2 * T::kB);
+          bulk_copy(sbase + j * T::kStage + 2 * T::kA, src + (size_t)s * (2 * T::kB), 2 * T::kB, &full[j]);
         }
       }
       // nothing may still be landing in shared memory when the CTA ends
-      for (int t = max(0, it - 2); t < it; ++t) ok = bar_wait(&full[t & 1], (t >> 1) & 1) && ok;
+      for (int t = max(0, it - 2); t < it; ++t) ok = bar_wait<kWaitLimit>(&full[t & 1], (t >> 1) & 1) && ok;
       if (!ok) atomicOr(&g_tc05_error, 1u);
     }
   } else {
@@ -702,15 +658,15 @@ k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, 
     const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 8 * (warp >> 2);
     auto drain = [&](int b) __attribute__((always_inline)) {   // block b
       const int set = b & 1;
-      ok = bar_wait(&accf[set], (b >> 1) & 1);
+      ok = bar_wait<kWaitLimit>(&accf[set], (b >> 1) & 1);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) return;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int c = 0; c < T::kG; ++c) {
         uint32_t x[8], y[8];
-        TC05_LD8(tq + set * T::N + 32 * c, x);
-        TC05_LD8(tq + set * T::N + NB + 32 * c, y);
+        TMEM_LD8(tq + set * T::N + 32 * c, x);
+        TMEM_LD8(tq + set * T::N + NB + 32 * c, y);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -720,7 +676,7 @@ k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, 
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&acce[set])) : "memory");
+      if (lane == 0) bar_arrive(&acce[set]);
     };
     auto finish = [&](int u) __attribute__((always_inline)) {
       const int bt = u % nbt, t = u / nbt, k = t / ntile;
@@ -750,13 +706,13 @@ k_apply_deep(const unsigned char *__restrict__ X, const float2 *__restrict__ A, 
     load(v1);
     auto stage = [&](float2 (&x)[2][2]) __attribute__((always_inline)) {
       const int j = it & 1;
-      if (it >= 2) ok = bar_wait(&free_[j], ((it >> 1) - 1) & 1);
+      if (it >= 2) ok = bar_wait<kWaitLimit>(&free_[j], ((it >> 1) - 1) & 1);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) return;
       put(j, x);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&full[j])) : "memory");
+      if (lane == 0) bar_arrive(&full[j]);
       load(x);
       ++it;
       if ((s & 1) || s == nst - 1) {   // end of block bl: take the one before, a unit's last one with its store
@@ -869,13 +825,13 @@ __global__ void __launch_bounds__(128, 1) k_peak_tc05(int iters) {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
   if (tid == 0) {
-    const uint64_t ad = sdesc(saddr(a_s), 128, 256), bd = sdesc(saddr(b_s), 128, 256);
+    const uint64_t ad = sdesc(smem_addr(a_s), 128, 256), bd = sdesc(smem_addr(b_s), 128, 256);
     const uint32_t idesc = idesc_tf32(128, kPeakN);
     for (int it = 0; it < iters; ++it) mma_tf32(tmem, ad, bd, idesc, it > 0 ? 1u : 0u);
-    commit(&bar);
+    mma_commit(&bar);
   }
   __syncthreads();   // the issuing loop is finite; only the MMAs still queued remain
-  const bool ok = __syncthreads_and(bar_wait(&bar, 0)) != 0;
+  const bool ok = __syncthreads_and(bar_wait<kWaitLimit>(&bar, 0)) != 0;
   if (!ok && tid == 0) atomicOr(&g_tc05_error, 1u);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
