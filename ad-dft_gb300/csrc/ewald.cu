@@ -18,10 +18,12 @@ struct EwaldParams {
   double omega, eta;
   int nat, nmax;
   int nr[3];       // translations per axis that reach within the real-space cut
-  double pos[kMaxAtomsE * 3];
-  Turns frac[kMaxAtomsE * 3];   // fractional coordinates (phases of the reciprocal sum)
   double z[kMaxAtomsE];
 };
+// positions (real-space sum) and fractional coordinates (phases of the reciprocal sum): each a parameter of the one
+// kernel that reads it
+struct EwaldPos { double r[kMaxAtomsE * 3]; };
+struct EwaldFracs { Turns f[kMaxAtomsE * 3]; };
 
 // Pairs further apart than this times 1/eta add erfc(10) < 3e-45 per unit charge: nothing that an
 // FP64 sum beside the self term could show, so they are not evaluated (Si64, nmax = 8: 27 of the
@@ -33,7 +35,7 @@ constexpr double kRealCut = 10.0;
 // the force on i from its pairs (i, j) and (j, i) is twice the sum over (i, j).
 // Bound by the FP64 pipe (erfc, exp, sqrt and two divisions per term): 7.85 ms with every
 // translation of every pair and one CTA per pair, 0.06 ms so (Si64).
-__global__ void __launch_bounds__(256) k_ewald_real(EwaldParams ep, double *__restrict__ partial) {
+__global__ void __launch_bounds__(256) k_ewald_real(EwaldParams ep, EwaldPos at, double *__restrict__ partial) {
   const int i = blockIdx.x, ns = gridDim.y;
   const int s1 = 2 * ep.nr[0] + 1, s2 = 2 * ep.nr[1] + 1, s3 = 2 * ep.nr[2] + 1, nt = s1 * s2 * s3;
   // translations of one pair fit 32 bits, pairs times translations need not (a small eta reaches far)
@@ -49,7 +51,7 @@ __global__ void __launch_bounds__(256) k_ewald_real(EwaldParams ep, double *__re
     if (i == j && a == 0 && b == 0 && c == 0) continue;
     double d[3];
     for (int x = 0; x < 3; ++x)
-      d[x] = ep.pos[3 * i + x] - ep.pos[3 * j + x] + a * ep.L[x] + b * ep.L[3 + x] + c * ep.L[6 + x];
+      d[x] = at.r[3 * i + x] - at.r[3 * j + x] + a * ep.L[x] + b * ep.L[3 + x] + c * ep.L[6 + x];
     const double d2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
     if (d2 > cut2) continue;
     const double zz = ep.z[i] * ep.z[j];
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(256) k_ewald_real(EwaldParams ep, double *__re
 // adds its atom's force.  A phase costs one complex product (the tables hold e^{-2 pi i m f}) where
 // a sincos per atom and G, once for S and again in every atom's force sum, took 5.0 ms (Si64):
 // 0.10 ms so.  partial[cta][10 + 3 nat] = {sum w |S|^2, sum coef |S|^2 G_a G_b, forces}.
-__global__ void __launch_bounds__(256) k_ewald_recip(EwaldParams ep, double *__restrict__ partial) {
+__global__ void __launch_bounds__(256) k_ewald_recip(EwaldParams ep, EwaldFracs fr, double *__restrict__ partial) {
   extern __shared__ double2 ew_smem[];
   const int nat = ep.nat, M = ep.nmax + 2, side = 2 * M + 1;
   double2 *e3 = ew_smem, *ph = e3 + kRecipChunk * nat;   // [chunk][atom]
@@ -100,11 +102,11 @@ __global__ void __launch_bounds__(256) k_ewald_recip(EwaldParams ep, double *__r
   for (int c0 = 0; c0 < side; c0 += kRecipChunk) {
     const int nc = min(kRecipChunk, side - c0);
     if (on)
-      for (int c = row; c < nc; c += nrow) e3[c * nat + i] = phase_exp(c0 + c - M, ep.frac[3 * i + 2]);
+      for (int c = row; c < nc; c += nrow) e3[c * nat + i] = phase_exp(c0 + c - M, fr.f[3 * i + 2]);
     for (int col = blockIdx.x; col < side * side; col += gridDim.x) {
       const int a = col / side - M, b = col % side - M;
       if (on) {
-        const double2 p1 = phase_exp(a, ep.frac[3 * i]), p2 = phase_exp(b, ep.frac[3 * i + 1]), e12 = cmul(p1, p2);
+        const double2 p1 = phase_exp(a, fr.f[3 * i]), p2 = phase_exp(b, fr.f[3 * i + 1]), e12 = cmul(p1, p2);
         for (int c = row; c < nc; c += nrow) ph[c * nat + i] = cmul(e12, e3[c * nat + i]);
       }
       __syncthreads();
@@ -153,13 +155,13 @@ __global__ void __launch_bounds__(256) k_ewald_recip(EwaldParams ep, double *__r
     }
   }
   double *out = partial + (size_t)blockIdx.x * (10 + 3 * nat);
-  double *fr = reinterpret_cast<double *>(ph);   // the rows' forces, added in row order
+  double *sums_of = reinterpret_cast<double *>(ph);   // the rows' forces, added in row order
   if (on)
-    for (int x = 0; x < 3; ++x) fr[(row * nat + i) * 3 + x] = F[x];
+    for (int x = 0; x < 3; ++x) sums_of[(row * nat + i) * 3 + x] = F[x];
   __syncthreads();
   for (int t = threadIdx.x; t < 3 * nat; t += blockDim.x) {
     double s = 0.0;
-    for (int r = 0; r < nrow; ++r) s += fr[r * nat * 3 + t];
+    for (int r = 0; r < nrow; ++r) s += sums_of[r * nat * 3 + t];
     out[10 + t] = s;
   }
   __shared__ double red[8][10];
@@ -256,7 +258,11 @@ addft_status addft_ewald(const double *lattice, int nat, const double *pos, cons
   ep.eta = eta;
   ep.nat = nat;
   ep.nmax = nmax;
-  for (int i = 0; i < 3 * nat; ++i) ep.pos[i] = pos[i];
+  EwaldPos at;
+  EwaldFracs fr;
+  memset(&at, 0, sizeof(at));
+  memset(&fr, 0, sizeof(fr));
+  for (int i = 0; i < 3 * nat; ++i) at.r[i] = pos[i];
   for (int i = 0; i < nat; ++i) ep.z[i] = charges[i];
   cudaStream_t st = as_stream(stream);
   char *w = (char *)work;
@@ -269,7 +275,7 @@ addft_status addft_ewald(const double *lattice, int nat, const double *pos, cons
       const double f = (r[0] * bv[0] + r[1] * bv[1] + r[2] * bv[2]) / (2.0 * M_PI);
       lo = i ? std::min(lo, f) : f;
       hi = i ? std::max(hi, f) : f;
-      ep.frac[3 * i + a] = phase_turns(bv, r);
+      fr.f[3 * i + a] = phase_turns(bv, r);
     }
     const double b = sqrt(ep.B[3 * a] * ep.B[3 * a] + ep.B[3 * a + 1] * ep.B[3 * a + 1] + ep.B[3 * a + 2] * ep.B[3 * a + 2]);
     const double reach = kRealCut / eta * b / (2.0 * M_PI) + (hi - lo) + 1e-6;
@@ -280,13 +286,13 @@ addft_status addft_ewald(const double *lattice, int nat, const double *pos, cons
   ADDFT_REQUIRE(cells <= 2147483647.0, ADDFT_UNSUPPORTED, "ewald: %.0f translations within reach", cells);
   const long terms = (long)nat * (long)cells;
   const int ns = (int)std::max<long>(1, std::min<long>(std::min<long>(nat, (terms + 255) / 256), (304 + nat - 1) / nat));
-  k_ewald_real<<<dim3(nat, ns), 256, 0, st>>>(ep, real_part);
+  k_ewald_real<<<dim3(nat, ns), 256, 0, st>>>(ep, at, real_part);
   ADDFT_TRY(check_launch("k_ewald_real"));
   const int side = 2 * (nmax + 2) + 1, nctas = (int)std::min<size_t>(std::min(kRecipCtas, side * side), (work_bytes - pairs) / per);
   const size_t sm = 2 * (size_t)kRecipChunk * nat * sizeof(double2);
   ADDFT_TRY(smem_optin(k_ewald_recip, sm));
   const int natp = (nat + 31) / 32 * 32;
-  k_ewald_recip<<<nctas, natp * std::max(1, 256 / natp), sm, st>>>(ep, recip);
+  k_ewald_recip<<<nctas, natp * std::max(1, 256 / natp), sm, st>>>(ep, fr, recip);
   ADDFT_TRY(check_launch("k_ewald_recip"));
   k_ewald_final<<<(1 + 3 * nat + 9 + 3) / 4, 128, 0, st>>>(ep, real_part, ns, recip, nctas, out);
   return check_launch("k_ewald_final");
