@@ -27,7 +27,7 @@
 // double-float form (2^-48) for S = 7.
 // Rows or columns that hold an infinity or a NaN are summed in plain FP64 at the end.
 //
-// Three kernels:
+// Three kernels (for up to 96 k the first two are one, k_oz_prep):
 //   k_oz_max   exponent of every row / column (one pass over each operand);
 //   k_oz_pack  digits into the operand layout of the MMA: per 16 k, real part then imaginary
 //              part, S slices each, a slice being 128 (A) or 32 (B) rows of 16 k in no-swizzle
@@ -132,6 +132,29 @@ __device__ __forceinline__ uint64_t oz_bytes(double x, int em) {
   return q + kBias;
 }
 
+// 8 k of one row: one 16-byte core-matrix row per part and slice
+template <int S, int R>
+__device__ __forceinline__ void oz_octet(const double2 *x, int em, int conj, unsigned char *dst) {
+  constexpr int kSlice = R * kStep * 2;   // bytes of one slice
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    uint64_t q[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double2 v = x[j];
+      // rows that are not finite are left to the FP64 sum of the GEMM's epilogue
+      q[j] = oz_bytes<S>(em == 0x7ff ? 0.0 : (part ? (conj ? -v.y : v.y) : v.x), em);
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      uint32_t h[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h[j] = digit_pair<S>(q[2 * j], q[2 * j + 1], s);
+      *reinterpret_cast<uint4 *>(dst + (size_t)(part * S + s) * kSlice) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+  }
+}
+
 // A CTA packs R rows x 2048 / R k: a coalesced read into shared memory, then a thread per row
 // and 8 k writes one 16-byte core-matrix row per part and slice.
 template <int S, int R>
@@ -160,24 +183,59 @@ k_oz_pack(const double2 *__restrict__ X, long s_row, long s_k, size_t s_batch, i
   const int em = ex[(size_t)blockIdx.z * rows + r0 + r];
   unsigned char *dst = out + blockIdx.z * out_batch + ((size_t)blockIdx.y * nks + step) * (2 * S * kSlice) +
                        (r >> 3) * 256 + (oct & 1) * 128 + (r & 7) * 16;
-#pragma unroll
-  for (int part = 0; part < 2; ++part) {
-    uint64_t q[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const double2 v = T[r * (KT + 1) + oct * 8 + j];
-      // rows that are not finite are left to the FP64 sum of the GEMM's epilogue
-      const double x = em == 0x7ff ? 0.0 : (part ? (conj ? -v.y : v.y) : v.x);
-      q[j] = oz_bytes<S>(x, em);
-    }
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      uint32_t h[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) h[j] = digit_pair<S>(q[2 * j], q[2 * j + 1], s);
-      *reinterpret_cast<uint4 *>(dst + (size_t)(part * S + s) * kSlice) = make_uint4(h[0], h[1], h[2], h[3]);
-    }
+  oz_octet<S, R>(T + r * (KT + 1) + oct * 8, em, conj, dst);
+}
+
+// Both operands of a product of few k (kPrepSteps stages) in one launch: a CTA holds 64 rows of A or 32 of B with all
+// their k, finds the exponents and writes the digits.  The passes by themselves are a memset and four launches, and these
+// small products are launches: rotations of 16 x 16 x 6,000 to 32 x 32 x 9,000 36 to 39 us with them (20 to 26
+// in double-float arithmetic, which holds fewer bits), 24 to 26 so.  Bits are those of the passes.
+constexpr int kPrepSteps = 6;      // 96 k: 99 KB of shared memory, two CTAs per SM
+constexpr int kPrepA = 64, kPrepB = kRowsB;
+inline size_t prep_smem(int nks) { return (size_t)kPrepA * (nks * kStep + 1) * sizeof(double2); }
+
+struct PrepArgs {
+  const double2 *X;
+  long s_row, s_k;
+  size_t s_batch;
+  int conj, rows;
+  int *ex;
+  unsigned char *out;
+  size_t out_batch;
+};
+
+template <int S, int R, int RB>   // RB rows per CTA, R per tile
+__device__ __forceinline__ void oz_prep(const PrepArgs &a, int blk, int K, int nks, double2 *T) {
+  constexpr int kPer = 256 / RB;   // threads per row
+  __shared__ int mx[256];
+  const int r0 = blk * RB, Kp = nks * kStep, pitch = Kp + 1;
+  const double2 *Xb = a.X + blockIdx.y * a.s_batch;
+  const bool kfast = a.s_k == 1;
+  for (int i = threadIdx.x; i < RB * Kp; i += 256) {
+    const int r = kfast ? i / Kp : i % RB, k = kfast ? i % Kp : i / RB;
+    T[r * pitch + k] = r0 + r < a.rows && k < K ? Xb[(r0 + r) * a.s_row + k * a.s_k] : make_double2(0.0, 0.0);
   }
+  __syncthreads();
+  const int r = threadIdx.x % RB, part = threadIdx.x / RB;
+  int em = 0;
+  for (int k = part; k < Kp; k += kPer) em = max(em, expo(T[r * pitch + k]));
+  mx[threadIdx.x] = em;
+  __syncthreads();
+  for (int p = 0; p < kPer; ++p) em = max(em, mx[p * RB + r]);
+  if (r0 + r >= a.rows) return;
+  if (part == 0) a.ex[(size_t)blockIdx.y * a.rows + r0 + r] = em;
+  const int rt = r0 % R + r;   // row in its tile
+  unsigned char *tile = a.out + blockIdx.y * a.out_batch + (size_t)(r0 / R) * nks * (2 * S * R * kStep * 2);
+  for (int oct = part; oct < 2 * nks; oct += kPer)
+    oz_octet<S, R>(T + r * pitch + oct * 8, em, a.conj,
+                   tile + (size_t)(oct / 2) * (2 * S * R * kStep * 2) + (rt >> 3) * 256 + (oct & 1) * 128 + (rt & 7) * 16);
+}
+
+template <int S>
+__global__ void __launch_bounds__(256) k_oz_prep(PrepArgs a, PrepArgs b, int ctas_a, int K, int nks) {
+  extern __shared__ __align__(16) double2 prep_smem_[];
+  if ((int)blockIdx.x < ctas_a) oz_prep<S, kRowsA, kPrepA>(a, blockIdx.x, K, nks, prep_smem_);
+  else oz_prep<S, kRowsB, kPrepB>(b, blockIdx.x - ctas_a, K, nks, prep_smem_);
 }
 
 // ---------------------------------------------------------------------------
@@ -653,11 +711,20 @@ addft_status oz_run(int rows, int cols, int K, int batch, const OzMat &A, const 
   char *w = (char *)work;
   int *ea = (int *)(w + l.o_ex), *eb = ea + (size_t)batch * rows;
   unsigned char *pa = (unsigned char *)w + l.o_pa, *pb = (unsigned char *)w + l.o_pb;
-  ADDFT_CUDA(cudaMemsetAsync(ea, 0, (size_t)batch * (rows + cols) * sizeof(int), st));
-  ADDFT_TRY(oz_max(A, rows, K, batch, ea, st));
-  ADDFT_TRY(oz_max(B, cols, K, batch, eb, st));
-  ADDFT_TRY((oz_pack<S, kRowsA>(A, rows, K, l.nks, batch, ea, pa, l.pa, st)));
-  ADDFT_TRY((oz_pack<S, kRowsB>(B, cols, K, l.nks, batch, eb, pb, l.pb, st)));
+  if (l.nks <= kPrepSteps) {
+    const PrepArgs a = {(const double2 *)A.p, A.s_row, A.s_k, A.s_batch, A.conj, rows, ea, pa, l.pa};
+    const PrepArgs b = {(const double2 *)B.p, B.s_row, B.s_k, B.s_batch, B.conj, cols, eb, pb, l.pb};
+    const int ca = (rows + kPrepA - 1) / kPrepA, cb = (cols + kPrepB - 1) / kPrepB;
+    ADDFT_TRY(smem_optin(k_oz_prep<S>, prep_smem(l.nks)));
+    k_oz_prep<S><<<dim3(ca + cb, batch), 256, prep_smem(l.nks), st>>>(a, b, ca, K, l.nks);
+    ADDFT_TRY(check_launch("k_oz_prep"));
+  } else {
+    ADDFT_CUDA(cudaMemsetAsync(ea, 0, (size_t)batch * (rows + cols) * sizeof(int), st));
+    ADDFT_TRY(oz_max(A, rows, K, batch, ea, st));
+    ADDFT_TRY(oz_max(B, cols, K, batch, eb, st));
+    ADDFT_TRY((oz_pack<S, kRowsA>(A, rows, K, l.nks, batch, ea, pa, l.pa, st)));
+    ADDFT_TRY((oz_pack<S, kRowsB>(B, cols, K, l.nks, batch, eb, pb, l.pb, st)));
+  }
   OzArgs g;
   g.pa = pa; g.pb = pb; g.pa_batch = l.pa; g.pb_batch = l.pb;
   g.ea = ea; g.eb = eb;

@@ -180,3 +180,38 @@ def test_graded_rows_meet_the_stated_bound(decades, K):
     fp64 = (math.sqrt(K) + 4.0) * 4 * U * (a.abs() @ b.abs().T)
     assert bool(((ops.zgemm_df(a, b.transpose(0, 1), conj_a=True) - ref).abs() <= K * 2.0 ** -50 * big + fp64).all())
     assert bool(((ops.becp(a[None], b[None])[0] - ref).abs() <= K * 2.0 ** -56 * big + fp64).all())
+
+
+@pytest.mark.parametrize("K", [15, 16, 17, 33, 48, 95, 96])
+@pytest.mark.parametrize("M,N", [(129, 1500), (63, 3100), (64, 3000), (65, 1200), (31, 5003), (33, 4097)])
+def test_few_k_in_one_launch_give_the_bits_of_the_passes(M, N, K):
+    """Products of up to 96 k find their exponents and digits in one launch; with zeros to 112 k the passes of longer
+    products run.  Every order of both operands, conjugates, graded rows, a row and a column that are not finite."""
+    if M * N * K < 2e6:
+        pytest.skip("a small product in plain FP64")
+    a, b = rnd(M, M, K, spread=6.0), rnd(N, K, N)
+    a[5] = 0
+    a[7, 3] = complex(float("inf"), 0.0)
+    b[2, 9] = complex(0.0, float("nan"))
+    a2 = torch.cat([a, torch.zeros((M, 112 - K), dtype=a.dtype, device="cuda")], 1)
+    b2 = torch.cat([b, torch.zeros((112 - K, N), dtype=a.dtype, device="cuda")], 0)
+    ok = torch.ones((M, N), dtype=torch.bool, device="cuda")
+    ok[7], ok[:, 9] = False, False                      # zeros against what is not finite are NaN in the longer one
+    for x, x2 in ((a, a2), (a.T.contiguous().T, a2.T.contiguous().T)):
+        for y, y2 in ((b, b2), (b.T.contiguous().T, b2.T.contiguous().T)):
+            for ca, cb in ((False, False), (True, False), (False, True)):
+                o, p = ops.zgemm_df(x, y, conj_a=ca, conj_b=cb), ops.zgemm_df(x2, y2, conj_a=ca, conj_b=cb)
+                assert torch.equal(torch.view_as_real(o)[ok], torch.view_as_real(p)[ok])
+                assert bool((torch.isfinite(torch.view_as_real(o)).all(-1) == ok).all())
+
+
+@pytest.mark.parametrize("nk,nb,P,nG", [(8, 24, 32, 700), (3, 31, 96, 1301)])
+def test_few_k_of_a_batch(nk, nb, P, nG):
+    """The V_NL apply of few projectors: all k points in one launch, added to H psi."""
+    proj, b = rnd(1, nk, P, nG, spread=6.0), rnd(2, nk, P, nb)
+    dion = torch.diag(torch.linspace(-2.0, 1.0, P, dtype=torch.float64, device="cuda"))
+    h0 = rnd(4, nk, nb, nG)
+    h = ops.vnl_apply(proj, dion, b, h0.clone())
+    for k in range(nk):
+        db = dion.to(torch.complex128) @ b[k]
+        assert bool(((h[k] - (h0[k] + db.T @ proj[k])).abs() <= bound(db.T, proj[k], 60) + 2 * U * h0[k].abs()).all())
