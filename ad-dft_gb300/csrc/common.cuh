@@ -105,6 +105,18 @@ struct D64Mat {
   long off;
 };
 
+// What the FP64 transforms on the tensor cores read beside the plan's tables: active y and z indices (in ascending
+// order), index tables per column, the transform matrices.  Kept by the plan and not part of PlanDev, which every
+// kernel takes by value: with 300 bytes more a density of three launches took 1.1 us longer, an H psi 1 to 2.
+struct D64Plan {
+  int nq, nz;
+  const int *col_zg;       // ncols * nz: G index at each active z, -1 where the sphere has no point
+  const int *col_of;       // np * nq: column at (active plane, active y), -1 where there is none
+  const int *col_pq;       // ncols: plane * nq + y index
+  D64Mat mat[6];           // x, y, z inverse, then forward
+  const unsigned char *F;
+};
+
 // Device view of a plan: sphere-aware layout of one G-shell in one FFT box.
 //   planes p = 0..np-1 are the x-planes (fixed i1) that hold sphere points;
 //   each plane owns a contiguous range [gptr[p], gptr[p+1]) of the
@@ -135,13 +147,7 @@ struct PlanDev {
   // (true for spheres around G = 0): row_lohi[p] = nlo | nhi << 16
   int xy_direct;
   const int *row_lohi;
-  // FP64 transforms on the tensor cores: active y and z indices (in ascending order), and per column
-  int nq, nz;
-  const int *col_zg;       // ncols * nz: G index at each active z, -1 where the sphere has no point
-  const int *col_of;       // np * nq: column at (active plane, active y), -1 where there is none
-  const int *col_pq;       // ncols: plane * nq + y index
-  D64Mat d64[6];           // x, y, z inverse, then forward
-  const unsigned char *d64_F;
+  const D64Plan *d64;      // host memory (of the plan)
   const void *tw_d;        // double2 twiddles: n1 | n2 | n3, e^{-2 pi i t/n}
   const void *tw_f;        // float2 twiddles, same layout
   AxisPlan ax[3];
@@ -258,6 +264,7 @@ addft_status finalize_sums(const double *partial, int nv, int nblk, double *out,
 
 struct addft_plan_s {
   addft::PlanDev dev;
+  addft::D64Plan d64;
   int ncols;
   void *blob;   // single device allocation holding all tables
   int device;

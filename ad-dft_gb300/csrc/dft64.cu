@@ -73,6 +73,8 @@ struct Args {
   PlanDev pd;
   D64Mat m;
   const unsigned char *F;
+  int nq, nz;              // as in D64Plan
+  const int *col_zg, *col_of, *col_pq;
   long lines;              // over all bands of the chunk (XI_D: per band)
   int nb;                  // bands of the chunk
   const double2 *in;
@@ -101,11 +103,11 @@ __device__ __forceinline__ Line line_at(const Args &a, unsigned l) {
   if (ST == ZI) {
     const unsigned b = l / (unsigned)pd.nrows;
     r.base = (long)b * pd.nG;
-    r.aux = (int)(l - b * pd.nrows) * pd.nz;
+    r.aux = (int)(l - b * pd.nrows) * a.nz;
   } else if (ST == YI) {
     const unsigned t = l / (unsigned)pd.n3, b = t / (unsigned)pd.np;
     r.base = (long)b * pd.nrows * pd.n3 + (l - t * pd.n3);
-    r.aux = (int)(t - b * pd.np) * pd.nq;
+    r.aux = (int)(t - b * pd.np) * a.nq;
   } else if (ST == XI_V || ST == XI_R || ST == XI_C || ST == XI_D) {
     const unsigned n = pd.n2 * pd.n3, b = l / n;
     r.base = (long)b * pd.np * n + (l - b * n);
@@ -119,7 +121,7 @@ __device__ __forceinline__ Line line_at(const Args &a, unsigned l) {
     r.base = (long)b * pd.n2 * pd.n3 * pd.np + (t - b * pd.n3) * a.sz + (l - t * pd.np);
   } else {
     const unsigned b = l / (unsigned)pd.nrows;
-    r.base = (long)b * pd.n3 * pd.np * pd.nq + pd.col_pq[l - b * pd.nrows];
+    r.base = (long)b * pd.n3 * pd.np * a.nq + a.col_pq[l - b * pd.nrows];
   }
   return r;
 }
@@ -135,10 +137,10 @@ __device__ __forceinline__ double2 load_at(const Args &a, const Line &l, int k) 
   const PlanDev &pd = a.pd;
   const double2 z = make_double2(0.0, 0.0);
   if (ST == ZI) {
-    const int g = pd.col_zg[l.aux + k];
+    const int g = a.col_zg[l.aux + k];
     return g >= 0 ? a.in[l.base + g] : z;
   } else if (ST == YI) {
-    const int c = pd.col_of[l.aux + k];
+    const int c = a.col_of[l.aux + k];
     return c >= 0 ? a.in[l.base + (long)c * pd.n3] : z;
   } else if (ST == XI_V || ST == XI_R || ST == XI_C || ST == XI_D || ST == XR_C) {
     return a.in[l.base + (long)k * pd.n2 * pd.n3];
@@ -149,7 +151,7 @@ __device__ __forceinline__ double2 load_at(const Args &a, const Line &l, int k) 
   } else if (ST == YF) {
     return a.in[l.base + k * a.sy];
   } else {
-    return a.in[l.base + (long)k * pd.np * pd.nq];
+    return a.in[l.base + (long)k * pd.np * a.nq];
   }
 }
 
@@ -159,7 +161,7 @@ template <int ST>
 __device__ __forceinline__ void pre_at(const Args &a, unsigned band, unsigned rem, int o, int comp, double &x, int &g) {
   const PlanDev &pd = a.pd;
   if (ST == XI_V) x = __ldg(a.V + (long)rem * pd.n1 + o);
-  if (ST == ZF || ST == ZF_H) g = __ldg(pd.col_zg + rem * pd.nz + o);
+  if (ST == ZF || ST == ZF_H) g = __ldg(a.col_zg + rem * a.nz + o);
   if (ST == ZF_H) {
     x = 0.0;
     if (g >= 0)
@@ -180,7 +182,7 @@ __device__ __forceinline__ void store_at(const Args &a, unsigned l, unsigned ban
   else if (ST == XI_C) out[2 * ((long)l * pd.n1 + o) + comp] = v * a.scale;
   else if (ST == XI_R) { if (!comp) out[(long)l * pd.n1 + o] = v * a.scale; }
   else if (ST == XF || ST == XR_R || ST == XR_C) out[2 * ((long)l * pd.np + o) + comp] = v;
-  else if (ST == YF) out[2 * ((long)l * pd.nq + o) + comp] = v;
+  else if (ST == YF) out[2 * ((long)l * a.nq + o) + comp] = v;
   else if (g >= 0) out[2 * ((long)band * pd.nG + g) + comp] = ST == ZF_H ? v + x : v * a.scale;
 }
 
@@ -571,15 +573,21 @@ inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // The two scratch regions of a band: Z, U, W in the first, Y, X in the second.
 inline size_t region1(const PlanDev &pd) {
-  const size_t z = (size_t)pd.nrows * pd.n3, u = (size_t)pd.n1 * pd.n2 * pd.n3, w = (size_t)pd.n3 * pd.np * pd.nq;
+  const size_t z = (size_t)pd.nrows * pd.n3, u = (size_t)pd.n1 * pd.n2 * pd.n3, w = (size_t)pd.n3 * pd.np * pd.d64->nq;
   return al256(std::max(std::max(z, u), w) * sizeof(double2));
 }
 inline size_t region2(const PlanDev &pd) { return al256((size_t)pd.np * pd.n2 * pd.n3 * sizeof(double2)); }
 
 template <int ST>
 addft_status stage(const PlanDev &pd, int axis, Args &a, long lines, cudaStream_t st) {
-  a.m = pd.d64[axis];
-  a.F = pd.d64_F;
+  const D64Plan &t = *pd.d64;
+  a.m = t.mat[axis];
+  a.F = t.F;
+  a.nq = t.nq;
+  a.nz = t.nz;
+  a.col_zg = t.col_zg;
+  a.col_of = t.col_of;
+  a.col_pq = t.col_pq;
   a.lines = lines;
   a.ring = std::min<int>(kMaxRing, (int)((kRoom - a.m.tile_bytes) / kItem));
   const int noct = 2 * a.m.nks;
@@ -636,9 +644,9 @@ int d64_chunk(const PlanDev &pd, int nbatch, size_t bytes) {
 
 bool d64_handles(const PlanDev &pd, D64Op op, int bands) {
   // tuning that asks for the split stages or for other kernels than the defaults keeps to the FFT kernels
-  if (!pd.d64_F || !pd.tun.colfft || pd.tun.plane_split) return false;
+  if (!pd.d64->F || !pd.tun.colfft || pd.tun.plane_split) return false;
   for (int a = 0; a < 6; ++a)
-    if (pd.d64[a].tiles == 0) return false;
+    if (pd.d64->mat[a].tiles == 0) return false;
   // Where the products start, in box points x bands at once, by (n1 n2 n3)^(1/3).  They take 65 to 80 (H psi) or
   // 36 to 48 us (density, one way) before the work shows, launches that load F first; the FFT kernels 40 to 60 and
   // 20 to 35, growing with the box.  Measured on 39 boxes from 9^3 to 80^3, cubes and 1 : 1 : 1.25 to 2, 1 to
@@ -714,7 +722,7 @@ addft_status d64_density(const PlanDev &pd, int nbatch, const double2 *psi, cons
   const long N = (long)pd.n1 * pd.n2 * pd.n3, lines = (long)pd.n2 * pd.n3;
   // band groups so that the CTAs of a tile share the (block, group) units evenly
   const long blocks = (lines + kLines - 1) / kLines;
-  int groups = (int)std::max<long>(1, std::min<long>(4, (8 * kSms / pd.d64[0].tiles + blocks - 1) / blocks));
+  int groups = (int)std::max<long>(1, std::min<long>(4, (8 * kSms / pd.d64->mat[0].tiles + blocks - 1) / blocks));
   groups = std::min(groups, nbatch);
   auto part_bytes = [N](int g) { return al256((size_t)g * 2 * N * sizeof(double)); };
   while (groups > 1 && bytes < part_bytes(groups) + d64_band_bytes(pd)) --groups;

@@ -783,14 +783,18 @@ static int becp_mode() {
   return m;
 }
 
-// K splits of the tcgen05 becp: the fewest waves of 32-G stages, each CTA about 6 stages' time on top
+// K splits of the tcgen05 becp: the fewest waves of 32-G stages, each CTA about 6 stages' time on top.  For each
+// number of waves up to two the splits that fill them, as few as give the same stages per CTA.
 static int becp_tc05_nsplit(int tiles, int nG) {
   const int steps = (nG + 31) / 32;
   int best = 1;
-  long least = 0;
-  for (int ns = 1; ns <= steps && (ns == 1 || (long)tiles * ns <= 2 * 152); ++ns) {
-    const long t = (((long)tiles * ns + 151) / 152) * ((steps + ns - 1) / ns + 6);
-    if (ns == 1 || t < least) {
+  long least = ((long)tiles + 151) / 152 * (steps + 6);
+  for (int w = 1; w <= 2; ++w) {
+    const int most = std::min(steps, 152 * w / tiles);
+    if (most < 1) continue;
+    const int per = (steps + most - 1) / most, ns = (steps + per - 1) / per;
+    const long t = ((long)tiles * ns + 151) / 152 * (per + 6);
+    if (t < least) {
       least = t;
       best = ns;
     }

@@ -302,10 +302,12 @@ addft_status addft_plan_create(addft_plan *plan, int n1, int n2, int n3, int nG,
   d.ncols_pad = ncols_pad; d.cgptr = ib + o_cgp; d.pt_pos = ib + o_ptp; d.col_xy = ib + o_cxy;
   d.pt_col = ib + o_ptc; d.col_m = ib + o_cm; d.col_uniform = col_uniform ? 1 : 0;
   d.xy_direct = xy_direct ? 1 : 0; d.row_lohi = ib + o_rlh;
-  d.nq = nq; d.nz = nz;
-  d.col_zg = ib + o_zg; d.col_of = ib + o_cof; d.col_pq = ib + o_cpq;
-  for (int a = 0; a < 6; ++a) d.d64[a] = dm[a];
-  d.d64_F = dF.empty() ? nullptr : (const unsigned char *)(b + off_F);
+  D64Plan &t = p->d64;
+  t.nq = nq; t.nz = nz;
+  t.col_zg = ib + o_zg; t.col_of = ib + o_cof; t.col_pq = ib + o_cpq;
+  for (int a = 0; a < 6; ++a) t.mat[a] = dm[a];
+  t.F = dF.empty() ? nullptr : (const unsigned char *)(b + off_F);
+  d.d64 = &t;
   d.tw_d = b + off_twd;
   d.tw_f = b + off_twf;
   for (int a = 0; a < 3; ++a) d.ax[a] = ax[a];
