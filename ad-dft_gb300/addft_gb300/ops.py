@@ -137,21 +137,21 @@ class Plan:
             self.handle = None
 
 
-def _bands_that_fit(nbytes, limit: int, nbatch: int) -> int:
-    """Largest number of bands up to nbatch (one at least) whose scratch nbytes(bands) stays within the
-    limit; nbytes grows with the bands, in steps where another form of the transforms starts."""
-    if nbytes(nbatch) <= limit:
-        return nbatch
+def _bytes_within(nbytes, limit: int, nbatch: int) -> int:
+    """nbytes(n), the scratch of n bands at once, for the largest n up to nbatch (one at least) with which it
+    stays within the limit; it grows with the bands, in steps where another form of the transforms starts."""
+    need = nbytes(nbatch)
+    if need <= limit or nbatch <= 1:
+        return need
     lo, hi = 1, nbatch
     while hi - lo > 1:
         mid = (lo + hi) // 2
         lo, hi = (mid, hi) if nbytes(mid) <= limit else (lo, mid)
-    return lo
+    return nbytes(lo)
 
 
 def _chunk_work(plan: Plan, dtype: int, nbatch: int, extra: int = 0, max_bytes: int = 1 << 30) -> torch.Tensor:
-    nfit = _bands_that_fit(lambda n: plan.work_bytes(n, dtype), max_bytes - extra, max(nbatch, 1))
-    return workspace(extra + plan.work_bytes(nfit, dtype))
+    return workspace(extra + _bytes_within(lambda n: plan.work_bytes(n, dtype), max_bytes - extra, max(nbatch, 1)))
 
 
 # ---------------------------------------------------------------------------
@@ -218,8 +218,7 @@ def hpsi(plan: Plan, psi: torch.Tensor, kin: torch.Tensor, v_r: torch.Tensor, pr
         dion = _c(torch.as_tensor(dion, device=psi.device).to(rdt), "dion")
     if out is None:
         out = torch.empty_like(psi)
-    chunk = _bands_that_fit(lambda c: hpsi_work_bytes(plan, dt, nk, nb, nproj, c), max_work, max(nk * nb, 1))
-    wb = hpsi_work_bytes(plan, dt, nk, nb, nproj, chunk)
+    wb = _bytes_within(lambda c: hpsi_work_bytes(plan, dt, nk, nb, nproj, c), max_work, max(nk * nb, 1))
     w = workspace(wb)
     check(LIB.addft_hpsi(plan.handle, dt, nk, nb, _p(psi), _p(kin), _p(v_r), nproj, _p(proj),
                          _p(dion), _p(out), _p(w), w.numel(), _stream()), "hpsi")
