@@ -748,6 +748,7 @@ k_kin_stress(PlanDev pd, GeoParams gp, const typename Cx<R>::T *__restrict__ psi
 // host drivers
 // ---------------------------------------------------------------------------
 inline int pick_nsplit(int tiles, int nG, int ctas_per_sm = 8) {
+  if (tiles < 1) return 1;   // an empty problem, in a size query
   int ns = (ctas_per_sm * 152 + tiles - 1) / tiles;
   const int maxs = (nG + 63) / 64;
   if (ns > maxs) ns = maxs;
@@ -1120,6 +1121,7 @@ addft_status projectors_t(const PlanDev &pd, const GeoParams &gp, void *proj, cu
 
 // splits of the gradients' G range per atom: about four CTAs per SM, at least 256 G each
 inline int nl_grad_splits(int nk, int nat, int nG) {
+  if (nk < 1 || nat < 1) return 1;
   return std::max(1, std::min((4 * 152 + nk * nat - 1) / (nk * nat), (nG + 255) / 256));
 }
 

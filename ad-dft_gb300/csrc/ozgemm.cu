@@ -641,6 +641,7 @@ int small_splits(int M, int N, int K, int batch) {
   return (int)std::max<long>(1, std::min<long>((K + 1023) / 1024, 4 * kSms / groups));
 }
 size_t small_bytes(int M, int N, int K, int batch) {
+  if (M < 1 || N < 1 || K < 1 || batch < 1) return 0;
   const int ns = small_splits(M, N, K, batch);
   return ns > 1 ? (size_t)ns * M * N * batch * sizeof(double2) : 0;
 }
@@ -649,6 +650,7 @@ size_t small_bytes(int M, int N, int K, int batch) {
 // beyond its launch; the digit slices 25 us for their small kernels, then 1.3 us per tile and 16 k
 // over the SMs).
 bool small_product(int M, int N, int K, int batch) {
+  if (M < 1 || N < 1 || K < 1 || batch < 1) return true;
   const double work = (double)M * N * K * batch;
   if (work > 2e7) return false;
   auto tiles = [](int r, int c) { return (double)((r + kRowsA - 1) / kRowsA) * ((c + kRowsB - 1) / kRowsB); };
